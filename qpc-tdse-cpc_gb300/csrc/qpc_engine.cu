@@ -46,6 +46,7 @@
 #include <cstdlib>
 #include "qpc_chain.cuh"
 #include "qpc_ltrans.cuh"
+#include "qpc_pos.cuh"
 
 namespace qpc {
 
@@ -476,6 +477,15 @@ struct qpc_lgwz {
 	std::vector<std::pair<int, int>> evuse;	// (kernel id, index of start event; end = +1)
 	double kms[QPC_NKERNEL] = {0};
 	int64_t kcount[QPC_NKERNEL] = {0};
+	// runs in the position basis (qpc_pos.cu), where the operators allow it; the banded solves otherwise
+	pos_path* pos = nullptr;
+	std::vector<double> h_R;	// the caller's R band: the in-loop dipole of R itself needs no band product
+	int* dperm = nullptr;		// device [B]: the instance of each sorted slot
+	// the state lives in st (r-major), in hostlay (the caller's order), or in both
+	bool st_valid = false, lay_valid = true;
+	size_t fac_elems = 0;
+	bool chains_ready = false;	// the banded solves' buffers exist
+	std::vector<double2> ffh;	// host copy of ff until they do
 	std::vector<double> h_lam;   // [M][L]
 	std::vector<double> h_P;     // [M][L][L]
 };
@@ -972,6 +982,71 @@ static void host_spikes(const double2* fac, size_t nblk, int N, int Q, int Ls, d
 		}
 }
 
+// the buffers of the banded solves, made when a run first needs them
+static int need_chains(qpc_lgwz* h)
+{
+	if (h->chains_ready) return QPC_OK;
+	const int N = h->N, P = h->P, NE = P + 1;
+	const long sl = state_len(h);
+	int rc;
+	if ((!h->st && (rc = dalloc(&h->st, sl))) || (!h->eo && (rc = dalloc(&h->eo, sl))) || (!h->wk && (rc = dalloc(&h->wk, sl))) ||
+		(!h->fac && (rc = dalloc(&h->fac, h->fac_elems))))
+		return rc;
+	if (h->seg_ok) {
+		const size_t nblk_ff = h->ffh.size() / ((size_t)N * NE), nblk_c = (size_t)h->K * h->B * h->M * h->npair;
+		std::vector<double2> sf(nblk_ff * N * P), sb(nblk_ff * N * P);
+		switch (P) {
+		case 3: host_spikes<3>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 4: host_spikes<4>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 5: host_spikes<5>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 6: host_spikes<6>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 7: host_spikes<7>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 8: host_spikes<8>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		}
+		if ((rc = dalloc(&h->spf_ff, sf.size())) || (rc = dalloc(&h->spb_ff, sb.size())) ||
+			(rc = dalloc(&h->spf_c, nblk_c * N * P)) || (rc = dalloc(&h->spb_c, nblk_c * N * P)))
+			return rc;
+		if (cudaMemcpy(h->spf_ff, sf.data(), sizeof(double2) * sf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+			cudaMemcpy(h->spb_ff, sb.data(), sizeof(double2) * sb.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+			cudaMemset(h->spf_c, 0, sizeof(double2) * nblk_c * N * P) != cudaSuccess ||
+			cudaMemset(h->spb_c, 0, sizeof(double2) * nblk_c * N * P) != cudaSuccess) {
+			set_error("initial device copies failed");
+			return QPC_ERR_CUDA;
+		}
+	}
+	h->ffh = std::vector<double2>();
+	h->chains_ready = true;
+	return QPC_OK;
+}
+
+// one field-free step of the factor set fi on J vectors X[J][N][nlh] (r-major), every l = 0..nlh-1 once, on the
+// handle's stream; act: device array of J ones
+template <int P, int G>
+static void fieldfree_columns_t(qpc_lgwz* h, double2* X, double2* wk, int J, int fi, const int64_t* act)
+{
+	using C = chain_cfg<P, G, false>;
+	const long nch = (long)J * h->nlh, warps = (nch + C::CPW - 1) / C::CPW;
+	const int wpb = h->chain_warps;
+	k_chain<P, G, false><<<(unsigned)((warps + wpb - 1) / wpb), 32 * wpb, h->chain_sstage ? h->chain_smem : 0, h->stream>>>(X, wk,
+		h->ff + (size_t)fi * h->nlh * h->N * (P + 1), h->S, act, 0, 0, J, 1, 0, h->N, h->nlh, h->npair, 0, nch, nullptr, nullptr, nullptr, 0, 0,
+		h->chain_sstage);
+	LAUNCH(h);
+}
+static int fieldfree_columns(qpc_lgwz* h, double2* X, double2* wk, int J, int fi, const int64_t* act)
+{
+	switch (h->P) {
+	case 3: fieldfree_columns_t<3, 3>(h, X, wk, J, fi, act); break;
+	case 4: fieldfree_columns_t<4, 2>(h, X, wk, J, fi, act); break;
+	case 5: fieldfree_columns_t<5, 5>(h, X, wk, J, fi, act); break;
+	case 6: fieldfree_columns_t<6, 3>(h, X, wk, J, fi, act); break;
+	case 7: fieldfree_columns_t<7, 7>(h, X, wk, J, fi, act); break;
+	case 8: fieldfree_columns_t<8, 4>(h, X, wk, J, fi, act); break;
+	default: set_error("unsupported B-spline degree %d", h->P); return QPC_ERR_ARGS;
+	}
+	QPC_CUDA(cudaGetLastError());
+	return QPC_OK;
+}
+
 extern "C" {
 
 const char* qpc_last_error(void) { return g_err; }
@@ -1110,11 +1185,11 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 	if (const char* e = getenv("QPC_FAC_BYTES")) fac_cap = std::max<size_t>(per_step, (size_t)atoll(e));
 	h->K = 1;
 	while (h->K < 4096 && (long)h->K * h->B * M * np < 40000 && per_step * (h->K * 2) <= fac_cap) h->K *= 2;
+	h->fac_elems = per_step / sizeof(double2) * h->K;
 	long sl = state_len(h);
 	if ((rc = dalloc(&h->S, (size_t)N * NE)) || (rc = dalloc(&h->R, (size_t)N * NE)) || (rc = dalloc(&h->Vh, Vh.size())) ||
-		(rc = dalloc(&h->lamp, lamp.size())) || (rc = dalloc(&h->ff, ffh.size())) || (rc = dalloc(&h->st, sl)) ||
-		(rc = dalloc(&h->eo, sl)) || (rc = dalloc(&h->wk, sl)) ||
-		(rc = dalloc(&h->hostlay, sl)) || (rc = dalloc(&h->fac, per_step / sizeof(double2) * h->K)) ||
+		(rc = dalloc(&h->lamp, lamp.size())) || (rc = dalloc(&h->ff, ffh.size())) ||
+		(rc = dalloc(&h->hostlay, sl)) || (rc = dalloc(&h->dperm, h->B)) ||
 		(rc = dalloc(&h->status, 1)) || (rc = dalloc(&h->red, (size_t)h->B * M * L * 2)) ||
 		(rc = dalloc(&h->ntf, h->B)) || (rc = dalloc(&h->ntt, h->B)))
 		return fail(rc);
@@ -1123,7 +1198,7 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 		cudaMemcpy(h->Vh, Vh.data(), sizeof(double) * Vh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->lamp, lamp.data(), sizeof(double) * lamp.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->ff, ffh.data(), sizeof(double2) * ffh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemset(h->st, 0, sizeof(double2) * sl) != cudaSuccess || cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess) {
+		cudaMemset(h->hostlay, 0, sizeof(double2) * sl) != cudaSuccess || cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess) {
 		set_error("initial device copies failed");
 		return fail(QPC_ERR_CUDA);
 	}
@@ -1147,28 +1222,6 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 			h->seg_sfac[cpl] = with <= budget;
 			h->seg_smem[cpl] = (size_t)(h->seg_sfac[cpl] ? with : without);
 			if (!h->seg_sfac[cpl] && without > budget) h->seg_ok = false;
-		}
-	}
-	if (h->seg_ok) {
-		const size_t nblk_ff = (size_t)nff * h->nlh, nblk_c = (size_t)h->K * h->B * M * np;
-		std::vector<double2> sf(nblk_ff * N * P), sb(nblk_ff * N * P);
-		switch (P) {
-		case 3: host_spikes<3>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 4: host_spikes<4>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 5: host_spikes<5>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 6: host_spikes<6>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 7: host_spikes<7>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 8: host_spikes<8>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		}
-		if ((rc = dalloc(&h->spf_ff, sf.size())) || (rc = dalloc(&h->spb_ff, sb.size())) ||
-			(rc = dalloc(&h->spf_c, nblk_c * N * P)) || (rc = dalloc(&h->spb_c, nblk_c * N * P)))
-			return fail(rc);
-		if (cudaMemcpy(h->spf_ff, sf.data(), sizeof(double2) * sf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-			cudaMemcpy(h->spb_ff, sb.data(), sizeof(double2) * sb.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-			cudaMemset(h->spf_c, 0, sizeof(double2) * nblk_c * N * P) != cudaSuccess ||
-			cudaMemset(h->spb_c, 0, sizeof(double2) * nblk_c * N * P) != cudaSuccess) {
-			set_error("initial device copies failed");
-			return fail(QPC_ERR_CUDA);
 		}
 	}
 	if (h->hpi) {
@@ -1208,6 +1261,22 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 	std::memset(h->gsel, 0, sizeof(h->gsel));
 	for (int g = 1; g <= P; ++g) if (P % g == 0 && (g <= 4 || g == P)) h->gcand.push_back(g);
 	if (h->seg_ok) h->gcand.push_back(QPC_SEG);	// the segmented solver
+	h->h_R.assign(R, R + (size_t)N * NE);
+	h->ffh.swap(ffh);
+	// the position basis, unless a switch asks for kernels of the banded solves (QPC_POS=1 keeps it all the same)
+	const char* ps = getenv("QPC_POS");
+	if (ps ? atoi(ps) != 0 : !getenv("QPC_CHAIN_G") && !getenv("QPC_LTRANS_TC")) {
+		pos_setup in{dev, N, P, L, M, d.m0, h->B, h->nlh, np, nff, dt, h->S, h->R, Vh.data(), lamp.data(), nullptr, h->stream};
+		int64_t* one = nullptr;
+		std::vector<int64_t> ones((size_t)N, 1);
+		if ((rc = dalloc(&one, (size_t)N))) return fail(rc);
+		if (cudaMemcpy(one, ones.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice) != cudaSuccess) { cudaFree(one); set_error("initial device copies failed"); return fail(QPC_ERR_CUDA); }
+		in.fieldfree = [&](double2* X, double2* wk, int J, int fi) { return fieldfree_columns(h, X, wk, J, fi, one); };
+		rc = pos_create(in, &h->pos);
+		cudaFree(one);
+		if (rc) return fail(rc);
+	}
+	if (!h->pos) if ((rc = need_chains(h))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }
@@ -1227,6 +1296,8 @@ int qpc_lgwz_destroy(qpc_lgwz* h)
 {
 	if (!h) return QPC_OK;
 	if (h->stream) cudaStreamSynchronize(h->stream);
+	pos_destroy(h->pos);
+	cudaFree(h->dperm);
 	cudaFree(h->S); cudaFree(h->R); cudaFree(h->Vh); cudaFree(h->lamp); cudaFree(h->ff); cudaFree(h->lt_dig); cudaFree(h->lt_fex);
 	cudaFree(h->ffmap); cudaFree(h->ffmap_id);
 	cudaFree(h->spf_c); cudaFree(h->spb_c); cudaFree(h->spf_ff); cudaFree(h->spb_ff);
@@ -1249,27 +1320,43 @@ int qpc_lgwz_destroy(qpc_lgwz* h)
 	return QPC_OK;
 }
 
-static int put_common(qpc_lgwz* h, const double* src, cudaMemcpyKind kind)
+// the state in st (r-major) / in hostlay (the caller's [inst][m][l][r])
+static int need_rmajor(qpc_lgwz* h)
 {
-	long sl = state_len(h);
-	// the stream idle first: a copy from pageable memory then never waits for queued work
-	if (kind == cudaMemcpyHostToDevice) if (int rc = wait_stream(h)) return rc;
-	QPC_CUDA(cudaMemcpyAsync(h->hostlay, src, sizeof(double2) * sl, kind, h->stream));
-	long nblk = (long)h->B * h->M;
-	k_to_rmajor<<<(unsigned)((sl + 255) / 256), 256, 0, h->stream>>>(h->hostlay, h->st, h->N, h->L, nblk);
+	const long sl = state_len(h);
+	if (!h->st) if (int rc = dalloc(&h->st, sl)) return rc;
+	if (h->st_valid) return QPC_OK;
+	k_to_rmajor<<<(unsigned)((sl + 255) / 256), 256, 0, h->stream>>>(h->hostlay, h->st, h->N, h->L, (long)h->B * h->M);
 	LAUNCH(h);
 	QPC_CUDA(cudaGetLastError());
+	h->st_valid = true;
+	return QPC_OK;
+}
+static int need_lmajor(qpc_lgwz* h)
+{
+	const long sl = state_len(h);
+	if (h->lay_valid) return QPC_OK;
+	k_to_lmajor<<<(unsigned)((sl + 255) / 256), 256, 0, h->stream>>>(h->st, h->hostlay, h->N, h->L, (long)h->B * h->M);
+	LAUNCH(h);
+	QPC_CUDA(cudaGetLastError());
+	h->lay_valid = true;
+	return QPC_OK;
+}
+
+static int put_common(qpc_lgwz* h, const double* src, cudaMemcpyKind kind)
+{
+	// the stream idle first: a copy from pageable memory then never waits for queued work
+	if (kind == cudaMemcpyHostToDevice) if (int rc = wait_stream(h)) return rc;
+	QPC_CUDA(cudaMemcpyAsync(h->hostlay, src, sizeof(double2) * state_len(h), kind, h->stream));
+	h->lay_valid = true;
+	h->st_valid = false;
 	return wait_stream(h);
 }
 static int get_common(qpc_lgwz* h, double* dst, cudaMemcpyKind kind)
 {
-	long sl = state_len(h);
-	long nblk = (long)h->B * h->M;
-	k_to_lmajor<<<(unsigned)((sl + 255) / 256), 256, 0, h->stream>>>(h->st, h->hostlay, h->N, h->L, nblk);
-	LAUNCH(h);
-	QPC_CUDA(cudaGetLastError());
-	if (kind == cudaMemcpyDeviceToHost) return copy_to_host(dst, h->hostlay, sizeof(double2) * sl, h->stream);
-	QPC_CUDA(cudaMemcpyAsync(dst, h->hostlay, sizeof(double2) * sl, kind, h->stream));
+	if (int rc = need_lmajor(h)) return rc;
+	if (kind == cudaMemcpyDeviceToHost) return copy_to_host(dst, h->hostlay, sizeof(double2) * state_len(h), h->stream);
+	QPC_CUDA(cudaMemcpyAsync(dst, h->hostlay, sizeof(double2) * state_len(h), kind, h->stream));
 	return wait_stream(h);
 }
 
@@ -1308,6 +1395,65 @@ int qpc_lgwz_stream(qpc_lgwz* h, void** stream)
 
 static int mask_prepare(qpc_lgwz* h);
 static void mask_enqueue(qpc_lgwz* h, cudaStream_t st, const int64_t* ntt, long step);
+
+// the loop in the position basis; pf, pt: nt_field and nt_total in the sorted order of perm
+static int run_pos(qpc_lgwz* h, const std::vector<int64_t>& pf, const std::vector<int64_t>& pt, const std::vector<int>& perm, long smax, long ntt_max,
+	const double* mband, bool dipole, double* zlist, int64_t ldz)
+{
+	const int B = h->B;
+	if (mband) {
+		if (int rc = mask_prepare(h)) return rc;
+		QPC_CUDA(cudaMemcpyAsync(h->mM, mband, sizeof(double) * h->N * (h->P + 1), cudaMemcpyHostToDevice, h->stream));
+	}
+	if (int rc = wait_stream(h)) return rc;
+	pos_run r{};
+	r.state = h->hostlay; r.perm = h->dperm; r.ntf = h->ntf; r.ntt = h->ntt; r.ftab = h->ftab; r.ld = h->ld;
+	r.mask = mband ? h->mM : nullptr;
+	r.z = dipole ? h->zdev : nullptr;
+	r.ldz = ldz;
+	r.launches = &h->launches;
+	r.stream = h->stream;
+	int open = -1;
+	if (h->profiling) {
+		r.prof_begin = [&](int, cudaStream_t st) {
+			open = (int)h->evuse.size() * 2;
+			while ((int)h->evpool.size() < open + 2) { cudaEvent_t e; cudaEventCreate(&e); h->evpool.push_back(e); }
+			cudaEventRecord(h->evpool[open], st);
+		};
+		r.prof_end = [&](int kind, cudaStream_t st) {
+			cudaEventRecord(h->evpool[open + 1], st);
+			h->evuse.push_back({kind, open});
+		};
+	}
+	h->st_valid = false;
+	QPC_CUDA(cudaEventRecord(h->ev0, h->stream));
+	if (int rc = pos_begin(h->pos, r)) return rc;
+	const long send = mband ? ntt_max + 1 : smax;
+	int Bc = 0, Bf = B;
+	while (Bc < B && pf[Bc] > 0) ++Bc;
+	for (long s = 0; s < send; ++s) {
+		while (Bc > 0 && pf[Bc - 1] < s) --Bc;
+		while (Bf > 0 && pt[Bf - 1] <= s) --Bf;
+		if (int rc = pos_step(h->pos, r, s, Bc, Bf)) return rc;
+	}
+	if (int rc = pos_end(h->pos, r)) return rc;
+	QPC_CUDA(cudaEventRecord(h->ev1, h->stream));
+	const long sl = state_len(h);
+	k_status_check<<<(unsigned)((sl + 255) / 256), 256, 0, h->stream>>>(h->hostlay, sl, h->status);
+	LAUNCH(h);
+	QPC_CUDA(cudaGetLastError());
+	const int rc = read_status(h);
+	float ms = 0.f;
+	cudaEventElapsedTime(&ms, h->ev0, h->ev1);
+	h->last_ms = ms;
+	collect_profile(h);
+	if (dipole && rc == QPC_OK) {
+		std::vector<double> zh((size_t)B * ldz);
+		if (int rc2 = copy_to_host(zh.data(), h->zdev, sizeof(double) * zh.size(), h->stream)) return rc2;
+		for (int k = 0; k < B; ++k) std::memcpy(zlist + (size_t)perm[k] * ldz, zh.data() + (size_t)k * ldz, sizeof(double) * ldz);
+	}
+	return rc;
+}
 
 static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* nt_field, const int64_t* nt_total,
 	const double* F, double* zlist, int64_t ldz, const qpc_run_opts* opts = nullptr)
@@ -1373,14 +1519,24 @@ static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* 
 		h->ffmap_cur = h->ffmap;
 	}
 	QPC_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
-	if (!ident) if (int rc = permute_instances(h, perm, false)) return rc;
+	// the position basis: plain runs, the absorbing mask, and the dipole of R itself (diagonal there)
+	const bool pos = h->pos && !tsf && (!F || std::memcmp(F, h->h_R.data(), sizeof(double) * h->h_R.size()) == 0);
+	if (pos) {
+		if (int rc = need_lmajor(h)) return rc;
+		QPC_CUDA(cudaMemcpyAsync(h->dperm, perm.data(), sizeof(int) * B, cudaMemcpyHostToDevice, h->stream));
+	} else {
+		int rc;
+		if ((rc = need_chains(h)) || (rc = need_rmajor(h))) return rc;
+		h->lay_valid = false;
+		if (!ident) if ((rc = permute_instances(h, perm, false))) return rc;
+	}
 	h->ld = anyfield ? (long)ld : 0;
 	if (F) {
 		const int N = h->N, NE = h->P + 1, M = h->M, L = h->L;
 		long ntmax = 0;
 		for (int k = 0; k < B; ++k) ntmax = std::max<long>(ntmax, nt_total[k]);
 		if (!zlist || ldz < ntmax) { set_error("zlist NULL or ldz=%lld < max nt_total=%ld", (long long)ldz, ntmax); return QPC_ERR_ARGS; }
-		if (!h->obsF) {
+		if (!pos && !h->obsF) {
 			std::vector<double> y((size_t)M * L);
 			for (int m = 0; m < M; ++m) qpc_y10_coupling(L, h->d.m0 + m, y.data() + (size_t)m * L);
 			int rc;
@@ -1395,12 +1551,13 @@ static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* 
 			if (int rc = dalloc(&h->zdev, (size_t)B * ldz)) return rc;
 			h->zcap = (size_t)B * ldz;
 		}
-		QPC_CUDA(cudaMemcpyAsync(h->obsF, F, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream));
+		if (!pos) QPC_CUDA(cudaMemcpyAsync(h->obsF, F, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream));
 		QPC_CUDA(cudaMemsetAsync(h->zdev, 0, sizeof(double) * B * ldz, h->stream));
 		if (int rc = wait_stream(h)) return rc;
 		h->ldz = ldz;
-		h->observing = true;
+		h->observing = !pos;
 	}
+	if (pos) return run_pos(h, pf, pt, perm, smax, ntt_max, mband, F != nullptr, zlist, ldz);
 	// Instance groups (contiguous in the sorted order, balanced by work) on their
 	// own streams; within a group, the instances still in their pulse at step s
 	// are a prefix, and the field-free ones lie below a bound.
@@ -1564,6 +1721,7 @@ int qpc_lgwz_propagate_free(qpc_lgwz* h)
 int qpc_lgwz_norm(qpc_lgwz* h, double* norm)
 {
 	if (!h || !norm) { set_error("NULL argument"); return QPC_ERR_ARGS; }
+	if (int rc = need_rmajor(h)) return rc;
 	long nch = (long)h->B * h->M * h->L;
 	k_band_inner<<<(unsigned)((nch + 127) / 128), 128, 0, h->stream>>>(h->st, h->S, h->P + 1, h->N, h->L, nch, 0, h->red);
 	LAUNCH(h);
@@ -1636,6 +1794,9 @@ int qpc_lgwz_mask(qpc_lgwz* h, const double* M)
 	const int N = h->N, NE = h->P + 1;
 	if (int rc = wait_stream(h)) return rc;
 	if (int rc = mask_prepare(h)) return rc;
+	if (int rc = need_rmajor(h)) return rc;
+	if (!h->wk) if (int rc = dalloc(&h->wk, (size_t)state_len(h))) return rc;
+	h->lay_valid = false;
 	QPC_CUDA(cudaMemcpyAsync(h->mM, M, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream));
 	mask_enqueue(h, h->stream, nullptr, 0);
 	QPC_CUDA(cudaGetLastError());
@@ -1647,6 +1808,7 @@ int qpc_lgwz_dipole(qpc_lgwz* h, const double* F, double* out)
 	if (!h || !F || !out) { set_error("NULL argument"); return QPC_ERR_ARGS; }
 	const int N = h->N, NE = h->P + 1, L = h->L, M = h->M;
 	if (int rc = wait_stream(h)) return rc;
+	if (int rc = need_rmajor(h)) return rc;
 	// stream-ordered scratch: freed in stream order, so no later wait can block on it
 	double* dF = nullptr;
 	if (cudaMallocAsync((void**)&dF, sizeof(double) * N * NE, h->stream) != cudaSuccess) { set_error("cudaMallocAsync failed"); return QPC_ERR_NOMEM; }
@@ -1701,6 +1863,7 @@ int qpc_lgwz_projection(qpc_lgwz* h, const int32_t* n_state, const double* basis
 	}
 	if (nmax == 0) return QPC_OK;
 	if (int rc = wait_stream(h)) return rc;
+	if (int rc = need_rmajor(h)) return rc;
 	// stream-ordered scratch: freed in stream order, so no later wait can block on it
 	void* buf[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 	const size_t bytes[5] = {sizeof(double) * (size_t)std::max<long>(boff[nl], 1), sizeof(long) * (nl + 1), sizeof(long) * (nch + 1),
