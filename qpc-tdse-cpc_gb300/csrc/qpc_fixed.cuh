@@ -1,0 +1,80 @@
+// Fixed-point products of FP64 vectors with fixed real or complex matrices, as the kernels of qpc_radial.cu,
+// qpc_pos.cu and qpc_vpos.cu form them (the arithmetic and its error: qpc_radial.cu): limbs, sums and the one
+// rounding back.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace qpc {
+
+constexpr int TM = 32;		// rows (positions) of a tile, one per lane
+constexpr int KC = 16;		// k per chunk of the stored operators
+
+__device__ __forceinline__ int bexp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+// v as limbs (hi, lo), v = (hi 2^28 + lo) 2^(E - 1078), |hi| <= 2^28, -2^27 <= lo < 2^27; E >= bexp(v)
+__device__ __forceinline__ int2 quant(double v, int E)
+{
+	const int h = __double2hiint(v);
+	const int ex = (h >> 20) & 0x7ff;
+	const int d = E - ex;
+	unsigned long long m = ((unsigned long long)(unsigned)((h & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(v);
+	m <<= 3;
+	m = (d > 57 || ex == 0) ? 0ull : (m + ((1ull << d) >> 1)) >> d;
+	long long x = h < 0 ? -(long long)m : (long long)m;
+	const int hi = (int)((x + (1ll << 27)) >> 28);
+	return make_int2(hi, (int)(x - ((long long)hi << 28)));
+}
+
+// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^61; nf: the operand was not finite
+__device__ __forceinline__ double to_double(long long h, long long m, int s, bool nf)
+{
+	long long q = (h << 2) | (m >> 26);
+	unsigned long long a = q < 0 ? 0ull - (unsigned long long)q : (unsigned long long)q;
+	const int lz = __clzll((long long)a);
+	const int e = 1023 + 63 - lz + s - 2;
+	a <<= (lz & 63);
+	unsigned long long b = ((unsigned long long)(unsigned)(e - 1) << 52) + (a >> 11) + ((a >> 10) & 1ull);
+	b |= (unsigned long long)q & 0x8000000000000000ull;
+	if (q == 0 || e < 1) b = 0ull;
+	if (nf) b = 0x7ff8000000000000ull;
+	return __longlong_as_double((long long)b);
+}
+
+__device__ __forceinline__ long long madw(int a, int b, long long c) { return c + (long long)a * b; }
+__device__ __forceinline__ void flush(long long& h, long long& m) { h += m >> 28; m &= (1ll << 28) - 1; }
+
+// v in [-1, 1] as limbs of unit 2^-56 (host side)
+inline int2 limbs_of(double v)
+{
+	const long long x = __builtin_llrint(v * 72057594037927936.0);
+	const int hi = (int)((x + (1ll << 27)) >> 28);
+	return make_int2(hi, (int)(x - ((long long)hi << 28)));
+}
+
+// outputs o0 .. o0+G-1 of a real matrix (element (o, k) at V[o * so + k * sk]) times the column in x[k * xk]; the
+// mixed sums hold 64 k (128 products below 2^55): LONG carries them into the high ones that often
+template <int G, bool LONG = false>
+__device__ __forceinline__ void local_product(const int2* __restrict__ V, int so, int sk, int nk, int no, const int4* __restrict__ x, int xk,
+	long long (&h)[G][2], long long (&m)[G][2])
+{
+#pragma unroll
+	for (int g = 0; g < G; ++g) h[g][0] = h[g][1] = m[g][0] = m[g][1] = 0;
+	for (int k0 = 0; k0 < nk; k0 += LONG ? 64 : nk) {
+		const int k1 = LONG ? min(nk, k0 + 64) : nk;
+#pragma unroll 4
+		for (int k = k0; k < k1; ++k) {
+			const int4 y = x[k * xk];
+#pragma unroll
+			for (int g = 0; g < G; ++g) {
+				const int2 a = __ldg(V + (g < no ? g : 0) * so + k * sk);
+				h[g][0] = madw(a.x, y.x, h[g][0]); h[g][1] = madw(a.x, y.z, h[g][1]);
+				m[g][0] = madw(a.x, y.y, m[g][0]); m[g][0] = madw(a.y, y.x, m[g][0]);
+				m[g][1] = madw(a.x, y.w, m[g][1]); m[g][1] = madw(a.y, y.z, m[g][1]);
+			}
+		}
+#pragma unroll
+		for (int g = 0; g < G; ++g) { flush(h[g][0], m[g][0]); flush(h[g][1], m[g][1]); }
+	}
+}
+
+} // namespace qpc

@@ -1,0 +1,107 @@
+// The radial operators of a grid in a localised orthonormal basis, stored for fixed-point banded products
+// (qpc_radial.cu).
+#pragma once
+#include "qpc_internal.h"
+#include "qpc_cuda_util.cuh"
+#include "qpc_fixed.cuh"
+#include <functional>
+#include <vector>
+
+namespace qpc {
+
+constexpr int WMAX = 176;	// widest band (either side of the diagonal) the products take
+
+struct band_args {
+	const char* A;		// operators, [set][nlh] of astride bytes
+	long astride, set_stride;
+	const int4* td;		// per tile: first chunk, first and end chunk with hi limbs, end chunk
+	const long* toff;	// per tile: byte offset
+	const int* lmap;	// channel -> operator of a set
+	const int* amap;	// destination slot -> set (NULL: one set)
+	int ea;			// |A| <= 2^ea
+	int N, ntile, nchan, ncols;
+	const double2 *s0, *s1;	// [slot][nchan][N]; s1 where par[slot] is odd
+	const int *e0, *e1;	// largest biased exponent per [slot][nchan][tile]
+	const int64_t* par;
+	const int* smap;	// slot -> source slot (NULL: the same)
+	const int* dmap;	// slot -> destination slot (NULL: the same)
+	double2* dst;
+	int* edst;
+	const int64_t* nta;	// slots with step < nta[slot] take part (NULL: all)
+	long step;
+	int tile0;		// first tile of the launch
+};
+
+// an operator (or one per l and set) in the layout k_band_apply reads: per tile of TM rows the chunks of KC columns
+// td = (first, first with hi limbs, end of those, end) at byte off
+struct band_store {
+	int w = 0, ea = 0;
+	long stride = 0;		// bytes of one operator
+	std::vector<int4> td;
+	std::vector<long> off;
+	int4* d_td = nullptr;
+	long* d_off = nullptr;
+	char* A = nullptr;
+	size_t cap = 0;
+	void release() { cudaFree(d_td); cudaFree(d_off); cudaFree(A); d_td = nullptr; d_off = nullptr; A = nullptr; }
+};
+
+// what radial_create reads: device bands S, R [N][P+1] (R: the operator the basis diagonalises, its eigenvalues
+// ascending with the row), nff sets of field-free operators for l = 0..nlh-1.  fieldfree(X, wk, J, fi) applies the
+// step of set fi to J vectors on `stream`: X[J][N][nlh] (r-major) when rmajor, else X[J][nlh][N]; wk the same size.
+struct radial_setup {
+	int N, P, nlh, nff;
+	const double *S, *R;
+	bool rmajor;
+	std::function<int(double2*, double2*, int, int)> fieldfree;
+	cudaStream_t stream;
+};
+
+// eigenvectors x_i of (R, S): X^T S X = 1, X^T R X = diag(r); c = X y
+struct radial_ops {
+	int N = 0, P = 0, nlh = 0, nff = 1, ntile = 0;
+	double *Xt = nullptr, *r = nullptr;	// x_i as rows, eigenvalues
+	band_store F, W, X;			// X^T S F_l X, X^T S, X
+	int* zero = nullptr;			// zeros [max(nlh, nmap)]
+	unsigned long long* prof = nullptr;
+};
+
+// ok = false (with QPC_OK): S not positive definite, eigenvalues not apart, or an operator that does not fall off
+// within WMAX of the diagonal (or takes more than 16 GB)
+int radial_create(radial_ops* p, const radial_setup& in, int nmap, bool* ok);
+void radial_destroy(radial_ops* p);
+
+// A (device, FP64, element (i, j) at A[i si + j sj]) into b, banded where it falls off (ok), or dense
+int store_banded(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st, bool* ok);
+int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st);
+// A [N][N] = X^T B X for a symmetric band B, or for an anti-symmetric one given by its upper entries (device
+// [N][P+1]), zero beyond ~WMAX of the diagonal; Bx scratch [N][N]
+int project_band(const radial_ops* p, const double* B, bool anti, double* Bx, double* A, cudaStream_t st);
+
+// rows of Qt [N][N] made orthonormal to rounding from nearly so (ok); E, T scratch [N][N]
+int orthonormalise(double* Qt, int N, double* E, double* T, cudaStream_t st, bool* ok);
+
+band_args band_args_of(const radial_ops* p, const band_store& b, int nchan, int ncols);
+void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st);
+// largest biased exponent of every TM-row tile of src [nvec][N]
+void exponents(const double2* src, int* ex, int N, int ntile, long nvec, cudaStream_t st);
+
+// device scratch of a set-up, given back at its end
+struct scratch {
+	cudaStream_t st;
+	std::vector<void*> ptr;
+	explicit scratch(cudaStream_t s) : st(s) {}
+	~scratch() { for (void* q : ptr) cudaFreeAsync(q, st); }
+	template <class T> int get(T** q, size_t n)
+	{
+		if (cudaMallocAsync((void**)q, sizeof(T) * std::max<size_t>(n, 1), st) != cudaSuccess) {
+			cudaGetLastError();
+			set_error("set-up scratch of %zu bytes", sizeof(T) * n);
+			return QPC_ERR_NOMEM;
+		}
+		ptr.push_back(*q);
+		return QPC_OK;
+	}
+};
+
+} // namespace qpc

@@ -33,6 +33,7 @@
 #include <cusolverDn.h>
 #include "qpc_gemm.cuh"
 #include "qpc_ozaki.cuh"
+#include "qpc_vpos.cuh"
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
@@ -576,6 +577,9 @@ struct qpc_vgwr {
 	double *dxs = nullptr, *dys = nullptr;
 	size_t dcap = 0;
 	int dnblk = 1;
+	// steps with diagonal radial couplings (qpc_vpos.cu) at the sizes that suit them
+	vpos_path* pos = nullptr;
+	int64_t* ntts = nullptr;                       // device [B]: nt_total by sorted slot
 };
 
 namespace {
@@ -584,6 +588,8 @@ void vg_free(qpc_vgwr* h)
 {
 	if (!h) return;
 	cudaSetDevice(h->dev);
+	vpos_destroy(h->pos);
+	if (h->ntts) cudaFree(h->ntts);
 	void* ps[] = {h->S, h->Ri, h->D, h->lam[0], h->lam[1], h->lam[2], h->lam[3], h->tmbuf, h->Lrow,
 		h->Dinv, h->X, h->W, h->U, h->atab, h->ntt, h->perm, h->nrm, h->chmap};
 	for (void* p : ps) if (p) cudaFree(p);
@@ -922,6 +928,57 @@ int device_transforms(qpc_vgwr* h, std::vector<int>& chmap, std::vector<double> 
 	return QPC_OK;
 }
 
+// one field-free step on J vectors X[J][nlh][N] (every l once), wk the same size; act: J ones, id: 0..nlh-1
+int fieldfree_columns(qpc_vgwr* h, double2* X, double2* wk, int J, const long long* act, const int* id)
+{
+	const int N = h->N;
+	const unsigned g = (unsigned)(((long)J * h->nlh + VG_THREADS - 1) / VG_THREADS);
+	auto run = [&](auto kern) { kern<<<g, VG_THREADS, 0, h->st>>>(X, wk, h->S, h->Lrow, h->Dinv, act, id, id, 0, N, h->nlh, 1, 0, h->nlh, J); };
+	switch (h->P) {
+	case 3: run(k_vg_ff<3>); break;
+	case 4: run(k_vg_ff<4>); break;
+	case 5: run(k_vg_ff<5>); break;
+	case 6: run(k_vg_ff<6>); break;
+	case 7: run(k_vg_ff<7>); break;
+	case 8: run(k_vg_ff<8>); break;
+	default: set_error("unsupported B-spline degree %d", h->P); return QPC_ERR_ARGS;
+	}
+	QPC_CUDA(cudaGetLastError());
+	return QPC_OK;
+}
+
+// the path with diagonal radial couplings, unless QPC_POS=0 or a switch asks for kernels of the other one
+int make_pos(qpc_vgwr* h, const std::vector<int>& chmap, const double* Ri)
+{
+	const char* ps = std::getenv("QPC_POS");
+	if (ps ? std::atoi(ps) == 0 : std::getenv("QPC_VG_GEMM") || std::getenv("QPC_OZ_TC") || std::getenv("QPC_OZ_TMA")) return QPC_OK;
+	vpos_setup in{};
+	in.N = h->N; in.P = h->P; in.nch = h->nch; in.nlh = h->nlh; in.B = h->B; in.n_l = h->d.n_l; in.m0 = h->d.m0; in.dt = h->dt;
+	in.S = h->S; in.D = h->D; in.Ri = Ri; in.chmap = chmap.data(); in.stream = h->st;
+	for (int b = 0; b < 2; ++b) {
+		in.off[b] = h->off[b]; in.na[b] = h->na[b]; in.nb[b] = h->nb[b];
+		for (int s = 0; s < 2; ++s) {
+			for (int m = 0; m < 5; ++m) in.tm[m][b][s] = h->tm[m][b][s];
+			for (int c = 0; c < 4; ++c) in.gam[c][b][s] = h->gam[c][b][s];
+		}
+	}
+	for (int c = 0; c < 4; ++c) in.lam[c] = h->lam[c];
+	const int n = std::max(h->N, h->nlh);
+	std::vector<long long> one(n, 1);
+	std::vector<int> id(n);
+	std::iota(id.begin(), id.end(), 0);
+	long long* done = nullptr;
+	int* did = nullptr;
+	int rc;
+	if ((rc = dalloc(&done, n)) || (rc = dalloc(&did, n)) || (rc = dalloc(&h->ntts, (size_t)h->B))) { cudaFree(done); cudaFree(did); return rc; }
+	if (cudaMemcpy(done, one.data(), sizeof(long long) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
+		cudaMemcpy(did, id.data(), sizeof(int) * n, cudaMemcpyHostToDevice) != cudaSuccess) { set_error("upload"); rc = QPC_ERR_CUDA; }
+	in.fieldfree = [&](double2* X, double2* wk, int J, int) { return fieldfree_columns(h, X, wk, J, done, did); };
+	if (!rc) rc = vpos_create(in, &h->pos);
+	cudaFree(done); cudaFree(did);
+	return rc;
+}
+
 } // namespace
 
 extern "C" {
@@ -1005,6 +1062,7 @@ int qpc_vgwr_create(const qpc_dims* dims, double dt, const double* S, const doub
 	}
 	for (int c = 0; c < 4; ++c)
 		if (cudaMemcpy(h->lam[c], lam[c].data(), sizeof(double) * nch, cudaMemcpyHostToDevice) != cudaSuccess) { set_error("upload"); return fail(QPC_ERR_CUDA); }
+	if ((rc = make_pos(h, chmap, Rinv))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }
@@ -1145,13 +1203,33 @@ static int run_impl(qpc_vgwr* h, const double* atab, int64_t ld, const int64_t* 
 	// instances running (nt_total) at step s: those with nt_total > s; the field-free kernel
 	// checks nt_total per instance, and covers the prefix up to the last running one
 	h->launches = 0;
-	QPC_CUDA(cudaEventRecord(h->ev0, h->st));
-	for (long s = 0; s < smax; ++s) {
-		int nlive = 0, nff = 0;
+	vpos_run vr{};
+	cudaEvent_t open_ev = nullptr;
+	if (h->pos) {
+		std::vector<int64_t> nts(B);
+		for (int k = 0; k < B; ++k) nts[k] = nt_total[perm[k]];
+		QPC_CUDA(cudaMemcpyAsync(h->ntts, nts.data(), sizeof(int64_t) * B, cudaMemcpyHostToDevice, h->st));
+		if (int rc = wait_on(h->st)) return rc;
+		vr.X = h->X; vr.atab = h->atab; vr.ld = anyfield ? ld : 0; vr.perm = h->perm; vr.ntt = h->ntts; vr.launches = &h->launches;
+		if (h->profiling) {
+			vr.prof_begin = [&](int) { open_ev = prof_begin(h); };
+			vr.prof_end = [&](int kind) { prof_end(h, kind, open_ev); };
+		}
+	}
+	auto counts = [&](long s, int& nlive, int& nff) {
+		nlive = nff = 0;
 		for (int k = 0; k < B; ++k) {
 			if (s < nt_field[perm[k]]) nlive = k + 1;
 			if (s < nt_total[perm[k]]) nff = k + 1;
 		}
+	};
+	QPC_CUDA(cudaEventRecord(h->ev0, h->st));
+	if (h->pos) if (int rc = vpos_begin(h->pos, vr)) return rc;
+	bool open = true;
+	for (long s = 0; s < smax; ++s) {
+		int nlive, nff;
+		counts(s, nlive, nff);
+		if (h->pos && F && s > 0) if (int rc = vpos_peek(h->pos, vr, s, nff)) return rc;
 		if (F && nff > 0 && h->ndpairs > 0) {
 			// the observation before step s (binsrc/sphTDSE.cpp:933-934)
 			k_vg_dip_part<<<dim3((unsigned)h->dnblk, (unsigned)nff), DIP_THREADS, 0, h->st>>>(h->X, h->dF, h->dpairs, h->dcoef,
@@ -1159,13 +1237,20 @@ static int run_impl(qpc_vgwr* h, const double* atab, int64_t ld, const int64_t* 
 			k_vg_dip_final<<<(unsigned)((nff + 127) / 128), 128, 0, h->st>>>(h->dpart, h->dnblk, nff, h->ntt, h->perm, s, ldz, h->dxs, h->dys);
 			h->launches += 2;
 		}
-		if (int rc = step_dispatch(h, s, anyfield ? ld : 0, nlive, nff)) return rc;
+		if (h->pos) {
+			int next, nff1;
+			counts(s + 1, next, nff1);
+			const bool close = F || next != nlive;
+			if (int rc = vpos_step(h->pos, vr, s, nlive, nff, open, close)) return rc;
+			open = close;
+		} else if (int rc = step_dispatch(h, s, anyfield ? ld : 0, nlive, nff)) return rc;
 	}
+	if (h->pos) if (int rc = vpos_end(h->pos, vr)) return rc;
 	QPC_CUDA(cudaGetLastError());
 	QPC_CUDA(cudaEventRecord(h->ev1, h->st));
 	if (!ident) if (int rc = permute(h, perm, true)) return rc;
 	if (int rc = wait_on(h->st)) return rc;
-	if (h->slices) if (int rc = oz_check(h->st)) return rc;
+	if (h->slices && !h->pos) if (int rc = oz_check(h->st)) return rc;
 	cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1);
 	prof_collect(h);
 	if (F) {
