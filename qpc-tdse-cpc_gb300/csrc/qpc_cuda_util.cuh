@@ -39,16 +39,20 @@ inline int wait_on(cudaStream_t st)
 	struct timespec t0, now;
 	clock_gettime(CLOCK_MONOTONIC, &t0);
 	const double limit = wait_limit_s();
-	for (long it = 0;; ++it) {
+	for (;;) {
 		cudaError_t e = cudaStreamQuery(st);
 		if (e == cudaSuccess) return QPC_OK;
 		if (e != cudaErrorNotReady) { set_error("stream error: %s", cudaGetErrorString(e)); return QPC_ERR_CUDA; }
 		clock_gettime(CLOCK_MONOTONIC, &now);
-		if ((double)(now.tv_sec - t0.tv_sec) + 1e-9 * (double)(now.tv_nsec - t0.tv_nsec) > limit) {
+		const double waited = (double)(now.tv_sec - t0.tv_sec) + 1e-9 * (double)(now.tv_nsec - t0.tv_nsec);
+		if (waited > limit) {
 			set_error("timed out after %.3g s waiting for the device", limit);
 			return QPC_ERR_TIMEOUT;
 		}
-		struct timespec ts = {0, it < 100 ? 2000L : 100000L};
+		// a sleep of any length takes ~55 us (the kernel's timer slack): poll without one for the first half millisecond
+		// (a single step is 30-100 us), then sleep between polls
+		if (waited < 5e-4) continue;
+		struct timespec ts = {0, waited < 0.05 ? 20000L : 100000L};
 		nanosleep(&ts, nullptr);
 	}
 }

@@ -8,6 +8,8 @@ namespace qpc {
 
 constexpr int TM = 32;		// rows (positions) of a tile, one per lane
 constexpr int KC = 16;		// k per chunk of the stored operators
+constexpr int TE = 8;		// rows that share a recorded exponent
+constexpr int EPT = TM / TE;
 
 __device__ __forceinline__ int bexp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
 
@@ -38,6 +40,14 @@ __device__ __forceinline__ double to_double(long long h, long long m, int s, boo
 	if (q == 0 || e < 1) b = 0ull;
 	if (nf) b = 0x7ff8000000000000ull;
 	return __longlong_as_double((long long)b);
+}
+
+// the largest of e over each group of TE lanes
+__device__ __forceinline__ int group_max(int e)
+{
+#pragma unroll
+	for (int o = 1; o < TE; o <<= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+	return e;
 }
 
 __device__ __forceinline__ long long madw(int a, int b, long long c) { return c + (long long)a * b; }

@@ -27,15 +27,17 @@ namespace {
 constexpr int LMAX = 128;	// most l channels
 
 // ------------------------------------------------------------------ the local part of a step
-// One block: TM positions of one (slot, m), all l; lane = position.  y -> E_k, O_k (the even-l and odd-l
-// halves of the transform by the eigenvectors of Y10; +-lambda share them), phases, and back:
+// One block: PT positions of one (slot, m), all l; PT lanes of a warp hold the positions, the 32 / PT groups of lanes
+// work as so many warps.  y -> E_k, O_k (the even-l and odd-l halves of the transform by the eigenvectors of Y10;
+// +-lambda share them), phases, and back:
 //   z+- = E +- O, z+' = phi z+, z-' = conj(phi) z-, s = z+' + z-' = 2 (c E + i s O), d = z+' - z-' = 2 (i s E + c O)
 // with phi = c + i s.  Both transforms in fixed point under each position's largest exponent, the phases in FP64
-// (28 instructions per pair and position: the kernel's largest single share).  The dipole of f(r) = r is
-// sum_k lambda_k r_j (|z+|^2 - |z-|^2) = sum_k 4 lambda_k r_j Re(conj(E_k) O_k).
+// (28 instructions per pair and position).  The dipole of f(r) = r is sum_k lambda_k r_j (|z+|^2 - |z-|^2) =
+// sum_k 4 lambda_k r_j Re(conj(E_k) O_k).  PT = 32 is bound by the multiply-adds; with too few blocks to fill the
+// SMs a block's own latency counts, and PT = 8 cuts it (four times the blocks, a quarter of the serial products).
 struct angle_args {
 	double2* y;		// [slot][M][L][N], in place
-	int* ex;		// [slot][M][L][ntile]
+	int* ex;		// [slot][M][L][ntile * EPT]
 	const int2* V;		// [M][npair+1][L] limbs, |V| <= 1
 	const double* lamp;	// [M][npair]
 	const double* r;	// [N]
@@ -46,7 +48,7 @@ struct angle_args {
 	int cmode;
 	double dt4;		// dt / 4
 	int N, ntile, L, M, npair;
-	double* zpart;		// [slot][M][ntile] of this step, or NULL
+	double* zpart;		// one per block, [slot][M][.], of this step, or NULL
 };
 
 __device__ __forceinline__ int power_of(long s, long nt, int cmode)
@@ -58,55 +60,56 @@ __device__ __forceinline__ int power_of(long s, long nt, int cmode)
 	return (s == 0 || s == nt) ? 1 : 2;
 }
 
-template <int G>
+template <int G, int PT>
 __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 {
+	constexpr int NV = 8 * 32 / PT, TPT = TM / PT;	// virtual warps; blocks per tile
 	extern __shared__ double2 sm[];
-	__shared__ int pe[8][32];
-	__shared__ double zs[8][32];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int tile = blockIdx.x % p.ntile;
-	const int im = blockIdx.x / p.ntile;	// slot * M + m
+	__shared__ int pe[NV][PT];
+	__shared__ double zs[NV][PT];
+	const int lane = threadIdx.x % PT, warp = threadIdx.x / PT;
+	const int tile = blockIdx.x % (p.ntile * TPT);
+	const int im = blockIdx.x / (p.ntile * TPT);	// slot * M + m
 	const int m = im % p.M, slot = im / p.M;
 	const int pw = power_of(p.step, p.ntf[slot], p.cmode);
 	const bool obs = p.zpart && p.step < p.ntt[slot];
 	if (pw == 0 && !obs) return;
 	const int L = p.L, np = p.npair, N = p.N;
-	double2* a = sm;		// [L][32]: y, then its limbs, then the eigen-channels' limbs
-	double2* b = sm + L * 32;	// [L][32]: E_k at 2k, O_k at 2k + 1, the zero channel at 2 npair
-	const int row = tile * TM + lane;
+	double2* a = sm;		// [L][PT]: y, then its limbs, then the eigen-channels' limbs
+	double2* b = sm + L * PT;	// [L][PT]: E_k at 2k, O_k at 2k + 1, the zero channel at 2 npair
+	const int row = tile * PT + lane;
 	const bool in = row < N;
 	double2* y = p.y + (long)im * L * N + row;
 	int e = 0;
-	for (int l = warp; l < L; l += 8) {
+	for (int l = warp; l < L; l += NV) {
 		const double2 v = in ? y[(long)l * N] : make_double2(0.0, 0.0);
-		a[l * 32 + lane] = v;
+		a[l * PT + lane] = v;
 		e = max(e, max(bexp(v.x), bexp(v.y)));
 	}
 	pe[warp][lane] = e;
 	__syncthreads();
 	e = 0;
 #pragma unroll
-	for (int w = 0; w < 8; ++w) e = max(e, pe[w][lane]);
-	for (int l = warp; l < L; l += 8) {
-		const double2 v = a[l * 32 + lane];
+	for (int w = 0; w < NV; ++w) e = max(e, pe[w][lane]);
+	for (int l = warp; l < L; l += NV) {
+		const double2 v = a[l * PT + lane];
 		const int2 q0 = quant(v.x, e), q1 = quant(v.y, e);
-		reinterpret_cast<int4*>(a)[l * 32 + lane] = make_int4(q0.x, q0.y, q1.x, q1.y);
+		reinterpret_cast<int4*>(a)[l * PT + lane] = make_int4(q0.x, q0.y, q1.x, q1.y);
 	}
 	__syncthreads();
 	const int4* qa = reinterpret_cast<const int4*>(a) + lane;
 	const int2* V = p.V + (long)m * (np + 1) * L;
 	const int nE = np + (L & 1), gE = (nE + G - 1) / G, gO = (np + G - 1) / G;
 	long long h[G][2], mm[G][2];
-	for (int t = warp; t < gE + gO; t += 8) {
+	for (int t = warp; t < gE + gO; t += NV) {
 		const bool odd = t >= gE;
 		const int k0 = (odd ? t - gE : t) * G, no = min(G, (odd ? np : nE) - k0);
-		local_product<G>(V + k0 * L + (odd ? 1 : 0), L, 2, odd ? L / 2 : (L + 1) / 2, no, qa + (odd ? 32 : 0), 64, h, mm);
+		local_product<G>(V + k0 * L + (odd ? 1 : 0), L, 2, odd ? L / 2 : (L + 1) / 2, no, qa + (odd ? PT : 0), 2 * PT, h, mm);
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
 				const int s = e - 1078;
-				b[(2 * (k0 + g) + (odd ? 1 : 0)) * 32 + lane] =
+				b[(2 * (k0 + g) + (odd ? 1 : 0)) * PT + lane] =
 					make_double2(to_double(h[g][0], mm[g][0], s, e == 0x7ff), to_double(h[g][1], mm[g][1], s, e == 0x7ff));
 			}
 	}
@@ -115,8 +118,8 @@ __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 	const double f = pw ? p.ftab[(long)slot * p.ld + p.step] * p.dt4 : 0.0;
 	double z = 0.0;
 	e = 0;
-	for (int k = warp; k < np; k += 8) {
-		const double2 E = b[(2 * k) * 32 + lane], O = b[(2 * k + 1) * 32 + lane];
+	for (int k = warp; k < np; k += NV) {
+		const double2 E = b[(2 * k) * PT + lane], O = b[(2 * k + 1) * PT + lane];
 		const double lam = p.lamp[m * np + k];
 		if (obs) z = fma(lam, fma(E.x, O.x, E.y * O.y), z);
 		if (pw) {
@@ -132,49 +135,52 @@ __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 			const double2 S = make_double2(fma(c, E.x, -s * O.y), fma(c, E.y, s * O.x));
 			const double2 D = make_double2(fma(c, O.x, -s * E.y), fma(c, O.y, s * E.x));
 			e = max(max(e, max(bexp(S.x), bexp(S.y))), max(bexp(D.x), bexp(D.y)));
-			b[(2 * k) * 32 + lane] = S;
-			b[(2 * k + 1) * 32 + lane] = D;
+			b[(2 * k) * PT + lane] = S;
+			b[(2 * k + 1) * PT + lane] = D;
 		}
 	}
 	if (obs) {
 		zs[warp][lane] = 4.0 * z * rj;
 		__syncthreads();
-		if (warp == 0) {
+		if (threadIdx.x < 32) {
 			double t = 0.0;
 #pragma unroll
-			for (int w = 0; w < 8; ++w) t += zs[w][lane];
+			for (int w = 0; w < NV; w += 32 / PT) t += zs[w + warp][lane];
 #pragma unroll
 			for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-			if (lane == 0) p.zpart[(long)im * p.ntile + tile] = t;
+			if (threadIdx.x == 0) p.zpart[(long)im * p.ntile * TPT + tile] = t;
 		}
 	}
 	if (pw == 0) return;
-	if ((L & 1) && warp == 7) { const double2 Z = b[2 * np * 32 + lane]; e = max(e, max(bexp(Z.x), bexp(Z.y))); }
+	if ((L & 1) && warp == NV - 1) { const double2 Z = b[2 * np * PT + lane]; e = max(e, max(bexp(Z.x), bexp(Z.y))); }
 	pe[warp][lane] = e;
 	__syncthreads();
 	e = 0;
 #pragma unroll
-	for (int w = 0; w < 8; ++w) e = max(e, pe[w][lane]);
-	for (int k = warp; k < L; k += 8) {
-		const double2 v = b[k * 32 + lane];
+	for (int w = 0; w < NV; ++w) e = max(e, pe[w][lane]);
+	for (int k = warp; k < L; k += NV) {
+		const double2 v = b[k * PT + lane];
 		const int2 q0 = quant(v.x, e), q1 = quant(v.y, e);
-		reinterpret_cast<int4*>(a)[k * 32 + lane] = make_int4(q0.x, q0.y, q1.x, q1.y);
+		reinterpret_cast<int4*>(a)[k * PT + lane] = make_int4(q0.x, q0.y, q1.x, q1.y);
 	}
 	__syncthreads();
 	const int nl0 = (L + 1) / 2, nl1 = L / 2, g0 = (nl0 + G - 1) / G, g1 = (nl1 + G - 1) / G;
-	for (int t = warp; t < g0 + g1; t += 8) {
+	const unsigned grp = PT == 32 ? 0xffffffffu : ((1u << PT) - 1) << (threadIdx.x & 31 & ~(PT - 1));
+	for (int t = warp; t < g0 + g1; t += NV) {
 		const int odd = t >= g0 ? 1 : 0;
 		const int o0 = (odd ? t - g0 : t) * G, no = min(G, (odd ? nl1 : nl0) - o0);
 		// even l: s_k (slots 2k) and, for odd n_l, the zero channel (slot 2 npair); odd l: d_k (slots 2k + 1)
-		local_product<G>(V + 2 * o0 + odd, 2, L, odd ? np : nE, no, qa + odd * 32, 64, h, mm);
+		local_product<G>(V + 2 * o0 + odd, 2, L, odd ? np : nE, no, qa + odd * PT, 2 * PT, h, mm);
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
 				const int s = e - 1078, l = 2 * (o0 + g) + odd;
 				const double2 v = make_double2(to_double(h[g][0], mm[g][0], s, e == 0x7ff), to_double(h[g][1], mm[g][1], s, e == 0x7ff));
 				if (in) y[(long)l * N] = v;
-				const int x = __reduce_max_sync(0xffffffffu, in ? max(bexp(v.x), bexp(v.y)) : 0);
-				if (lane == 0) p.ex[((long)im * L + l) * p.ntile + tile] = x;
+				int x = in ? max(bexp(v.x), bexp(v.y)) : 0;
+#pragma unroll
+				for (int o = 1; o < TE; o <<= 1) x = max(x, __shfl_xor_sync(grp, x, o));
+				if (lane % TE == 0) p.ex[((long)im * L + l) * p.ntile * EPT + row / TE] = x;
 			}
 	}
 }
@@ -211,8 +217,8 @@ struct pos_path {
 	static constexpr int ZB = 32;		// steps between two sums of the dipole's parts
 	long zfirst = 0;
 	int zcount = 0;
-	int angle_g = 3;
-	size_t angle_smem = 0;
+	int angle_g = 3;		// outputs per task of k_angle, PT = 32
+	bool angle_small = false;	// PT = 8, one output per task
 };
 
 
@@ -221,7 +227,7 @@ namespace {
 template <int G>
 void angle_launch(const pos_path* p, const angle_args& a, int slots, cudaStream_t st)
 {
-	k_angle<G><<<(unsigned)((long)slots * p->M * p->ntile), 256, p->angle_smem, st>>>(a);
+	k_angle<G, 32><<<(unsigned)((long)slots * p->M * p->ntile), 256, sizeof(double2) * 2 * 32 * p->L, st>>>(a);
 }
 
 int build(pos_path* p, const pos_setup& in, bool* ok)
@@ -239,19 +245,20 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 	QPC_CUDA(cudaMemcpy(p->V, V.data(), sizeof(int2) * V.size(), cudaMemcpyHostToDevice));
 	QPC_CUDA(cudaMemcpy(p->lamp, in.lamp, sizeof(double) * M * std::max(p->npair, 1), cudaMemcpyHostToDevice));
 	for (int i = 0; i < 2; ++i)
-		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile))) return rc;
-	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile))) return rc;
+		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
+	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
 	// outputs per task of k_angle: the fewest rounds of eight warps
 	int best = 1 << 30;
 	for (int g = 2; g <= 4; ++g) {
 		const int ne = p->npair + (L & 1), tasks = (ne + g - 1) / g + (p->npair + g - 1) / g, cost = (tasks + 7) / 8 * (g * 6 + 4);
 		if (cost < best) { best = cost; p->angle_g = g; }
 	}
-	p->angle_smem = sizeof(double2) * 2 * 32 * L;
+	// fewer blocks than SMs with 32 positions each: 8
+	p->angle_small = (long)p->B * M * p->ntile <= 304;
 	const int smem = (int)(sizeof(double2) * 64 * LMAX);
-	cudaFuncSetAttribute(k_angle<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-	cudaFuncSetAttribute(k_angle<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-	cudaFuncSetAttribute(k_angle<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<3, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<4, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	return QPC_OK;
 }
 
@@ -308,7 +315,7 @@ int pos_begin(pos_path* p, const pos_run& r)
 		if ((rc = store_banded(&p->ops, p->K, A, p->N, 1, st, &ok))) return rc;
 		if (!ok) { set_error("the mask does not fall off the diagonal in the position basis"); return QPC_ERR_NUMERIC; }
 	}
-	if (r.z && !p->zpart) if (int rc = dalloc(&p->zpart, (size_t)pos_path::ZB * p->B * p->M * p->ntile)) return rc;
+	if (r.z && !p->zpart) if (int rc = dalloc(&p->zpart, (size_t)pos_path::ZB * p->B * p->M * p->ntile * EPT)) return rc;
 	p->zcount = 0;
 	POS_PROF(QPC_KERNEL_TRANSFORM_FWD);
 	exponents(r.state, p->exin, p->N, p->ntile, nvec, st);
@@ -324,7 +331,7 @@ static void sum_dipole(pos_path* p, const pos_run& r)
 {
 	if (!p->zcount) return;
 	const int n = p->B * p->zcount;
-	k_dipole_sum<<<(n + 127) / 128, 128, 0, r.stream>>>(p->zpart, r.z, r.ldz, r.ntt, p->B, p->M * p->ntile, p->zfirst, p->zcount);
+	k_dipole_sum<<<(n + 127) / 128, 128, 0, r.stream>>>(p->zpart, r.z, r.ldz, r.ntt, p->B, p->M * p->ntile * (p->angle_small ? EPT : 1), p->zfirst, p->zcount);
 	++*r.launches;
 	p->zcount = 0;
 }
@@ -343,10 +350,11 @@ int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf)
 		a.step = s; a.cmode = cmode; a.dt4 = 0.25 * p->dt; a.N = p->N; a.ntile = p->ntile; a.L = p->L; a.M = p->M; a.npair = p->npair;
 		if (observe) {
 			if (!p->zcount) p->zfirst = s;
-			a.zpart = p->zpart + (size_t)p->zcount * p->B * p->M * p->ntile;
+			a.zpart = p->zpart + (size_t)p->zcount * p->B * p->M * p->ntile * (p->angle_small ? EPT : 1);
 			++p->zcount;
 		}
-		switch (p->angle_g) {
+		if (p->angle_small) k_angle<1, 8><<<(unsigned)((long)slots * p->M * p->ntile * EPT), 256, sizeof(double2) * 2 * 8 * p->L, st>>>(a);
+		else switch (p->angle_g) {
 		case 2: angle_launch<2>(p, a, slots, st); break;
 		case 3: angle_launch<3>(p, a, slots, st); break;
 		default: angle_launch<4>(p, a, slots, st); break;

@@ -16,6 +16,7 @@
 #include "qpc_radial.cuh"
 #include <cstring>
 #include <cmath>
+#include <type_traits>
 
 namespace qpc {
 
@@ -49,20 +50,21 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 	const int col0 = cg * COLS;
 	if (p.nta && KS == 8 && NB == 1 && !(p.step < p.nta[col0])) return;
 	const int4 td = p.td[tile];
-	const int t0 = td.x * KC / TM, t1 = min(p.ntile, (td.w * KC + TM - 1) / TM);
-	if (threadIdx.x < COLS) {
-		const int c = col0 + threadIdx.x;
+	// every column's largest exponent over the tile's k range, one warp per column
+	const int nex = p.ntile * EPT, x0 = td.x * KC / TE, x1 = td.w * KC / TE;
+	for (int cl = warp; cl < COLS; cl += 8) {
+		const int c = col0 + cl;
 		int e = 0;
 		const double2* src = nullptr;
 		if (c < p.ncols && (!p.nta || p.step < p.nta[c])) {
 			const bool odd = p.par && (p.par[c] & 1);
 			const long v = (long)(p.smap ? p.smap[c] : c) * p.nchan + ch;
-			const int* ex = (odd ? p.e1 : p.e0) + v * p.ntile;
-			for (int t = t0; t < t1; ++t) e = max(e, ex[t]);
+			const int* ex = (odd ? p.e1 : p.e0) + v * nex;
+			for (int t = x0 + lane; t < x1; t += 32) e = max(e, ex[t]);
 			src = (odd ? p.s1 : p.s0) + v * p.N;
 		}
-		sE[threadIdx.x] = e;
-		sp[threadIdx.x] = src;
+		e = __reduce_max_sync(0xffffffffu, e);
+		if (lane == 0) { sE[cl] = e; sp[cl] = src; }
 	}
 	// the stage's raw values arrive by cp.async in the order they are converted in (this thread's own elements)
 	const int lk = threadIdx.x % SK;
@@ -98,73 +100,85 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 		}
 		__syncthreads();
 		if (c0 + 2 * KS < td.w) load((c0 + 2 * KS) * KC + lk);
+		// the stage's chunks before, with and after the hi limbs.  Of every chunk a warp takes KC / KS k, so that the
+		// warps of a column have equal work whatever the kind of a chunk; with eight warps to a column (few columns,
+		// bound by the latency of the operator's loads) two whole chunks, all their loads in flight
+		constexpr int KW = KS == 8 ? KC : KC / KS;
+		const int k0 = KS == 8 ? 0 : ks * KW;
+		const int ce = min(c0 + 2 * KS, td.w);
+		auto span = [&](int ca, int cb, const char* seg, auto full) {
+			constexpr bool FULL = decltype(full)::value;
+			const int n = (cb - ca) * KW;
+			const int4* x = xs + ((ca - c0) * KC + k0) * XS + wc;
+			using elem = std::conditional_t<CX, std::conditional_t<FULL, int4, int2>, std::conditional_t<FULL, int2, int>>;
+			const elem* src = reinterpret_cast<const elem*>(seg) + k0 * TM + lane;
+			// UN loads in flight, then their products (elements past the end: zero)
+			for (int i0 = 0; i0 < n; i0 += UN) {
+				elem av[UN];
 #pragma unroll
-		for (int half = 0; half < 2; ++half) {
-			const int c = c0 + 2 * ks + half;
-			if (c >= td.w) break;
-			const int4* x = xs + (ks * 32 + half * KC) * XS + wc;
-			if (c >= td.y && c < td.z) {
-				const char* a0 = A + tl + (long)(c - td.y) * FB;
-				if (CX) {
-					const int4* ap = reinterpret_cast<const int4*>(a0) + lane;
-#pragma unroll UN
-					for (int k = 0; k < KC; ++k) {
-						const int4 a = __ldg(ap + k * TM);
-						const int nz = -a.z, nw = -a.w;
-#pragma unroll
-						for (int j = 0; j < NB; ++j) {
-							const int4 y = x[k * XS + j];
-							rh[j] = madw(a.x, y.x, rh[j]); rh[j] = madw(nz, y.z, rh[j]);
-							ih[j] = madw(a.x, y.z, ih[j]); ih[j] = madw(a.z, y.x, ih[j]);
-							rm[j] = madw(a.x, y.y, rm[j]); rm[j] = madw(a.y, y.x, rm[j]);
-							rm[j] = madw(nz, y.w, rm[j]); rm[j] = madw(nw, y.z, rm[j]);
-							im[j] = madw(a.x, y.w, im[j]); im[j] = madw(a.y, y.z, im[j]);
-							im[j] = madw(a.z, y.y, im[j]); im[j] = madw(a.w, y.x, im[j]);
-						}
-					}
-				} else {
-					const int2* ap = reinterpret_cast<const int2*>(a0) + lane;
-#pragma unroll UN
-					for (int k = 0; k < KC; ++k) {
-						const int2 a = __ldg(ap + k * TM);
-#pragma unroll
-						for (int j = 0; j < NB; ++j) {
-							const int4 y = x[k * XS + j];
-							rh[j] = madw(a.x, y.x, rh[j]); ih[j] = madw(a.x, y.z, ih[j]);
-							rm[j] = madw(a.x, y.y, rm[j]); rm[j] = madw(a.y, y.x, rm[j]);
-							im[j] = madw(a.x, y.w, im[j]); im[j] = madw(a.y, y.z, im[j]);
-						}
-					}
+				for (int u = 0; u < UN; ++u) {
+					const int i = i0 + u;
+					if constexpr (KW % UN == 0) av[u] = __ldg(src + ((i / KW) * KC + i % KW) * TM);
+					else av[u] = i < n ? __ldg(src + ((i / KW) * KC + i % KW) * TM) : elem{};
 				}
-			} else {
-				const char* a0 = A + (c < td.y ? (long)(c - td.x) * TB : tf + (long)(c - td.z) * TB);
-				if (CX) {
-					const int2* ap = reinterpret_cast<const int2*>(a0) + lane;
-#pragma unroll UN
-					for (int k = 0; k < KC; ++k) {
-						const int2 a = __ldg(ap + k * TM);
-						const int nb = -a.y;
+#pragma unroll
+				for (int u = 0; u < UN; ++u) {
+					const int i = KW % UN == 0 ? i0 + u : min(i0 + u, n - 1);
+					const int4* y0 = x + ((i / KW) * KC + i % KW) * XS;
+					if constexpr (CX && FULL) {
+						const int4 A4 = av[u];
+						const int nz = -A4.z, nw = -A4.w;
 #pragma unroll
 						for (int j = 0; j < NB; ++j) {
-							const int4 y = x[k * XS + j];
-							rm[j] = madw(a.x, y.x, rm[j]); rm[j] = madw(nb, y.z, rm[j]);
-							im[j] = madw(a.x, y.z, im[j]); im[j] = madw(a.y, y.x, im[j]);
+							const int4 y = y0[j];
+							rh[j] = madw(A4.x, y.x, rh[j]); ih[j] = madw(A4.x, y.z, ih[j]); rm[j] = madw(A4.x, y.y, rm[j]); im[j] = madw(A4.x, y.w, im[j]);
+							rh[j] = madw(nz, y.z, rh[j]); ih[j] = madw(A4.z, y.x, ih[j]); rm[j] = madw(nz, y.w, rm[j]); im[j] = madw(A4.z, y.y, im[j]);
+							rm[j] = madw(A4.y, y.x, rm[j]); im[j] = madw(A4.y, y.z, im[j]);
+							rm[j] = madw(nw, y.z, rm[j]); im[j] = madw(A4.w, y.x, im[j]);
 						}
-					}
-				} else {
-					const int* ap = reinterpret_cast<const int*>(a0) + lane;
-#pragma unroll UN
-					for (int k = 0; k < KC; ++k) {
-						const int a = __ldg(ap + k * TM);
+					} else if constexpr (CX) {
+						const int2 A2 = av[u];
+						const int nb = -A2.y;
 #pragma unroll
 						for (int j = 0; j < NB; ++j) {
-							const int4 y = x[k * XS + j];
-							rm[j] = madw(a, y.x, rm[j]); im[j] = madw(a, y.z, im[j]);
+							const int4 y = y0[j];
+							rm[j] = madw(A2.x, y.x, rm[j]); im[j] = madw(A2.x, y.z, im[j]);
+							rm[j] = madw(nb, y.z, rm[j]); im[j] = madw(A2.y, y.x, im[j]);
+						}
+					} else if constexpr (FULL) {
+						const int2 A2 = av[u];
+#pragma unroll
+						for (int j = 0; j < NB; ++j) {
+							const int4 y = y0[j];
+							rh[j] = madw(A2.x, y.x, rh[j]); ih[j] = madw(A2.x, y.z, ih[j]); rm[j] = madw(A2.x, y.y, rm[j]); im[j] = madw(A2.x, y.w, im[j]);
+							rm[j] = madw(A2.y, y.x, rm[j]); im[j] = madw(A2.y, y.z, im[j]);
+						}
+					} else {
+						const int A1 = av[u];
+#pragma unroll
+						for (int j = 0; j < NB; ++j) {
+							const int4 y = y0[j];
+							rm[j] = madw(A1, y.x, rm[j]); im[j] = madw(A1, y.z, im[j]);
 						}
 					}
 				}
 			}
-		}
+		};
+		auto spans = [&](int from, int to) {
+			if (from < td.y) span(from, min(to, td.y), A + (long)(from - td.x) * TB, std::false_type());
+			if (from < td.z && to > td.y) {
+				const int ca = max(from, td.y);
+				span(ca, min(to, td.z), A + tl + (long)(ca - td.y) * FB, std::true_type());
+			}
+			if (to > td.z) {
+				const int ca = max(from, td.z);
+				span(ca, to, A + tf + (long)(ca - td.z) * TB, std::false_type());
+			}
+		};
+		if constexpr (KS == 8) {
+			if (c0 + ks < td.w) spans(c0 + ks, c0 + ks + 1);
+			if (c0 + ks + 8 < td.w) spans(c0 + ks + 8, c0 + ks + 9);
+		} else spans(c0, ce);
 		// at most 32 k since the last flush: 128 mixed products below 2^55
 #pragma unroll
 		for (int j = 0; j < NB; ++j) { flush(rh[j], rm[j]); flush(ih[j], im[j]); }
@@ -178,8 +192,8 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 		const double2 y = make_double2(to_double(hr, mr, s, E == 0x7ff), to_double(hi, mi, s, E == 0x7ff));
 		const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 		if (row < p.N) p.dst[o * p.N + row] = y;
-		const int e = __reduce_max_sync(0xffffffffu, row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);
-		if (lane == 0) p.edst[o * p.ntile + tile] = e;
+		const int e = group_max(row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);
+		if (lane % TE == 0) p.edst[o * nex + tile * EPT + lane / TE] = e;
 	};
 	if constexpr (KS == 1) {
 #pragma unroll
@@ -205,7 +219,7 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 	}
 }
 
-// largest exponent of every TM-row tile of src [nvec][N]
+// largest exponent of every TE rows of src [nvec][N]
 __global__ void k_exponents(const double2* __restrict__ src, int* __restrict__ ex, int N, int ntile, long nvec)
 {
 	const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -215,8 +229,8 @@ __global__ void k_exponents(const double2* __restrict__ src, int* __restrict__ e
 	const int row = (int)(w % ntile) * TM + lane;
 	int e = 0;
 	if (row < N) { const double2 v = src[vec * N + row]; e = max(bexp(v.x), bexp(v.y)); }
-	e = __reduce_max_sync(0xffffffffu, e);
-	if (lane == 0) ex[w] = e;
+	e = group_max(e);
+	if (lane % TE == 0) ex[w * EPT + lane / TE] = e;
 }
 
 // ------------------------------------------------------------------ set-up: the eigenvectors of (R, S)
@@ -772,8 +786,8 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 	double2 *c0, *c1, *Fb;
 	int *ce, *cd;
 	const size_t band = (size_t)nlh * N * (2 * WMAX + 1);
-	if ((rc = tmp.get(&c0, chunk)) || (rc = tmp.get(&c1, chunk)) || (rc = tmp.get(&Fb, band)) || (rc = tmp.get(&ce, (size_t)J * nlh * p->ntile)) ||
-		(rc = tmp.get(&cd, (size_t)J * nlh * p->ntile)))
+	if ((rc = tmp.get(&c0, chunk)) || (rc = tmp.get(&c1, chunk)) || (rc = tmp.get(&Fb, band)) || (rc = tmp.get(&ce, (size_t)J * nlh * p->ntile * EPT)) ||
+		(rc = tmp.get(&cd, (size_t)J * nlh * p->ntile * EPT)))
 		return rc;
 	std::vector<unsigned long long> prof;
 	for (int fi = 0; fi < p->nff; ++fi) {

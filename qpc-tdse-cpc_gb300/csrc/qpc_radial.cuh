@@ -21,7 +21,7 @@ struct band_args {
 	int ea;			// |A| <= 2^ea
 	int N, ntile, nchan, ncols;
 	const double2 *s0, *s1;	// [slot][nchan][N]; s1 where par[slot] is odd
-	const int *e0, *e1;	// largest biased exponent per [slot][nchan][tile]
+	const int *e0, *e1;	// largest biased exponent of every TE rows, [slot][nchan][ntile * EPT]
 	const int64_t* par;
 	const int* smap;	// slot -> source slot (NULL: the same)
 	const int* dmap;	// slot -> destination slot (NULL: the same)
@@ -83,7 +83,7 @@ int orthonormalise(double* Qt, int N, double* E, double* T, cudaStream_t st, boo
 
 band_args band_args_of(const radial_ops* p, const band_store& b, int nchan, int ncols);
 void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st);
-// largest biased exponent of every TM-row tile of src [nvec][N]
+// largest biased exponent of every TE rows of src [nvec][N]
 void exponents(const double2* src, int* ex, int N, int ntile, long nvec, cudaStream_t st);
 
 // device scratch of a set-up, given back at its end

@@ -23,12 +23,12 @@ namespace qpc {
 
 namespace {
 
-constexpr int NBMAX = 448;	// most channels of a parity block (its 32-position tile sits in shared memory)
+constexpr int NBMAX = 452;	// most channels of a parity block (its 32-position tile sits in shared memory)
 
 struct set_args {
 	const double2* in;	// [slot][nch][N]
 	double2* out;
-	int* eout;		// [slot][nch][ntile]
+	int* eout;		// [slot][nch][ntile * EPT]
 	const int2* A[2][2];	// real matrices of the angular transform, [block][set], limbs
 	int off[2], na[2], ns[2];
 	int kind;		// 0: no coupling, 1: phase, 2: rotation of position pairs
@@ -49,7 +49,7 @@ struct set_args {
 __global__ void __launch_bounds__(256) k_couple(const set_args p)
 {
 	extern __shared__ double2 sm[];
-	__shared__ int pe[2][8][32];
+	__shared__ unsigned short pe[2][8][32];
 	constexpr int G = 4;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int tile = blockIdx.x, blk = blockIdx.y & 1, slot = blockIdx.y >> 1, slice = blockIdx.z;
@@ -96,12 +96,12 @@ __global__ void __launch_bounds__(256) k_couple(const set_args p)
 		const int e = max(bexp(v.x), bexp(v.y));
 		if (q < na) e0 = max(e0, e); else e1 = max(e1, e);
 	}
-	pe[0][warp][lane] = e0;
-	pe[1][warp][lane] = e1;
+	pe[0][warp][lane] = (unsigned short)e0;
+	pe[1][warp][lane] = (unsigned short)e1;
 	__syncthreads();
 	e0 = e1 = 0;
 #pragma unroll
-	for (int w = 0; w < 8; ++w) { e0 = max(e0, pe[0][w][lane]); e1 = max(e1, pe[1][w][lane]); }
+	for (int w = 0; w < 8; ++w) { e0 = max(e0, (int)pe[0][w][lane]); e1 = max(e1, (int)pe[1][w][lane]); }
 	for (int q = warp; q < n; q += 8) {
 		const double2 v = sm[q * 32 + lane];
 		const int e = q < na ? e0 : e1;
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256) k_couple(const set_args p)
 				const double2 v = make_double2(to_double(h[g][0], m[g][0], e - 1078, e == 0x7ff), to_double(h[g][1], m[g][1], e - 1078, e == 0x7ff));
 				const int ch = (set ? na : 0) + o0 + g;
 				if (in) p.out[base + (long)ch * N] = v;
-				const int x = __reduce_max_sync(0xffffffffu, in ? max(bexp(v.x), bexp(v.y)) : 0);
-				if (lane == 0) p.eout[((long)slot * p.nch + p.off[blk] + ch) * p.ntile + tile] = x;
+				const int x = group_max(in ? max(bexp(v.x), bexp(v.y)) : 0);
+				if (lane % TE == 0) p.eout[(((long)slot * p.nch + p.off[blk] + ch) * p.ntile + tile) * EPT + lane / TE] = x;
 			}
 	}
 }
@@ -282,8 +282,8 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	QPC_CUDA(cudaMemcpy(p->lmap, lm.data(), sizeof(int) * nch, cudaMemcpyHostToDevice));
 	const long nvec = (long)p->B * nch;
 	for (int i = 0; i < 2; ++i)
-		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile))) return rc;
-	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile))) return rc;
+		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
+	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
 	p->smem = sizeof(double2) * 32 * std::max(in.nb[0], in.nb[1]);
 	QPC_CUDA(cudaFuncSetAttribute(k_couple, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double2) * 32 * NBMAX)));
 	QPC_CUDA(cudaGetLastError());
@@ -379,8 +379,8 @@ void fieldfree(vpos_path* p, const vpos_run& r, int src, long s, int k0, int n)
 	band_args a = band_args_of(&p->ops, p->ops.F, p->nch, n);
 	a.lmap = p->lmap;
 	const long o = (long)k0 * p->nch;
-	a.s0 = p->buf[src] + o * p->N; a.e0 = p->ex[src] + o * p->ntile;
-	a.dst = p->buf[1 - src] + o * p->N; a.edst = p->ex[1 - src] + o * p->ntile;
+	a.s0 = p->buf[src] + o * p->N; a.e0 = p->ex[src] + o * p->ntile * EPT;
+	a.dst = p->buf[1 - src] + o * p->N; a.edst = p->ex[1 - src] + o * p->ntile * EPT;
 	a.nta = r.ntt + k0; a.step = s;
 	band_apply(a, true, p->ntile, p->stream);
 	++*r.launches;
