@@ -34,8 +34,7 @@ namespace qpc {
 namespace {
 
 constexpr int AR_THREADS = 256;
-constexpr int AR_PER_THREAD = 4;
-constexpr int AR_TILE = AR_THREADS * AR_PER_THREAD; // elements per block of the element-wise kernels
+// elements per thread of the element-wise kernels: 4, or 1 for batches whose blocks would leave SMs idle
 constexpr int AR_KMAX = 32;                          // largest Krylov dimension accepted
 constexpr int CH_THREADS = 32;                       // real recurrences per block of k_ar_sinv
 
@@ -51,6 +50,7 @@ struct ar_args {
 	long hstride; // doubles between the Hamiltonians of consecutive instances (0: shared)
 	double dt, emin, emax;
 	const double *S, *R, *Lrow, *Lcol, *dinv, *H, *y10;
+	const double *SM, *SN, *SI;	// block substitution (k_ar_sinv_blk): M_t, N_t, L11^-1 per block [P][P]
 	double2 *X, *U, *V0, *V1;
 	double2* partX;
 	double* partN;
@@ -115,18 +115,6 @@ __device__ bool arrive_last(unsigned* cnt, int nb)
 	return last;
 }
 
-// fixed-order sum of nb partials by warp 0 (lanes stride, then the shuffle tree); valid in lane 0
-__device__ double2 sum_partials(const double2* p, long stride, int nb)
-{
-	double2 s = make_double2(0.0, 0.0);
-	for (int j = threadIdx.x; j < nb; j += 32) s = cadd(s, __ldcg(p + (long)j * stride));
-	for (int o = 16; o; o >>= 1) {
-		s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-		s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-	}
-	return s;
-}
-
 // ---------------------------------------------------------------- layout
 __global__ void k_ar_to_rmajor(const double2* __restrict__ src, double2* __restrict__ dst, int N, int nch, long total)
 {
@@ -151,6 +139,7 @@ __global__ void k_ar_to_lmajor(const double2* __restrict__ src, double2* __restr
 //        or the instance idles this step (step >= nt).
 // k >= 0: end of iteration k (orthogonalize_ip, la_1e.hpp:221-238): nu < 1e-13 ends the
 //        expansion with m = k+1; else sfac = 1/sqrt(nu), b[k+1] = sqrt(nu).
+template <int PT>
 __global__ void __launch_bounds__(AR_THREADS) k_ar_snorm(ar_args g, const double2* __restrict__ src, int k, long step)
 {
 	const int b = g.b0 + blockIdx.y;
@@ -164,8 +153,8 @@ __global__ void __launch_bounds__(AR_THREADS) k_ar_snorm(ar_args g, const double
 	const int P = g.P, nch = g.nch, N = g.N;
 	const double2* x = src + (long)b * g.n;
 	double acc = 0.0;
-	for (int j = 0; j < AR_PER_THREAD; ++j) {
-		long e = (long)blockIdx.x * AR_TILE + j * AR_THREADS + threadIdx.x;
+	for (int j = 0; j < PT; ++j) {
+		long e = (long)blockIdx.x * (AR_THREADS * PT) + j * AR_THREADS + threadIdx.x;
 		if (e >= g.n) break;
 		int r = (int)(e / nch);
 		double2 t = make_double2(0.0, 0.0);
@@ -223,12 +212,12 @@ __global__ void __launch_bounds__(AR_THREADS) k_ar_snorm(ar_args g, const double
 // x_i = <u_i|dst> for i <= k (orthogonalize_ip, la_1e.hpp:204-209), a[k] = Re x_k.
 // The band sums run on the unscaled src and are scaled once, H (s x) = s (H x): the
 // same value to rounding, for a third of the FP64 instructions.
+template <int PT>
 __global__ void __launch_bounds__(AR_THREADS) k_ar_expand(ar_args g, const double2* __restrict__ src, double2* __restrict__ dst,
 	int k, long step)
 {
 	const int b = g.b0 + blockIdx.y;
 	if (g.flag[b] != AR_LIVE) return;
-	__shared__ double2 sm[32];
 	const int P = g.P, nch = g.nch, N = g.N, L = g.L;
 	const long n = g.n;
 	const double s = g.sfac[b];
@@ -238,11 +227,11 @@ __global__ void __launch_bounds__(AR_THREADS) k_ar_expand(ar_args g, const doubl
 	double2* Uk = g.U + ((long)b * g.kmax + k) * n;
 	const double* __restrict__ H = g.H + (long)b * g.hstride;
 	const double* __restrict__ Rb = g.R;
-	double2 yv[AR_PER_THREAD], uv[AR_PER_THREAD];
+	double2 yv[PT], uv[PT];
 #pragma unroll
-	for (int j = 0; j < AR_PER_THREAD; ++j) {
+	for (int j = 0; j < PT; ++j) {
 		yv[j] = uv[j] = make_double2(0.0, 0.0);
-		long e = (long)blockIdx.x * AR_TILE + j * AR_THREADS + threadIdx.x;
+		long e = (long)blockIdx.x * (AR_THREADS * PT) + j * AR_THREADS + threadIdx.x;
 		if (e >= n) continue;
 		int r = (int)(e / nch), ch = (int)(e - (long)r * nch);
 		int im = ch / L, il = ch - im * L;
@@ -285,29 +274,48 @@ __global__ void __launch_bounds__(AR_THREADS) k_ar_expand(ar_args g, const doubl
 		y[e] = acc;
 		yv[j] = acc;
 	}
-	// projections x_i = <u_i|v>, i <= k, one fixed-order block sum each
+	// projections x_i = <u_i|v>, i <= k: eight at a time, every thread's part to shared memory, one warp per sum (a
+	// block-wide sum each had two barriers and a shuffle tree of its own: 4.5 us per projection)
+	constexpr int ND = 8;
+	__shared__ double2 sp[ND][AR_THREADS + 1];
 	double2* part = g.partX + ((long)b * g.nbe + blockIdx.x) * g.kmax;
-	for (int i = 0; i <= k; ++i) {
-		const double2* Ui = g.U + ((long)b * g.kmax + i) * n;
-		double2 acc = make_double2(0.0, 0.0);
-		for (int j = 0; j < AR_PER_THREAD; ++j) {
-			long e = (long)blockIdx.x * AR_TILE + j * AR_THREADS + threadIdx.x;
-			if (e >= n) break;
-			double2 ui = (i == k) ? uv[j] : Ui[e];
-			acc = cadd(acc, cdot(ui, yv[j]));
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	for (int i0 = 0; i0 <= k; i0 += ND) {
+		const int ni = min(ND, k + 1 - i0);
+		for (int i = 0; i < ni; ++i) {
+			const double2* Ui = g.U + ((long)b * g.kmax + i0 + i) * n;
+			double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+			for (int j = 0; j < PT; ++j) {
+				const long e = (long)blockIdx.x * (AR_THREADS * PT) + j * AR_THREADS + threadIdx.x;
+				if (e >= n) break;
+				acc = cadd(acc, cdot(i0 + i == k ? uv[j] : Ui[e], yv[j]));
+			}
+			sp[i][threadIdx.x] = acc;
 		}
-		double2 tot = block_sum(acc, sm);
-		if (threadIdx.x == 0) part[i] = tot;
+		__syncthreads();
+		if (warp < ni) {
+			double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+			for (int j = 0; j < AR_THREADS / 32; ++j) t = cadd(t, sp[warp][j * 32 + lane]);
+			for (int o = 16; o; o >>= 1) { t.x += __shfl_xor_sync(0xffffffffu, t.x, o); t.y += __shfl_xor_sync(0xffffffffu, t.y, o); }
+			if (lane == 0) part[i0 + warp] = t;
+		}
+		__syncthreads();
 	}
+	// the barrier above orders the warps' partials before thread 0's fence
 	if (!arrive_last(g.cnt + b, g.nbe)) return;
-	if (threadIdx.x < 32) {
-		for (int i = 0; i <= k; ++i) {
-			double2 xi = sum_partials(g.partX + (long)b * g.nbe * g.kmax + i, g.kmax, g.nbe);
-			if (threadIdx.x == 0) g.xfin[(long)b * g.kmax + i] = xi;
-			if (threadIdx.x == 0 && i == k) g.a[(long)b * g.kmax + k] = xi.x;
+	for (int i = warp; i <= k; i += AR_THREADS / 32) {
+		double2 t = make_double2(0.0, 0.0);
+		const double2* q = g.partX + (long)b * g.nbe * g.kmax + i;
+		for (int j = lane; j < g.nbe; j += 32) t = cadd(t, __ldcg(q + (long)j * g.kmax));
+		for (int o = 16; o; o >>= 1) { t.x += __shfl_xor_sync(0xffffffffu, t.x, o); t.y += __shfl_xor_sync(0xffffffffu, t.y, o); }
+		if (lane == 0) {
+			g.xfin[(long)b * g.kmax + i] = t;
+			if (i == k) g.a[(long)b * g.kmax + k] = t.x;
 		}
-		if (threadIdx.x == 0) g.cnt[b] = 0u;
 	}
+	if (threadIdx.x == 0) g.cnt[b] = 0u;
 }
 
 // ---------------------------------------------------------------- S^-1
@@ -386,94 +394,104 @@ __global__ void __launch_bounds__(CH_THREADS) k_ar_sinv(ar_args g, double2* __re
 	sinv_sweep<P, false>(g, v, stride, act, Lt);
 }
 
-// The same solve with P lanes per real recurrence, column-oriented (for batches too small
-// to occupy the GPU one lane per recurrence): lane j of a recurrence holds the pending sum
-// of one of the next P rows; when row r is complete its owner's sum is broadcast, every lane
-// computes x_r, and each lane adds L(row_j, r) x_r to its own row's sum.  Three FP64
-// instructions per row instead of P + 1, on P times as many warps.
+// The same solve for batches too small to occupy the GPU one lane per recurrence: block substitution in blocks of
+// P rows, P lanes per recurrence.  With L21(t) the factor's block left of the diagonal block L11(t),
+//   a(t) = v(t) - M_t a(t-1),  M_t = L21(t) L11(t-1)^-1      y(t) = L11(t)^-1 a(t)
+//   b(t) = y(t) - N_t b(t+1),  N_t = (L11(t+1)^-1 L21(t+1))^T    x(t) = L11(t)^-T b(t):
+// only a and b are sequences, P rows per link of a few dependent FMAs (one warp), the rest is done by the whole block.
+// The vector stays in shared memory in between.  Bound by the FP64 issue of the sequences (P FMAs of 64 cycles per P
+// rows); measured at groups of 4 wavefunctions of 400 x 21: 68 us, against ~270 for one dependent chain of three
+// FP64 instructions and two shuffles per row (122 with the factor rows scaled to one FMA and one shuffle).
+constexpr int SB_THREADS = 128;
+constexpr size_t SB_SMEM = 200 * 1024;	// longest vectors it takes: 5 recurrences of 5 000 rows at p = 6
 template <int P>
-__global__ void __launch_bounds__(128) k_ar_sinv_sys(ar_args g, double2* __restrict__ vbuf)
+__global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* __restrict__ vbuf)
 {
 	const int b = g.b0 + blockIdx.y;
 	if (g.flag[b] != AR_LIVE) return;
-	constexpr int CPW = 32 / P;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int cs = lane / P, j = lane - cs * P;
-	const int c = (blockIdx.x * (int)(blockDim.x >> 5) + warp) * CPW + cs;
-	const bool act = cs < CPW && c < 2 * g.nch;
-	const int base = (cs < CPW ? cs : 0) * P;
+	constexpr int CPW = 32 / P, PP = P * P;
+	extern __shared__ double xs[];	// [CPW][nt P]
+	const int N = g.N, nt = (N + P - 1) / P, np = nt * P;
 	const long stride = 2L * g.nch;
-	const int N = g.N;
-	double* v = reinterpret_cast<double*>(vbuf + (long)b * g.n) + (act ? c : 0);
-	const double* __restrict__ Lcol = g.Lcol;
-	const double* __restrict__ Lrow = g.Lrow;
-	const double* __restrict__ dinv = g.dinv;
-	// forward: rows r ascending, owner o = r mod P
-	{
-		double acc = 0.0, cur[SV_D], nxt[SV_D];
-		const int ntile = (N + SV_D - 1) / SV_D;
-#pragma unroll
-		for (int q = 0; q < SV_D; ++q) cur[q] = (act && q < N) ? v[(long)q * stride] : 0.0;
-		int o = 0;
-		for (int t = 0; t < ntile; ++t) {
-#pragma unroll
-			for (int q = 0; q < SV_D; ++q) {
-				int r = (t + 1) * SV_D + q;
-				nxt[q] = (act && r < N) ? v[(long)r * stride] : 0.0;
-			}
-#pragma unroll
-			for (int q = 0; q < SV_D; ++q) {
-				const int r = t * SV_D + q;
-				if (r < N) {
-					double ao = __shfl_sync(0xffffffffu, acc, base + o);
-					double x = (cur[q] - ao) * dinv[r];
-					if (j == o) acc = 0.0;
-					int k = (j - o - 1 + P) % P + 1;
-					acc = fma(Lcol[(long)r * P + k - 1], x, acc);
-					if (act && j == o) v[(long)r * stride] = x;
-					o = (o + 1 == P) ? 0 : o + 1;
-				}
-			}
-#pragma unroll
-			for (int q = 0; q < SV_D; ++q) cur[q] = nxt[q];
-		}
+	const int c0 = blockIdx.x * CPW, nc = min(CPW, 2 * g.nch - c0);
+	double* v = reinterpret_cast<double*>(vbuf + (long)b * g.n) + c0;
+	for (int i = threadIdx.x; i < np * CPW; i += SB_THREADS) {
+		const int r = i / CPW, c = i - r * CPW;
+		xs[c * np + r] = (r < N && c < nc) ? v[(long)r * stride + c] : 0.0;
 	}
-	__syncwarp();
-	// backward: rows s = N-1-i descending, owner o = i mod P
-	{
-		double acc = 0.0, cur[SV_D], nxt[SV_D];
-		const int ntile = (N + SV_D - 1) / SV_D;
+	__syncthreads();
+	const int lane = threadIdx.x, cs = lane / P, j = lane - cs * P;
+	auto sequence = [&](const double* __restrict__ C, bool fwd) {
+		if (threadIdx.x >= 32) return;
+		const bool act = cs < CPW;
+		double* x = xs + (act ? cs : 0) * np;
+		const int base = (act ? cs : 0) * P;
+		auto blk = [&](int i) { return fwd ? i : nt - 1 - i; };
+		// coefficients of the next D - 1 blocks on their way (a read from L2 takes two links)
+		constexpr int D = 4;
+		double cf[D][P], vl[D];
+		auto fetch = [&](int i, double* c, double& w) {
 #pragma unroll
-		for (int q = 0; q < SV_D; ++q) cur[q] = (act && q < N) ? v[(long)(N - 1 - q) * stride] : 0.0;
-		int o = 0;
-		for (int t = 0; t < ntile; ++t) {
+			for (int k = 0; k < P; ++k) c[k] = i < nt ? __ldg(C + (long)blk(i) * PP + j * P + k) : 0.0;
+			w = (act && i < nt) ? x[blk(i) * P + j] : 0.0;
+		};
+		double a = act ? x[blk(0) * P + j] : 0.0;
 #pragma unroll
-			for (int q = 0; q < SV_D; ++q) {
-				int i = (t + 1) * SV_D + q;
-				nxt[q] = (act && i < N) ? v[(long)(N - 1 - i) * stride] : 0.0;
-			}
+		for (int d = 0; d < D - 1; ++d) fetch(1 + d, cf[d], vl[d]);
+		for (int i0 = 1; i0 < nt; i0 += D) {
 #pragma unroll
-			for (int q = 0; q < SV_D; ++q) {
-				const int i = t * SV_D + q;
-				if (i < N) {
-					const int sr = N - 1 - i;
-					double ao = __shfl_sync(0xffffffffu, acc, base + o);
-					double x = (cur[q] - ao) * dinv[sr];
-					if (j == o) acc = 0.0;
-					int k = (j - o - 1 + P) % P + 1;
-					acc = fma(Lrow[(long)sr * P + k - 1], x, acc);
-					if (act && j == o) v[(long)sr * stride] = x;
-					o = (o + 1 == P) ? 0 : o + 1;
+			for (int d = 0; d < D; ++d) {
+				const int i = i0 + d;
+				if (i >= nt) break;
+				fetch(i + D - 1, cf[(d + D - 1) % D], vl[(d + D - 1) % D]);
+				double p = vl[d], q = 0.0;
+#pragma unroll
+				for (int k = 0; k < P; ++k) {
+					const double ak = __shfl_sync(0xffffffffu, a, base + k);
+					if (k & 1) q = fma(-cf[d][k], ak, q); else p = fma(-cf[d][k], ak, p);
 				}
+				a = p + q;
+				if (act) x[blk(i) * P + j] = a;
+			}
+		}
+	};
+	auto blocks = [&](bool trans) {	// every block times L11^-1 or its transpose
+		for (int i = threadIdx.x; i < nt * CPW; i += SB_THREADS) {
+			const int t = i / CPW, c = i - t * CPW;
+			double* x = xs + c * np + t * P;
+			const double* Li = g.SI + (long)t * PP;
+			double in[P], out[P];
+#pragma unroll
+			for (int k = 0; k < P; ++k) in[k] = x[k];
+#pragma unroll
+			for (int r = 0; r < P; ++r) {
+				double s = 0.0;
+#pragma unroll
+				for (int k = 0; k < P; ++k)
+					if (trans ? k >= r : k <= r) s = fma(__ldg(Li + (trans ? k * P + r : r * P + k)), in[k], s);
+				out[r] = s;
 			}
 #pragma unroll
-			for (int q = 0; q < SV_D; ++q) cur[q] = nxt[q];
+			for (int k = 0; k < P; ++k) x[k] = out[k];
 		}
+	};
+	sequence(g.SM, true);
+	__syncthreads();
+	blocks(false);
+	__syncthreads();
+	sequence(g.SN, false);
+	__syncthreads();
+	blocks(true);
+	__syncthreads();
+	for (int i = threadIdx.x; i < N * CPW; i += SB_THREADS) {
+		const int r = i / CPW, c = i - r * CPW;
+		if (c < nc) v[(long)r * stride + c] = xs[c * np + r];
 	}
 }
 
 // ---------------------------------------------------------------- Gram-Schmidt
 // v -= u_i x_i for i <= k with i == k or |x_i|^2 > 4e-27, i ascending (la_1e.hpp:212-219)
+template <int PT>
 __global__ void __launch_bounds__(AR_THREADS) k_ar_orth(ar_args g, double2* __restrict__ vbuf, int k)
 {
 	const int b = g.b0 + blockIdx.y;
@@ -488,8 +506,8 @@ __global__ void __launch_bounds__(AR_THREADS) k_ar_orth(ar_args g, double2* __re
 	__syncthreads();
 	const long n = g.n;
 	double2* v = vbuf + (long)b * n;
-	for (int j = 0; j < AR_PER_THREAD; ++j) {
-		long e = (long)blockIdx.x * AR_TILE + j * AR_THREADS + threadIdx.x;
+	for (int j = 0; j < PT; ++j) {
+		long e = (long)blockIdx.x * (AR_THREADS * PT) + j * AR_THREADS + threadIdx.x;
 		if (e >= n) break;
 		double2 t = v[e];
 		for (int i = 0; i <= k; ++i)
@@ -517,6 +535,11 @@ __global__ void __launch_bounds__(32) k_ar_small(ar_args g, long step)
 		e[i] = i + 1 < m ? g.b[(long)b * (g.kmax + 1) + i + 1] : 0.0;
 		z[i] = (i == lane) ? 1.0 : 0.0;
 	}
+	// scaled by the largest entry, so that sums of squares neither overflow nor lose what matters
+	double big = 0.0;
+	for (int i = 0; i < m; ++i) big = fmax(big, fmax(fabs(d[i]), fabs(e[i])));
+	const double up = big > 0.0 ? big : 1.0, down = 1.0 / up;
+	for (int i = 0; i < m; ++i) { d[i] *= down; e[i] *= down; }
 	bool ok = true;
 	for (int l = 0; l < m && ok; ++l) {
 		int iter = 0, mm;
@@ -528,14 +551,17 @@ __global__ void __launch_bounds__(32) k_ar_small(ar_args g, long step)
 			if (mm == l) break;
 			if (iter++ == 60) { ok = false; break; }
 			double gg = (d[l + 1] - d[l]) / (2.0 * e[l]);
-			double r = hypot(gg, 1.0);
+			double r = sqrt(fma(gg, gg, 1.0));
 			gg = d[mm] - d[l] + e[l] / (gg + (gg >= 0 ? r : -r));
 			double s = 1.0, c = 1.0, pp = 0.0;
 			int i;
 			bool underflow = false;
 			for (i = mm - 1; i >= l; --i) {
 				double f = s * e[i], bb = c * e[i];
-				r = hypot(f, gg);
+				// one reciprocal root in place of a hypot and two divisions (m = 12: 325 -> 210 us)
+				const double rr = fma(f, f, gg * gg), ri = rsqrt(rr);
+				r = rr * ri;
+				if (!(rr > 0.0)) r = 0.0;
 				e[i + 1] = r;
 				if (r == 0.0) {
 					d[i + 1] -= pp;
@@ -543,8 +569,8 @@ __global__ void __launch_bounds__(32) k_ar_small(ar_args g, long step)
 					underflow = true;
 					break;
 				}
-				s = f / r;
-				c = gg / r;
+				s = f * ri;
+				c = gg * ri;
 				gg = d[i + 1] - pp;
 				r = (d[i] - gg) * s + 2.0 * c * bb;
 				pp = s * r;
@@ -570,7 +596,7 @@ __global__ void __launch_bounds__(32) k_ar_small(ar_args g, long step)
 	for (int i = 0; i < m; ++i) {
 		double z0 = __shfl_sync(0xffffffffu, z[i], 0);
 		double sn, cs;
-		sincos(-(g.dt * d[i]), &sn, &cs);
+		sincos(-(g.dt * (d[i] * up)), &sn, &cs);
 		double2 wi = make_double2(z0 * cs, z0 * sn);
 		xj = i == 0 ? rmul(wi, z[i]) : cadd(xj, rmul(wi, z[i]));
 	}
@@ -585,6 +611,7 @@ __global__ void __launch_bounds__(32) k_ar_small(ar_args g, long step)
 }
 
 // w = sum_{i<m} u_i x_i (eliminate_sub, la_1e.hpp:176-193)
+template <int PT>
 __global__ void __launch_bounds__(AR_THREADS) k_ar_combine(ar_args g)
 {
 	const int b = g.b0 + blockIdx.y;
@@ -596,8 +623,8 @@ __global__ void __launch_bounds__(AR_THREADS) k_ar_combine(ar_args g)
 	__syncthreads();
 	const long n = g.n;
 	bool bad = false;
-	for (int j = 0; j < AR_PER_THREAD; ++j) {
-		long e = (long)blockIdx.x * AR_TILE + j * AR_THREADS + threadIdx.x;
+	for (int j = 0; j < PT; ++j) {
+		long e = (long)blockIdx.x * (AR_THREADS * PT) + j * AR_THREADS + threadIdx.x;
 		if (e >= n) break;
 		const double2* U = g.U + (long)b * g.kmax * n + e;
 		double2 w = cmul(U[0], xs[0]);
@@ -617,12 +644,12 @@ using namespace qpc;
 struct qpc_arnoldi {
 	int dev = 0;
 	qpc_dims d{};
-	int P = 0, nch = 0, nlh = 0, kmax = 0, nbe = 0, hper = 0;
+	int P = 0, nch = 0, nlh = 0, kmax = 0, nbe = 0, hper = 0, pt = 4;
 	long n = 0;
 	double dt = 0, emin = 0, emax = 0;
 	cudaStream_t stream = nullptr, stream2 = nullptr;	// stream2: second instance group (n_inst >= 2)
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-	double *S = nullptr, *R = nullptr, *Lrow = nullptr, *Lcol = nullptr, *dinv = nullptr, *H = nullptr, *y10 = nullptr;
+	double *S = nullptr, *R = nullptr, *Lrow = nullptr, *Lcol = nullptr, *SM = nullptr, *SN = nullptr, *SI = nullptr, *dinv = nullptr, *H = nullptr, *y10 = nullptr;
 	double2 *X = nullptr, *U = nullptr, *V0 = nullptr, *V1 = nullptr, *tmp = nullptr;
 	double2* partX = nullptr;
 	double* partN = nullptr;
@@ -645,7 +672,7 @@ void ar_free(qpc_arnoldi* h)
 {
 	if (!h) return;
 	cudaSetDevice(h->dev);
-	void* ptrs[] = {h->S, h->R, h->Lrow, h->Lcol, h->dinv, h->H, h->y10, h->X, h->U, h->V0, h->V1, h->tmp, h->partX, h->partN,
+	void* ptrs[] = {h->S, h->R, h->Lrow, h->Lcol, h->SM, h->SN, h->SI, h->dinv, h->H, h->y10, h->X, h->U, h->V0, h->V1, h->tmp, h->partX, h->partN,
 		h->cnt, h->xfin, h->xc, h->a, h->b, h->sfac, h->nu0, h->msub, h->flag, h->status, h->ez, h->nt, h->crit, h->msub_out};
 	for (void* p : ptrs)
 		if (p) cudaFree(p);
@@ -664,7 +691,7 @@ ar_args make_args(qpc_arnoldi* h)
 	g.B = h->d.n_inst; g.kmax = h->kmax; g.nbe = h->nbe; g.n = h->n; g.b0 = 0;
 	g.hstride = h->hper ? (long)h->d.n_r * (h->P + 1) * h->nlh : 0;
 	g.dt = h->dt; g.emin = h->emin; g.emax = h->emax;
-	g.S = h->S; g.R = h->R; g.Lrow = h->Lrow; g.Lcol = h->Lcol; g.dinv = h->dinv; g.H = h->H; g.y10 = h->y10;
+	g.S = h->S; g.R = h->R; g.Lrow = h->Lrow; g.Lcol = h->Lcol; g.SM = h->SM; g.SN = h->SN; g.SI = h->SI; g.dinv = h->dinv; g.H = h->H; g.y10 = h->y10;
 	g.X = h->X; g.U = h->U; g.V0 = h->V0; g.V1 = h->V1;
 	g.partX = h->partX; g.partN = h->partN; g.cnt = h->cnt; g.xfin = h->xfin;
 	g.a = h->a; g.b = h->b; g.sfac = h->sfac; g.nu0 = h->nu0; g.msub = h->msub; g.flag = h->flag; g.xc = h->xc;
@@ -674,21 +701,24 @@ ar_args make_args(qpc_arnoldi* h)
 
 void launch_sinv(const ar_args& g, int Bg, double2* v, cudaStream_t st)
 {
-	// one lane per recurrence when that fills the GPU, else P lanes per recurrence
+	// one lane per recurrence when that fills the GPU, else block substitution
 	const long chains = 2L * g.nch * Bg;
 	const char* e = getenv("QPC_AR_SINV");
-	const bool sys = e ? atoi(e) == 2 : chains < 32L * 304;
-	if (sys && g.P >= 2) {
+	const bool blk = e ? atoi(e) == 2 : chains < 32L * 304;
+	if (blk && g.P >= 2) {
 		const int cpw = 32 / g.P;
-		dim3 gs((unsigned)((2 * g.nch + 4 * cpw - 1) / (4 * cpw)), Bg);
-		switch (g.P) {
-		case 2: k_ar_sinv_sys<2><<<gs, 128, 0, st>>>(g, v); return;
-		case 3: k_ar_sinv_sys<3><<<gs, 128, 0, st>>>(g, v); return;
-		case 4: k_ar_sinv_sys<4><<<gs, 128, 0, st>>>(g, v); return;
-		case 5: k_ar_sinv_sys<5><<<gs, 128, 0, st>>>(g, v); return;
-		case 6: k_ar_sinv_sys<6><<<gs, 128, 0, st>>>(g, v); return;
-		case 7: k_ar_sinv_sys<7><<<gs, 128, 0, st>>>(g, v); return;
-		default: k_ar_sinv_sys<8><<<gs, 128, 0, st>>>(g, v); return;
+		const size_t smem = sizeof(double) * cpw * ((g.N + g.P - 1) / g.P) * g.P;
+		if (smem <= SB_SMEM) {
+			const dim3 gs((unsigned)((2 * g.nch + cpw - 1) / cpw), Bg);
+			switch (g.P) {
+			case 2: k_ar_sinv_blk<2><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			case 3: k_ar_sinv_blk<3><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			case 4: k_ar_sinv_blk<4><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			case 5: k_ar_sinv_blk<5><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			case 6: k_ar_sinv_blk<6><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			case 7: k_ar_sinv_blk<7><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			default: k_ar_sinv_blk<8><<<gs, SB_THREADS, smem, st>>>(g, v); return;
+			}
 		}
 	}
 	dim3 grid((2 * g.nch + CH_THREADS - 1) / CH_THREADS, Bg);
@@ -705,24 +735,30 @@ void launch_sinv(const ar_args& g, int Bg, double2* v, cudaStream_t st)
 }
 
 // one Arnoldi step of instances [g.b0, g.b0 + Bg) on stream st: 4 kmax launches
-long launch_step(qpc_arnoldi* h, const ar_args& g, int Bg, cudaStream_t st, long step)
+template <int PT>
+long launch_step_t(qpc_arnoldi* h, const ar_args& g, int Bg, cudaStream_t st, long step)
 {
 	dim3 ge(g.nbe, Bg);
 	long nl = 0;
-	k_ar_snorm<<<ge, AR_THREADS, 0, st>>>(g, h->X, -1, step); ++nl;
+	k_ar_snorm<PT><<<ge, AR_THREADS, 0, st>>>(g, h->X, -1, step); ++nl;
 	double2* src = h->X;
 	for (int k = 0; k < g.kmax; ++k) {
 		double2* dst = (k & 1) ? h->V1 : h->V0;
-		k_ar_expand<<<ge, AR_THREADS, 0, st>>>(g, src, dst, k, step); ++nl;
+		k_ar_expand<PT><<<ge, AR_THREADS, 0, st>>>(g, src, dst, k, step); ++nl;
 		if (k == g.kmax - 1) break; // u_kmax is never used (eliminate_sub sums i < m)
 		launch_sinv(g, Bg, dst, st); ++nl;
-		k_ar_orth<<<ge, AR_THREADS, 0, st>>>(g, dst, k); ++nl;
-		k_ar_snorm<<<ge, AR_THREADS, 0, st>>>(g, dst, k, step); ++nl;
+		k_ar_orth<PT><<<ge, AR_THREADS, 0, st>>>(g, dst, k); ++nl;
+		k_ar_snorm<PT><<<ge, AR_THREADS, 0, st>>>(g, dst, k, step); ++nl;
 		src = dst;
 	}
 	k_ar_small<<<Bg, 32, 0, st>>>(g, step); ++nl;
-	k_ar_combine<<<ge, AR_THREADS, 0, st>>>(g); ++nl;
+	k_ar_combine<PT><<<ge, AR_THREADS, 0, st>>>(g); ++nl;
 	return nl;
+}
+
+long launch_step(qpc_arnoldi* h, const ar_args& g, int Bg, cudaStream_t st, long step)
+{
+	return h->pt == 1 ? launch_step_t<1>(h, g, Bg, st, step) : launch_step_t<4>(h, g, Bg, st, step);
 }
 
 int read_status(qpc_arnoldi* h)
@@ -769,7 +805,8 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 	h->nlh = mmax + d.n_l;
 	h->kmax = kmax;
 	h->n = (long)h->nch * d.n_r;
-	h->nbe = (int)((h->n + AR_TILE - 1) / AR_TILE);
+	h->pt = h->n * d.n_inst < 4L * AR_THREADS * 608 ? 1 : 4;
+	h->nbe = (int)((h->n + AR_THREADS * h->pt - 1) / (AR_THREADS * h->pt));
 	h->hper = h_per_instance ? 1 : 0;
 	h->dt = dt; h->emin = emin; h->emax = emax;
 	const int N = d.n_r, P = d.p, NE = P + 1, B = d.n_inst;
@@ -785,6 +822,34 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 			if (r + j < N) lcol[(size_t)r * P + j - 1] = Lc[(size_t)r * NE + j];
 		}
 	}
+	// the tables of the block substitution, blocks of P rows (rows past the last: the identity)
+	const int nt = (N + P - 1) / P;
+	auto Lat = [&](int r, int c) -> double {	// L(r, c)
+		if (r >= N || c >= N) return r == c ? 1.0 : 0.0;
+		return (c > r || r - c > P) ? 0.0 : Lc[(size_t)c * NE + (r - c)];
+	};
+	std::vector<double> sM((size_t)nt * P * P, 0.0), sN((size_t)nt * P * P, 0.0), sI((size_t)nt * P * P, 0.0);
+	for (int t = 0; t < nt; ++t) {
+		double* I = sI.data() + (size_t)t * P * P;
+		for (int c = 0; c < P; ++c)
+			for (int r = c; r < P; ++r) {
+				double x = r == c ? 1.0 : 0.0;
+				for (int k = c; k < r; ++k) x -= Lat(t * P + r, t * P + k) * I[k * P + c];
+				I[r * P + c] = x / Lat(t * P + r, t * P + r);
+			}
+	}
+	for (int t = 1; t < nt; ++t)
+		for (int r = 0; r < P; ++r)
+			for (int c = 0; c < P; ++c) {
+				const double *Ip = sI.data() + (size_t)(t - 1) * P * P, *It = sI.data() + (size_t)t * P * P;
+				double x = 0.0, y = 0.0;
+				for (int k = 0; k < P; ++k) {
+					x += Lat(t * P + r, (t - 1) * P + k) * Ip[k * P + c];
+					y += It[r * P + k] * Lat(t * P + k, (t - 1) * P + c);
+				}
+				sM[((size_t)t * P + r) * P + c] = x;
+				sN[((size_t)(t - 1) * P + c) * P + r] = y;
+			}
 	// Hamiltonian bands r-major: Hr[hs][r][k][l]
 	const int nhs = h->hper ? B : 1;
 	std::vector<double> Hr((size_t)nhs * N * NE * h->nlh);
@@ -805,7 +870,7 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 		if ((cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking)) != cudaSuccess) { set_error("cudaStreamCreateWithFlags failed"); return fail(QPC_ERR_CUDA); }
 	const long nst = (long)B * h->n;
 	if ((rc = dalloc(&h->S, (size_t)N * NE)) || (rc = dalloc(&h->R, (size_t)N * NE)) || (rc = dalloc(&h->Lrow, (size_t)N * P)) ||
-		(rc = dalloc(&h->Lcol, (size_t)N * P)) || (rc = dalloc(&h->dinv, (size_t)N)) || (rc = dalloc(&h->H, Hr.size())) ||
+		(rc = dalloc(&h->Lcol, (size_t)N * P)) || (rc = dalloc(&h->SM, sM.size())) || (rc = dalloc(&h->SN, sN.size())) || (rc = dalloc(&h->SI, sI.size())) || (rc = dalloc(&h->dinv, (size_t)N)) || (rc = dalloc(&h->H, Hr.size())) ||
 		(rc = dalloc(&h->y10, (size_t)d.n_m * d.n_l)) || (rc = dalloc(&h->X, nst)) || (rc = dalloc(&h->U, nst * kmax)) ||
 		(rc = dalloc(&h->V0, nst)) || (rc = dalloc(&h->V1, nst)) || (rc = dalloc(&h->tmp, nst)) ||
 		(rc = dalloc(&h->partX, (size_t)B * h->nbe * kmax)) || (rc = dalloc(&h->partN, (size_t)B * h->nbe)) ||
@@ -818,6 +883,9 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 		cudaMemcpy(h->R, R, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->Lrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->Lcol, lcol.data(), sizeof(double) * lcol.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+		cudaMemcpy(h->SM, sM.data(), sizeof(double) * sM.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+		cudaMemcpy(h->SN, sN.data(), sizeof(double) * sN.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+		cudaMemcpy(h->SI, sI.data(), sizeof(double) * sI.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->dinv, di.data(), sizeof(double) * N, cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->H, Hr.data(), sizeof(double) * Hr.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->y10, y10, sizeof(double) * d.n_m * d.n_l, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -826,6 +894,9 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 		set_error("device upload failed");
 		return fail(QPC_ERR_CUDA);
 	}
+	auto attr = [](auto kern) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SB_SMEM); };
+	attr(k_ar_sinv_blk<2>); attr(k_ar_sinv_blk<3>); attr(k_ar_sinv_blk<4>); attr(k_ar_sinv_blk<5>); attr(k_ar_sinv_blk<6>); attr(k_ar_sinv_blk<7>);
+	attr(k_ar_sinv_blk<8>);
 	*out = h;
 	return QPC_OK;
 }
@@ -966,7 +1037,8 @@ int qpc_arnoldi_norm(qpc_arnoldi* h, double* norm)
 	if (int rc = wait_on(h->stream)) return rc;
 	QPC_CUDA(cudaMemcpyAsync(h->nt, one.data(), sizeof(long long) * B, cudaMemcpyHostToDevice, h->stream));
 	ar_args g = make_args(h);
-	k_ar_snorm<<<dim3(h->nbe, B), AR_THREADS, 0, h->stream>>>(g, h->X, -1, 0);
+	if (h->pt == 1) k_ar_snorm<1><<<dim3(h->nbe, B), AR_THREADS, 0, h->stream>>>(g, h->X, -1, 0);
+	else k_ar_snorm<4><<<dim3(h->nbe, B), AR_THREADS, 0, h->stream>>>(g, h->X, -1, 0);
 	QPC_CUDA(cudaGetLastError());
 	std::vector<double> nu(B);
 	if (int rc = copy_to_host(nu.data(), h->nu0, sizeof(double) * B, h->stream)) return rc;

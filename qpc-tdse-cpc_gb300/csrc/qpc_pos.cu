@@ -401,6 +401,7 @@ int pos_end(pos_path* p, const pos_run& r)
 	band_args a = band_args_of(&p->ops, p->ops.X, nchan, p->B);
 	a.s0 = p->buf[0]; a.e0 = p->ex[0]; a.s1 = p->buf[1]; a.e1 = p->ex[1]; a.par = r.mask ? nullptr : r.ntt; a.dmap = r.perm;
 	a.dst = r.state; a.edst = p->exin;
+	a.nta = r.ntt; a.step = 0;	// a slot without steps stays as it is
 	band_apply(a, false, p->ntile, r.stream);
 	++*r.launches;
 	QPC_CUDA(cudaGetLastError());

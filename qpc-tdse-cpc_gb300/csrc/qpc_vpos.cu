@@ -444,6 +444,7 @@ int vpos_end(vpos_path* p, const vpos_run& r)
 	band_args a = band_args_of(&p->ops, p->ops.X, p->nch, p->B);
 	a.s0 = p->buf[0]; a.e0 = p->ex[0]; a.s1 = p->buf[1]; a.e1 = p->ex[1]; a.par = r.ntt;
 	a.dst = r.X; a.edst = p->exin;
+	a.nta = r.ntt; a.step = 0;	// a slot without steps stays as it is
 	band_apply(a, false, p->ntile, p->stream);
 	++*r.launches;
 	QPC_CUDA(cudaGetLastError());
