@@ -49,7 +49,8 @@ def build_engine(force=False, verbose=False):
                                              "qpc_mlp.cu", "qpc_vgwr.cu", "qpc_momentum.cu", "qpc_momentum.cpp",
                                              "qpc_gemm.cuh", "qpc_hhg.cu", "qpc_ozaki.cu", "qpc_ozaki.cuh",
                                              "qpc_tcgen05.cuh", "qpc_ltrans.cu", "qpc_ltrans.cuh", "qpc_pos.cu", "qpc_pos.cuh",
-                                             "qpc_fixed.cuh", "qpc_radial.cu", "qpc_radial.cuh", "qpc_vpos.cu", "qpc_vpos.cuh")]
+                                             "qpc_fixed.cuh", "qpc_radial.cu", "qpc_radial.cuh", "qpc_vpos.cu", "qpc_vpos.cuh",
+                                             "qpc_tcband.cu", "qpc_tcband.cuh")]
     srcs.append(os.path.join(ROOT, "include", "qpc_gb300.h"))
     if not force and not _stale(LIB, srcs):
         return LIB
@@ -69,6 +70,7 @@ def build_engine(force=False, verbose=False):
     o_po = os.path.join(OBJDIR, "qpc_pos.o")
     o_ra = os.path.join(OBJDIR, "qpc_radial.o")
     o_vp = os.path.join(OBJDIR, "qpc_vpos.o")
+    o_tb = os.path.join(OBJDIR, "qpc_tcband.o")
     nv = [_nvcc()] + NVCC_ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"] + os.environ.get("QPC_NVCC_EXTRA", "").split()
     jobs = [
         nv + ["-c", os.path.join(CSRC, "qpc_engine.cu"), "-o", o_cu],
@@ -83,13 +85,14 @@ def build_engine(force=False, verbose=False):
         nv + ["-c", os.path.join(CSRC, "qpc_pos.cu"), "-o", o_po],
         nv + ["-c", os.path.join(CSRC, "qpc_radial.cu"), "-o", o_ra],
         nv + ["-c", os.path.join(CSRC, "qpc_vpos.cu"), "-o", o_vp],
+        nv + ["-c", os.path.join(CSRC, "qpc_tcband.cu"), "-o", o_tb],
         ["g++", "-O2", "-std=c++17", "-fPIC", "-c", os.path.join(CSRC, "qpc_momentum.cpp"), "-o", o_mt],
         ["g++", "-O2", "-std=c++17", "-fPIC", "-c", os.path.join(CSRC, "qpc_setup.cpp"), "-o", o_cc],
         ["g++", "-O2", "-std=c++17", "-fPIC", "-c", os.path.join(CSRC, "qpc_spectra.cpp"), "-o", o_sp],
     ]
     with cf.ThreadPoolExecutor(len(jobs)) as ex:
         outs = list(ex.map(_run, jobs))
-    _run([_nvcc()] + NVCC_ARCH + ["-shared", o_cu, o_na, o_ar, o_ml, o_vg, o_mo, o_hh, o_oz, o_lt, o_po, o_ra, o_vp, o_mt, o_cc, o_sp, "-o", LIB + ".tmp", "-lcudart", "-lcusolver", "-lpthread"])
+    _run([_nvcc()] + NVCC_ARCH + ["-shared", o_cu, o_na, o_ar, o_ml, o_vg, o_mo, o_hh, o_oz, o_lt, o_po, o_ra, o_vp, o_tb, o_mt, o_cc, o_sp, "-o", LIB + ".tmp", "-lcudart", "-lcusolver", "-lpthread"])
     os.replace(LIB + ".tmp", LIB)
     if verbose:
         print("".join(outs))

@@ -581,7 +581,7 @@ int read_status(qpc_lgwz* h)
 	}
 	if (st & ST_PIVOT) { set_error("zero pivot in a Crank-Nicolson factorisation"); return QPC_ERR_SINGULAR; }
 	if (st & ST_NONFINITE) { set_error("non-finite value in the state"); return QPC_ERR_NUMERIC; }
-	if (st & ST_TIMEOUT) { set_error("a tensor-core wait of the l-space transform ran out"); return QPC_ERR_TIMEOUT; }
+	if (st & ST_TIMEOUT) { set_error("a tensor-core wait ran out"); return QPC_ERR_TIMEOUT; }
 	return QPC_OK;
 }
 
@@ -1412,6 +1412,8 @@ static int run_pos(qpc_lgwz* h, const std::vector<int64_t>& pf, const std::vecto
 	r.z = dipole ? h->zdev : nullptr;
 	r.ldz = ldz;
 	r.launches = &h->launches;
+	r.status = h->status;
+	r.stbit = ST_TIMEOUT;
 	r.stream = h->stream;
 	int open = -1;
 	if (h->profiling) {

@@ -11,9 +11,9 @@
 // A step is two kernels: k_angle (l transform, phases, l transform back, everything local in j) and
 // k_band_apply (the banded products, everything local in l).
 //
-// Both products run in fixed point (qpc_radial.cu).
+// Both products run in fixed point (qpc_radial.cu), for batches on the tensor cores (qpc_tcband.cu).
 // Against the banded solves (GB300, per step): one wavefunction of 800 x 41 with its dipole 1340 -> 60 us,
-// 400 x 21 287 -> 26 us, 24 wavefunctions of 517 x 30 1120 -> 200 us, 256 of 800 x 41 8.0 -> 3.3 ms; error against
+// 400 x 21 287 -> 26 us, 24 wavefunctions of 517 x 30 1120 -> 86 us, 256 of 800 x 41 8.0 -> 1.2 ms; error against
 // extended precision after 60 steps 3.3e-13 against 4.7e-13.
 #include "qpc_pos.cuh"
 #include "qpc_radial.cuh"
@@ -235,7 +235,7 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 	const int N = p->N, L = p->L, M = p->M;
 	int rc;
 	const long nvec = (long)p->B * M * L;
-	if ((rc = radial_create(&p->ops, radial_setup{N, p->P, p->nlh, p->nff, in.S, in.R, true, in.fieldfree, in.stream}, M * L, ok)) || !*ok) return rc;
+	if ((rc = radial_create(&p->ops, radial_setup{N, p->P, p->nlh, p->nff, in.S, in.R, true, in.fieldfree, in.stream, p->B}, M * L, ok)) || !*ok) return rc;
 	std::vector<int> lm(M * L);
 	for (int c = 0; c < M * L; ++c) lm[c] = c % L + std::abs(p->m0 + c / L);
 	std::vector<int2> V((size_t)M * (p->npair + 1) * L);
@@ -322,7 +322,7 @@ int pos_begin(pos_path* p, const pos_run& r)
 	band_args a = band_args_of(&p->ops, p->ops.W, nchan, p->B);
 	a.s0 = r.state; a.e0 = p->exin; a.smap = r.perm;
 	a.dst = p->buf[0]; a.edst = p->ex[0];
-	band_apply(a, false, p->ntile, st);
+	band_apply(a, false, p->ntile, st, &p->ops.W, r.status, r.stbit);
 	*r.launches += 2;
 	return QPC_OK;
 }
@@ -386,7 +386,7 @@ int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf)
 		if (p->nff > 1) a.amap = r.perm;
 		a.s0 = p->buf[cur]; a.e0 = p->ex[cur]; a.dst = p->buf[1 - cur]; a.edst = p->ex[1 - cur];
 		a.nta = r.ntt; a.step = s;
-		band_apply(a, true, p->ntile, st);
+		band_apply(a, true, p->ntile, st, &p->ops.F, r.status, r.stbit);
 		++*r.launches;
 	}
 	QPC_CUDA(cudaGetLastError());
@@ -402,7 +402,7 @@ int pos_end(pos_path* p, const pos_run& r)
 	a.s0 = p->buf[0]; a.e0 = p->ex[0]; a.s1 = p->buf[1]; a.e1 = p->ex[1]; a.par = r.mask ? nullptr : r.ntt; a.dmap = r.perm;
 	a.dst = r.state; a.edst = p->exin;
 	a.nta = r.ntt; a.step = 0;	// a slot without steps stays as it is
-	band_apply(a, false, p->ntile, r.stream);
+	band_apply(a, false, p->ntile, r.stream, &p->ops.X, r.status, r.stbit);
 	++*r.launches;
 	QPC_CUDA(cudaGetLastError());
 	return QPC_OK;

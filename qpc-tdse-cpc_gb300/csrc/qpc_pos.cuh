@@ -37,6 +37,8 @@ struct pos_run {
 	double* z;			// device [B][ldz], the dipole of f(r) = r before every step, or nullptr
 	long ldz;
 	int64_t* launches;
+	int* status;			// device word, or-ed with stbit when a wait on the tensor cores ran out
+	int stbit;
 	std::function<void(int, cudaStream_t)> prof_begin, prof_end;	// per-kernel timing, or empty
 	cudaStream_t stream;
 };

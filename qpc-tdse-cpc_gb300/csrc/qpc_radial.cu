@@ -14,7 +14,9 @@
 // 2^-57 of the largest element of the ~250 a sum covers, below the FP64 rounding of the sum itself.  Entries of
 // F~ below 2^-29 have no hi limb: the outer part of the band costs one multiply-add and half the bytes.
 #include "qpc_radial.cuh"
+#include "qpc_tcband.cuh"
 #include <cstring>
+#include <cstdlib>
 #include <cmath>
 #include <type_traits>
 
@@ -741,6 +743,13 @@ int eigenvectors(radial_ops* p, const radial_setup& in, scratch& tmp, double** Y
 }
 
 
+std::vector<double> as_doubles(const std::vector<unsigned long long>& prof)
+{
+	std::vector<double> d(prof.size());
+	std::memcpy(d.data(), prof.data(), 8 * d.size());
+	return d;
+}
+
 // scale and profile of a real operator; ok as in decay()
 int store_banded_impl(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st, bool dense, bool* ok)
 {
@@ -759,6 +768,7 @@ int store_banded_impl(radial_ops* p, band_store& b, const double* A, long si, lo
 		std::frexp(big, &b.ea);
 		*ok = decay(prof, p->N, std::ldexp(1.0, b.ea), w, wf, 29);
 		if (!*ok) return QPC_OK;
+		b.prof = as_doubles(prof);
 	}
 	lay_out(b, p->N, w, wf, false);
 	if (int rc = upload(b, (size_t)b.stride)) return rc;
@@ -780,6 +790,14 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 	if ((rc = eigenvectors(p, in, tmp, &Yt, ok)) || !*ok) return rc;
 	if ((rc = store_banded(p, p->W, Yt, N, 1, st, ok)) || !*ok) return rc;
 	if ((rc = store_banded(p, p->X, p->Xt, 1, N, st, ok)) || !*ok) return rc;
+	const char* mode = std::getenv("QPC_POS_TC");	// 0: multiply-adds only, 1: tensor cores wherever they can
+	const bool always = mode && mode[0] == '1';
+	p->F.tc_always = p->W.tc_always = p->X.tc_always = always;
+	const bool tcp = p->nff == 1 && (always || (in.batch >= TC_MIN && N >= 128 && !(mode && mode[0] == '0')));
+	if (tcp) {
+		if ((rc = tc_make(p->W.tc, nullptr, Yt, 0, N, 1, N, N, 1, p->W.w, p->W.prof.data(), p->W.ea, nullptr, st, &p->W.has_tc))) return rc;
+		if ((rc = tc_make(p->X.tc, nullptr, p->Xt, 0, 1, N, N, N, 1, p->X.w, p->X.prof.data(), p->X.ea, nullptr, st, &p->X.has_tc))) return rc;
+	}
 	// F~_l, a set of columns at a time: the engine's field-free solve on the eigenvectors, then X^T S
 	const int J = (int)std::min<long>(N, std::max<long>(32, (64l << 20) / ((long)N * nlh * 16)));
 	const size_t chunk = (size_t)J * N * nlh;
@@ -823,6 +841,10 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 		}
 		k_store<true><<<dim3(p->ntile, nlh), 256, 0, st>>>(Fb, nullptr, 0, 0, N, p->F.w, std::ldexp(1.0, 56), p->F.d_td, p->F.d_off,
 			p->F.A + (size_t)fi * nlh * p->F.stride, p->F.stride);
+		if (tcp) {
+			const std::vector<double> pd = as_doubles(prof);
+			if ((rc = tc_make(p->F.tc, Fb, nullptr, 0, 0, 0, N, N, nlh, p->F.w, pd.data(), 0, nullptr, st, &p->F.has_tc))) return rc;
+		}
 	}
 	if (p->nff > 1) {
 		int w, wf;
@@ -862,8 +884,22 @@ band_args band_args_of(const radial_ops* p, const band_store& b, int nchan, int 
 	return a;
 }
 
-void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st)
+// Microseconds of k_band_apply: its multiply-adds at 8e12 a second (26 per cycle and SM), 6 us of latency.  Measured against
+// the tensor cores (F~, us): 800 x 41, 4 columns 56 to 76, 8 98 to 78, 48 613 to 131; 400 x 21, 8 30 to 41, 12 50 to 41,
+// 48 164 to 56; 250 x 30 (p = 7), 8 30 to 33, 16 50 to 34.  The two estimates cross where these do
+static double madd_cost(const band_store& b, bool cx, int nchan, int ncols)
 {
+	double k = 0.0;
+	for (const int4& t : b.td) k += KC * ((t.z - t.y) * (cx ? 12.0 : 6.0) + (t.y - t.x + t.w - t.z) * (cx ? 4.0 : 2.0));
+	return 6.0 + k * TM * nchan * ((ncols + 7) & ~7) / 8e6;
+}
+
+void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st, const band_store* b, int* status, int stbit)
+{
+	if (b && b->has_tc && !a.amap && (b->tc_always || tc_cost(b->tc, a.nchan, a.ncols) < madd_cost(*b, cx, a.nchan, a.ncols))) {
+		tc_apply(b->tc, a, status, stbit, st);
+		return;
+	}
 	if (cx) dispatch<true>(a, tiles, st);
 	else dispatch<false>(a, tiles, st);
 }

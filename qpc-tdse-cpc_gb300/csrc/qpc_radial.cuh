@@ -32,6 +32,22 @@ struct band_args {
 	int tile0;		// first tile of the launch
 };
 
+// digit planes of a set of operators (one per l) for k_tc_apply; made from the FP64 entries
+struct tc_store {
+	bool cx = false;
+	int ea = 0;			// |A| <= 2^ea
+	int db = 8;			// bits of a digit
+	int N = 0, ntile = 0;		// columns, 128-row tiles
+	int nrow = 0;
+	size_t stride = 0;		// bytes of one operator
+	int2* d_list = nullptr;		// per tile: its (first k, first digit) stages, those with every digit first
+	int4* d_first = nullptr;	// per tile: its entries of d_list, the k they cover
+	size_t* d_off = nullptr;	// per tile: byte offset of its first plane
+	char* A = nullptr;
+	std::vector<int> work;		// per tile: cycles of tensor-core math
+	void release();
+};
+
 // an operator (or one per l and set) in the layout k_band_apply reads: per tile of TM rows the chunks of KC columns
 // td = (first, first with hi limbs, end of those, end) at byte off
 struct band_store {
@@ -43,7 +59,10 @@ struct band_store {
 	long* d_off = nullptr;
 	char* A = nullptr;
 	size_t cap = 0;
-	void release() { cudaFree(d_td); cudaFree(d_off); cudaFree(A); d_td = nullptr; d_off = nullptr; A = nullptr; }
+	std::vector<double> prof;	// largest entry per distance, as laid out
+	tc_store tc;			// the same for the tensor cores, for batches
+	bool has_tc = false, tc_always = false;
+	void release() { tc.release(); has_tc = false; cudaFree(d_td); cudaFree(d_off); cudaFree(A); d_td = nullptr; d_off = nullptr; A = nullptr; }
 };
 
 // what radial_create reads: device bands S, R [N][P+1] (R: the operator the basis diagonalises, its eigenvalues
@@ -55,7 +74,9 @@ struct radial_setup {
 	bool rmajor;
 	std::function<int(double2*, double2*, int, int)> fieldfree;
 	cudaStream_t stream;
+	int batch;		// most columns of a product: from TC_MIN on the operators are kept for the tensor cores too
 };
+constexpr int TC_MIN = 6;	// below, the multiply-adds win at every size (16 MB to 300 MB of planes saved)
 
 // eigenvectors x_i of (R, S): X^T S X = 1, X^T R X = diag(r); c = X y
 struct radial_ops {
@@ -82,7 +103,9 @@ int project_band(const radial_ops* p, const double* B, bool anti, double* Bx, do
 int orthonormalise(double* Qt, int N, double* E, double* T, cudaStream_t st, bool* ok);
 
 band_args band_args_of(const radial_ops* p, const band_store& b, int nchan, int ncols);
-void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st);
+// status, stbit: device word or-ed with stbit when a wait of the tensor-core kernel ran out; b: the store behind a (its
+// planes are used where that is the faster way), or NULL
+void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st, const band_store* b = nullptr, int* status = nullptr, int stbit = 0);
 // largest biased exponent of every TE rows of src [nvec][N]
 void exponents(const double2* src, int* ex, int N, int ntile, long nvec, cudaStream_t st);
 

@@ -1,0 +1,19 @@
+// The banded and dense products of qpc_radial.cu on the tensor cores (qpc_tcband.cu), for batches.
+#pragma once
+#include "qpc_radial.cuh"
+
+namespace qpc {
+
+// From the band Fb [nop][N][2 WMAX + 1] (complex), or a real matrix A(i, j) = A[op * sop + i * si + j * sj] of nrow x N;
+// prof: largest |entry| per distance as in radial_create (NULL: every entry counts).  ok = false: an exact sum could
+// exceed 2^24, or the planes would take more than 4 GB.
+int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, long sj, int nrow, int N, int nop, int w, const double* prof, int ea,
+	const int* ear, cudaStream_t st, bool* ok);
+
+// the product of band_args a with the planes t (a.A, a.td, a.toff unused); status: device word or-ed with stbit when a
+// wait ran out
+void tc_apply(const tc_store& t, const band_args& a, int* status, int stbit, cudaStream_t st);
+// microseconds it takes: twice the tensor-core math and 9 us of a block's own, one block per SM
+double tc_cost(const tc_store& t, int nchan, int ncols);
+
+} // namespace qpc

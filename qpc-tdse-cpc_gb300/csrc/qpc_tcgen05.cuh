@@ -80,6 +80,12 @@ __device__ __forceinline__ void ld8(uint32_t taddr, uint32_t (&v)[8])
 		: "r"(taddr));
 }
 
+// 4 of them
+__device__ __forceinline__ void ld4(uint32_t taddr, uint32_t (&v)[4])
+{
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(taddr));
+}
+
 __device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }

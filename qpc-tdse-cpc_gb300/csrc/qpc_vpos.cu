@@ -250,7 +250,7 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	if ((rc = dalloc(&R, nb))) return rc;
 	struct guard { double* p; ~guard() { cudaFree(p); } } g{R};
 	QPC_CUDA(cudaMemcpy(R, neg.data(), sizeof(double) * nb, cudaMemcpyHostToDevice));
-	if ((rc = radial_create(&p->ops, radial_setup{N, in.P, in.nlh, 1, in.S, R, false, in.fieldfree, st}, nch, ok)) || !*ok) return rc;
+	if ((rc = radial_create(&p->ops, radial_setup{N, in.P, in.nlh, 1, in.S, R, false, in.fieldfree, st, 0}, nch, ok)) || !*ok) return rc;
 	if ((rc = dalloc(&p->om, N)) || (rc = dalloc(&p->rinv, N))) return rc;
 	k_negate<<<(N + 255) / 256, 256, 0, st>>>(p->ops.r, p->rinv, N);
 	if ((rc = momentum_basis(p, in, ok)) || !*ok) return rc;
