@@ -35,10 +35,13 @@ constexpr int LMAX = 128;	// most l channels
 // (28 instructions per pair and position).  The dipole of f(r) = r is sum_k lambda_k r_j (|z+|^2 - |z-|^2) =
 // sum_k 4 lambda_k r_j Re(conj(E_k) O_k).  PT = 32 is bound by the multiply-adds; with too few blocks to fill the
 // SMs a block's own latency counts, and PT = 8 cuts it (four times the blocks, a quarter of the serial products).
+// 80 registers (a few spilled at G = 3) for three blocks per SM, coefficients stored in the order a task reads them:
+// 256 wavefunctions of 800 x 41 570 -> 450 us (multiply-adds alone 270), 24 of 517 x 30 36 -> 28 us.
 struct angle_args {
 	double2* y;		// [slot][M][L][N], in place
 	int* ex;		// [slot][M][L][ntile * EPT]
-	const int2* V;		// [M][npair+1][L] limbs, |V| <= 1
+	const int2 *V, *W;	// limbs of the transform and of its transpose, [M][task][k][G] (|V| <= 1)
+	int nV, nW;		// of one m
 	const double* lamp;	// [M][npair]
 	const double* r;	// [N]
 	const double* ftab;
@@ -60,8 +63,41 @@ __device__ __forceinline__ int power_of(long s, long nt, int cmode)
 	return (s == 0 || s == nt) ? 1 : 2;
 }
 
+// 1 / x, x >= 1: two Newton steps from the fp32 approximation (relative error 2^-23 -> 2^-46 -> rounding)
+__device__ __forceinline__ double reciprocal(double x)
+{
+	if (!(x < 1e30)) return 1.0 / x;
+	float r0;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(__int_as_float(((__double2hiint(x) - 0x38000000) << 3) | (int)((unsigned)__double2loint(x) >> 29))));
+	const int b = __float_as_int(r0);
+	double r = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+	r = fma(r, fma(-x, r, 1.0), r);
+	return fma(r, fma(-x, r, 1.0), r);
+}
+
+// G outputs of a real matrix, A = [k][G] limbs, times the column at x[k * XK]
+template <int G, int XK>
+__device__ __forceinline__ void task_product(const int2* __restrict__ A, int nk, const int4* __restrict__ x, long long (&h)[G][2], long long (&m)[G][2])
+{
+#pragma unroll
+	for (int g = 0; g < G; ++g) h[g][0] = h[g][1] = m[g][0] = m[g][1] = 0;
+#pragma unroll 4
+	for (int k = 0; k < nk; ++k) {
+		const int4 y = x[k * XK];
+#pragma unroll
+		for (int g = 0; g < G; ++g) {
+			const int2 a = __ldg(A + k * G + g);
+			h[g][0] = madw(a.x, y.x, h[g][0]); h[g][1] = madw(a.x, y.z, h[g][1]);
+			m[g][0] = madw(a.x, y.y, m[g][0]); m[g][0] = madw(a.y, y.x, m[g][0]);
+			m[g][1] = madw(a.x, y.w, m[g][1]); m[g][1] = madw(a.y, y.z, m[g][1]);
+		}
+	}
+#pragma unroll
+	for (int g = 0; g < G; ++g) { flush(h[g][0], m[g][0]); flush(h[g][1], m[g][1]); }
+}
+
 template <int G, int PT>
-__global__ void __launch_bounds__(256) k_angle(const angle_args p)
+__global__ void __launch_bounds__(256, 3) k_angle(const angle_args p)
 {
 	constexpr int NV = 8 * 32 / PT, TPT = TM / PT;	// virtual warps; blocks per tile
 	extern __shared__ double2 sm[];
@@ -98,13 +134,14 @@ __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 	}
 	__syncthreads();
 	const int4* qa = reinterpret_cast<const int4*>(a) + lane;
-	const int2* V = p.V + (long)m * (np + 1) * L;
+	const int2* V = p.V + (long)m * p.nV;
+	const int nl0 = (L + 1) / 2, nl1 = L / 2;	// even and odd l
 	const int nE = np + (L & 1), gE = (nE + G - 1) / G, gO = (np + G - 1) / G;
 	long long h[G][2], mm[G][2];
 	for (int t = warp; t < gE + gO; t += NV) {
 		const bool odd = t >= gE;
 		const int k0 = (odd ? t - gE : t) * G, no = min(G, (odd ? np : nE) - k0);
-		local_product<G>(V + k0 * L + (odd ? 1 : 0), L, 2, odd ? L / 2 : (L + 1) / 2, no, qa + (odd ? PT : 0), 2 * PT, h, mm);
+		task_product<G, 2 * PT>(V + t * G * nl0, odd ? nl1 : nl0, qa + (odd ? PT : 0), h, mm);
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
@@ -115,7 +152,7 @@ __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 	}
 	__syncthreads();
 	const double rj = in ? p.r[row] : 0.0;
-	const double f = pw ? p.ftab[(long)slot * p.ld + p.step] * p.dt4 : 0.0;
+	const double f = pw ? p.ftab[(long)slot * p.ld + p.step] * p.dt4 * rj : 0.0;
 	double z = 0.0;
 	e = 0;
 	for (int k = warp; k < np; k += NV) {
@@ -123,15 +160,14 @@ __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 		const double lam = p.lamp[m * np + k];
 		if (obs) z = fma(lam, fma(E.x, O.x, E.y * O.y), z);
 		if (pw) {
-			const double beta = lam * f * rj;
-			const double inv = 1.0 / fma(beta, beta, 1.0);
-			double c = fma(-beta, beta, 1.0) * inv, s = -2.0 * beta * inv;
+			// 2 (c + i s), c + i s = ((1 - i beta) / (1 + i beta))^pw
+			const double beta = lam * f, inv = reciprocal(fma(beta, beta, 1.0));
+			double s = -4.0 * beta * inv, c = fma(s, beta, 2.0);	// a rounding of inv moves |c + i s| by beta^2 of it
 			if (pw == 2) {
-				const double c1 = c;
-				c = fma(-2.0 * s, s, 1.0);
-				s = 2.0 * s * c1;
+				const double s1 = s;
+				s *= c;
+				c = fma(-s1, s1, 2.0);
 			}
-			c *= 2.0; s *= 2.0;
 			const double2 S = make_double2(fma(c, E.x, -s * O.y), fma(c, E.y, s * O.x));
 			const double2 D = make_double2(fma(c, O.x, -s * E.y), fma(c, O.y, s * E.x));
 			e = max(max(e, max(bexp(S.x), bexp(S.y))), max(bexp(D.x), bexp(D.y)));
@@ -164,13 +200,14 @@ __global__ void __launch_bounds__(256) k_angle(const angle_args p)
 		reinterpret_cast<int4*>(a)[k * PT + lane] = make_int4(q0.x, q0.y, q1.x, q1.y);
 	}
 	__syncthreads();
-	const int nl0 = (L + 1) / 2, nl1 = L / 2, g0 = (nl0 + G - 1) / G, g1 = (nl1 + G - 1) / G;
+	const int g0 = (nl0 + G - 1) / G, g1 = (nl1 + G - 1) / G;
+	V = p.W + (long)m * p.nW;
 	const unsigned grp = PT == 32 ? 0xffffffffu : ((1u << PT) - 1) << (threadIdx.x & 31 & ~(PT - 1));
 	for (int t = warp; t < g0 + g1; t += NV) {
 		const int odd = t >= g0 ? 1 : 0;
 		const int o0 = (odd ? t - g0 : t) * G, no = min(G, (odd ? nl1 : nl0) - o0);
 		// even l: s_k (slots 2k) and, for odd n_l, the zero channel (slot 2 npair); odd l: d_k (slots 2k + 1)
-		local_product<G>(V + 2 * o0 + odd, 2, L, odd ? np : nE, no, qa + odd * PT, 2 * PT, h, mm);
+		task_product<G, 2 * PT>(V + t * G * nE, odd ? np : nE, qa + odd * PT, h, mm);
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
@@ -210,7 +247,8 @@ struct pos_path {
 	double2* buf[2] = {nullptr, nullptr};
 	int* ex[2] = {nullptr, nullptr};
 	int* exin = nullptr;
-	int2* V = nullptr;
+	int2 *V = nullptr, *W = nullptr;
+	int nV = 0, nW = 0;
 	double* lamp = nullptr;
 	int* lmap = nullptr;		// channel -> l
 	double* zpart = nullptr;
@@ -238,15 +276,6 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 	if ((rc = radial_create(&p->ops, radial_setup{N, p->P, p->nlh, p->nff, in.S, in.R, true, in.fieldfree, in.stream, p->B}, M * L, ok)) || !*ok) return rc;
 	std::vector<int> lm(M * L);
 	for (int c = 0; c < M * L; ++c) lm[c] = c % L + std::abs(p->m0 + c / L);
-	std::vector<int2> V((size_t)M * (p->npair + 1) * L);
-	for (size_t i = 0; i < V.size(); ++i) V[i] = limbs_of(in.Vh[i]);
-	if ((rc = dalloc(&p->lmap, lm.size())) || (rc = dalloc(&p->V, V.size())) || (rc = dalloc(&p->lamp, (size_t)M * std::max(p->npair, 1)))) return rc;
-	QPC_CUDA(cudaMemcpy(p->lmap, lm.data(), sizeof(int) * lm.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(p->V, V.data(), sizeof(int2) * V.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(p->lamp, in.lamp, sizeof(double) * M * std::max(p->npair, 1), cudaMemcpyHostToDevice));
-	for (int i = 0; i < 2; ++i)
-		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
-	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
 	// outputs per task of k_angle: the fewest rounds of eight warps
 	int best = 1 << 30;
 	for (int g = 2; g <= 4; ++g) {
@@ -255,6 +284,28 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 	}
 	// fewer blocks than SMs with 32 positions each: 8
 	p->angle_small = (long)p->B * M * p->ntile <= 304;
+	// the transforms' limbs as the tasks read them; a task's outputs beyond the last are zero
+	const int np = p->npair, nE = np + (L & 1), nl0 = (L + 1) / 2, nl1 = L / 2, G = p->angle_small ? 1 : p->angle_g;
+	const int gE = (nE + G - 1) / G, gO = (np + G - 1) / G, g0 = (nl0 + G - 1) / G, g1 = (nl1 + G - 1) / G;
+	p->nV = (gE + gO) * nl0 * G;
+	p->nW = (g0 + g1) * nE * G;
+	std::vector<int2> V((size_t)M * p->nV, make_int2(0, 0)), W((size_t)M * p->nW, make_int2(0, 0));
+	for (int m = 0; m < M; ++m)
+		for (int odd = 0; odd < 2; ++odd)
+			for (int k = 0; k < (odd ? np : nE); ++k)
+				for (int l = 0; l < (odd ? nl1 : nl0); ++l) {
+					const int2 v = limbs_of(in.Vh[((size_t)m * (np + 1) + k) * L + 2 * l + odd]);
+					V[(size_t)m * p->nV + (((odd ? gE : 0) + k / G) * nl0 + l) * G + k % G] = v;
+					W[(size_t)m * p->nW + (((odd ? g0 : 0) + l / G) * nE + k) * G + l % G] = v;
+				}
+	if ((rc = dalloc(&p->lmap, lm.size())) || (rc = dalloc(&p->V, V.size())) || (rc = dalloc(&p->W, std::max<size_t>(W.size(), 1))) || (rc = dalloc(&p->lamp, (size_t)M * std::max(p->npair, 1)))) return rc;
+	QPC_CUDA(cudaMemcpy(p->lmap, lm.data(), sizeof(int) * lm.size(), cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpy(p->V, V.data(), sizeof(int2) * V.size(), cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpy(p->W, W.data(), sizeof(int2) * W.size(), cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpy(p->lamp, in.lamp, sizeof(double) * M * std::max(p->npair, 1), cudaMemcpyHostToDevice));
+	for (int i = 0; i < 2; ++i)
+		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
+	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
 	const int smem = (int)(sizeof(double2) * 64 * LMAX);
 	cudaFuncSetAttribute(k_angle<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	cudaFuncSetAttribute(k_angle<3, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -287,7 +338,7 @@ int pos_create(const pos_setup& in, pos_path** out)
 void pos_destroy(pos_path* p)
 {
 	if (!p) return;
-	cudaFree(p->lmap); cudaFree(p->V); cudaFree(p->lamp);
+	cudaFree(p->lmap); cudaFree(p->V); cudaFree(p->W); cudaFree(p->lamp);
 	for (int i = 0; i < 2; ++i) { cudaFree(p->buf[i]); cudaFree(p->ex[i]); }
 	cudaFree(p->exin); cudaFree(p->zpart);
 	p->K.release();
@@ -346,7 +397,7 @@ int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf)
 	auto angle = [&](int cmode, int slots, bool observe) {
 		POS_PROF(QPC_KERNEL_SWEEP);
 		angle_args a{};
-		a.y = p->buf[cur]; a.ex = p->ex[cur]; a.V = p->V; a.lamp = p->lamp; a.r = p->ops.r; a.ftab = r.ftab; a.ld = r.ld; a.ntf = r.ntf; a.ntt = r.ntt;
+		a.y = p->buf[cur]; a.ex = p->ex[cur]; a.V = p->V; a.W = p->W; a.nV = p->nV; a.nW = p->nW; a.lamp = p->lamp; a.r = p->ops.r; a.ftab = r.ftab; a.ld = r.ld; a.ntf = r.ntf; a.ntt = r.ntt;
 		a.step = s; a.cmode = cmode; a.dt4 = 0.25 * p->dt; a.N = p->N; a.ntile = p->ntile; a.L = p->L; a.M = p->M; a.npair = p->npair;
 		if (observe) {
 			if (!p->zcount) p->zfirst = s;
