@@ -10,9 +10,12 @@
 //   tSURF per step: the surface values (N_ch * nb), the flux term per (kr, channel), the
 //         l-sum against Y_lm (nkr * nkt * N_ch per instance) and the m-sum with the Volkov
 //         phase (nkr * nkt * nkp * n_m per instance).
-// Every kernel is a plain FP64 loop: one thread per output element, operands staged in
-// shared memory where a block shares them.
+// The projections run as exact digit sums on the tensor cores (qpc_tcband.cu; each row of the table under its own
+// largest exponent); where the table does not suit that (values that are not finite, planes beyond 4 GB) and for
+// everything else the kernels are plain FP64 loops: one thread per output element, operands staged in shared memory
+// where a block shares them.
 #include "qpc_cuda_util.cuh"
+#include "qpc_tcband.cuh"
 #include <cmath>
 #include <vector>
 
@@ -74,7 +77,62 @@ __global__ void __launch_bounds__(128) k_pcs_proj(const double* __restrict__ ijl
 	}
 }
 
-// With Q = cps <ijl|c> from k_pcs_proj:
+// The projections on the tensor cores: P[seg][inst][ch][kr] = sum over the columns of a segment (at most TCK of them: an
+// exact sum of 8 digits of 7 bits holds about 1000).  64 wavefunctions of 800 x 41 on 250 momenta
+// 2.06 -> 0.16 ms (FP64: 1.05e9 multiply-adds at 2 per cycle and SM are 1.7 ms), and an error of 6.0e-16 against extended
+// precision where the plain sums leave 1.0e-15.
+constexpr int TCK = 896;
+
+// Q[inst][kr][ch] = cps[kr][l] sum_seg P[seg][inst][ch][kr], 32 x 32 of (kr, ch) at a time
+__global__ void __launch_bounds__(256) k_pcs_join(const double2* __restrict__ P, int nseg, size_t stride, const double2* __restrict__ cps, double2* __restrict__ Q, int nkr,
+	int n_l, int m0, int nch, int nl_tot)
+{
+	__shared__ double2 t[32][33];
+	const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, kr0 = blockIdx.x * 32, ch0 = blockIdx.y * 32;
+	const size_t inst = blockIdx.z;
+	for (int i = ty; i < 32; i += 8)
+		if (ch0 + i < nch && kr0 + tx < nkr) {
+			double2 v = make_double2(0.0, 0.0);
+			for (int s = 0; s < nseg; ++s) v = cadd(v, P[s * stride + (inst * nch + ch0 + i) * nkr + kr0 + tx]);
+			t[i][tx] = v;
+		}
+	__syncthreads();
+	const int ch = ch0 + tx;
+	if (ch >= nch) return;
+	const int l = abs(m0 + ch / n_l) + ch % n_l;
+	for (int i = ty; i < 32; i += 8)
+		if (kr0 + i < nkr) Q[(inst * nkr + kr0 + i) * nch + ch] = cmul(cps[(size_t)(kr0 + i) * nl_tot + l], t[tx][i]);
+}
+
+// |ijl[kr][l][.]| <= 2^ear[l][kr]
+__global__ void k_pcs_rows(const double* __restrict__ ijl, int* __restrict__ ear, int nkr, int nl, int n_r)
+{
+	const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+	if (row >= nkr * nl) return;
+	const int l = row / nkr, k = row % nkr;
+	const double* a = ijl + ((size_t)k * nl + l) * n_r;
+	double v = 0.0;
+	for (int r = threadIdx.x & 31; r < n_r; r += 32) v = fmax(v, fabs(a[r]));
+	for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+	if ((threadIdx.x & 31) == 0) ear[row] = v > 0.0 && v < 1e300 ? ilogb(v) + 1 : 0;
+}
+
+// ijlT[l][r][kr] = ijl[kr][l][r]
+__global__ void __launch_bounds__(256) k_pcs_transpose(const double* __restrict__ ijl, double* __restrict__ ijlT, int nkr, int nl, int n_r)
+{
+	__shared__ double t[32][33];
+	const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+	for (int l = blockIdx.z; l < nl; l += gridDim.z) {
+		__syncthreads();
+		for (int i = ty; i < 32; i += 8)
+			if (k0 + i < nkr && r0 + tx < n_r) t[i][tx] = ijl[((size_t)(k0 + i) * nl + l) * n_r + r0 + tx];
+		__syncthreads();
+		for (int i = ty; i < 32; i += 8)
+			if (r0 + i < n_r && k0 + tx < nkr) ijlT[((size_t)l * n_r + r0 + i) * nkr + k0 + tx] = t[tx][i];
+	}
+}
+
+// With Q = cps <ijl|c>:
 // LMD[inst][kr][ch] = sqrt(2/pi) Q                                   (measure_lmd, 386-403)
 // PMD[inst][kr][kt][kp] = sqrt(2/pi) sum_m exm[kp][m] sum_l plm Q     (measure_prj, 337-355)
 // PAD[inst][kr][kt] = 2 sqrt(kr) sum_m sum_l plm Q                    (measure_pad, 358-383)
@@ -272,8 +330,11 @@ struct qpc_pcs {
 	float last_ms = 0.f;
 	double *ijlT = nullptr, *plm = nullptr, *kr = nullptr;
 	double2 *exm = nullptr, *cps = nullptr;
-	double2 *cbuf = nullptr, *Q = nullptr, *out = nullptr;
-	long cap_c = 0, cap_q = 0, cap_o = 0;
+	double2 *cbuf = nullptr, *Q = nullptr, *out = nullptr, *P = nullptr;
+	long cap_c = 0, cap_q = 0, cap_o = 0, cap_p = 0, cap_x = 0;
+	std::vector<tc_store> seg;	// the table's digit planes, a segment of columns each (none: ijlT)
+	int *ear = nullptr, *lmap = nullptr, *ex = nullptr, *status = nullptr;
+	int* hstatus = nullptr;		// pinned
 };
 
 struct qpc_tsurff {
@@ -299,7 +360,9 @@ void pcs_free(qpc_pcs* h)
 {
 	if (!h) return;
 	cudaSetDevice(h->dev);
-	void* ps[] = {h->ijlT, h->plm, h->kr, h->exm, h->cps, h->cbuf, h->Q, h->out};
+	void* ps[] = {h->ijlT, h->plm, h->kr, h->exm, h->cps, h->cbuf, h->Q, h->out, h->P, h->ear, h->lmap, h->ex, h->status};
+	for (tc_store& t : h->seg) t.release();
+	if (h->hstatus) cudaFreeHost(h->hstatus);
 	for (void* p : ps) if (p) cudaFree(p);
 	if (h->ev0) cudaEventDestroy(h->ev0);
 	if (h->ev1) cudaEventDestroy(h->ev1);
@@ -339,17 +402,73 @@ int pcs_run(qpc_pcs* h, int kind, const double2* c, int n_inst, double* out)
 	long total = kind == QPC_SPEC_LMD ? (long)n_inst * h->nkr * nch
 		: kind == QPC_SPEC_PMD ? (long)n_inst * h->nkr * h->nkt * h->nkp : (long)n_inst * h->nkr * h->nkt;
 	if (int rc = grow(&h->out, &h->cap_o, total)) return rc;
-	dim3 g1((n_inst + PG - 1) / PG, (h->nkr + 127) / 128, nch);
+	const int nseg = (int)h->seg.size(), ntile = (d.n_r + TM - 1) / TM;
+	const long nvec = (long)n_inst * nch;
+	if (nseg)
+		if (int rc = grow(&h->P, &h->cap_p, nseg * nvec * h->nkr)) return rc;
+	if (nseg)
+		if (int rc = grow(&h->ex, &h->cap_x, nvec * ntile * EPT)) return rc;
 	QPC_CUDA(cudaEventRecord(h->ev0, h->st));
-	k_pcs_proj<<<g1, 128, 0, h->st>>>(h->ijlT, h->cps, c, h->Q, h->nkr, d.n_r, d.n_l, d.m0, nch, h->nl, n_inst);
+	if (nseg) {
+		QPC_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), h->st));
+		exponents(c, h->ex, d.n_r, ntile, nvec, h->st);
+		for (int s = 0; s < nseg; ++s) {
+			band_args a{};
+			a.lmap = h->lmap; a.N = d.n_r; a.ntile = ntile; a.nchan = nch; a.ncols = n_inst;
+			a.s0 = c; a.e0 = h->ex; a.dst = h->P + s * nvec * h->nkr;
+			tc_apply(h->seg[s], a, h->status, 1, h->st);
+		}
+		QPC_CUDA(cudaGetLastError());
+		for (int i0 = 0; i0 < n_inst; i0 += 65535) {
+			const size_t o = (size_t)i0 * nch * h->nkr;
+			k_pcs_join<<<dim3((h->nkr + 31) / 32, (nch + 31) / 32, std::min(65535, n_inst - i0)), 256, 0, h->st>>>(h->P + o, nseg, (size_t)nvec * h->nkr,
+				h->cps, h->Q + o, h->nkr, d.n_l, d.m0, nch, h->nl);
+		}
+		QPC_CUDA(cudaMemcpyAsync(h->hstatus, h->status, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+	} else {
+		dim3 g1((n_inst + PG - 1) / PG, (h->nkr + 127) / 128, nch);
+		k_pcs_proj<<<g1, 128, 0, h->st>>>(h->ijlT, h->cps, c, h->Q, h->nkr, d.n_r, d.n_l, d.m0, nch, h->nl, n_inst);
+	}
 	QPC_CUDA(cudaGetLastError());
 	k_pcs_out<<<(unsigned)((total + 255) / 256), 256, 0, h->st>>>(kind, h->Q, h->plm, h->exm, h->kr, h->out, h->nkr, h->nkt, h->nkp,
 		d.n_l, d.n_m, total);
 	QPC_CUDA(cudaGetLastError());
 	QPC_CUDA(cudaEventRecord(h->ev1, h->st));
 	if (int rc = copy_to_host(out, h->out, sizeof(double2) * total, h->st)) return rc;
+	if (nseg && *h->hstatus) { set_error("a tensor-core wait ran out"); return QPC_ERR_TIMEOUT; }
 	QPC_CUDA(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
 	return QPC_OK;
+}
+
+// the projector's table on the device: digit planes where it suits them, or transposed for k_pcs_proj
+int pcs_table(qpc_pcs* h, const double* ijl)
+{
+	const qpc_dims& d = h->d;
+	const int n = d.n_r, nl = h->nl, nk = h->nkr, nch = d.n_m * d.n_l;
+	int rc;
+	scratch tmp(h->st);
+	double* raw;
+	if ((rc = tmp.get(&raw, (size_t)nk * nl * n))) return rc;
+	QPC_CUDA(cudaStreamSynchronize(h->st));
+	QPC_CUDA(cudaMemcpy(raw, ijl, sizeof(double) * (size_t)nk * nl * n, cudaMemcpyHostToDevice));
+	std::vector<int> lm(nch);
+	for (int c = 0; c < nch; ++c) lm[c] = std::abs(d.m0 + c / d.n_l) + c % d.n_l;
+	if ((rc = upload(&h->lmap, lm.data(), lm.size())) || (rc = dalloc(&h->ear, (size_t)nk * nl)) || (rc = dalloc(&h->status, 1))) return rc;
+	QPC_CUDA(cudaMallocHost(&h->hstatus, sizeof(int)));
+	k_pcs_rows<<<(unsigned)(((long)nk * nl + 7) / 8), 256, 0, h->st>>>(raw, h->ear, nk, nl, n);
+	QPC_CUDA(cudaGetLastError());
+	bool ok = nl <= 65535;
+	for (int k0 = 0; ok && k0 < n; k0 += TCK) {
+		h->seg.emplace_back();
+		if ((rc = tc_make(h->seg.back(), nullptr, raw, n, (long)nl * n, 1, nk, n, nl, -1, nullptr, 0, h->ear, h->st, &ok, k0, std::min(n, k0 + TCK)))) return rc;
+	}
+	if (ok) return QPC_OK;
+	for (tc_store& t : h->seg) t.release();
+	h->seg.clear();
+	if ((rc = dalloc(&h->ijlT, (size_t)nl * n * nk))) return rc;
+	k_pcs_transpose<<<dim3((n + 31) / 32, (nk + 31) / 32, std::min(nl, 65535)), 256, 0, h->st>>>(raw, h->ijlT, nk, nl, n);
+	QPC_CUDA(cudaGetLastError());
+	return wait_on(h->st);
 }
 
 // one accumulate, enqueued on st without a wait: the surface values come from c (host layout
@@ -439,12 +558,8 @@ int qpc_pcs_create(const qpc_dims* dims, const qpc_kgrid* g, const double* kr, c
 	auto fail = [&](int r) { pcs_free(h); return r; };
 	if (cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreate(&h->ev0) != cudaSuccess ||
 		cudaEventCreate(&h->ev1) != cudaSuccess) { set_error("stream or event creation failed"); return fail(QPC_ERR_CUDA); }
-	const int n = dims->n_r, nl = h->nl, nk = g->nkr, nch = dims->n_m * dims->n_l;
-	std::vector<double> t((size_t)nl * n * nk);
-	for (int k = 0; k < nk; ++k)
-		for (int l = 0; l < nl; ++l)
-			for (int r = 0; r < n; ++r) t[((size_t)l * n + r) * nk + k] = ijl[((size_t)k * nl + l) * n + r];
-	if ((rc = upload(&h->ijlT, t.data(), t.size()))) return fail(rc);
+	const int nl = h->nl, nk = g->nkr, nch = dims->n_m * dims->n_l;
+	if ((rc = pcs_table(h, ijl))) return fail(rc);
 	if ((rc = upload(&h->plm, plm, (size_t)g->nkt * nch))) return fail(rc);
 	if ((rc = upload(&h->kr, kr, (size_t)nk))) return fail(rc);
 	if ((rc = upload(&h->exm, (const double2*)exm, (size_t)g->nkp * dims->n_m))) return fail(rc);

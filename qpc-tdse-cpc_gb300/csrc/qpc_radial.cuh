@@ -36,6 +36,7 @@ struct band_args {
 struct tc_store {
 	bool cx = false;
 	int ea = 0;			// |A| <= 2^ea
+	const int* ear = nullptr;	// per operator and row instead, or NULL (not owned)
 	int db = 8;			// bits of a digit
 	int N = 0, ntile = 0;		// columns, 128-row tiles
 	int nrow = 0;

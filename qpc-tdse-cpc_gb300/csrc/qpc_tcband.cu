@@ -41,6 +41,7 @@ constexpr int NA = 6;			// operator planes in the ring
 constexpr int PLANE_A = TR * 128, PLANE_B = 2 * TCOLS * 128;
 constexpr int COLUMNS = 1024;	// bytes of barriers and column data, in front
 constexpr int B_MAX = 16 * PLANE_B, SMEM = COLUMNS + B_MAX + NA * PLANE_A + 1024;	// the last for alignment
+constexpr int DROP = 9;			// bits of an output's sum that are rounded off (the dropped pairs are worth 10)
 constexpr int SPLIT = 512, THREADS = 64 + SPLIT;
 
 // DB: bits of a digit.  x = sum_s d_s 2^(DB (ND - 1 - s)) with d_s in [-HALF, HALF) (the leading one up to HALF);
@@ -296,23 +297,23 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 #pragma unroll
 					for (int j = 0; j < 4; ++j) {
 						long long h = 0;
-						int m = 128;	// the last 8 bits are rounded off: the dropped pairs are worth 10
+						int m = 1 << (DROP - 1);
 #pragma unroll
 						for (int l = 0; l < ND; ++l) {
 							const int f = __float2int_rn(__uint_as_float(lv[l][j])), sh = DB * (ND - 1 - l);
-							if (sh >= 40) h += ((long long)f << 32) << (sh - 40);
-							else if (sh >= 8) h += (long long)f * (1ll << (sh - 8));
+							if (sh >= DROP + 32) h += ((long long)f << 32) << (sh - DROP - 32);
+							else if (sh >= DROP) h += (long long)f * (1ll << (sh - DROP));
 							else if (sh == 0) m += f;
-							else { h += f >> (8 - sh); m += (f & ((1 << (8 - sh)) - 1)) << sh; }
+							else { h += f >> (DROP - sh); m += (f & ((1 << (DROP - sh)) - 1)) << sh; }
 						}
-						sum[part][j] = h + (m >> 8);
+						sum[part][j] = h + (m >> DROP);
 					}
 				}
 #pragma unroll
 				for (int j = 0; j < 4; ++j) {
 					const int cl = c0 + j, cc = col0 + cl;
 					if (cc >= p.ncols || !sp[cl]) continue;
-					const int Ec = sE[cl], s = ea + Ec - (DB == 8 ? 1076 : 1075);
+					const int Ec = sE[cl], s = ea + Ec + DROP - (DB == 8 ? 1084 : 1083);
 					const double2 y = make_double2(int_double(sum[0][j], s, Ec == 0x7ff), int_double(sum[1][j], s, Ec == 0x7ff));
 					const long o = (long)(p.dmap ? p.dmap[cc] : cc) * p.nchan + ch;
 					if (in) p.dst[o * t.nrow + row] = y;
@@ -338,12 +339,13 @@ struct make_args {
 	long sop, si, sj;
 	int nrow, N, w, ea;
 	const int* ear;
+	int kb, ke;		// columns that take part; kb a multiple of KS
 };
 
 __device__ __forceinline__ double2 entry(const make_args& m, int op, int i, int j)
 {
 	double2 v = make_double2(0.0, 0.0);
-	if (i < m.nrow && j < m.N && (m.w < 0 || abs(i - j) <= m.w)) {
+	if (i < m.nrow && j < m.ke && (m.w < 0 || abs(i - j) <= m.w)) {
 		if (m.Fb) v = m.Fb[((long)op * m.N + i) * (2 * WMAX + 1) + (j - i + WMAX)];
 		else v.x = m.A[op * m.sop + i * m.si + j * m.sj];
 	}
@@ -363,8 +365,8 @@ __global__ void k_tc_planes(const make_args m, const int2* __restrict__ list, co
 	for (int q = threadIdx.x; q < TR * KS; q += blockDim.x) {
 		const int r = q / KS, k = q % KS;
 		const double2 v = entry(m, op, row0 + r, k0 + k);
-		const double sc = ldexp(1.0, 55 - ((m.ear && row0 + r < m.nrow) ? m.ear[(long)op * m.nrow + row0 + r] : m.ea));
-		const unsigned long long x = (unsigned long long)(__double2ll_rn(v.x * sc) + BIAS), y = (unsigned long long)(__double2ll_rn(v.y * sc) + BIAS);
+		const int sc = 55 - ((m.ear && row0 + r < m.nrow) ? m.ear[(long)op * m.nrow + row0 + r] : m.ea);
+		const unsigned long long x = (unsigned long long)(__double2ll_rn(ldexp(v.x, sc)) + BIAS), y = (unsigned long long)(__double2ll_rn(ldexp(v.y, sc)) + BIAS);
 		for (int s = s0; s < ND; ++s) {
 			const int plane = cx ? s - s0 : (s - s0) / 2, part = cx ? 0 : (s - s0) & 1;
 			const int b = plane * PLANE_A + r * 128 + (k & 7) * 2;
@@ -382,14 +384,15 @@ __global__ void k_tc_bound(const make_args m, int* __restrict__ worst)
 	constexpr int ND = digits<DB>::ND;
 	constexpr long long BIAS = digits<DB>::BIAS;
 	const int i = blockIdx.x, op = blockIdx.y;
-	const double sc = ldexp(1.0, 55 - (m.ear ? m.ear[(long)op * m.nrow + i] : m.ea));
+	const int sc = 55 - (m.ear ? m.ear[(long)op * m.nrow + i] : m.ea);
 	int sum = 0, lead = 0;
-	const int j0 = m.w < 0 ? 0 : max(0, i - m.w), j1 = m.w < 0 ? m.N : min(m.N, i + m.w + 1);
+	const int j0 = m.w < 0 ? m.kb : max(m.kb, i - m.w), j1 = m.w < 0 ? m.ke : min(m.ke, i + m.w + 1);
 	for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-		const double2 v = entry(m, op, i, j);
-		if (!(fabs(v.x) * sc <= 36028797018963968.0) || !(fabs(v.y) * sc <= 36028797018963968.0)) sum = lead = 1 << 28;	// 2^55
+		double2 v = entry(m, op, i, j);
+		v.x = ldexp(v.x, sc); v.y = ldexp(v.y, sc);
+		if (!(fabs(v.x) <= 36028797018963968.0) || !(fabs(v.y) <= 36028797018963968.0)) sum = lead = 1 << 28;	// 2^55
 		else {
-			const unsigned long long x = (unsigned long long)(__double2ll_rn(v.x * sc) + BIAS), y = (unsigned long long)(__double2ll_rn(v.y * sc) + BIAS);
+			const unsigned long long x = (unsigned long long)(__double2ll_rn(v.x) + BIAS), y = (unsigned long long)(__double2ll_rn(v.y) + BIAS);
 			lead += abs((int)__uint_as_float(digit_bits<DB>(x, 0))) + abs((int)__uint_as_float(digit_bits<DB>(y, 0)));
 			for (int s = 0; s < ND; ++s) sum += abs((int)__uint_as_float(digit_bits<DB>(x, s))) + abs((int)__uint_as_float(digit_bits<DB>(y, s)));
 		}
@@ -408,8 +411,8 @@ template <int DB>
 int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStream_t st, bool* ok)
 {
 	constexpr int ND = digits<DB>::ND;
-	const int nrow = m.nrow, N = m.N, w = m.w, ea = m.ea;
-	t.cx = m.Fb != nullptr; t.ea = ea; t.N = N; t.nrow = nrow; t.ntile = (nrow + TR - 1) / TR; t.db = DB;
+	const int nrow = m.nrow, w = m.w, ea = m.ea;
+	t.cx = m.Fb != nullptr; t.ea = ea; t.ear = m.ear; t.N = m.N; t.nrow = nrow; t.ntile = (nrow + TR - 1) / TR; t.db = DB;
 	int rc;
 	scratch tmp(st);
 	int* d_worst;
@@ -419,8 +422,8 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 	QPC_CUDA(cudaGetLastError());
 	int worst[2];
 	if ((rc = copy_to_host(worst, d_worst, sizeof(worst), st))) return rc;
-	// exact fp32 sums; and the sum of the levels, 2^(48 or 49) times the first one, less 8 bits, within 2^62
-	if (worst[0] > (1 << 24) / digits<DB>::HALF || worst[1] > (1 << 20) / digits<DB>::HALF) return QPC_OK;
+	// exact fp32 sums; and the first level, 2^(48 or 49 - DROP) of the sum, within 2^62
+	if (worst[0] > (1 << 24) / digits<DB>::HALF || worst[1] > (1 << (62 - DB * (ND - 1) + DROP)) / digits<DB>::HALF) return QPC_OK;
 	std::vector<int2> list;
 	std::vector<int4> first;
 	std::vector<int> tile_of;
@@ -430,7 +433,7 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 	for (int tl = 0; tl < t.ntile; ++tl) {
 		const int r0 = tl * TR, r1 = std::min(nrow, r0 + TR) - 1;
 		std::vector<int2> mine;
-		for (int k0 = 0; k0 < N; k0 += KS) {
+		for (int k0 = m.kb; k0 < m.ke; k0 += KS) {
 			const int k1 = k0 + KS - 1, gap = w < 0 ? 0 : std::max(0, std::max(k0 - r1, r0 - k1));
 			if (w >= 0 && gap > w) continue;
 			int s0 = 0;
@@ -479,10 +482,10 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 } // namespace
 
 int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, long sj, int nrow, int N, int nop, int w, const double* prof, int ea,
-	const int* ear, cudaStream_t st, bool* ok)
+	const int* ear, cudaStream_t st, bool* ok, int kb, int ke)
 {
 	*ok = false;
-	const make_args m{Fb, A, sop, si, sj, nrow, N, w, ea, ear};
+	const make_args m{Fb, A, sop, si, sj, nrow, N, w, ea, ear, kb, ke < 0 ? N : ke};
 	int rc = make<8>(t, m, nop, prof, st, ok);
 	if (!rc && !*ok) rc = make<7>(t, m, nop, prof, st, ok);
 	return rc;
@@ -490,7 +493,7 @@ int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, 
 
 void tc_apply(const tc_store& t, const band_args& a, int* status, int stbit, cudaStream_t st)
 {
-	const tc_args q{t.A, t.stride, t.d_list, t.d_first, t.d_off, t.nrow, t.ea, nullptr, status, stbit};
+	const tc_args q{t.A, t.stride, t.d_list, t.d_first, t.d_off, t.nrow, t.ea, t.ear, status, stbit};
 	const dim3 g((unsigned)(t.ntile * ((a.ncols + TCOLS - 1) / TCOLS)), (unsigned)a.nchan);
 	if (t.db == 8) {
 		if (t.cx) k_tc_apply<true, 8><<<g, THREADS, SMEM, st>>>(a, q);
