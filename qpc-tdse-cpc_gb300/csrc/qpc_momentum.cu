@@ -104,19 +104,6 @@ __global__ void __launch_bounds__(256) k_pcs_join(const double2* __restrict__ P,
 		if (kr0 + i < nkr) Q[(inst * nkr + kr0 + i) * nch + ch] = cmul(cps[(size_t)(kr0 + i) * nl_tot + l], t[tx][i]);
 }
 
-// |ijl[kr][l][.]| <= 2^ear[l][kr]
-__global__ void k_pcs_rows(const double* __restrict__ ijl, int* __restrict__ ear, int nkr, int nl, int n_r)
-{
-	const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
-	if (row >= nkr * nl) return;
-	const int l = row / nkr, k = row % nkr;
-	const double* a = ijl + ((size_t)k * nl + l) * n_r;
-	double v = 0.0;
-	for (int r = threadIdx.x & 31; r < n_r; r += 32) v = fmax(v, fabs(a[r]));
-	for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-	if ((threadIdx.x & 31) == 0) ear[row] = v > 0.0 && v < 1e300 ? ilogb(v) + 1 : 0;
-}
-
 // ijlT[l][r][kr] = ijl[kr][l][r]
 __global__ void __launch_bounds__(256) k_pcs_transpose(const double* __restrict__ ijl, double* __restrict__ ijlT, int nkr, int nl, int n_r)
 {
@@ -333,7 +320,7 @@ struct qpc_pcs {
 	double2 *cbuf = nullptr, *Q = nullptr, *out = nullptr, *P = nullptr;
 	long cap_c = 0, cap_q = 0, cap_o = 0, cap_p = 0, cap_x = 0;
 	std::vector<tc_store> seg;	// the table's digit planes, a segment of columns each (none: ijlT)
-	int *ear = nullptr, *lmap = nullptr, *ex = nullptr, *status = nullptr;
+	int *lmap = nullptr, *ex = nullptr, *status = nullptr;
 	int* hstatus = nullptr;		// pinned
 };
 
@@ -360,7 +347,7 @@ void pcs_free(qpc_pcs* h)
 {
 	if (!h) return;
 	cudaSetDevice(h->dev);
-	void* ps[] = {h->ijlT, h->plm, h->kr, h->exm, h->cps, h->cbuf, h->Q, h->out, h->P, h->ear, h->lmap, h->ex, h->status};
+	void* ps[] = {h->ijlT, h->plm, h->kr, h->exm, h->cps, h->cbuf, h->Q, h->out, h->P, h->lmap, h->ex, h->status};
 	for (tc_store& t : h->seg) t.release();
 	if (h->hstatus) cudaFreeHost(h->hstatus);
 	for (void* p : ps) if (p) cudaFree(p);
@@ -453,14 +440,12 @@ int pcs_table(qpc_pcs* h, const double* ijl)
 	QPC_CUDA(cudaMemcpy(raw, ijl, sizeof(double) * (size_t)nk * nl * n, cudaMemcpyHostToDevice));
 	std::vector<int> lm(nch);
 	for (int c = 0; c < nch; ++c) lm[c] = std::abs(d.m0 + c / d.n_l) + c % d.n_l;
-	if ((rc = upload(&h->lmap, lm.data(), lm.size())) || (rc = dalloc(&h->ear, (size_t)nk * nl)) || (rc = dalloc(&h->status, 1))) return rc;
+	if ((rc = upload(&h->lmap, lm.data(), lm.size())) || (rc = dalloc(&h->status, 1))) return rc;
 	QPC_CUDA(cudaMallocHost(&h->hstatus, sizeof(int)));
-	k_pcs_rows<<<(unsigned)(((long)nk * nl + 7) / 8), 256, 0, h->st>>>(raw, h->ear, nk, nl, n);
-	QPC_CUDA(cudaGetLastError());
 	bool ok = nl <= 65535;
 	for (int k0 = 0; ok && k0 < n; k0 += TCK) {
 		h->seg.emplace_back();
-		if ((rc = tc_make(h->seg.back(), nullptr, raw, n, (long)nl * n, 1, nk, n, nl, -1, nullptr, 0, h->ear, h->st, &ok, k0, std::min(n, k0 + TCK)))) return rc;
+		if ((rc = tc_make(h->seg.back(), nullptr, raw, n, (long)nl * n, 1, nk, n, nl, -1, nullptr, 0, true, h->st, &ok, k0, std::min(n, k0 + TCK)))) return rc;
 	}
 	if (ok) return QPC_OK;
 	for (tc_store& t : h->seg) t.release();

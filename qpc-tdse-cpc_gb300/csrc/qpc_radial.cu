@@ -795,8 +795,8 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 	p->F.tc_always = p->W.tc_always = p->X.tc_always = always;
 	const bool tcp = p->nff == 1 && (always || (in.batch >= TC_MIN && N >= 128 && !(mode && mode[0] == '0')));
 	if (tcp) {
-		if ((rc = tc_make(p->W.tc, nullptr, Yt, 0, N, 1, N, N, 1, p->W.w, p->W.prof.data(), p->W.ea, nullptr, st, &p->W.has_tc))) return rc;
-		if ((rc = tc_make(p->X.tc, nullptr, p->Xt, 0, 1, N, N, N, 1, p->X.w, p->X.prof.data(), p->X.ea, nullptr, st, &p->X.has_tc))) return rc;
+		if ((rc = tc_make(p->W.tc, nullptr, Yt, 0, N, 1, N, N, 1, p->W.w, p->W.prof.data(), p->W.ea, false, st, &p->W.has_tc))) return rc;
+		if ((rc = tc_make(p->X.tc, nullptr, p->Xt, 0, 1, N, N, N, 1, p->X.w, p->X.prof.data(), p->X.ea, false, st, &p->X.has_tc))) return rc;
 	}
 	// F~_l, a set of columns at a time: the engine's field-free solve on the eigenvectors, then X^T S
 	const int J = (int)std::min<long>(N, std::max<long>(32, (64l << 20) / ((long)N * nlh * 16)));
@@ -843,7 +843,7 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 			p->F.A + (size_t)fi * nlh * p->F.stride, p->F.stride);
 		if (tcp) {
 			const std::vector<double> pd = as_doubles(prof);
-			if ((rc = tc_make(p->F.tc, Fb, nullptr, 0, 0, 0, N, N, nlh, p->F.w, pd.data(), 0, nullptr, st, &p->F.has_tc))) return rc;
+			if ((rc = tc_make(p->F.tc, Fb, nullptr, 0, 0, 0, N, N, nlh, p->F.w, pd.data(), 0, false, st, &p->F.has_tc))) return rc;
 		}
 	}
 	if (p->nff > 1) {
@@ -909,10 +909,14 @@ int store_banded(radial_ops* p, band_store& b, const double* A, long si, long sj
 	return store_banded_impl(p, b, A, si, sj, st, false, ok);
 }
 
-int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st)
+int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, int ncols, cudaStream_t st)
 {
 	bool ok;
-	return store_banded_impl(p, b, A, si, sj, st, true, &ok);
+	if (int rc = store_banded_impl(p, b, A, si, sj, st, true, &ok)) return rc;
+	const char* mode = std::getenv("QPC_POS_TC");
+	b.tc_always = mode && mode[0] == '1';
+	if (ncols < TC_MIN || (mode && mode[0] == '0')) return QPC_OK;
+	return tc_make(b.tc, nullptr, A, 0, si, sj, p->N, p->N, 1, -1, nullptr, 0, true, st, &b.has_tc);
 }
 
 int project_band(const radial_ops* p, const double* B, bool anti, double* Bx, double* A, cudaStream_t st)

@@ -36,7 +36,7 @@ struct band_args {
 struct tc_store {
 	bool cx = false;
 	int ea = 0;			// |A| <= 2^ea
-	const int* ear = nullptr;	// per operator and row instead, or NULL (not owned)
+	int* ear = nullptr;		// per operator and row instead, or NULL
 	int db = 8;			// bits of a digit
 	int N = 0, ntile = 0;		// columns, 128-row tiles
 	int nrow = 0;
@@ -95,7 +95,8 @@ void radial_destroy(radial_ops* p);
 
 // A (device, FP64, element (i, j) at A[i si + j sj]) into b, banded where it falls off (ok), or dense
 int store_banded(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st, bool* ok);
-int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st);
+// an orthogonal matrix; ncols: most columns of a product
+int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, int ncols, cudaStream_t st);
 // A [N][N] = X^T B X for a symmetric band B, or for an anti-symmetric one given by its upper entries (device
 // [N][P+1]), zero beyond ~WMAX of the diagonal; Bx scratch [N][N]
 int project_band(const radial_ops* p, const double* B, bool anti, double* Bx, double* A, cudaStream_t st);

@@ -28,8 +28,8 @@ namespace qpc {
 
 void tc_store::release()
 {
-	cudaFree(d_list); cudaFree(d_first); cudaFree(d_off); cudaFree(A);
-	d_list = nullptr; d_first = nullptr; d_off = nullptr; A = nullptr;
+	cudaFree(d_list); cudaFree(d_first); cudaFree(d_off); cudaFree(A); cudaFree(ear);
+	d_list = nullptr; d_first = nullptr; d_off = nullptr; A = nullptr; ear = nullptr;
 }
 
 namespace {
@@ -407,12 +407,22 @@ __global__ void k_tc_bound(const make_args m, int* __restrict__ worst)
 	if (threadIdx.x < 2) { const int* q = part + 4 * threadIdx.x; atomicMax(worst + threadIdx.x, q[0] + q[1] + q[2] + q[3]); }
 }
 
+// |entry| <= 2^ear of each row
+__global__ void k_tc_rows(const make_args m, int* __restrict__ ear)
+{
+	const int i = blockIdx.x, op = blockIdx.y;
+	double v = 0.0;
+	for (int j = m.kb + threadIdx.x; j < m.ke; j += 32) { const double2 a = entry(m, op, i, j); v = fmax(v, fmax(fabs(a.x), fabs(a.y))); }
+	for (int o = 16; o; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+	if (threadIdx.x == 0) ear[(long)op * m.nrow + i] = v > 0.0 && v < 1e300 ? ilogb(v) + 1 : 0;
+}
+
 template <int DB>
 int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStream_t st, bool* ok)
 {
 	constexpr int ND = digits<DB>::ND;
 	const int nrow = m.nrow, w = m.w, ea = m.ea;
-	t.cx = m.Fb != nullptr; t.ea = ea; t.ear = m.ear; t.N = m.N; t.nrow = nrow; t.ntile = (nrow + TR - 1) / TR; t.db = DB;
+	t.cx = m.Fb != nullptr; t.ea = ea; t.N = m.N; t.nrow = nrow; t.ntile = (nrow + TR - 1) / TR; t.db = DB;
 	int rc;
 	scratch tmp(st);
 	int* d_worst;
@@ -482,11 +492,18 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 } // namespace
 
 int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, long sj, int nrow, int N, int nop, int w, const double* prof, int ea,
-	const int* ear, cudaStream_t st, bool* ok, int kb, int ke)
+	bool rows, cudaStream_t st, bool* ok, int kb, int ke)
 {
 	*ok = false;
-	const make_args m{Fb, A, sop, si, sj, nrow, N, w, ea, ear, kb, ke < 0 ? N : ke};
-	int rc = make<8>(t, m, nop, prof, st, ok);
+	make_args m{Fb, A, sop, si, sj, nrow, N, w, ea, nullptr, kb, ke < 0 ? N : ke};
+	int rc;
+	if (rows) {
+		if ((rc = dalloc(&t.ear, (size_t)nrow * nop))) return rc;
+		k_tc_rows<<<dim3(nrow, nop), 32, 0, st>>>(m, t.ear);
+		QPC_CUDA(cudaGetLastError());
+		m.ear = t.ear;
+	}
+	rc = make<8>(t, m, nop, prof, st, ok);
 	if (!rc && !*ok) rc = make<7>(t, m, nop, prof, st, ok);
 	return rc;
 }

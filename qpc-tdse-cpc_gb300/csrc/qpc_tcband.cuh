@@ -5,12 +5,12 @@
 namespace qpc {
 
 // From the band Fb [nop][N][2 WMAX + 1] (complex), or a real matrix A(i, j) = A[op * sop + i * si + j * sj] of nrow x N;
-// w: half-band, or -1 for a dense one; ear: exponents per operator and
-// row in place of ea (device, kept), or NULL; kb, ke: the columns that take part (kb a multiple of 32).
+// w: half-band, or -1 for a dense one; rows: each row under its own
+// largest exponent in place of ea; kb, ke: the columns that take part (kb a multiple of 32).
 // prof: largest |entry| per distance as in radial_create (NULL: every entry counts).  ok = false: an exact sum could
 // exceed 2^24, or the planes would take more than 4 GB.
 int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, long sj, int nrow, int N, int nop, int w, const double* prof, int ea,
-	const int* ear, cudaStream_t st, bool* ok, int kb = 0, int ke = -1);
+	bool rows, cudaStream_t st, bool* ok, int kb = 0, int ke = -1);
 
 // the product of band_args a with the planes t (a.A, a.td, a.toff unused); status: device word or-ed with stbit when a
 // wait ran out

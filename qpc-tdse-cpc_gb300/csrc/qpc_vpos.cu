@@ -5,14 +5,16 @@
 // anti-symmetric matrix, Q^T A Q = blocks omega [[0, -1], [1, 0]], and in the basis D = I Q the second is a rotation
 // of position pairs.  Radial transforms commute with the angular ones, so a step is a chain of
 //   k_couple: coupling of one component, then its merged angular transform (both local in position), and
-//   k_band_apply: the dense real Q or Q^T on every channel, or the banded F~_l in the basis I,
+//   k_band_apply: the dense real Q or Q^T on every channel (from ~200 columns on tensor cores, qpc_tcband.cu), or the
+//   banded F~_l in the basis I,
 // with no factorisation and no recurrence.  The pairing of the angular eigenvectors (u, +-v)/sqrt 2 folds into the
 // coupling: with a, b the two m-parity halves, M+- = c +- i s (phase) or c -+ s J (rotation),
 //   a' = c a + i s kappa b, b' = c b + i s conj(kappa) a   or   a' = c a - s kappa J b, b' = c b - s conj(kappa) J a,
 // kappa = conj(g_A) g_B.  Between two steps the closing and the opening x1 coupling (same field) are one of power 2.
 // All products in fixed point (qpc_radial.cu).  The banded solves cost the latency of eight recurrences over N rows
 // (4.85 us per row, whatever the batch, until ~10^4 chains fill the FP64 pipe); this form costs 8 N^2 products per
-// channel.  Measured on GB300 at 400 x (25 x 13), two wavefunctions: 22.6 -> 1.85 ms per step.
+// channel.  Measured on GB300 at 400 x (25 x 13), two wavefunctions: 22.6 -> 1.2 ms per step (1.85 with Q on the
+// multiply-adds: 136 -> 40 us each).
 #include "qpc_vpos.cuh"
 #include "qpc_radial.cuh"
 #include <cusolverDn.h>
@@ -193,6 +195,7 @@ struct vpos_path {
 	int* ex[2] = {nullptr, nullptr};
 	int* exin = nullptr;
 	size_t smem = 0;
+	int *status = nullptr, *hstatus = nullptr;	// a tensor-core wait ran out (device, pinned)
 	cudaStream_t stream = nullptr;
 };
 
@@ -234,7 +237,7 @@ int momentum_basis(vpos_path* p, const vpos_setup& in, bool* ok)
 	*ok = hinfo == 0;
 	if (!*ok) return QPC_OK;
 	if ((rc = orthonormalise(Qt, N, A, T, st, ok)) || !*ok) return rc;
-	if ((rc = store_dense(&p->ops, p->TD, Qt, N, 1, st)) || (rc = store_dense(&p->ops, p->TI, Qt, 1, N, st))) return rc;
+	if ((rc = store_dense(&p->ops, p->TD, Qt, N, 1, p->B * p->nch, st)) || (rc = store_dense(&p->ops, p->TI, Qt, 1, N, p->B * p->nch, st))) return rc;
 	return wait_on(st);
 }
 
@@ -283,7 +286,9 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	const long nvec = (long)p->B * nch;
 	for (int i = 0; i < 2; ++i)
 		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
-	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
+	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT)) || (rc = dalloc(&p->status, 1))) return rc;
+	QPC_CUDA(cudaMallocHost(&p->hstatus, sizeof(int)));
+	*p->hstatus = 0;
 	p->smem = sizeof(double2) * 32 * std::max(in.nb[0], in.nb[1]);
 	QPC_CUDA(cudaFuncSetAttribute(k_couple, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double2) * 32 * NBMAX)));
 	QPC_CUDA(cudaGetLastError());
@@ -321,7 +326,8 @@ void vpos_destroy(vpos_path* p)
 	if (!p) return;
 	cudaFree(p->om); cudaFree(p->rinv); cudaFree(p->tab); cudaFree(p->lmap);
 	for (int i = 0; i < 2; ++i) { cudaFree(p->buf[i]); cudaFree(p->ex[i]); }
-	cudaFree(p->exin);
+	cudaFree(p->exin); cudaFree(p->status);
+	if (p->hstatus) cudaFreeHost(p->hstatus);
 	p->TD.release(); p->TI.release();
 	radial_destroy(&p->ops);
 	delete p;
@@ -369,7 +375,7 @@ void radial(vpos_path* p, const vpos_run& r, int src, const band_store& b, int n
 	prof_scope ps(r, 0);
 	band_args a = band_args_of(&p->ops, b, 1, nlive * p->nch);
 	a.s0 = p->buf[src]; a.e0 = p->ex[src]; a.dst = p->buf[1 - src]; a.edst = p->ex[1 - src];
-	band_apply(a, false, p->ntile, p->stream);
+	band_apply(a, false, p->ntile, p->stream, &b, p->status, 1);
 	++*r.launches;
 }
 
@@ -391,6 +397,7 @@ void fieldfree(vpos_path* p, const vpos_run& r, int src, long s, int k0, int n)
 int vpos_begin(vpos_path* p, const vpos_run& r)
 {
 	prof_scope ps(r, 0);
+	if (p->TD.has_tc) QPC_CUDA(cudaMemsetAsync(p->status, 0, sizeof(int), p->stream));
 	exponents(r.X, p->exin, p->N, p->ntile, (long)p->B * p->nch, p->stream);
 	band_args a = band_args_of(&p->ops, p->ops.W, p->nch, p->B);
 	a.s0 = r.X; a.e0 = p->exin; a.dst = p->buf[0]; a.edst = p->ex[0];
@@ -448,7 +455,15 @@ int vpos_end(vpos_path* p, const vpos_run& r)
 	band_apply(a, false, p->ntile, p->stream);
 	++*r.launches;
 	QPC_CUDA(cudaGetLastError());
+	if (p->TD.has_tc) QPC_CUDA(cudaMemcpyAsync(p->hstatus, p->status, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
 	return QPC_OK;
+}
+
+int vpos_check(const vpos_path* p)
+{
+	if (*p->hstatus == 0) return QPC_OK;
+	set_error("a tensor-core wait ran out");
+	return QPC_ERR_TIMEOUT;
 }
 
 } // namespace qpc

@@ -43,5 +43,7 @@ int vpos_step(vpos_path* p, const vpos_run& r, long s, int nlive, int nff, bool 
 // the B-spline coefficients of the first n slots before step s (all of them in the l basis) into r.X
 int vpos_peek(vpos_path* p, const vpos_run& r, long s, int n);
 int vpos_end(vpos_path* p, const vpos_run& r);
+// after the stream has been waited for: an error if a wait in a kernel of the run ran out
+int vpos_check(const vpos_path* p);
 
 } // namespace qpc

@@ -55,3 +55,12 @@ def test_zero_and_not_finite(q, monkeypatch):
         prop.put(c0)
         prop.run(0.05 * np.ones((14, 5)), np.full(14, 4), np.full(14, 4))
     prop.close()
+
+
+@pytest.mark.parametrize("n_r,p,n_l,n_m,m0,B", [(64, 6, 4, 5, -2, 1), (129, 5, 3, 6, -3, 2), (160, 7, 5, 3, -1, 5), (97, 4, 2, 3, 1, 1)])
+def test_dense_transforms_agree(q, monkeypatch, n_r, p, n_l, n_m, m0, B):
+    """the velocity gauge's dense radial transforms: about 9 of them in each of 6 steps, so 1.2e-12"""
+    from test_gpu_vpos import _run as vrun
+    (a, _), (b, _) = _both(monkeypatch, lambda: vrun(q, n_r, p, n_l, n_m, m0, B))
+    for k in range(B):
+        assert rel_l2(b[k], a[k]) < 1.2e-12, k
