@@ -61,11 +61,22 @@ inline int2 limbs_of(double v)
 	return make_int2(hi, (int)(x - ((long long)hi << 28)));
 }
 
-// outputs o0 .. o0+G-1 of a real matrix (element (o, k) at V[o * so + k * sk]) times the column in x[k * xk]; the
-// mixed sums hold 64 k (128 products below 2^55): LONG carries them into the high ones that often
-template <int G, bool LONG = false>
-__device__ __forceinline__ void local_product(const int2* __restrict__ V, int so, int sk, int nk, int no, const int4* __restrict__ x, int xk,
-	long long (&h)[G][2], long long (&m)[G][2])
+// 1 / x, x >= 1: two Newton steps from the fp32 approximation (relative error 2^-23 -> 2^-46 -> rounding)
+__device__ __forceinline__ double reciprocal(double x)
+{
+	if (!(x < 1e30)) return 1.0 / x;
+	float r0;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(__int_as_float(((__double2hiint(x) - 0x38000000) << 3) | (int)((unsigned)__double2loint(x) >> 29))));
+	const int b = __float_as_int(r0);
+	double r = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+	r = fma(r, fma(-x, r, 1.0), r);
+	return fma(r, fma(-x, r, 1.0), r);
+}
+
+// G outputs of a real matrix, A = [k][G] limbs, times the column at x[k * XK]; the mixed sums hold 64 k (128 products
+// below 2^55): LONG carries them into the high ones that often
+template <int G, int XK, bool LONG>
+__device__ __forceinline__ void task_product(const int2* __restrict__ A, int nk, const int4* __restrict__ x, long long (&h)[G][2], long long (&m)[G][2])
 {
 #pragma unroll
 	for (int g = 0; g < G; ++g) h[g][0] = h[g][1] = m[g][0] = m[g][1] = 0;
@@ -73,10 +84,10 @@ __device__ __forceinline__ void local_product(const int2* __restrict__ V, int so
 		const int k1 = LONG ? min(nk, k0 + 64) : nk;
 #pragma unroll 4
 		for (int k = k0; k < k1; ++k) {
-			const int4 y = x[k * xk];
+			const int4 y = x[k * XK];
 #pragma unroll
 			for (int g = 0; g < G; ++g) {
-				const int2 a = __ldg(V + (g < no ? g : 0) * so + k * sk);
+				const int2 a = __ldg(A + k * G + g);
 				h[g][0] = madw(a.x, y.x, h[g][0]); h[g][1] = madw(a.x, y.z, h[g][1]);
 				m[g][0] = madw(a.x, y.y, m[g][0]); m[g][0] = madw(a.y, y.x, m[g][0]);
 				m[g][1] = madw(a.x, y.w, m[g][1]); m[g][1] = madw(a.y, y.z, m[g][1]);

@@ -63,39 +63,6 @@ __device__ __forceinline__ int power_of(long s, long nt, int cmode)
 	return (s == 0 || s == nt) ? 1 : 2;
 }
 
-// 1 / x, x >= 1: two Newton steps from the fp32 approximation (relative error 2^-23 -> 2^-46 -> rounding)
-__device__ __forceinline__ double reciprocal(double x)
-{
-	if (!(x < 1e30)) return 1.0 / x;
-	float r0;
-	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(__int_as_float(((__double2hiint(x) - 0x38000000) << 3) | (int)((unsigned)__double2loint(x) >> 29))));
-	const int b = __float_as_int(r0);
-	double r = __hiloint2double((b >> 3) + 0x38000000, b << 29);
-	r = fma(r, fma(-x, r, 1.0), r);
-	return fma(r, fma(-x, r, 1.0), r);
-}
-
-// G outputs of a real matrix, A = [k][G] limbs, times the column at x[k * XK]
-template <int G, int XK>
-__device__ __forceinline__ void task_product(const int2* __restrict__ A, int nk, const int4* __restrict__ x, long long (&h)[G][2], long long (&m)[G][2])
-{
-#pragma unroll
-	for (int g = 0; g < G; ++g) h[g][0] = h[g][1] = m[g][0] = m[g][1] = 0;
-#pragma unroll 4
-	for (int k = 0; k < nk; ++k) {
-		const int4 y = x[k * XK];
-#pragma unroll
-		for (int g = 0; g < G; ++g) {
-			const int2 a = __ldg(A + k * G + g);
-			h[g][0] = madw(a.x, y.x, h[g][0]); h[g][1] = madw(a.x, y.z, h[g][1]);
-			m[g][0] = madw(a.x, y.y, m[g][0]); m[g][0] = madw(a.y, y.x, m[g][0]);
-			m[g][1] = madw(a.x, y.w, m[g][1]); m[g][1] = madw(a.y, y.z, m[g][1]);
-		}
-	}
-#pragma unroll
-	for (int g = 0; g < G; ++g) { flush(h[g][0], m[g][0]); flush(h[g][1], m[g][1]); }
-}
-
 template <int G, int PT>
 __global__ void __launch_bounds__(256, 3) k_angle(const angle_args p)
 {
@@ -141,7 +108,7 @@ __global__ void __launch_bounds__(256, 3) k_angle(const angle_args p)
 	for (int t = warp; t < gE + gO; t += NV) {
 		const bool odd = t >= gE;
 		const int k0 = (odd ? t - gE : t) * G, no = min(G, (odd ? np : nE) - k0);
-		task_product<G, 2 * PT>(V + t * G * nl0, odd ? nl1 : nl0, qa + (odd ? PT : 0), h, mm);
+		task_product<G, 2 * PT, false>(V + t * G * nl0, odd ? nl1 : nl0, qa + (odd ? PT : 0), h, mm);
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
@@ -207,7 +174,7 @@ __global__ void __launch_bounds__(256, 3) k_angle(const angle_args p)
 		const int odd = t >= g0 ? 1 : 0;
 		const int o0 = (odd ? t - g0 : t) * G, no = min(G, (odd ? nl1 : nl0) - o0);
 		// even l: s_k (slots 2k) and, for odd n_l, the zero channel (slot 2 npair); odd l: d_k (slots 2k + 1)
-		task_product<G, 2 * PT>(V + t * G * nE, odd ? np : nE, qa + odd * PT, h, mm);
+		task_product<G, 2 * PT, false>(V + t * G * nE, odd ? np : nE, qa + odd * PT, h, mm);
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {

@@ -25,13 +25,15 @@ namespace qpc {
 
 namespace {
 
+constexpr int AG = 3;		// outputs per task of k_couple
+constexpr int CW = 16;		// its warps
 constexpr int NBMAX = 452;	// most channels of a parity block (its 32-position tile sits in shared memory)
 
 struct set_args {
 	const double2* in;	// [slot][nch][N]
 	double2* out;
 	int* eout;		// [slot][nch][ntile * EPT]
-	const int2* A[2][2];	// real matrices of the angular transform, [block][set], limbs
+	const int2* A[2][2];	// real matrices of the angular transform, [block][set], limbs as [task][k][AG]
 	int off[2], na[2], ns[2];
 	int kind;		// 0: no coupling, 1: phase, 2: rotation of position pairs
 	int power;
@@ -47,32 +49,35 @@ struct set_args {
 };
 
 // One block: TM positions of one parity block of one slot, an interleaved share of the outputs; lane = position.
-// Bound by the integer multiply-adds of the two real products (6 n per output).
-__global__ void __launch_bounds__(256) k_couple(const set_args p)
+// Bound by the integer multiply-adds of the two real products (6 n per output) and the FP64 of the coupling (35 per pair
+// and position, in every share): 16 warps, two blocks per SM, shares to give every SM a block once.  400 x 325 channels,
+// two wavefunctions 96 -> 76 us, 800 x 861 channels 440 -> 275 us (8 warps, an IEEE division per phase, row-major
+// coefficients before).
+__global__ void __launch_bounds__(CW * 32, 2) k_couple(const set_args p)
 {
 	extern __shared__ double2 sm[];
-	__shared__ unsigned short pe[2][8][32];
-	constexpr int G = 4;
+	__shared__ int pe[2][32];
+	constexpr int G = AG;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int tile = blockIdx.x, blk = blockIdx.y & 1, slot = blockIdx.y >> 1, slice = blockIdx.z;
 	const int na = p.na[blk], ns = p.ns[blk], n = na + ns, N = p.N;
 	const int row = tile * TM + lane;
 	const bool in = row < N;
 	const long base = ((long)slot * p.nch + p.off[blk]) * N + row;
-	for (int q = warp; q < n; q += 8) sm[q * 32 + lane] = in ? p.in[base + (long)q * N] : make_double2(0.0, 0.0);
+	if (warp < 2) pe[warp][lane] = 0;
+	for (int q = warp; q < n; q += CW) sm[q * 32 + lane] = in ? p.in[base + (long)q * N] : make_double2(0.0, 0.0);
 	__syncthreads();
 	if (p.kind) {
 		const double f = p.atab[((long)p.perm[slot] * p.ld + p.at) * 2 + p.axis] * p.scale * (in ? p.rad[row] : 0.0);
 		const double2 kp = p.kap[blk];
-		for (int k = warp; k < ns; k += 8) {
+		for (int k = warp; k < ns; k += CW) {
 			const double2 a = sm[k * 32 + lane], b = sm[(na + k) * 32 + lane];
 			const double x = p.sig[p.off[blk] + k] * f;
-			const double inv = 1.0 / fma(x, x, 1.0);
-			double c = fma(-x, x, 1.0) * inv, s = -2.0 * x * inv;
+			double s = -2.0 * x * reciprocal(fma(x, x, 1.0)), c = fma(s, x, 1.0);
 			if (p.power == 2) {
-				const double c1 = c;
-				c = fma(-2.0 * s, s, 1.0);
-				s = 2.0 * s * c1;
+				const double s1 = 2.0 * s;
+				s = s1 * c;
+				c = fma(-0.5 * s1, s1, 1.0);
 			}
 			double2 u = b, v = a, g;	// a' = c a + s g u, b' = c b + s h v with g = i kappa, h = i conj(kappa), or kappa
 			double2 h;
@@ -93,18 +98,17 @@ __global__ void __launch_bounds__(256) k_couple(const set_args p)
 		__syncthreads();
 	}
 	int e0 = 0, e1 = 0;
-	for (int q = warp; q < n; q += 8) {
+	for (int q = warp; q < n; q += CW) {
 		const double2 v = sm[q * 32 + lane];
 		const int e = max(bexp(v.x), bexp(v.y));
 		if (q < na) e0 = max(e0, e); else e1 = max(e1, e);
 	}
-	pe[0][warp][lane] = (unsigned short)e0;
-	pe[1][warp][lane] = (unsigned short)e1;
+	atomicMax(&pe[0][lane], e0);
+	atomicMax(&pe[1][lane], e1);
 	__syncthreads();
-	e0 = e1 = 0;
-#pragma unroll
-	for (int w = 0; w < 8; ++w) { e0 = max(e0, (int)pe[0][w][lane]); e1 = max(e1, (int)pe[1][w][lane]); }
-	for (int q = warp; q < n; q += 8) {
+	e0 = pe[0][lane];
+	e1 = pe[1][lane];
+	for (int q = warp; q < n; q += CW) {
 		const double2 v = sm[q * 32 + lane];
 		const int e = q < na ? e0 : e1;
 		const int2 x = quant(v.x, e), y = quant(v.y, e);
@@ -114,10 +118,10 @@ __global__ void __launch_bounds__(256) k_couple(const set_args p)
 	const int4* qs = reinterpret_cast<const int4*>(sm) + lane;
 	const int ga = (na + G - 1) / G, gb = (ns + G - 1) / G;
 	long long h[G][2], m[G][2];
-	for (int t = warp + 8 * slice; t < ga + gb; t += 8 * p.slices) {
+	for (int t = warp + CW * slice; t < ga + gb; t += CW * p.slices) {
 		const int set = t >= ga ? 1 : 0;
 		const int o0 = (set ? t - ga : t) * G, nn = set ? ns : na, no = min(G, nn - o0);
-		local_product<G, true>(p.A[blk][set] + (long)o0 * nn, nn, 1, nn, no, qs + (set ? na : 0) * 32, 32, h, m);
+		task_product<G, 32, true>(p.A[blk][set] + (long)o0 * nn, nn, qs + (set ? na : 0) * 32, h, m);
 		const int e = set ? e1 : e0;
 #pragma unroll
 		for (int g = 0; g < G; ++g)
@@ -160,7 +164,7 @@ __global__ void k_pairs(const cuDoubleComplex* __restrict__ U, const double* __r
 	}
 }
 
-// limbs of op(A), row-major n x n
+// limbs of op(A), row-major n x n, as [task][k][AG]
 __global__ void k_limbs(const double* __restrict__ A, int n, int trans, int2* __restrict__ out)
 {
 	const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -168,7 +172,7 @@ __global__ void k_limbs(const double* __restrict__ A, int n, int trans, int2* __
 	const long i = t / n, k = t % n;
 	const long long x = __double2ll_rn((trans ? A[k * n + i] : A[t]) * 72057594037927936.0);
 	const int hi = (int)((x + (1ll << 27)) >> 28);
-	out[t] = make_int2(hi, (int)(x - ((long long)hi << 28)));
+	out[(i / AG * n + k) * AG + i % AG] = make_int2(hi, (int)(x - ((long long)hi << 28)));
 }
 
 __global__ void k_negate(const double* __restrict__ a, double* __restrict__ b, int n)
@@ -259,8 +263,10 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	if ((rc = momentum_basis(p, in, ok)) || !*ok) return rc;
 	// angular tables
 	size_t tot = 0;
-	for (int b = 0; b < 2; ++b) tot += (size_t)p->na[b] * p->na[b] + (size_t)p->ns[b] * p->ns[b];
+	auto room = [](int n) { return (size_t)((n + AG - 1) / AG) * AG * n; };	// a task's outputs beyond the last are zero
+	for (int b = 0; b < 2; ++b) tot += room(p->na[b]) + room(p->ns[b]);
 	if ((rc = dalloc(&p->tab, tot * 10))) return rc;
+	QPC_CUDA(cudaMemsetAsync(p->tab, 0, sizeof(int2) * tot * 10, st));
 	size_t o = 0;
 	for (int m = 0; m < 5; ++m)
 		for (int b = 0; b < 2; ++b)
@@ -269,7 +275,7 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 				for (int t = 0; t < 2; ++t) {
 					p->A[m][b][s][t] = p->tab + o;
 					if (n) k_limbs<<<(unsigned)(((long)n * n + 255) / 256), 256, 0, st>>>(in.tm[m][b][s], n, t, p->tab + o);
-					o += (size_t)n * n;
+					o += room(n);
 				}
 			}
 	for (int c = 0; c < 4; ++c) {
@@ -364,8 +370,8 @@ void couple(vpos_path* p, const vpos_run& r, int src, int c, long at, int power,
 	}
 	a.perm = r.perm;
 	a.N = p->N; a.ntile = p->ntile; a.nch = p->nch;
-	a.slices = std::max(1, std::min(4, 304 / std::max(1, 2 * nlive * p->ntile)));
-	k_couple<<<dim3(p->ntile, 2 * nlive, a.slices), 256, p->smem, p->stream>>>(a);
+	a.slices = std::max(1, std::min(4, 152 / std::max(1, 2 * nlive * p->ntile)));
+	k_couple<<<dim3(p->ntile, 2 * nlive, a.slices), CW * 32, p->smem, p->stream>>>(a);
 	++*r.launches;
 }
 
