@@ -25,20 +25,45 @@
 namespace qpc {
 namespace {
 
-constexpr int MT = 64;          // block tile (rows and columns)
-constexpr int MLP_THREADS = 128; // 4 warps, 2 x 2 warp tiles of 32 x 32
+constexpr int MT = 64;           // block tile (rows and columns)
+constexpr int KT = 64;           // k of a stage
+constexpr int NSTG = 4;          // stages in flight
+constexpr int PITCH = KT + 8;    // of a staged row: ldmatrix without bank conflicts
+constexpr int MLP_THREADS = 256; // 8 warps, 2 x 4 warp tiles of 32 x 16
+constexpr int MLP_SMEM = NSTG * 2 * MT * PITCH * (int)sizeof(__nv_bfloat16);
 
-enum { EPI_STORE = 0, EPI_HIDDEN = 1, EPI_BACK = 2 };
+// what becomes of a product v (bias added)
+enum {
+	EPI_STORE = 0,   // out = v
+	EPI_HIDDEN = 1,  // out = v, outb/outt = gelu(v)
+	EPI_BACK = 2,    // outb/outt = v gelu'(aux), cs = sums over the tile's rows
+	EPI_LOSS = 3     // d = v - aux on valid rows: outb/outt = 2 d scale, cs as above, part = the tile's sum of d^2
+};
 
 struct gemm_args {
 	const __nv_bfloat16* A; long sA;  // [M][K] per member, member stride
 	const __nv_bfloat16* B; long sB;  // [N][K]
-	int M, N, K;
+	int M, N, K, epi;
 	const float* bias; long sbias;    // [N] or null
-	const float* aux; long saux;      // EPI_BACK: pre-activation Z [M][N]
+	const float* aux; long saux;      // EPI_BACK: pre-activation Z [M][N]; EPI_LOSS: targets
 	float* out; long sout;            // fp32 [M][N]
-	__nv_bfloat16* outb; long soutb;  // bf16 [M][N] (EPI_HIDDEN/EPI_BACK)
+	__nv_bfloat16* outb; long soutb;  // bf16 [M][N]
 	__nv_bfloat16* outt; long soutt;  // bf16 [N][M]
+	float* cs; long scs;              // [ceil(M / MT)][N]
+	const int* idx;                   // [E][M]: rows < 0 do not count
+	float scale;
+	float* part;                      // [E][tiles]
+	__host__ __device__ int tiles() const { return ((M + MT - 1) / MT) * ((N + MT - 1) / MT); }
+};
+
+// the last stage of a reduction, a block of a backward launch: gb[n] = sum over the row tiles, in order; and the loss
+struct sum_args {
+	const float* cs; long scs;
+	int nt, N;
+	float* gb; long sgb;
+	const float* part; int npart;     // null: no loss
+	float scale;
+	float* loss;
 };
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
@@ -47,82 +72,178 @@ __device__ __forceinline__ float gelu_grad(float z)
 	return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-__device__ __forceinline__ uint32_t ld_pair(const __nv_bfloat16* base, int row, int col, int nrow, int ld)
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t a)
 {
-	if (row >= nrow) return 0u;
-	return *reinterpret_cast<const uint32_t*>(base + (long)row * ld + col);
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(MLP_THREADS) k_mlp_gemm(gemm_args a)
+// rows row0.. of X [nrow][K] into a stage, zero beyond the rows and beyond K (a multiple of 8)
+__device__ __forceinline__ void stage_rows(__nv_bfloat16* to, const __nv_bfloat16* X, int row0, int nrow, int K, int k0)
 {
-	const int e = blockIdx.z;
+#pragma unroll
+	for (int i = 0; i < MT * KT / 8 / MLP_THREADS; ++i) {
+		const int q = threadIdx.x + i * MLP_THREADS, r = q / (KT / 8), k = q % (KT / 8) * 8;
+		const bool in = row0 + r < nrow && k0 + k < K;
+		const __nv_bfloat16* src = in ? X + (long)(row0 + r) * K + k0 + k : X;
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_at(to + r * PITCH + k)), "l"(src), "r"(in ? 16 : 0) : "memory");
+	}
+}
+
+// One 64 x 64 tile.  The products of the surrogate (256 x 256 x 256 per member) are bound by latency, not by the tensor
+// cores: the whole K = 256 is in flight at once (16 dependent rounds of loads from global memory took 12-24 us a product,
+// now 7).  Sums over rows leave as partial sums of the tile, the transposed copies through shared memory.  A gradient of
+// five members on 256 rows: 26 launches and 1.00 ms before, 11 and 0.31 ms now, mostly the copies to and from the host.
+__device__ void gemm_tile(const gemm_args& a, int tile, int e, __nv_bfloat16* sm)
+{
+	const int nbx = (a.N + MT - 1) / MT, m0 = tile / nbx * MT, n0 = tile % nbx * MT;
 	const __nv_bfloat16* A = a.A + e * a.sA;
 	const __nv_bfloat16* B = a.B + e * a.sB;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int gid = lane >> 2, tig = lane & 3;
-	const int m0 = blockIdx.y * MT + (warp >> 1) * 32;
-	const int n0 = blockIdx.x * MT + (warp & 1) * 32;
-	float acc[2][4][4];
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+	const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+	const int nk = (a.K + KT - 1) / KT;
+	auto stage = [&](int t) {
+		if (t < nk) {
+			__nv_bfloat16* to = sm + (t % NSTG) * 2 * MT * PITCH;
+			stage_rows(to, A, m0, a.M, a.K, t * KT);
+			stage_rows(to + MT * PITCH, B, n0, a.N, a.K, t * KT);
+		}
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
+	for (int t = 0; t < NSTG; ++t) stage(t);
+	float acc[2][2][4];
 #pragma unroll
 	for (int i = 0; i < 2; ++i)
 #pragma unroll
-		for (int j = 0; j < 4; ++j)
+		for (int j = 0; j < 2; ++j)
 #pragma unroll
 			for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.f;
-	for (int k0 = 0; k0 < a.K; k0 += 16) {
-		uint32_t af[2][4], bf[4][2];
+	for (int t = 0; t < nk; ++t) {
+		asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTG - 1) : "memory");
+		__syncthreads();
+		const __nv_bfloat16* As = sm + (t % NSTG) * 2 * MT * PITCH;
+		const uint32_t aa = smem_at(As + (wm + (lane & 15)) * PITCH + (lane >> 4) * 8);
+		const uint32_t ba = smem_at(As + (MT + wn + (lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 8);
 #pragma unroll
-		for (int i = 0; i < 2; ++i) {
-			int r = m0 + i * 16 + gid;
-			af[i][0] = ld_pair(A, r, k0 + tig * 2, a.M, a.K);
-			af[i][1] = ld_pair(A, r + 8, k0 + tig * 2, a.M, a.K);
-			af[i][2] = ld_pair(A, r, k0 + tig * 2 + 8, a.M, a.K);
-			af[i][3] = ld_pair(A, r + 8, k0 + tig * 2 + 8, a.M, a.K);
-		}
+		for (int k = 0; k < KT; k += 16) {
+			uint32_t af[2][4], bf[4];
+			ldmatrix4(af[0], aa + k * 2);
+			ldmatrix4(af[1], aa + (16 * PITCH + k) * 2);
+			ldmatrix4(bf, ba + k * 2);
 #pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			int c = n0 + j * 8 + gid;
-			bf[j][0] = ld_pair(B, c, k0 + tig * 2, a.N, a.K);
-			bf[j][1] = ld_pair(B, c, k0 + tig * 2 + 8, a.N, a.K);
+			for (int i = 0; i < 2; ++i)
+#pragma unroll
+				for (int j = 0; j < 2; ++j)
+					asm volatile(
+						"mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+						: "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
+						: "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bf[2 * j]), "r"(bf[2 * j + 1]));
 		}
+		__syncthreads();
+		stage(t + NSTG);
+	}
+	// acc[i][j][c] is C(row, col) with row = m0 + wm + 16 i + gid + 8 (c >> 1), col = n0 + wn + 8 j + 2 tig + (c & 1);
+	// N is a multiple of 8: a pair of columns is inside or outside
+	asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+	__nv_bfloat16* T = sm;	// [64][PITCH], bf16 results
+	float* cs = reinterpret_cast<float*>(sm + MT * PITCH);	// [2][64] column sums, then 8 sums of squares
+	float sq = 0.f;
+#pragma unroll
+	for (int j = 0; j < 2; ++j) {
+		const int lc = wn + 8 * j + 2 * tig, col = n0 + lc;
+		float s0 = 0.f, s1 = 0.f;
 #pragma unroll
 		for (int i = 0; i < 2; ++i)
 #pragma unroll
-			for (int j = 0; j < 4; ++j)
-				asm volatile(
-					"mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-					: "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
-					: "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bf[j][0]), "r"(bf[j][1]));
-	}
-	// epilogue: acc[i][j][c] is C(row, col) with row = m0+16i+gid+8(c>>1), col = n0+8j+2tig+(c&1)
-#pragma unroll
-	for (int i = 0; i < 2; ++i)
-#pragma unroll
-		for (int j = 0; j < 4; ++j)
-#pragma unroll
-			for (int c = 0; c < 4; ++c) {
-				int row = m0 + i * 16 + gid + 8 * (c >> 1);
-				int col = n0 + j * 8 + tig * 2 + (c & 1);
+			for (int c = 0; c < 4; c += 2) {
+				const int lr = wm + 16 * i + gid + 4 * c, row = m0 + lr;
 				if (row >= a.M || col >= a.N) continue;
-				float v = acc[i][j][c];
-				long o = (long)row * a.N + col;
-				if (a.bias) v += a.bias[e * a.sbias + col];
-				if (EPI == EPI_STORE) {
-					a.out[e * a.sout + o] = v;
-				} else if (EPI == EPI_HIDDEN) {
-					a.out[e * a.sout + o] = v;
-					__nv_bfloat16 h = __float2bfloat16_rn(gelu(v));
-					a.outb[e * a.soutb + o] = h;
-					a.outt[e * a.soutt + (long)col * a.M + row] = h;
-				} else {
-					float d = v * gelu_grad(a.aux[e * a.saux + o]);
-					a.out[e * a.sout + o] = d;
-					__nv_bfloat16 hb = __float2bfloat16_rn(d);
-					a.outb[e * a.soutb + o] = hb;
-					a.outt[e * a.soutt + (long)col * a.M + row] = hb;
+				float v0 = acc[i][j][c], v1 = acc[i][j][c + 1];
+				const long o = (long)row * a.N + col;
+				if (a.bias) { v0 += a.bias[e * a.sbias + col]; v1 += a.bias[e * a.sbias + col + 1]; }
+				if (a.epi <= EPI_HIDDEN) *reinterpret_cast<float2*>(a.out + e * a.sout + o) = make_float2(v0, v1);
+				if (a.epi == EPI_HIDDEN) { v0 = gelu(v0); v1 = gelu(v1); }
+				if (a.epi >= EPI_BACK) {
+					const float2 x = *reinterpret_cast<const float2*>(a.aux + e * a.saux + o);
+					if (a.epi == EPI_BACK) { v0 *= gelu_grad(x.x); v1 *= gelu_grad(x.y); }
+					else {
+						const bool valid = a.idx[(long)e * a.M + row] >= 0;
+						v0 = valid ? v0 - x.x : 0.f;
+						v1 = valid ? v1 - x.y : 0.f;
+						sq += v0 * v0 + v1 * v1;
+						v0 = 2.f * v0 * a.scale;
+						v1 = 2.f * v1 * a.scale;
+					}
+					s0 += v0;
+					s1 += v1;
 				}
+				if (a.epi) *reinterpret_cast<__nv_bfloat162*>(T + lr * PITCH + lc) = __floats2bfloat162_rn(v0, v1);
 			}
+		if (a.epi >= EPI_BACK) {
+#pragma unroll
+			for (int o = 4; o < 32; o <<= 1) { s0 += __shfl_xor_sync(0xffffffffu, s0, o); s1 += __shfl_xor_sync(0xffffffffu, s1, o); }
+			if (gid == 0) { cs[(warp >> 2) * 64 + lc] = s0; cs[(warp >> 2) * 64 + lc + 1] = s1; }
+		}
+	}
+	if (a.epi == EPI_STORE) return;
+	if (a.epi == EPI_LOSS) {
+#pragma unroll
+		for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+		if (lane == 0) cs[128 + warp] = sq;
+	}
+	__syncthreads();
+	for (int q = threadIdx.x; q < MT * MT / 8; q += MLP_THREADS) {
+		const int r = q / (MT / 8), x = q % (MT / 8) * 8;
+		if (m0 + r < a.M && n0 + x < a.N)
+			*reinterpret_cast<uint4*>(a.outb + e * a.soutb + (long)(m0 + r) * a.N + n0 + x) = *reinterpret_cast<const uint4*>(T + r * PITCH + x);
+		// transposed: column r of the tile, rows x .. x + 7 (M is a multiple of 64)
+		if (n0 + r < a.N) {
+			uint32_t w[4];
+#pragma unroll
+			for (int i = 0; i < 4; ++i) {
+				const uint16_t lo = *reinterpret_cast<const uint16_t*>(T + (x + 2 * i) * PITCH + r), hi = *reinterpret_cast<const uint16_t*>(T + (x + 2 * i + 1) * PITCH + r);
+				w[i] = lo | (uint32_t)hi << 16;
+			}
+			*reinterpret_cast<uint4*>(a.outt + e * a.soutt + (long)(n0 + r) * a.M + m0 + x) = make_uint4(w[0], w[1], w[2], w[3]);
+		}
+	}
+	if (a.epi >= EPI_BACK && threadIdx.x < MT && n0 + threadIdx.x < a.N)
+		a.cs[e * a.scs + (long)(m0 / MT) * a.N + n0 + threadIdx.x] = cs[threadIdx.x] + cs[64 + threadIdx.x];
+	if (a.epi == EPI_LOSS && threadIdx.x == 0) {
+		float t = 0.f;
+		for (int w = 0; w < MLP_THREADS / 32; ++w) t += cs[128 + w];
+		a.part[(long)e * a.tiles() + tile] = t;
+	}
+}
+
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_gemm(const gemm_args a)
+{
+	extern __shared__ __align__(16) __nv_bfloat16 mlp_sm[];
+	gemm_tile(a, blockIdx.x, blockIdx.z, mlp_sm);
+}
+
+// one layer backwards: the tiles of the weight gradient, those of the input gradient (na of them, 0 for the first layer),
+// and the bias gradient (with the loss), none of which waits for another
+__global__ void __launch_bounds__(MLP_THREADS) k_mlp_back(const gemm_args w, const gemm_args a, const sum_args s, int nw, int na)
+{
+	extern __shared__ __align__(16) __nv_bfloat16 mlp_sm[];
+	const int e = blockIdx.z, t = blockIdx.x;
+	if (t < nw) gemm_tile(w, t, e, mlp_sm);
+	else if (t < nw + na) gemm_tile(a, t - nw, e, mlp_sm);
+	else {
+		const int n = (t - nw - na) * MLP_THREADS + threadIdx.x;
+		if (n < s.N) {
+			float v = 0.f;
+			for (int i = 0; i < s.nt; ++i) v += s.cs[e * s.scs + (long)i * s.N + n];
+			s.gb[e * s.sgb + n] = v;
+		}
+		if (s.part && t == nw + na && threadIdx.x < 32) {
+			double v = 0.0;
+			for (int i = threadIdx.x; i < s.npart; i += 32) v += s.part[(long)e * s.npart + i];
+			for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+			if (threadIdx.x == 0) s.loss[e] = (float)(v * s.scale);
+		}
+	}
 }
 
 // rows of the dataset into the first layer's input (bf16, zero-padded to K0, both
@@ -143,56 +264,6 @@ __global__ void k_mlp_gather(const float* __restrict__ X, const float* __restric
 		for (int k = threadIdx.x; k < n_out; k += blockDim.x) Yb[((long)e * M + m) * n_out + k] = id >= 0 ? Y[(long)id * n_out + k] : 0.f;
 }
 
-// G = 2 (Yhat - Y) / (M_valid n_out) on valid rows, 0 on padding rows; per-member sum of
-// squared errors, per block then in fixed order by k_mlp_loss_sum
-__global__ void k_mlp_loss(const float* __restrict__ Yh, const float* __restrict__ Y, const int* __restrict__ idx, int M, int n_out,
-	float scale, long sg, float* G, __nv_bfloat16* Gb, __nv_bfloat16* Gt, float* part)
-{
-	const int e = blockIdx.y, m = blockIdx.x;
-	const bool valid = idx[e * M + m] >= 0;
-	__shared__ float sm[32];
-	float s = 0.f;
-	for (int k = threadIdx.x; k < n_out; k += blockDim.x) {
-		long o = ((long)e * M + m) * n_out + k;
-		float d = valid ? Yh[o] - Y[o] : 0.f;
-		s += d * d;
-		float g = 2.f * d * scale;
-		long og = e * sg + (long)m * n_out + k;
-		G[og] = g;
-		__nv_bfloat16 b = __float2bfloat16_rn(g);
-		Gb[og] = b;
-		Gt[e * sg + (long)k * M + m] = b;
-	}
-	for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-	if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		float t = 0.f;
-		for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sm[w];
-		part[e * M + m] = t;
-	}
-}
-
-__global__ void k_mlp_loss_sum(const float* __restrict__ part, int M, float scale, float* loss)
-{
-	const int e = blockIdx.x;
-	if (threadIdx.x) return;
-	double t = 0.0;
-	for (int m = 0; m < M; ++m) t += part[e * M + m];
-	loss[e] = (float)(t * scale);
-}
-
-// gb[n] = sum_m G[m][n], rows in order
-__global__ void k_mlp_bias_grad(const float* __restrict__ G, long sg, int M, int N, float* gb, long sgb)
-{
-	const int e = blockIdx.y;
-	const int n = blockIdx.x * blockDim.x + threadIdx.x;
-	if (n >= N) return;
-	float s = 0.f;
-	for (int m = 0; m < M; ++m) s += G[e * sg + (long)m * N + n];
-	gb[e * sgb + n] = s;
-}
-
 // Adam (Kingma & Ba 2015) on the fp32 masters of one member's parameters, then the
 // bf16 copies of the weights in both orientations
 struct adam_layer {
@@ -201,14 +272,14 @@ struct adam_layer {
 	int N, K;
 };
 
-__global__ void k_mlp_adam(adam_layer L, long sW, long sb, long sWb, float lr, float b1, float b2, float c1, float c2, float eps)
+__global__ void k_mlp_adam(adam_layer L, long sW, long sb, long sg, float lr, float b1, float b2, float c1, float c2, float eps)
 {
 	const int e = blockIdx.y;
 	const long nw = (long)L.N * L.K;
 	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < nw + L.N; i += (long)gridDim.x * blockDim.x) {
 		const bool isw = i < nw;
 		float* p = isw ? L.W + e * sW + i : L.b + e * sb + (i - nw);
-		const float g = isw ? L.gW[e * sW + i] : L.gb[e * sb + (i - nw)];
+		const float g = isw ? L.gW[e * sg + i] : L.gb[e * sg + (i - nw)];
 		float* m = isw ? L.mW + e * sW + i : L.mb + e * sb + (i - nw);
 		float* v = isw ? L.vW + e * sW + i : L.vb + e * sb + (i - nw);
 		float mm = b1 * *m + (1.f - b1) * g;
@@ -220,8 +291,8 @@ __global__ void k_mlp_adam(adam_layer L, long sW, long sb, long sWb, float lr, f
 		if (isw) {
 			int n = (int)(i / L.K), k = (int)(i - (long)n * L.K);
 			__nv_bfloat16 b = __float2bfloat16_rn(w);
-			L.Wb[e * sWb + i] = b;
-			L.Wt[e * sWb + (long)k * L.N + n] = b;
+			L.Wb[e * sW + i] = b;
+			L.Wt[e * sW + (long)k * L.N + n] = b;
 		}
 	}
 }
@@ -248,17 +319,19 @@ struct qpc_mlp {
 	int n_in = 0, K0 = 0, n_hidden = 0, n_layers = 0, n_out = 0, E = 0, J = 0;
 	std::vector<int> Ns, Ks;          // per linear layer j: out, in
 	std::vector<long> offW, offb;     // offsets of layer j in the per-member flat arrays
+	std::vector<long> goff;           // of its weights in the gradient [E][nW + nb] (W_0, b_0, W_1, ..): the caller's layout
 	long nW = 0, nb = 0;              // per-member totals
 	cudaStream_t st = nullptr;
-	float *W = nullptr, *b = nullptr, *gW = nullptr, *gb = nullptr, *mW = nullptr, *vW = nullptr, *mb = nullptr, *vb = nullptr;
+	float *W = nullptr, *b = nullptr, *grad = nullptr, *mW = nullptr, *vW = nullptr, *mb = nullptr, *vb = nullptr;
 	__nv_bfloat16 *Wb = nullptr, *Wt = nullptr;
 	long t = 0;                       // Adam step count
 	// batch work space (capacity M)
 	int Mcap = 0;
 	std::vector<__nv_bfloat16*> Act, ActT;  // layer inputs j = 0..J-1: [E][M][K_j] and [E][K_j][M]
 	std::vector<float*> Z;                  // pre-activations of hidden layers [E][M][N_j]
-	float *Yh = nullptr, *Yb = nullptr, *G = nullptr, *part = nullptr, *loss = nullptr;
-	__nv_bfloat16 *Gb = nullptr, *Gt = nullptr;
+	float *Yh = nullptr, *Yb = nullptr, *part = nullptr, *loss = nullptr;
+	__nv_bfloat16 *Gb[2] = {}, *Gt[2] = {}; // a layer's output gradient and the one below it, in turn
+	float* cs[2] = {};                      // their sums over 64 rows
 	int* idx = nullptr;
 	// dataset on the device
 	float *dX = nullptr, *dY = nullptr;
@@ -273,10 +346,10 @@ void mlp_free_batch(qpc_mlp* h)
 	for (auto p : h->ActT) cudaFree(p);
 	for (auto p : h->Z) cudaFree(p);
 	h->Act.clear(); h->ActT.clear(); h->Z.clear();
-	void* ps[] = {h->Yh, h->Yb, h->G, h->part, h->loss, h->Gb, h->Gt, h->idx};
+	void* ps[] = {h->Yh, h->Yb, h->part, h->loss, h->Gb[0], h->Gb[1], h->Gt[0], h->Gt[1], h->cs[0], h->cs[1], h->idx};
 	for (void* p : ps) if (p) cudaFree(p);
-	h->Yh = h->Yb = h->G = h->part = h->loss = nullptr;
-	h->Gb = h->Gt = nullptr;
+	h->Yh = h->Yb = h->part = h->loss = nullptr;
+	for (int i = 0; i < 2; ++i) { h->Gb[i] = h->Gt[i] = nullptr; h->cs[i] = nullptr; }
 	h->idx = nullptr;
 	h->Mcap = 0;
 }
@@ -286,7 +359,7 @@ void mlp_free(qpc_mlp* h)
 	if (!h) return;
 	cudaSetDevice(h->dev);
 	mlp_free_batch(h);
-	void* ps[] = {h->W, h->b, h->gW, h->gb, h->mW, h->vW, h->mb, h->vb, h->Wb, h->Wt, h->dX, h->dY};
+	void* ps[] = {h->W, h->b, h->grad, h->mW, h->vW, h->mb, h->vb, h->Wb, h->Wt, h->dX, h->dY};
 	for (void* p : ps) if (p) cudaFree(p);
 	if (h->st) cudaStreamDestroy(h->st);
 	delete h;
@@ -306,85 +379,75 @@ int ensure_batch(qpc_mlp* h, int M)
 	}
 	const int maxN = *std::max_element(h->Ns.begin(), h->Ns.end());
 	if ((rc = dalloc(&h->Yh, (size_t)E * M * h->n_out)) || (rc = dalloc(&h->Yb, (size_t)E * M * h->n_out)) ||
-		(rc = dalloc(&h->G, (size_t)E * M * maxN)) || (rc = dalloc(&h->Gb, (size_t)E * M * maxN)) ||
-		(rc = dalloc(&h->Gt, (size_t)E * M * maxN)) || (rc = dalloc(&h->part, (size_t)E * M)) || (rc = dalloc(&h->loss, (size_t)E)) ||
+		(rc = dalloc(&h->part, (size_t)E * (M / MT) * ((h->n_out + MT - 1) / MT))) || (rc = dalloc(&h->loss, (size_t)E)) ||
 		(rc = dalloc(&h->idx, (size_t)E * M)))
 		return rc;
+	for (int i = 0; i < 2; ++i)
+		if ((rc = dalloc(&h->Gb[i], (size_t)E * M * maxN)) || (rc = dalloc(&h->Gt[i], (size_t)E * M * maxN)) || (rc = dalloc(&h->cs[i], (size_t)E * (M / MT) * maxN)))
+			return rc;
 	h->Mcap = M;
 	return QPC_OK;
 }
 
-// second buffer for the gradient chain: G (fp32/bf16) alternate with the Act-sized
-// scratch of the layer below; the backward pass writes layer j-1's gradient into
-// dedicated buffers allocated on first use
-struct back_bufs {
-	float* G2 = nullptr;
-	__nv_bfloat16 *G2b = nullptr, *G2t = nullptr;
-};
-
-template <int EPI>
-void gemm(cudaStream_t st, int E, const __nv_bfloat16* A, long sA, const __nv_bfloat16* B, long sB, int M, int N, int K,
-	const float* bias, long sbias, const float* aux, long saux, float* out, long sout, __nv_bfloat16* outb, long soutb,
-	__nv_bfloat16* outt, long soutt)
+gemm_args product(int epi, const __nv_bfloat16* A, long sA, const __nv_bfloat16* B, long sB, int M, int N, int K)
 {
-	gemm_args a{A, sA, B, sB, M, N, K, bias, sbias, aux, saux, out, sout, outb, soutb, outt, soutt};
-	dim3 grid((N + MT - 1) / MT, (M + MT - 1) / MT, E);
-	k_mlp_gemm<EPI><<<grid, MLP_THREADS, 0, st>>>(a);
+	gemm_args a{};
+	a.A = A; a.sA = sA; a.B = B; a.sB = sB; a.M = M; a.N = N; a.K = K; a.epi = epi;
+	return a;
 }
 
-// forward of the Mcap rows gathered into Act[0]; output in Yh
-void forward(qpc_mlp* h)
-{
-	const int E = h->E, J = h->J, M = h->Mcap;
-	for (int j = 0; j < J; ++j) {
-		const int N = h->Ns[j], K = h->Ks[j];
-		const __nv_bfloat16* W = h->Wb + h->offW[j];
-		if (j < J - 1)
-			gemm<EPI_HIDDEN>(h->st, E, h->Act[j], (long)h->Mcap * K, W, h->nW, M, N, K, h->b + h->offb[j], h->nb, nullptr, 0,
-				h->Z[j], (long)h->Mcap * N, h->Act[j + 1], (long)h->Mcap * N, h->ActT[j + 1], (long)h->Mcap * N);
-		else
-			gemm<EPI_STORE>(h->st, E, h->Act[j], (long)h->Mcap * K, W, h->nW, M, N, K, h->b + h->offb[j], h->nb, nullptr, 0,
-				h->Yh, (long)h->Mcap * N, nullptr, 0, nullptr, 0);
-	}
-}
-
-// loss and gradients of the batch in Act[0] / Yb (idx marks valid rows); gW, gb filled
-int backward(qpc_mlp* h, int Mvalid, back_bufs& bb)
+// forward of the Mcap rows gathered into Act[0]; the output into Yh, or with Mvalid > 0 the loss gradient of that many
+// rows into G[0] (and its partial sums)
+void forward(qpc_mlp* h, int Mvalid)
 {
 	const int E = h->E, J = h->J, M = h->Mcap;
 	const int maxN = *std::max_element(h->Ns.begin(), h->Ns.end());
-	if (!bb.G2) {
-		// stream-ordered: freed in stream order by free_back, which never blocks
-		const size_t n = (size_t)E * h->Mcap * maxN;
-		if (cudaMallocAsync((void**)&bb.G2, sizeof(float) * n, h->st) != cudaSuccess ||
-			cudaMallocAsync((void**)&bb.G2b, sizeof(__nv_bfloat16) * n, h->st) != cudaSuccess ||
-			cudaMallocAsync((void**)&bb.G2t, sizeof(__nv_bfloat16) * n, h->st) != cudaSuccess) {
-			set_error("cudaMallocAsync of the gradient scratch failed");
-			return QPC_ERR_NOMEM;
+	for (int j = 0; j < J; ++j) {
+		const int N = h->Ns[j], K = h->Ks[j];
+		const bool last = j == J - 1;
+		gemm_args a = product(!last ? EPI_HIDDEN : Mvalid ? EPI_LOSS : EPI_STORE, h->Act[j], (long)M * K, h->Wb + h->offW[j], h->nW, M, N, K);
+		a.bias = h->b + h->offb[j]; a.sbias = h->nb;
+		a.out = last ? h->Yh : h->Z[j]; a.sout = (long)M * N;
+		if (!last) {
+			a.outb = h->Act[j + 1]; a.outt = h->ActT[j + 1];
+			a.soutb = a.soutt = (long)M * N;
+		} else {
+			a.outb = h->Gb[0]; a.outt = h->Gt[0]; a.cs = h->cs[0];
+			a.soutb = a.soutt = (long)M * maxN;
+			a.scs = (long)(M / MT) * maxN;
+			a.aux = h->Yb; a.saux = (long)M * N; a.idx = h->idx; a.part = h->part;
+			a.scale = 1.0f / ((float)std::max(Mvalid, 1) * (float)h->n_out);
 		}
+		k_mlp_gemm<<<dim3(a.tiles(), 1, E), MLP_THREADS, MLP_SMEM, h->st>>>(a);
 	}
-	const float scale = 1.0f / ((float)Mvalid * (float)h->n_out);
-	const long sg = (long)h->Mcap * maxN;
-	k_mlp_loss<<<dim3(M, E), 128, 0, h->st>>>(h->Yh, h->Yb, h->idx, M, h->n_out, scale, sg, h->G, h->Gb, h->Gt, h->part);
-	k_mlp_loss_sum<<<E, 32, 0, h->st>>>(h->part, h->Mcap, scale, h->loss);
-	float* G = h->G;
-	__nv_bfloat16 *Gb = h->Gb, *Gt = h->Gt;
-	float* G2 = bb.G2;
-	__nv_bfloat16 *G2b = bb.G2b, *G2t = bb.G2t;
-	for (int j = J - 1; j >= 0; --j) {
+}
+
+// gradients and loss after forward(h, Mvalid)
+void backward(qpc_mlp* h, int Mvalid)
+{
+	const int E = h->E, J = h->J, M = h->Mcap, nt = M / MT;
+	const int maxN = *std::max_element(h->Ns.begin(), h->Ns.end());
+	const long sg = (long)M * maxN, np = h->nW + h->nb;
+	for (int j = J - 1, g = 0; j >= 0; --j, g = 1 - g) {
 		const int N = h->Ns[j], K = h->Ks[j];
 		// gW_j[n][k] = sum_m G[m][n] A_j[m][k]: A = G^T [N][M], B = A_j^T [K][M]
-		gemm<EPI_STORE>(h->st, E, Gt, sg, h->ActT[j], (long)h->Mcap * K, N, K, M, nullptr, 0, nullptr, 0,
-			h->gW + h->offW[j], h->nW, nullptr, 0, nullptr, 0);
-		k_mlp_bias_grad<<<dim3((N + 127) / 128, E), 128, 0, h->st>>>(G, sg, M, N, h->gb + h->offb[j], h->nb);
+		gemm_args w = product(EPI_STORE, h->Gt[g], sg, h->ActT[j], (long)M * K, N, K, M), a{};
+		w.out = h->grad + h->goff[j]; w.sout = np;
 		if (j > 0) {
 			// dA[m][k] = sum_n G[m][n] W[n][k]: A = G [M][N], B = W^T [K][N]; times gelu'(Z_{j-1})
-			gemm<EPI_BACK>(h->st, E, Gb, sg, h->Wt + h->offW[j], h->nW, M, K, N, nullptr, 0, h->Z[j - 1], (long)h->Mcap * K,
-				G2, sg, G2b, sg, G2t, sg);
-			std::swap(G, G2); std::swap(Gb, G2b); std::swap(Gt, G2t);
+			a = product(EPI_BACK, h->Gb[g], sg, h->Wt + h->offW[j], h->nW, M, K, N);
+			a.aux = h->Z[j - 1]; a.saux = (long)M * K;
+			a.outb = h->Gb[1 - g]; a.outt = h->Gt[1 - g]; a.soutb = a.soutt = sg;
+			a.cs = h->cs[1 - g]; a.scs = (long)nt * maxN;
 		}
+		sum_args s{h->cs[g], (long)nt * maxN, nt, N, h->grad + h->goff[j] + (long)N * K, np, nullptr, 0, 0.f, h->loss};
+		if (j == J - 1) {
+			s.part = h->part; s.npart = nt * ((h->n_out + MT - 1) / MT);
+			s.scale = 1.0f / ((float)Mvalid * (float)h->n_out);
+		}
+		const int nw = w.tiles(), na = j > 0 ? a.tiles() : 0;
+		k_mlp_back<<<dim3(nw + na + (N + MLP_THREADS - 1) / MLP_THREADS, 1, E), MLP_THREADS, MLP_SMEM, h->st>>>(w, a, s, nw, na);
 	}
-	return QPC_OK;
 }
 
 void adam(qpc_mlp* h, float lr)
@@ -393,11 +456,11 @@ void adam(qpc_mlp* h, float lr)
 	h->t += 1;
 	const float c1 = 1.f - powf(b1, (float)h->t), c2 = 1.f - powf(b2, (float)h->t);
 	for (int j = 0; j < h->J; ++j) {
-		adam_layer L{h->W + h->offW[j], h->b + h->offb[j], h->gW + h->offW[j], h->gb + h->offb[j], h->mW + h->offW[j], h->vW + h->offW[j],
+		adam_layer L{h->W + h->offW[j], h->b + h->offb[j], h->grad + h->goff[j], h->grad + h->goff[j] + (long)h->Ns[j] * h->Ks[j], h->mW + h->offW[j], h->vW + h->offW[j],
 			h->mb + h->offb[j], h->vb + h->offb[j], h->Wb + h->offW[j], h->Wt + h->offW[j], h->Ns[j], h->Ks[j]};
 		long n = (long)h->Ns[j] * h->Ks[j] + h->Ns[j];
 		int blocks = (int)std::min<long>((n + 255) / 256, 1024);
-		k_mlp_adam<<<dim3(blocks, h->E), 256, 0, h->st>>>(L, h->nW, h->nb, h->nW, lr, b1, b2, c1, c2, eps);
+		k_mlp_adam<<<dim3(blocks, h->E), 256, 0, h->st>>>(L, h->nW, h->nb, h->nW + h->nb, lr, b1, b2, c1, c2, eps);
 	}
 }
 
@@ -434,14 +497,6 @@ int upload_data(qpc_mlp* h, const float* X, const float* Y, long n)
 	return QPC_OK;
 }
 
-void free_back(back_bufs& bb, cudaStream_t st)
-{
-	if (bb.G2) cudaFreeAsync(bb.G2, st);
-	if (bb.G2b) cudaFreeAsync(bb.G2b, st);
-	if (bb.G2t) cudaFreeAsync(bb.G2t, st);
-	bb = back_bufs{};
-}
-
 int round_m(int m) { return (m + MT - 1) / MT * MT; }
 
 } // namespace
@@ -470,13 +525,14 @@ int qpc_mlp_create(int32_t n_in, int32_t n_hidden, int32_t n_layers, int32_t n_o
 		h->Ns.push_back(j == h->J - 1 ? n_out : n_hidden);
 		h->offW.push_back(h->nW);
 		h->offb.push_back(h->nb);
+		h->goff.push_back(h->nW + h->nb);
 		h->nW += (long)h->Ns[j] * h->Ks[j];
 		h->nb += h->Ns[j];
 	}
 	if ((cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking)) != cudaSuccess) { set_error("cudaStreamCreateWithFlags failed"); return fail(QPC_ERR_CUDA); }
 	const size_t tw = (size_t)h->E * h->nW, tb = (size_t)h->E * h->nb;
 	int rc;
-	if ((rc = dalloc(&h->W, tw)) || (rc = dalloc(&h->b, tb)) || (rc = dalloc(&h->gW, tw)) || (rc = dalloc(&h->gb, tb)) ||
+	if ((rc = dalloc(&h->W, tw)) || (rc = dalloc(&h->b, tb)) || (rc = dalloc(&h->grad, tw + tb)) ||
 		(rc = dalloc(&h->mW, tw)) || (rc = dalloc(&h->vW, tw)) || (rc = dalloc(&h->mb, tb)) || (rc = dalloc(&h->vb, tb)) ||
 		(rc = dalloc(&h->Wb, tw)) || (rc = dalloc(&h->Wt, tw)))
 		return fail(rc);
@@ -500,6 +556,8 @@ int qpc_mlp_create(int32_t n_in, int32_t n_hidden, int32_t n_layers, int32_t n_o
 		set_error("device upload failed");
 		return fail(QPC_ERR_CUDA);
 	}
+	cudaFuncSetAttribute(k_mlp_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM);
+	cudaFuncSetAttribute(k_mlp_back, cudaFuncAttributeMaxDynamicSharedMemorySize, MLP_SMEM);
 	cast_all(h);
 	if (cudaGetLastError() != cudaSuccess) { set_error("cast failed"); return fail(QPC_ERR_CUDA); }
 	if (int rc2 = wait_on(h->st)) return fail(rc2);
@@ -568,29 +626,11 @@ int qpc_mlp_loss_grad(qpc_mlp* h, const float* X, const float* Y, int32_t n, flo
 		for (int m = 0; m < n; ++m) idx[(size_t)e * h->Mcap + m] = m;
 	QPC_CUDA(cudaMemcpyAsync(h->idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, h->st));
 	k_mlp_gather<<<dim3(M, h->E), 64, 0, h->st>>>(h->dX, h->dY, h->idx, h->n_in, h->K0, h->n_out, M, h->Act[0], h->ActT[0], h->Yb);
-	forward(h);
-	back_bufs bb;
-	int rc = backward(h, n, bb);
-	if (!rc && cudaGetLastError() != cudaSuccess) { set_error("kernel launch failed"); rc = QPC_ERR_CUDA; }
-	if (!rc) rc = wait_on(h->st);
-	if (rc) { free_back(bb, h->st); return rc; }
-	free_back(bb, h->st);
-	if (int rc2 = copy_to_host(loss, h->loss, sizeof(float) * h->E, h->st)) return rc2;
-	if (grad) {
-		const long np = h->nW + h->nb;
-		std::vector<float> gw((size_t)h->E * h->nW), gbv((size_t)h->E * h->nb);
-		if (int rc2 = copy_to_host(gw.data(), h->gW, sizeof(float) * gw.size(), h->st)) return rc2;
-		if (int rc2 = copy_to_host(gbv.data(), h->gb, sizeof(float) * gbv.size(), h->st)) return rc2;
-		for (int e = 0; e < h->E; ++e) {
-			long o = 0;
-			for (int j = 0; j < h->J; ++j) {
-				const size_t nw = (size_t)h->Ns[j] * h->Ks[j];
-				std::copy(gw.begin() + (size_t)e * h->nW + h->offW[j], gw.begin() + (size_t)e * h->nW + h->offW[j] + nw, grad + e * np + o);
-				std::copy(gbv.begin() + (size_t)e * h->nb + h->offb[j], gbv.begin() + (size_t)e * h->nb + h->offb[j] + h->Ns[j], grad + e * np + o + nw);
-				o += nw + h->Ns[j];
-			}
-		}
-	}
+	forward(h, n);
+	backward(h, n);
+	QPC_CUDA(cudaGetLastError());
+	if (int rc = copy_to_host(loss, h->loss, sizeof(float) * h->E, h->st)) return rc;
+	if (grad) return copy_to_host(grad, h->grad, sizeof(float) * (size_t)h->E * (h->nW + h->nb), h->st);
 	return QPC_OK;
 }
 
@@ -608,7 +648,6 @@ int qpc_mlp_train(qpc_mlp* h, const float* X, const float* Y, int32_t n, int32_t
 	std::vector<int> perm((size_t)h->E * n), idx((size_t)h->E * h->Mcap);
 	std::vector<float> lsum(h->E), lb(h->E);
 	uint64_t sd = seed;
-	back_bufs bb;
 	int rc = QPC_OK;
 	for (int ep = 0; ep < epochs && !rc; ++ep) {
 		for (int e = 0; e < h->E; ++e) {
@@ -623,8 +662,8 @@ int qpc_mlp_train(qpc_mlp* h, const float* X, const float* Y, int32_t n, int32_t
 				for (int m = 0; m < h->Mcap; ++m) idx[(size_t)e * h->Mcap + m] = m < mv ? perm[(size_t)e * n + m0 + m] : -1;
 			if (cudaMemcpyAsync(h->idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, h->st) != cudaSuccess) { rc = QPC_ERR_CUDA; break; }
 			k_mlp_gather<<<dim3(M, h->E), 64, 0, h->st>>>(h->dX, h->dY, h->idx, h->n_in, h->K0, h->n_out, M, h->Act[0], h->ActT[0], h->Yb);
-			forward(h);
-			if ((rc = backward(h, mv, bb))) break;
+			forward(h, mv);
+			backward(h, mv);
 			adam(h, lr);
 			if (loss_hist) {
 				if ((rc = copy_to_host(lb.data(), h->loss, sizeof(float) * h->E, h->st))) break;
@@ -635,7 +674,6 @@ int qpc_mlp_train(qpc_mlp* h, const float* X, const float* Y, int32_t n, int32_t
 	}
 	if (!rc && cudaGetLastError() != cudaSuccess) { rc = QPC_ERR_CUDA; set_error("training step failed on the device"); }
 	if (!rc) rc = wait_on(h->st);
-	free_back(bb, h->st);
 	return rc;
 }
 
@@ -656,7 +694,7 @@ int qpc_mlp_predict(qpc_mlp* h, const float* X, int32_t n, float* out)
 			for (int m = 0; m < h->Mcap; ++m) idx[(size_t)e * h->Mcap + m] = m < mv ? m0 + m : -1;
 		QPC_CUDA(cudaMemcpyAsync(h->idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, h->st));
 		k_mlp_gather<<<dim3(M, h->E), 64, 0, h->st>>>(h->dX, nullptr, h->idx, h->n_in, h->K0, h->n_out, M, h->Act[0], h->ActT[0], nullptr);
-		forward(h);
+		forward(h, 0);
 		QPC_CUDA(cudaGetLastError());
 		if (int rc = copy_to_host(yh.data(), h->Yh, sizeof(float) * yh.size(), h->st)) return rc;
 		for (int e = 0; e < h->E; ++e)
