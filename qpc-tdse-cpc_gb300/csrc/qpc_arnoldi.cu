@@ -51,6 +51,7 @@ struct ar_args {
 	double dt, emin, emax;
 	const double *S, *R, *Lrow, *Lcol, *dinv, *H, *y10;
 	const double *SM, *SN, *SI;	// block substitution (k_ar_sinv_blk): M_t, N_t, L11^-1 per block [P][P]
+	const double *SF, *SB;		// products of -M, -N from the start of a segment
 	double2 *X, *U, *V0, *V1;
 	double2* partX;
 	double* partN;
@@ -398,11 +399,14 @@ __global__ void __launch_bounds__(CH_THREADS) k_ar_sinv(ar_args g, double2* __re
 // P rows, P lanes per recurrence.  With L21(t) the factor's block left of the diagonal block L11(t),
 //   a(t) = v(t) - M_t a(t-1),  M_t = L21(t) L11(t-1)^-1      y(t) = L11(t)^-1 a(t)
 //   b(t) = y(t) - N_t b(t+1),  N_t = (L11(t+1)^-1 L21(t+1))^T    x(t) = L11(t)^-T b(t):
-// only a and b are sequences, P rows per link of a few dependent FMAs (one warp), the rest is done by the whole block.
-// The vector stays in shared memory in between.  Bound by the FP64 issue of the sequences (P FMAs of 64 cycles per P
-// rows); measured at groups of 4 wavefunctions of 400 x 21: 68 us, against ~270 for one dependent chain of three
-// FP64 instructions and two shuffles per row (122 with the factor rows scaled to one FMA and one shuffle).
+// only a and b are sequences, P rows per link of a few dependent FMAs, the rest is done by the whole block.  The sequences
+// are cut into four segments, a warp each, started from zero; what a segment should have started from then adds
+// Phi_t a(end of the segment before), Phi_t the product of -M (or -N) from the segment's start to t.
+// The vector stays in shared memory in between.  Bound by the latency of the sequences (P FMAs of 64 cycles per P
+// rows); measured at groups of 4 wavefunctions of 400 x 21: 38 us (68 with one segment, ~270 for one dependent chain
+// of three FP64 instructions and two shuffles per row).
 constexpr int SB_THREADS = 128;
+constexpr int SB_SEG = SB_THREADS / 32;
 constexpr size_t SB_SMEM = 200 * 1024;	// longest vectors it takes: 5 recurrences of 5 000 rows at p = 6
 template <int P>
 __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* __restrict__ vbuf)
@@ -411,6 +415,7 @@ __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* 
 	if (g.flag[b] != AR_LIVE) return;
 	constexpr int CPW = 32 / P, PP = P * P;
 	extern __shared__ double xs[];	// [CPW][nt P]
+	__shared__ double carry[SB_SEG][CPW * P];	// what enters each segment
 	const int N = g.N, nt = (N + P - 1) / P, np = nt * P;
 	const long stride = 2L * g.nch;
 	const int c0 = blockIdx.x * CPW, nc = min(CPW, 2 * g.nch - c0);
@@ -420,10 +425,11 @@ __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* 
 		xs[c * np + r] = (r < N && c < nc) ? v[(long)r * stride + c] : 0.0;
 	}
 	__syncthreads();
-	const int lane = threadIdx.x, cs = lane / P, j = lane - cs * P;
-	auto sequence = [&](const double* __restrict__ C, bool fwd) {
-		if (threadIdx.x >= 32) return;
+	const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, cs = lane / P, j = lane - cs * P;
+	const int sl = (nt + SB_SEG - 1) / SB_SEG;	// blocks of a segment
+	auto sequence = [&](const double* __restrict__ C, const double* __restrict__ Phi, bool fwd) {
 		const bool act = cs < CPW;
+		const int ib = seg * sl, ie = min(nt, ib + sl);
 		double* x = xs + (act ? cs : 0) * np;
 		const int base = (act ? cs : 0) * P;
 		auto blk = [&](int i) { return fwd ? i : nt - 1 - i; };
@@ -432,17 +438,17 @@ __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* 
 		double cf[D][P], vl[D];
 		auto fetch = [&](int i, double* c, double& w) {
 #pragma unroll
-			for (int k = 0; k < P; ++k) c[k] = i < nt ? __ldg(C + (long)blk(i) * PP + j * P + k) : 0.0;
-			w = (act && i < nt) ? x[blk(i) * P + j] : 0.0;
+			for (int k = 0; k < P; ++k) c[k] = (act && i < ie) ? __ldg(C + (long)blk(i) * PP + j * P + k) : 0.0;
+			w = (act && i < ie) ? x[blk(i) * P + j] : 0.0;
 		};
-		double a = act ? x[blk(0) * P + j] : 0.0;
+		double a = (act && ib < ie) ? x[blk(ib) * P + j] : 0.0;
 #pragma unroll
-		for (int d = 0; d < D - 1; ++d) fetch(1 + d, cf[d], vl[d]);
-		for (int i0 = 1; i0 < nt; i0 += D) {
+		for (int d = 0; d < D - 1; ++d) fetch(ib + 1 + d, cf[d], vl[d]);
+		for (int i0 = ib + 1; i0 < ie; i0 += D) {
 #pragma unroll
 			for (int d = 0; d < D; ++d) {
 				const int i = i0 + d;
-				if (i >= nt) break;
+				if (i >= ie) break;
 				fetch(i + D - 1, cf[(d + D - 1) % D], vl[(d + D - 1) % D]);
 				double p = vl[d], q = 0.0;
 #pragma unroll
@@ -454,8 +460,24 @@ __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* 
 				if (act) x[blk(i) * P + j] = a;
 			}
 		}
+		if (act) carry[seg][lane] = a;	// the segment's end; turned into what enters it
+		__syncthreads();
+		if (seg) return;
+		double in = 0.0;
+		for (int s = 0; s < SB_SEG; ++s) {
+			const int e = min(nt, (s + 1) * sl) - 1;
+			double out = act ? carry[s][lane] : 0.0;
+#pragma unroll
+			for (int k = 0; k < P; ++k) {
+				const double ik = __shfl_sync(0xffffffffu, in, base + k);
+				if (s && act && s * sl < nt) out = fma(__ldg(Phi + (long)blk(e) * PP + j * P + k), ik, out);
+			}
+			if (act) carry[s][lane] = in;
+			in = out;
+		}
 	};
-	auto blocks = [&](bool trans) {	// every block times L11^-1 or its transpose
+	auto blocks = [&](bool trans) {	// every block, with what entered its segment, times L11^-1 or its transpose
+		const double* __restrict__ Phi = trans ? g.SB : g.SF;
 		for (int i = threadIdx.x; i < nt * CPW; i += SB_THREADS) {
 			const int t = i / CPW, c = i - t * CPW;
 			double* x = xs + c * np + t * P;
@@ -463,6 +485,13 @@ __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* 
 			double in[P], out[P];
 #pragma unroll
 			for (int k = 0; k < P; ++k) in[k] = x[k];
+			const int s = (trans ? nt - 1 - t : t) / sl;
+			if (s) {
+#pragma unroll
+				for (int k = 0; k < P; ++k)
+#pragma unroll
+					for (int q = 0; q < P; ++q) in[k] = fma(__ldg(Phi + (long)t * PP + k * P + q), carry[s][c * P + q], in[k]);
+			}
 #pragma unroll
 			for (int r = 0; r < P; ++r) {
 				double s = 0.0;
@@ -475,11 +504,11 @@ __global__ void __launch_bounds__(SB_THREADS) k_ar_sinv_blk(ar_args g, double2* 
 			for (int k = 0; k < P; ++k) x[k] = out[k];
 		}
 	};
-	sequence(g.SM, true);
+	sequence(g.SM, g.SF, true);
 	__syncthreads();
 	blocks(false);
 	__syncthreads();
-	sequence(g.SN, false);
+	sequence(g.SN, g.SB, false);
 	__syncthreads();
 	blocks(true);
 	__syncthreads();
@@ -649,7 +678,7 @@ struct qpc_arnoldi {
 	double dt = 0, emin = 0, emax = 0;
 	cudaStream_t stream = nullptr, stream2 = nullptr;	// stream2: second instance group (n_inst >= 2)
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-	double *S = nullptr, *R = nullptr, *Lrow = nullptr, *Lcol = nullptr, *SM = nullptr, *SN = nullptr, *SI = nullptr, *dinv = nullptr, *H = nullptr, *y10 = nullptr;
+	double *S = nullptr, *R = nullptr, *Lrow = nullptr, *Lcol = nullptr, *SM = nullptr, *SN = nullptr, *SI = nullptr, *SF = nullptr, *SB = nullptr, *dinv = nullptr, *H = nullptr, *y10 = nullptr;
 	double2 *X = nullptr, *U = nullptr, *V0 = nullptr, *V1 = nullptr, *tmp = nullptr;
 	double2* partX = nullptr;
 	double* partN = nullptr;
@@ -672,7 +701,7 @@ void ar_free(qpc_arnoldi* h)
 {
 	if (!h) return;
 	cudaSetDevice(h->dev);
-	void* ptrs[] = {h->S, h->R, h->Lrow, h->Lcol, h->SM, h->SN, h->SI, h->dinv, h->H, h->y10, h->X, h->U, h->V0, h->V1, h->tmp, h->partX, h->partN,
+	void* ptrs[] = {h->S, h->R, h->Lrow, h->Lcol, h->SM, h->SN, h->SI, h->SF, h->SB, h->dinv, h->H, h->y10, h->X, h->U, h->V0, h->V1, h->tmp, h->partX, h->partN,
 		h->cnt, h->xfin, h->xc, h->a, h->b, h->sfac, h->nu0, h->msub, h->flag, h->status, h->ez, h->nt, h->crit, h->msub_out};
 	for (void* p : ptrs)
 		if (p) cudaFree(p);
@@ -691,7 +720,7 @@ ar_args make_args(qpc_arnoldi* h)
 	g.B = h->d.n_inst; g.kmax = h->kmax; g.nbe = h->nbe; g.n = h->n; g.b0 = 0;
 	g.hstride = h->hper ? (long)h->d.n_r * (h->P + 1) * h->nlh : 0;
 	g.dt = h->dt; g.emin = h->emin; g.emax = h->emax;
-	g.S = h->S; g.R = h->R; g.Lrow = h->Lrow; g.Lcol = h->Lcol; g.SM = h->SM; g.SN = h->SN; g.SI = h->SI; g.dinv = h->dinv; g.H = h->H; g.y10 = h->y10;
+	g.S = h->S; g.R = h->R; g.Lrow = h->Lrow; g.Lcol = h->Lcol; g.SM = h->SM; g.SN = h->SN; g.SI = h->SI; g.SF = h->SF; g.SB = h->SB; g.dinv = h->dinv; g.H = h->H; g.y10 = h->y10;
 	g.X = h->X; g.U = h->U; g.V0 = h->V0; g.V1 = h->V1;
 	g.partX = h->partX; g.partN = h->partN; g.cnt = h->cnt; g.xfin = h->xfin;
 	g.a = h->a; g.b = h->b; g.sfac = h->sfac; g.nu0 = h->nu0; g.msub = h->msub; g.flag = h->flag; g.xc = h->xc;
@@ -850,6 +879,22 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 				sM[((size_t)t * P + r) * P + c] = x;
 				sN[((size_t)(t - 1) * P + c) * P + r] = y;
 			}
+	// Phi of the segments (zero in the first, where nothing enters)
+	std::vector<double> sF((size_t)nt * P * P, 0.0), sB((size_t)nt * P * P, 0.0);
+	const int sl = (nt + SB_SEG - 1) / SB_SEG;
+	for (int back = 0; back < 2; ++back)
+		for (int i = sl; i < nt; ++i) {
+			const int t = back ? nt - 1 - i : i, prev = back ? t + 1 : t - 1;
+			const double* C = (back ? sN : sM).data() + (size_t)t * P * P;
+			double* F = (back ? sB : sF).data();
+			for (int r = 0; r < P; ++r)
+				for (int c = 0; c < P; ++c) {
+					double x = 0.0;
+					if (i % sl == 0) x = -C[r * P + c];
+					else for (int k = 0; k < P; ++k) x -= C[r * P + k] * F[((size_t)prev * P + k) * P + c];
+					F[((size_t)t * P + r) * P + c] = x;
+				}
+		}
 	// Hamiltonian bands r-major: Hr[hs][r][k][l]
 	const int nhs = h->hper ? B : 1;
 	std::vector<double> Hr((size_t)nhs * N * NE * h->nlh);
@@ -870,7 +915,7 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 		if ((cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking)) != cudaSuccess) { set_error("cudaStreamCreateWithFlags failed"); return fail(QPC_ERR_CUDA); }
 	const long nst = (long)B * h->n;
 	if ((rc = dalloc(&h->S, (size_t)N * NE)) || (rc = dalloc(&h->R, (size_t)N * NE)) || (rc = dalloc(&h->Lrow, (size_t)N * P)) ||
-		(rc = dalloc(&h->Lcol, (size_t)N * P)) || (rc = dalloc(&h->SM, sM.size())) || (rc = dalloc(&h->SN, sN.size())) || (rc = dalloc(&h->SI, sI.size())) || (rc = dalloc(&h->dinv, (size_t)N)) || (rc = dalloc(&h->H, Hr.size())) ||
+		(rc = dalloc(&h->Lcol, (size_t)N * P)) || (rc = dalloc(&h->SM, sM.size())) || (rc = dalloc(&h->SN, sN.size())) || (rc = dalloc(&h->SI, sI.size())) || (rc = dalloc(&h->SF, sF.size())) || (rc = dalloc(&h->SB, sB.size())) || (rc = dalloc(&h->dinv, (size_t)N)) || (rc = dalloc(&h->H, Hr.size())) ||
 		(rc = dalloc(&h->y10, (size_t)d.n_m * d.n_l)) || (rc = dalloc(&h->X, nst)) || (rc = dalloc(&h->U, nst * kmax)) ||
 		(rc = dalloc(&h->V0, nst)) || (rc = dalloc(&h->V1, nst)) || (rc = dalloc(&h->tmp, nst)) ||
 		(rc = dalloc(&h->partX, (size_t)B * h->nbe * kmax)) || (rc = dalloc(&h->partN, (size_t)B * h->nbe)) ||
@@ -886,6 +931,8 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 		cudaMemcpy(h->SM, sM.data(), sizeof(double) * sM.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->SN, sN.data(), sizeof(double) * sN.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->SI, sI.data(), sizeof(double) * sI.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+		cudaMemcpy(h->SF, sF.data(), sizeof(double) * sF.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+		cudaMemcpy(h->SB, sB.data(), sizeof(double) * sB.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->dinv, di.data(), sizeof(double) * N, cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->H, Hr.data(), sizeof(double) * Hr.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
 		cudaMemcpy(h->y10, y10, sizeof(double) * d.n_m * d.n_l, cudaMemcpyHostToDevice) != cudaSuccess ||
