@@ -32,13 +32,14 @@ constexpr int SEEDW = 40;	// half-width of the windows the starting vectors are 
 // column and split its k.  The operator is stored per tile as chunks of KC k x TM rows, so that a warp's load is
 // 32 consecutive elements; the columns are quantised into shared memory once per block and read as broadcasts.
 // Bound by the integer multiply-adds from ~8 columns on (12 NB per k and lane against one 16-byte load), by the
-// operator's bytes below.
+// operator's bytes below; with one column per block four blocks share an SM, eight k in flight each (F~ of 800 x 41, one
+// column: 30 us with two blocks and sixteen, 24 us now, 105 MB; four operators of 400 x 21 30 -> 26 us).
 template <int NB, int KS, bool CX>
-__global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
+__global__ void __launch_bounds__(256, NB <= 1 ? 4 : 2) k_band_apply(const band_args p)
 {
 	constexpr int CG = 8 / KS, COLS = NB * CG, SK = 32 * KS, XS = COLS | 1;
 	constexpr int FB = KC * TM * (CX ? 16 : 8), TB = FB / 2;
-	constexpr int UN = NB <= 1 ? 16 : (NB <= 2 ? 8 : (NB <= 4 ? 4 : 2));
+	constexpr int UN = NB <= 2 ? 8 : (NB <= 4 ? 4 : 2);
 	constexpr size_t XBYTES = sizeof(int4) * SK * XS, RBYTES = KS > 1 ? sizeof(long long) * 8 * NB * 4 * 32 : 0;
 	constexpr size_t QBYTES = XBYTES > RBYTES ? XBYTES : RBYTES;
 	extern __shared__ __align__(16) char smem[];
