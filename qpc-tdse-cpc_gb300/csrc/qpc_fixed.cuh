@@ -42,6 +42,30 @@ __device__ __forceinline__ double to_double(long long h, long long m, int s, boo
 	return __longlong_as_double((long long)b);
 }
 
+// Kernels of a step follow each other on one stream by programmatic dependent launch (launch_after): a block may become
+// resident and read what no kernel of a run writes (operators, tables) before the previous kernel has ended; prev_wait()
+// holds it until that kernel, and so every one before it, is complete and its writes are visible.  Every block calls it
+// before it reads or writes a state and before it can return, so a kernel never ends before the previous one.
+// One wavefunction of 400 x 21, 120 steps of two kernels: 2.39 -> 1.77 ms; four with own potentials 1.57 -> 1.24 ms.
+// Launches of many waves start in the usual order (256 wavefunctions: 13.6 against 13.8 ms).
+__device__ __forceinline__ void prev_wait()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+void launch_after(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... a)
+{
+	cudaLaunchConfig_t c{};
+	c.gridDim = grid; c.blockDim = dim3(threads); c.dynamicSmemBytes = smem; c.stream = st;
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[0].val.programmaticStreamSerializationAllowed = 1;
+	c.attrs = at; c.numAttrs = (long)grid.x * grid.y <= 2000 ? 1 : 0;
+	cudaLaunchKernelEx(&c, k, P(a)...);	// errors: the caller's cudaGetLastError
+}
+
 // the largest of e over each group of TE lanes
 __device__ __forceinline__ int group_max(int e)
 {

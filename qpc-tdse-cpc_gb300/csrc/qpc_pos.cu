@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(256, 3) k_angle(const angle_args p)
 	const int m = im % p.M, slot = im / p.M;
 	const int pw = power_of(p.step, p.ntf[slot], p.cmode);
 	const bool obs = p.zpart && p.step < p.ntt[slot];
+	prev_wait();
 	if (pw == 0 && !obs) return;
 	const int L = p.L, np = p.npair, N = p.N;
 	double2* a = sm;		// [L][PT]: y, then its limbs, then the eigen-channels' limbs
@@ -232,7 +233,7 @@ namespace {
 template <int G>
 void angle_launch(const pos_path* p, const angle_args& a, int slots, cudaStream_t st)
 {
-	k_angle<G, 32><<<(unsigned)((long)slots * p->M * p->ntile), 256, sizeof(double2) * 2 * 32 * p->L, st>>>(a);
+	launch_after(k_angle<G, 32>, dim3((unsigned)((long)slots * p->M * p->ntile)), 256, sizeof(double2) * 2 * 32 * p->L, st, a);
 }
 
 int build(pos_path* p, const pos_setup& in, bool* ok)
@@ -371,7 +372,7 @@ int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf)
 			a.zpart = p->zpart + (size_t)p->zcount * p->B * p->M * p->ntile * (p->angle_small ? EPT : 1);
 			++p->zcount;
 		}
-		if (p->angle_small) k_angle<1, 8><<<(unsigned)((long)slots * p->M * p->ntile * EPT), 256, sizeof(double2) * 2 * 8 * p->L, st>>>(a);
+		if (p->angle_small) launch_after(k_angle<1, 8>, dim3((unsigned)((long)slots * p->M * p->ntile * EPT)), 256, sizeof(double2) * 2 * 8 * p->L, st, a);
 		else switch (p->angle_g) {
 		case 2: angle_launch<2>(p, a, slots, st); break;
 		case 3: angle_launch<3>(p, a, slots, st); break;

@@ -32,10 +32,9 @@ constexpr int SEEDW = 40;	// half-width of the windows the starting vectors are 
 // column and split its k.  The operator is stored per tile as chunks of KC k x TM rows, so that a warp's load is
 // 32 consecutive elements; the columns are quantised into shared memory once per block and read as broadcasts.
 // Bound by the integer multiply-adds from ~8 columns on (12 NB per k and lane against one 16-byte load), by the
-// operator's bytes below; with one column per block four blocks share an SM, eight k in flight each (F~ of 800 x 41, one
-// column: 30 us with two blocks and sixteen, 24 us now, 105 MB; four operators of 400 x 21 30 -> 26 us).
+// operator's bytes below.
 template <int NB, int KS, bool CX>
-__global__ void __launch_bounds__(256, NB <= 1 ? 4 : 2) k_band_apply(const band_args p)
+__global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 {
 	constexpr int CG = 8 / KS, COLS = NB * CG, SK = 32 * KS, XS = COLS | 1;
 	constexpr int FB = KC * TM * (CX ? 16 : 8), TB = FB / 2;
@@ -51,8 +50,8 @@ __global__ void __launch_bounds__(256, NB <= 1 ? 4 : 2) k_band_apply(const band_
 	const int ncg = (p.ncols + COLS - 1) / COLS;
 	const int cg = blockIdx.x % ncg, tile = p.tile0 + blockIdx.x / ncg, ch = blockIdx.y;
 	const int col0 = cg * COLS;
-	if (p.nta && KS == 8 && NB == 1 && !(p.step < p.nta[col0])) return;
 	const int4 td = p.td[tile];
+	prev_wait();
 	// every column's largest exponent over the tile's k range, one warp per column
 	const int nex = p.ntile * EPT, x0 = td.x * KC / TE, x1 = td.w * KC / TE;
 	for (int cl = warp; cl < COLS; cl += 8) {
@@ -85,8 +84,7 @@ __global__ void __launch_bounds__(256, NB <= 1 ? 4 : 2) k_band_apply(const band_
 	__syncthreads();
 	load(td.x * KC + lk);
 	const int ks = warp % KS, wc = (warp / KS) * NB;
-	const int set = p.amap ? p.amap[p.dmap ? p.dmap[col0] : col0] : 0;
-	const char* A = p.A + set * p.set_stride + (long)p.lmap[ch] * p.astride + p.toff[tile];
+	const char* A = p.A + (long)p.lmap[ch] * p.astride + p.toff[tile];
 	const long tl = (long)(td.y - td.x) * TB, tf = tl + (long)(td.z - td.y) * FB;
 	long long rh[NB], rm[NB], ih[NB], im[NB];
 #pragma unroll
@@ -220,6 +218,119 @@ __global__ void __launch_bounds__(256, NB <= 1 ? 4 : 2) k_band_apply(const band_
 			emit(cl, a, b, c, d);
 		}
 	}
+}
+
+// The same for one column per block (one wavefunction, or an operator of its own for each): eight warps split k by whole
+// chunks.  Bound by the latency of its loads and the operator's bytes, so a warp's first eight k of the operator are on
+// their way before the column is, four blocks share an SM, and only one barrier stands between the loads and the
+// products.  F~ of 800 x 41 (105 MB) 30 -> 24 us, 4 x (400 x 21) with own potentials 30 -> 25 us against k_band_apply<1, 8>
+// (two blocks, 16 k in flight after two barriers); what comes before prev_wait() then overlaps the kernel before.
+template <bool CX>
+__global__ void __launch_bounds__(256, 4) k_band_one(const band_args p)
+{
+	constexpr int FB = KC * TM * (CX ? 16 : 8), TB = FB / 2, UN = 8, RC = 32;	// RC: chunks of a round
+	__shared__ int4 xs[RC * KC];
+	__shared__ long long red[8][4][32];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int c = blockIdx.x % p.ncols, tile = p.tile0 + blockIdx.x / p.ncols, ch = blockIdx.y;
+	const int4 td = p.td[tile];
+	const long toff = p.toff[tile];
+	const bool on = !p.nta || p.step < p.nta[c];
+	const int nex = p.ntile * EPT;
+	const bool odd = p.par && (p.par[c] & 1);
+	const long v = (long)(p.smap ? p.smap[c] : c) * p.nchan + ch;
+	const int set = p.amap ? p.amap[p.dmap ? p.dmap[c] : c] : 0;
+	const char* A = p.A + set * p.set_stride + (long)p.lmap[ch] * p.astride + toff;
+	const long tl = (long)(td.y - td.x) * TB, tf = tl + (long)(td.z - td.y) * FB;
+	using full_t = std::conditional_t<CX, int4, int2>;
+	using tail_t = std::conditional_t<CX, int2, int>;
+	int4 av[UN];
+	auto fetch = [&](int k, int half) {	// eight k of chunk k
+		if (k >= td.y && k < td.z) {
+			const full_t* q = reinterpret_cast<const full_t*>(A + tl + (long)(k - td.y) * FB) + half * UN * TM + lane;
+#pragma unroll
+			for (int u = 0; u < UN; ++u) {
+				const full_t a = __ldg(q + u * TM);
+				if constexpr (CX) av[u] = a; else av[u] = make_int4(a.x, a.y, 0, 0);
+			}
+		} else {
+			const tail_t* q = reinterpret_cast<const tail_t*>(A + (k < td.y ? (long)(k - td.x) * TB : tf + (long)(k - td.z) * TB)) + half * UN * TM + lane;
+#pragma unroll
+			for (int u = 0; u < UN; ++u) {
+				const tail_t a = __ldg(q + u * TM);
+				if constexpr (CX) av[u] = make_int4(a.x, a.y, 0, 0); else av[u] = make_int4(a, 0, 0, 0);
+			}
+		}
+	};
+	const double2* src = (odd ? p.s1 : p.s0) + v * p.N;
+	const int* ex = (odd ? p.e1 : p.e0) + v * nex;
+	const int kend = min(p.N, td.w * KC);
+	long long rh = 0, rm = 0, ih = 0, im = 0;
+	int E = 0;
+	for (int c0 = td.x; c0 < td.w; c0 += RC) {
+		if (on && c0 + warp < td.w) fetch(c0 + warp, 0);
+		if (c0 == td.x) {
+			prev_wait();
+			if (!on) return;
+		}
+		double2 raw[RC * KC / 256];
+#pragma unroll
+		for (int i = 0; i < RC * KC / 256; ++i) {
+			const int k = c0 * KC + i * 256 + threadIdx.x;
+			raw[i] = k < kend ? src[k] : make_double2(0.0, 0.0);
+		}
+		if (c0 == td.x) {	// the column's largest exponent over the tile's k range
+			for (int t = td.x * KC / TE + lane; t < td.w * KC / TE; t += 32) E = max(E, ex[t]);
+			E = __reduce_max_sync(0xffffffffu, E);
+		} else __syncthreads();
+#pragma unroll
+		for (int i = 0; i < RC * KC / 256; ++i) {
+			const int2 a = quant(raw[i].x, E), b = quant(raw[i].y, E);
+			xs[i * 256 + threadIdx.x] = make_int4(a.x, a.y, b.x, b.y);
+		}
+		__syncthreads();
+		const int ce = min(c0 + RC, td.w);
+		for (int k = c0 + warp; k < ce; k += 8) {
+#pragma unroll
+			for (int half = 0; half < 2; ++half) {
+				const int4* x = xs + (k - c0) * KC + half * UN;
+				if (half || k >= c0 + 8) fetch(k, half);
+				if (k >= td.y && k < td.z) {
+#pragma unroll
+					for (int u = 0; u < UN; ++u) {
+						const int4 y = x[u], a = av[u];
+						rh = madw(a.x, y.x, rh); ih = madw(a.x, y.z, ih); rm = madw(a.x, y.y, rm); im = madw(a.x, y.w, im);
+						rm = madw(a.y, y.x, rm); im = madw(a.y, y.z, im);
+						if constexpr (CX) {
+							const int nz = -a.z, nw = -a.w;
+							rh = madw(nz, y.z, rh); ih = madw(a.z, y.x, ih); rm = madw(nz, y.w, rm); im = madw(a.z, y.y, im);
+							rm = madw(nw, y.z, rm); im = madw(a.w, y.x, im);
+						}
+					}
+				} else {
+#pragma unroll
+					for (int u = 0; u < UN; ++u) {
+						const int4 y = x[u], a = av[u];
+						rm = madw(a.x, y.x, rm); im = madw(a.x, y.z, im);
+						if constexpr (CX) { rm = madw(-a.y, y.z, rm); im = madw(a.y, y.x, im); }
+					}
+				}
+			}
+			flush(rh, rm); flush(ih, im);	// every 16 k: 64 mixed products below 2^55
+		}
+	}
+	red[warp][0][lane] = rh; red[warp][1][lane] = rm; red[warp][2][lane] = ih; red[warp][3][lane] = im;
+	__syncthreads();
+	if (warp) return;
+#pragma unroll
+	for (int w = 1; w < 8; ++w) { rh += red[w][0][lane]; rm += red[w][1][lane]; ih += red[w][2][lane]; im += red[w][3][lane]; }
+	flush(rh, rm); flush(ih, im);
+	const int row = tile * TM + lane, s = p.ea + E - 1078;
+	const double2 y = make_double2(to_double(rh, rm, s, E == 0x7ff), to_double(ih, im, s, E == 0x7ff));
+	const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
+	if (row < p.N) p.dst[o * p.N + row] = y;
+	const int e = group_max(row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);
+	if (lane % TE == 0) p.edst[o * nex + tile * EPT + lane / TE] = e;
 }
 
 // largest exponent of every TE rows of src [nvec][N]
@@ -670,7 +781,7 @@ void band_launch(const band_args& a, int tiles, cudaStream_t st)
 	constexpr int COLS = NB * 8 / KS;
 	constexpr size_t smem = band_smem<NB, KS>();
 	const int ncg = (a.ncols + COLS - 1) / COLS;
-	k_band_apply<NB, KS, CX><<<dim3((unsigned)(tiles * ncg), (unsigned)a.nchan), 256, smem, st>>>(a);
+	launch_after(k_band_apply<NB, KS, CX>, dim3((unsigned)(tiles * ncg), (unsigned)a.nchan), 256, smem, st, a);
 }
 
 template <int NB, int KS>
@@ -690,7 +801,7 @@ void dispatch(const band_args& a, int tiles, cudaStream_t st)
 	const int n = a.ncols;
 	const long per = (long)tiles * a.nchan;
 	auto blocks = [&](int cols) { return per * ((n + cols - 1) / cols); };
-	if (a.amap || n == 1) band_launch<1, 8, CX>(a, tiles, st);
+	if (a.amap || n == 1) launch_after(k_band_one<CX>, dim3((unsigned)(tiles * n), (unsigned)a.nchan), 256, 0, st, a);
 	else if (n == 2) band_launch<2, 8, CX>(a, tiles, st);
 	else if (n <= 4) band_launch<4, 8, CX>(a, tiles, st);
 	else if (n <= 8) band_launch<4, 4, CX>(a, tiles, st);
@@ -866,7 +977,7 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 
 void set_attrs()
 {
-	band_attr<1, 8>(); band_attr<2, 8>(); band_attr<4, 8>(); band_attr<4, 4>(); band_attr<4, 2>(); band_attr<4, 1>(); band_attr<8, 1>();
+	band_attr<2, 8>(); band_attr<4, 8>(); band_attr<4, 4>(); band_attr<4, 2>(); band_attr<4, 1>(); band_attr<8, 1>();
 }
 
 } // namespace

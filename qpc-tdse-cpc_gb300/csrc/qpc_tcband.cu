@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 		const bool odd = p.par && (p.par[cl] & 1);
 		const long o = (long)(p.smap ? p.smap[cl] : cl) * p.nchan + ch;
 		if (cc < p.ncols && (!p.nta || p.step < p.nta[cl])) x = (odd ? p.s1 : p.s0) + o * p.N;
+		prev_wait();
 		load(k0);
 		if (x) {
 			const int* ex = (odd ? p.e1 : p.e0) + o * nex;
@@ -513,10 +514,10 @@ void tc_apply(const tc_store& t, const band_args& a, int* status, int stbit, cud
 	const tc_args q{t.A, t.stride, t.d_list, t.d_first, t.d_off, t.nrow, t.ea, t.ear, status, stbit};
 	const dim3 g((unsigned)(t.ntile * ((a.ncols + TCOLS - 1) / TCOLS)), (unsigned)a.nchan);
 	if (t.db == 8) {
-		if (t.cx) k_tc_apply<true, 8><<<g, THREADS, SMEM, st>>>(a, q);
-		else k_tc_apply<false, 8><<<g, THREADS, SMEM, st>>>(a, q);
-	} else if (t.cx) k_tc_apply<true, 7><<<g, THREADS, SMEM, st>>>(a, q);
-	else k_tc_apply<false, 7><<<g, THREADS, SMEM, st>>>(a, q);
+		if (t.cx) launch_after(k_tc_apply<true, 8>, g, THREADS, SMEM, st, a, q);
+		else launch_after(k_tc_apply<false, 8>, g, THREADS, SMEM, st, a, q);
+	} else if (t.cx) launch_after(k_tc_apply<true, 7>, g, THREADS, SMEM, st, a, q);
+	else launch_after(k_tc_apply<false, 7>, g, THREADS, SMEM, st, a, q);
 }
 
 double tc_cost(const tc_store& t, int nchan, int ncols)
