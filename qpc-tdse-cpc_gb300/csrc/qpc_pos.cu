@@ -12,8 +12,8 @@
 // k_band_apply (the banded products, everything local in l).
 //
 // Both products run in fixed point (qpc_radial.cu), for batches on the tensor cores (qpc_tcband.cu).
-// Against the banded solves (GB300, per step): one wavefunction of 800 x 41 with its dipole 1340 -> 60 us,
-// 400 x 21 287 -> 26 us, 24 wavefunctions of 517 x 30 1120 -> 86 us, 256 of 800 x 41 8.0 -> 1.2 ms; error against
+// Against the banded solves (GB300, per step): one wavefunction of 800 x 41 with its dipole 1340 -> 37 us,
+// 400 x 21 287 -> 15 us, 24 wavefunctions of 517 x 30 1120 -> 77 us, 256 of 800 x 41 8.0 -> 1.13 ms; error against
 // extended precision after 60 steps 3.3e-13 against 4.7e-13.
 #include "qpc_pos.cuh"
 #include "qpc_radial.cuh"

@@ -13,7 +13,7 @@
 // kappa = conj(g_A) g_B.  Between two steps the closing and the opening x1 coupling (same field) are one of power 2.
 // All products in fixed point (qpc_radial.cu).  The banded solves cost the latency of eight recurrences over N rows
 // (4.85 us per row, whatever the batch, until ~10^4 chains fill the FP64 pipe); this form costs 8 N^2 products per
-// channel.  Measured on GB300 at 400 x (25 x 13), two wavefunctions: 22.6 -> 1.2 ms per step (1.85 with Q on the
+// channel.  Measured on GB300 at 400 x (25 x 13), two wavefunctions: 22.6 -> 1.07 ms per step (1.7 with Q on the
 // multiply-adds: 136 -> 40 us each).
 #include "qpc_vpos.cuh"
 #include "qpc_radial.cuh"
