@@ -18,8 +18,9 @@ window sits).  Metric: wavefunction-steps/s.
              (device -> host) per timed step, wall clock
   plain_1wf  the plain one-wavefunction-at-a-time GPU path (n_inst = 1, same
              kernels) on the same grid and fields, device time
-  roofline   the dominant kernel (the coupling sweeps), FP64 flops per launch
-             over its CUDA-event duration, against the measured FP64 peak
+  roofline   the dominant kernel (the banded field-free products as bf16 digit sums), its
+             digit flops per launch over its CUDA-event duration, against the measured
+             bf16 peak (the coupling sweeps against the FP64 peak where the banded solves run)
   cpu_baseline  the CPU oracle (a port of the reference's propagator) on the
              host cores, a bounded sample of the same workload
 
@@ -160,6 +161,37 @@ def chain_flops(n_r, p, chains, power):
     return chains * n_r * power * 2 * per_part
 
 
+def band_digit_flops(n_r, n_l, B, per=15.5):
+    """bf16 flops of one launch of k_tc_apply for the field-free operators (csrc/qpc_tcband.cu): 128-row tiles,
+    stages of 32 k, seven digits of which the leading one vanishes every `per` rows off the diagonal (p = 6),
+    pairs s + t <= 6, a complex product as four real ones."""
+    total = 0.0
+    for r0 in range(0, n_r, 128):
+        r1 = min(n_r, r0 + 128) - 1
+        for k0 in range(0, n_r, 32):
+            s0 = int(max(0, k0 - r1, r0 - k0 - 31) / per)
+            if s0 < 7:
+                total += (7 - s0) * (8 - s0) / 2 * 128 * 32 * 4 * 2.0
+    return total * n_l * B
+
+
+def pos_roofline(ktimes, n_r, n_l, B):
+    """the step's dominant kernel in the position basis"""
+    ms, n = ktimes["fieldfree"]
+    peaks = load_peaks()
+    fl, bf = band_digit_flops(n_r, n_l, B), peaks.get("bf16_tflops")
+    launch_ms = ms / n
+    ach = fl / (launch_ms * 1e-3) / 1e12
+    state = 16.0 * B * n_l * n_r
+    roof = {"bound": "tensor", "kernel": "k_tc_apply (banded field-free products, exact bf16 digits)", "achieved": ach, "peak": bf,
+            "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst, cuBLAS)", "unit": "TFLOP/s", "frac": ach / bf if bf else None,
+            "flops_per_launch": fl, "launch_ms": launch_ms, "traffic": None,
+            "hbm": {"achieved_gbs": 2 * state / (launch_ms * 1e-3) / 1e9, "peak_gbs": peaks.get("hbm_gbs"), "bytes_per_launch": 2 * state}}
+    if peaks.get("hbm_gbs"):
+        roof["hbm"]["frac"] = roof["hbm"]["achieved_gbs"] / peaks["hbm_gbs"]
+    return roof
+
+
 def path_flops(n_r, p, n_l, power=2):
     """FP64 flops of one wavefunction-step of the batched run (FMA = 2): coupling
     chains (n_l - n_l%2 chains, M^2), field-free chains (n_l), the complex-symmetric
@@ -283,6 +315,10 @@ def run_engine(args, sync=None):
                      "frac": path_tflops / fp64_peak()["tflops"]}}
     if roof["hbm"]["achieved_gbs"] and peaks.get("hbm_gbs"):
         roof["hbm"]["frac"] = roof["hbm"]["achieved_gbs"] / peaks["hbm_gbs"]
+    if not ktimes["factor"][1] and ktimes["fieldfree"][1]:  # no factorisations: the position basis
+        roof = pos_roofline(ktimes, n_r, n_l, B)
+        roof["fp64_equivalent"] = {"flops_per_wf_step": path_flops(n_r, p, n_l), "achieved_tflops": path_tflops,
+                                   "ratio_to_fp64_peak": path_tflops / fp64_peak()["tflops"], "note": "FP64 flops of the banded solves this replaces"}
     kt = {k: {"ms_total": v[0], "launches": v[1]} for k, v in ktimes.items()}
     tuning = prop.tuning()
     prop.close()
@@ -639,11 +675,10 @@ def run_c0(args):
         "e2e": {"value": nt / e2e_s, "unit": "wf-steps/s", "h2d_bytes_per_step": (c0.nbytes + f.nbytes) / nt,
                 "d2h_bytes_per_step": out.nbytes / nt},
         "gpu_launches": int(launches), "final_norm": float(norm), "tuning": tuning, "kernel_times": ktimes,
-        "roofline": {"bound": "fp64 (latency: one wavefunction's recurrences are sequential in r)",
-                     "kernel": "whole step", "achieved": path_flops(n_r, p, n_l) * nt / (dev_ms * 1e-3) / 1e12,
-                     "peak": fp64_peak()["tflops"], "unit": "TFLOP/s",
-                     "frac": path_flops(n_r, p, n_l) * nt / (dev_ms * 1e-3) / 1e12 / fp64_peak()["tflops"],
-                     "flops_per_step": path_flops(n_r, p, n_l)},
+        "roofline": {"bound": "latency (two dependent kernels per step)", "kernel": "whole step",
+                     "achieved": None, "peak": fp64_peak()["tflops"], "unit": "TFLOP/s", "frac": None,
+                     "fp64_equivalent": {"achieved": path_flops(n_r, p, n_l) * nt / (dev_ms * 1e-3) / 1e12,
+                                         "flops_per_step": path_flops(n_r, p, n_l), "note": "FP64 flops of the banded solves this replaces"}},
         "cpu_baseline": cpu, "clocks": clk.summary(),
     }
 
@@ -773,10 +808,12 @@ def run_pcs(args):
                                "theta in [0,pi] x 181, one phi" % B, "inputs": "resident batch (134 MB) > L2"},
         "e2e": {"value": B / e2e_s, "unit": "wavefunctions/s", "h2d_bytes_per_step": int(states.nbytes),
                 "d2h_bytes_per_step": int(out.nbytes)},
-        "gpu_launches": 2 * K,
-        "roofline": {"bound": "fp64", "kernel": "k_pcs_proj + k_pcs_out (one measurement)", "achieved": tfl,
-                     "peak": fp64_peak()["tflops"], "unit": "TFLOP/s", "frac": tfl / fp64_peak()["tflops"],
-                     "flops_per_launch": fl_proj + fl_out, "flops_projection": fl_proj},
+        "gpu_launches": 4 * K,
+        "roofline": {"bound": "fp64 (k_pcs_out; the projections run as bf16 digits on the tensor cores)",
+                     "kernel": "k_exponents + k_tc_apply + k_pcs_join + k_pcs_out (one measurement)",
+                     "achieved": fl_out / (dev_ms * 1e-3) / 1e12, "peak": fp64_peak()["tflops"], "unit": "TFLOP/s",
+                     "frac": fl_out / (dev_ms * 1e-3) / 1e12 / fp64_peak()["tflops"], "flops_per_launch": fl_out,
+                     "fp64_equivalent": {"achieved": tfl, "flops_projection": fl_proj}},
         "cpu_baseline": {"value": cpu_rate, "unit": "wavefunctions/s", "cores": os.cpu_count(), "kind": "port",
                          "sample": "%d wavefunctions through the numpy oracle of measure_prj (numpy's BLAS may use every host core)" % n_cpu},
         "tables_setup_s": setup_s, "clocks": clk.summary(),

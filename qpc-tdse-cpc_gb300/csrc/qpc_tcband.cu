@@ -7,10 +7,10 @@
 // output are combined as integers and rounded once to FP64; what the dropped pairs carry is 2^-53 of the column's largest
 // element in one sum of ~250 (the banded solves this replaces stood at 2^-47).
 //
-// One block: 128 rows of one operator, 32 columns (64 with the imaginary parts).  Warp 0 brings the operator's digit
+// One block: 128 rows of one operator, TC = 16, 24 or 32 columns (twice with the imaginary parts).  Warp 0 brings the operator's digit
 // planes (16 KB: 128 rows, 32 k, real | imaginary part, or two digits of a real operator) by bulk copies into a ring;
-// warp 1 issues the MMAs (M 128, K 16): digit t of the columns is rows 64 t .. of one tile and level l columns 64 l .. of
-// the accumulators, so digit s meets all the digits it pairs with in one or two instructions of N <= 256 (one pair at a
+// warp 1 issues the MMAs (M 128, K 16): digit t of the columns is rows 2 TC t .. of one tile and level l columns 2 TC l ..
+// of the accumulators, so digit s meets all the digits it pairs with in one or two instructions of N <= 256 (one pair at a
 // time, N = 64, took 85 cycles for 32 of math); sixteen warps split the columns into digit planes, two halves of 32 k in
 // turn, and at the end read the accumulators.  For a complex operator the columns are there as (xr, xi) and (-xi, xr), so
 // that Fr and Fi take one plane each.  Digits that vanish are not formed: the entries of F~ lose a leading digit every ~15
@@ -35,12 +35,12 @@ void tc_store::release()
 namespace {
 
 constexpr int TR = 128;			// rows of a block
-constexpr int TCOLS = 32;		// columns of a block
+constexpr int TCMAX = 32;		// most columns of a block (TC: 16, 24 or 32)
 constexpr int KS = 32;			// k of a stage
 constexpr int NA = 6;			// operator planes in the ring
-constexpr int PLANE_A = TR * 128, PLANE_B = 2 * TCOLS * 128;
+constexpr int PLANE_A = TR * 128;
 constexpr int COLUMNS = 1024;	// bytes of barriers and column data, in front
-constexpr int B_MAX = 16 * PLANE_B, SMEM = COLUMNS + B_MAX + NA * PLANE_A + 1024;	// the last for alignment
+constexpr int B_MAX = 16 * 2 * TCMAX * 128, SMEM = COLUMNS + B_MAX + NA * PLANE_A + 1024;	// the last for alignment
 constexpr int DROP = 9;			// bits of an output's sum that are rounded off (the dropped pairs are worth 10)
 constexpr int SPLIT = 512, THREADS = 64 + SPLIT;
 
@@ -106,28 +106,29 @@ __device__ __forceinline__ uint32_t desc_lo(uint32_t a) { return (a >> 4) | (1u 
 __device__ __forceinline__ uint64_t desc(uint32_t lo) { return ((tc::sw128_desc(0) >> 32) << 32) | lo; }
 
 // every product of digit D of an operator plane (two halves of 32 k: real | imaginary, or D | D + 1) with the digits of
-// the columns.  Digit t of the columns are rows 64 t .. 64 t + 63 of one tile and level l is tensor-memory columns
-// 64 l .., so one instruction multiplies by up to four digits at once
-template <bool CX, int ND, int D>
+// the columns.  Digit t of the columns are rows 2 TC t .. of one tile and level l is tensor-memory columns
+// 2 TC l .., so one instruction multiplies by up to four digits at once
+template <bool CX, int ND, int TC, int D>
 __device__ __forceinline__ void plane_products(uint32_t tmem, uint32_t a, uint32_t b, bool start)
 {
 #pragma unroll
 	for (int part = 0; part < 2; ++part) {
-		const int d = CX ? D : D + part, cols = (ND - d) * 2 * TCOLS, n = cols > 256 ? cols / 2 : cols;
-		const uint32_t o = (CX && part) ? (ND * PLANE_B) >> 4 : 0u;	// Fi meets (-xi, xr), else (xr, xi)
+		const int d = CX ? D : D + part, cols = (ND - d) * 2 * TC;
+		const int n = cols > 256 ? (cols / 2 + 15) & ~15 : cols;	// N: a multiple of 16, at most 256
+		const uint32_t o = (CX && part) ? (ND * 2 * TC * 128) >> 4 : 0u;	// Fi meets (-xi, xr), else (xr, xi)
 #pragma unroll
 		for (int c = 0; c < cols; c += n)
 #pragma unroll
 			for (int k = 0; k < 2; ++k)
-				tc::mma_bf16(tmem + (uint32_t)(d * 2 * TCOLS + c), desc(a + 4u * part + 2u * k), desc(b + o + (uint32_t)c * 8u + 2u * k), tc::idesc_bf16(TR, n),
-					(D == 0 && part == 0 && k == 0) ? (start ? 0u : 1u) : 1u);
+				tc::mma_bf16(tmem + (uint32_t)(d * 2 * TC + c), desc(a + 4u * part + 2u * k), desc(b + o + (uint32_t)c * 8u + 2u * k),
+					tc::idesc_bf16(TR, cols - c < n ? cols - c : n), (D == 0 && part == 0 && k == 0) ? (start ? 0u : 1u) : 1u);
 	}
 }
 
-template <bool CX, int DB>
+template <bool CX, int DB, int TC>
 __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, const tc_args t)
 {
-	constexpr int ND = digits<DB>::ND;
+	constexpr int ND = digits<DB>::ND, PLANE_B = 2 * TC * 128;
 	constexpr long long BIAS = digits<DB>::BIAS;
 	extern __shared__ char dyn[];
 	const uint32_t raw = tc::smem_u32(dyn), base = (raw + 1023u) & ~1023u;
@@ -138,8 +139,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 	const double2** sp = reinterpret_cast<const double2**>(sm + 320);
 	volatile int* bad = reinterpret_cast<volatile int*>(sm + 576);
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int ncg = (p.ncols + TCOLS - 1) / TCOLS;
-	const int cg = blockIdx.x % ncg, tile = blockIdx.x / ncg, ch = blockIdx.y, col0 = cg * TCOLS;
+	const int ncg = (p.ncols + TC - 1) / TC;
+	const int cg = blockIdx.x % ncg, tile = blockIdx.x / ncg, ch = blockIdx.y, col0 = cg * TC;
 	const int4 span = t.first[tile];	// stages, and the k they cover
 	const int e0 = span.x, e1 = span.y;
 	if (threadIdx.x == 0) {
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
 	// a splitter thread has two consecutive k of one column in every stage; a warp columns c and c + 4, whose swizzled rows
-	// fall on different banks
+	// fall on different banks (those of columns beyond TC only take part in the waits)
 	const int kq = lane & 15, c = ((warp - 2) & 3) + 4 * (lane >> 4) + 8 * ((warp - 2) >> 2);
 	const double2* x = nullptr;
 	int E = 0;
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 		const int cc = col0 + c, cl = min(cc, p.ncols - 1), k0 = t.list[e0].x, nex = p.ntile * EPT;
 		const bool odd = p.par && (p.par[cl] & 1);
 		const long o = (long)(p.smap ? p.smap[cl] : cl) * p.nchan + ch;
-		if (cc < p.ncols && (!p.nta || p.step < p.nta[cl])) x = (odd ? p.s1 : p.s0) + o * p.N;
+		if (c < TC && cc < p.ncols && (!p.nta || p.step < p.nta[cl])) x = (odd ? p.s1 : p.s0) + o * p.N;
 		prev_wait();
 		load(k0);
 		if (x) {
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 			for (int i = span.z / TE + kq; i < min(nex, span.w / TE); i += 16) E = max(E, ex[i]);
 		}
 		for (int s = 1; s < 16; s <<= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, s));
-		if (kq == 0) { sE[c] = E; sp[c] = x; }
+		if (kq == 0 && c < TC) { sE[c] = E; sp[c] = x; }
 	}
 	tc::fence_before();
 	__syncthreads();
@@ -220,14 +221,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 				const uint32_t a = desc_lo(planeA + slot * PLANE_A);
 				if (lane == 0) {
 					switch (s) {	// the first stage has every digit: all levels start there
-					case 0: plane_products<CX, ND, 0>(tmem, a, b, i == 0); break;
-					case 1: if (CX) plane_products<CX, ND, 1>(tmem, a, b, false); break;
-					case 2: plane_products<CX, ND, 2>(tmem, a, b, false); break;
-					case 3: if (CX) plane_products<CX, ND, 3>(tmem, a, b, false); break;
-					case 4: plane_products<CX, ND, 4>(tmem, a, b, false); break;
-					case 5: if (CX) plane_products<CX, ND, 5>(tmem, a, b, false); break;
-					case 6: plane_products<CX, ND, 6>(tmem, a, b, false); break;
-					case 7: if (CX && ND == 8) plane_products<CX, ND, ND - 1>(tmem, a, b, false); break;
+					case 0: plane_products<CX, ND, TC, 0>(tmem, a, b, i == 0); break;
+					case 1: if (CX) plane_products<CX, ND, TC, 1>(tmem, a, b, false); break;
+					case 2: plane_products<CX, ND, TC, 2>(tmem, a, b, false); break;
+					case 3: if (CX) plane_products<CX, ND, TC, 3>(tmem, a, b, false); break;
+					case 4: plane_products<CX, ND, TC, 4>(tmem, a, b, false); break;
+					case 5: if (CX) plane_products<CX, ND, TC, 5>(tmem, a, b, false); break;
+					case 6: plane_products<CX, ND, TC, 6>(tmem, a, b, false); break;
+					case 7: if (CX && ND == 8) plane_products<CX, ND, TC, ND - 1>(tmem, a, b, false); break;
 					}
 					tc::commit(emptyA + 8 * slot);
 				}
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 		// ---- the columns' digits
 		uint32_t at[2];
 #pragma unroll
-		for (int h = 0; h < 2; ++h)	// 128-byte swizzle; rows c and c + 32 alike
+		for (int h = 0; h < 2; ++h)	// 128-byte swizzle; rows c and c + TC alike
 			at[h] = planeB + (uint32_t)c * 128u + (((uint32_t)(4 * h + (kq >> 2)) ^ (uint32_t)(c & 7)) << 4) + 4u * (kq & 3);
 		int2 at_e = t.list[e0], next = t.list[min(e0 + 1, e1 - 1)];
 		bool ok = true;
@@ -261,9 +262,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 			if (i >= 2 && !tc::mbar_wait(emptyB + 8 * h, ((i >> 1) - 1) & 1)) { ok = false; break; }
 #pragma unroll
 			for (int s = 0; s < ND; ++s) {
-				if (s >= nd) break;
+				if (s >= nd || c >= TC) break;
 				const uint32_t r = __byte_perm(digit_bits<DB>(re[0], s), digit_bits<DB>(re[1], s), 0x7632), m = __byte_perm(digit_bits<DB>(im[0], s), digit_bits<DB>(im[1], s), 0x7632);
-				const uint32_t q = at[h] + (uint32_t)s * PLANE_B, half = TCOLS * 128u;
+				const uint32_t q = at[h] + (uint32_t)s * PLANE_B, half = TC * 128u;
 				st_shared(q, r);
 				st_shared(q + half, m);
 				if (CX) {
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 		// ---- the levels of 128 rows x 64 columns: a warp its quarter of the rows and 8 columns
 		const bool fin = tc::mbar_wait(done, 0);
 		tc::fence_after();
-		if (__all_sync(0xffffffffu, fin && ok && !*bad)) {
+		if (__all_sync(0xffffffffu, fin && ok && !*bad) && (warp - 2) >> 2 < TC / 8) {
 			const int qr = warp & 3, c8 = 8 * ((warp - 2) >> 2);
 			const int row = tile * TR + qr * 32 + lane;
 			const bool in = row < t.nrow;
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 				for (int part = 0; part < 2; ++part) {
 					uint32_t lv[ND][4];
 #pragma unroll
-					for (int l = 0; l < ND; ++l) tc::ld4(tl + (uint32_t)(l * 2 * TCOLS + part * TCOLS + c0), lv[l]);
+					for (int l = 0; l < ND; ++l) tc::ld4(tl + (uint32_t)(l * 2 * TC + part * TC + c0), lv[l]);
 					tc::wait_ld();
 #pragma unroll
 					for (int j = 0; j < 4; ++j) {
@@ -484,8 +485,12 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 	QPC_CUDA(cudaMemcpy(d_at, at.data(), sizeof(size_t) * at.size(), cudaMemcpyHostToDevice));
 	k_tc_planes<DB><<<dim3((unsigned)list.size(), nop), 256, 0, st>>>(m, t.d_list, d_tile, d_at, t.stride, t.A, t.cx);
 	QPC_CUDA(cudaGetLastError());
-	QPC_CUDA(cudaFuncSetAttribute(k_tc_apply<true, DB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-	QPC_CUDA(cudaFuncSetAttribute(k_tc_apply<false, DB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+	auto attr = [](auto kern) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); };
+	if (t.cx) {
+		QPC_CUDA(attr(k_tc_apply<true, DB, 16>)); QPC_CUDA(attr(k_tc_apply<true, DB, 24>)); QPC_CUDA(attr(k_tc_apply<true, DB, 32>));
+	} else {
+		QPC_CUDA(attr(k_tc_apply<false, DB, 16>)); QPC_CUDA(attr(k_tc_apply<false, DB, 24>)); QPC_CUDA(attr(k_tc_apply<false, DB, 32>));
+	}
 	*ok = true;
 	return wait_on(st);
 }
@@ -509,23 +514,49 @@ int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, 
 	return rc;
 }
 
-void tc_apply(const tc_store& t, const band_args& a, int* status, int stbit, cudaStream_t st)
-{
-	const tc_args q{t.A, t.stride, t.d_list, t.d_first, t.d_off, t.nrow, t.ea, t.ear, status, stbit};
-	const dim3 g((unsigned)(t.ntile * ((a.ncols + TCOLS - 1) / TCOLS)), (unsigned)a.nchan);
-	if (t.db == 8) {
-		if (t.cx) launch_after(k_tc_apply<true, 8>, g, THREADS, SMEM, st, a, q);
-		else launch_after(k_tc_apply<false, 8>, g, THREADS, SMEM, st, a, q);
-	} else if (t.cx) launch_after(k_tc_apply<true, 7>, g, THREADS, SMEM, st, a, q);
-	else launch_after(k_tc_apply<false, 7>, g, THREADS, SMEM, st, a, q);
-}
+namespace {
 
-double tc_cost(const tc_store& t, int nchan, int ncols)
+// cycles of a launch with blocks of tc columns: twice the tensor-core math of an average tile and 18 thousand of a block's
+// own, one block per SM.  (Blocks of 32 only before: 48 wavefunctions
+// of 800 x 41, 20 steps 5.60 -> 5.39 ms, 24 of 517 x 30, 30 steps 2.30 -> 2.23, 8 of 640 x 25, 20 steps 2.53 -> 2.44.)
+double cycles(const tc_store& t, int nchan, int ncols, int tc)
 {
 	double mma = 0.0;
 	for (int w : t.work) mma += w;
-	const double blocks = (double)t.ntile * nchan * ((ncols + TCOLS - 1) / TCOLS), one = (2.0 * mma / t.ntile + 18e3) / 2000.0;
-	return std::ceil(blocks / 152.0) * one;
+	const double blocks = (double)t.ntile * nchan * ((ncols + tc - 1) / tc);
+	return std::ceil(blocks / 152.0) * (2.0 * mma / t.ntile * tc / 32.0 + 18e3);
 }
+
+int columns(const tc_store& t, int nchan, int ncols)
+{
+	int best = 32;
+	for (int tc : {24, 16})
+		if (cycles(t, nchan, ncols, tc) < cycles(t, nchan, ncols, best)) best = tc;
+	return best;
+}
+
+template <bool CX, int DB>
+void launch(const tc_args& q, const tc_store& t, const band_args& a, cudaStream_t st)
+{
+	const int tc = columns(t, a.nchan, a.ncols);
+	const dim3 g((unsigned)(t.ntile * ((a.ncols + tc - 1) / tc)), (unsigned)a.nchan);
+	if (tc == 16) launch_after(k_tc_apply<CX, DB, 16>, g, THREADS, SMEM, st, a, q);
+	else if (tc == 24) launch_after(k_tc_apply<CX, DB, 24>, g, THREADS, SMEM, st, a, q);
+	else launch_after(k_tc_apply<CX, DB, 32>, g, THREADS, SMEM, st, a, q);
+}
+
+} // namespace
+
+void tc_apply(const tc_store& t, const band_args& a, int* status, int stbit, cudaStream_t st)
+{
+	const tc_args q{t.A, t.stride, t.d_list, t.d_first, t.d_off, t.nrow, t.ea, t.ear, status, stbit};
+	if (t.db == 8) {
+		if (t.cx) launch<true, 8>(q, t, a, st);
+		else launch<false, 8>(q, t, a, st);
+	} else if (t.cx) launch<true, 7>(q, t, a, st);
+	else launch<false, 7>(q, t, a, st);
+}
+
+double tc_cost(const tc_store& t, int nchan, int ncols) { return cycles(t, nchan, ncols, columns(t, nchan, ncols)) / 2000.0; }
 
 } // namespace qpc

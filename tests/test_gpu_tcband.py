@@ -1,5 +1,5 @@
 """The digit products on the tensor cores (csrc/qpc_tcband.cu) against the multiply-adds (QPC_POS_TC=0) where the kernel
-changes shape: the edges of its 128 rows, 32 columns and 32-deep stages, grids below a stage, every spline degree, several
+changes shape: the edges of its 128 rows, 16, 24 or 32 columns and 32-deep stages, grids below a stage, every spline degree, several
 m, uneven runs, the mask, zero states.  A product drops less than 2^-49 of a column's largest element per output, so
 sqrt(N) 2^-49 of the norm: 14 products of up to 400 rows stay below 5e-13."""
 import numpy as np
@@ -22,7 +22,8 @@ def _both(monkeypatch, run):
 
 @pytest.mark.parametrize("n_r,p,n_l,B", [
     (31, 6, 2, 1), (33, 5, 3, 2), (97, 3, 9, 3), (127, 4, 8, 31), (128, 7, 16, 32), (129, 8, 5, 33), (160, 6, 3, 63), (161, 6, 4, 64),
-    (255, 5, 6, 65), (257, 7, 4, 12), (385, 6, 3, 17), (400, 6, 5, 97)])
+    (255, 5, 6, 65), (257, 7, 4, 12), (385, 6, 3, 17), (400, 6, 5, 97),
+    (257, 6, 20, 48), (270, 6, 20, 41), (257, 6, 30, 96), (300, 5, 30, 85)])	# blocks of 24 and of 32 columns, full and ragged; 16 above
 def test_runs_agree(q, monkeypatch, n_r, p, n_l, B):
     a, b = _both(monkeypatch, lambda: _run(q, n_r, p, n_l, B)[0])
     for k in range(B):
