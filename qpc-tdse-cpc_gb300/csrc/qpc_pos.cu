@@ -35,8 +35,8 @@ constexpr int LMAX = 128;	// most l channels
 // (28 instructions per pair and position).  The dipole of f(r) = r is sum_k lambda_k r_j (|z+|^2 - |z-|^2) =
 // sum_k 4 lambda_k r_j Re(conj(E_k) O_k).  PT = 32 is bound by the multiply-adds; with too few blocks to fill the
 // SMs a block's own latency counts, and PT = 8 cuts it (four times the blocks, a quarter of the serial products).
-// 80 registers (a few spilled at G = 3) for three blocks per SM, coefficients stored in the order a task reads them:
-// 256 wavefunctions of 800 x 41 570 -> 450 us (multiply-adds alone 270), 24 of 517 x 30 36 -> 28 us.
+// Three or four blocks per SM (80 or 64 registers, a few spilled), coefficients stored in the order a task reads them:
+// 256 wavefunctions of 800 x 41 570 -> 438 us (multiply-adds alone 270), 24 of 517 x 30 36 -> 28 us.
 struct angle_args {
 	double2* y;		// [slot][M][L][N], in place
 	int* ex;		// [slot][M][L][ntile * EPT]
@@ -63,8 +63,8 @@ __device__ __forceinline__ int power_of(long s, long nt, int cmode)
 	return (s == 0 || s == nt) ? 1 : 2;
 }
 
-template <int G, int PT>
-__global__ void __launch_bounds__(256, 3) k_angle(const angle_args p)
+template <int G, int PT, int BPS>
+__global__ void __launch_bounds__(256, BPS) k_angle(const angle_args p)
 {
 	constexpr int NV = 8 * 32 / PT, TPT = TM / PT;	// virtual warps; blocks per tile
 	extern __shared__ double2 sm[];
@@ -225,15 +225,16 @@ struct pos_path {
 	int zcount = 0;
 	int angle_g = 3;		// outputs per task of k_angle, PT = 32
 	bool angle_small = false;	// PT = 8, one output per task
+	bool angle_many = false;	// four blocks per SM
 };
 
 
 namespace {
 
-template <int G>
+template <int G, int BPS>
 void angle_launch(const pos_path* p, const angle_args& a, int slots, cudaStream_t st)
 {
-	launch_after(k_angle<G, 32>, dim3((unsigned)((long)slots * p->M * p->ntile)), 256, sizeof(double2) * 2 * 32 * p->L, st, a);
+	launch_after(k_angle<G, 32, BPS>, dim3((unsigned)((long)slots * p->M * p->ntile)), 256, sizeof(double2) * 2 * 32 * p->L, st, a);
 }
 
 int build(pos_path* p, const pos_setup& in, bool* ok)
@@ -252,6 +253,10 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 	}
 	// fewer blocks than SMs with 32 positions each: 8
 	p->angle_small = (long)p->B * M * p->ntile <= 304;
+	// more than three per SM: four, with two outputs per task (256 wavefunctions of 800 x 41 460 -> 438 us, 48 108 -> 98;
+	// 24 of 517 x 30, where three hold every block at once, 28 -> 29.6)
+	p->angle_many = (long)p->B * M * p->ntile > 456;
+	if (p->angle_many) p->angle_g = 2;
 	// the transforms' limbs as the tasks read them; a task's outputs beyond the last are zero
 	const int np = p->npair, nE = np + (L & 1), nl0 = (L + 1) / 2, nl1 = L / 2, G = p->angle_small ? 1 : p->angle_g;
 	const int gE = (nE + G - 1) / G, gO = (np + G - 1) / G, g0 = (nl0 + G - 1) / G, g1 = (nl1 + G - 1) / G;
@@ -275,9 +280,10 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
 	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
 	const int smem = (int)(sizeof(double2) * 64 * LMAX);
-	cudaFuncSetAttribute(k_angle<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-	cudaFuncSetAttribute(k_angle<3, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-	cudaFuncSetAttribute(k_angle<4, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<2, 32, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<3, 32, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<2, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	cudaFuncSetAttribute(k_angle<4, 32, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	return QPC_OK;
 }
 
@@ -372,11 +378,14 @@ int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf)
 			a.zpart = p->zpart + (size_t)p->zcount * p->B * p->M * p->ntile * (p->angle_small ? EPT : 1);
 			++p->zcount;
 		}
-		if (p->angle_small) launch_after(k_angle<1, 8>, dim3((unsigned)((long)slots * p->M * p->ntile * EPT)), 256, sizeof(double2) * 2 * 8 * p->L, st, a);
+		if (p->angle_small) launch_after(k_angle<1, 8, 3>, dim3((unsigned)((long)slots * p->M * p->ntile * EPT)), 256, sizeof(double2) * 2 * 8 * p->L, st, a);
 		else switch (p->angle_g) {
-		case 2: angle_launch<2>(p, a, slots, st); break;
-		case 3: angle_launch<3>(p, a, slots, st); break;
-		default: angle_launch<4>(p, a, slots, st); break;
+		case 2:
+			if (p->angle_many) angle_launch<2, 4>(p, a, slots, st);
+			else angle_launch<2, 3>(p, a, slots, st);
+			break;
+		case 3: angle_launch<3, 3>(p, a, slots, st); break;
+		default: angle_launch<4, 3>(p, a, slots, st); break;
 		}
 		++*r.launches;
 	};

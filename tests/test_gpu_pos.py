@@ -51,7 +51,7 @@ def _run(q, n_r, p, n_l, B, n_m=1, m0=0, own=False, kind="run", steps=9, seed=0)
 
 @pytest.mark.parametrize("n_r,p,n_l,B", [
     (32, 6, 2, 1), (33, 5, 3, 2), (63, 3, 9, 3), (64, 4, 8, 5), (65, 7, 16, 9), (96, 8, 17, 17), (97, 6, 33, 33), (289, 6, 5, 1),
-    (300, 5, 6, 65), (321, 7, 4, 97), (256, 6, 41, 2), (160, 4, 64, 4), (40, 6, 128, 2)])
+    (300, 5, 6, 65), (321, 7, 4, 97), (256, 6, 41, 2), (160, 4, 64, 4), (40, 6, 128, 2), (161, 6, 7, 90), (64, 4, 41, 229), (33, 5, 2, 228)])
 def test_runs_agree(q, monkeypatch, n_r, p, n_l, B):
     a, b = _both(q, monkeypatch, lambda: _run(q, n_r, p, n_l, B)[0])
     for k in range(B):
