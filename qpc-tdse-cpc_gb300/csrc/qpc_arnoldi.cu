@@ -924,26 +924,27 @@ int qpc_arnoldi_create(const qpc_dims* dims, const double* S, const double* R, c
 		(rc = dalloc(&h->msub, (size_t)B)) || (rc = dalloc(&h->flag, (size_t)B)) || (rc = dalloc(&h->status, 1)) ||
 		(rc = dalloc(&h->nt, (size_t)B)))
 		return fail(rc);
-	if (cudaMemcpy(h->S, S, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->R, R, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->Lrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->Lcol, lcol.data(), sizeof(double) * lcol.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->SM, sM.data(), sizeof(double) * sM.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->SN, sN.data(), sizeof(double) * sN.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->SI, sI.data(), sizeof(double) * sI.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->SF, sF.data(), sizeof(double) * sF.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->SB, sB.data(), sizeof(double) * sB.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->dinv, di.data(), sizeof(double) * N, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->H, Hr.data(), sizeof(double) * Hr.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->y10, y10, sizeof(double) * d.n_m * d.n_l, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemset(h->X, 0, sizeof(double2) * nst) != cudaSuccess || cudaMemset(h->cnt, 0, sizeof(unsigned) * B) != cudaSuccess ||
-		cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess) {
+	if (cudaMemcpyAsync(h->S, S, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->R, R, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->Lrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->Lcol, lcol.data(), sizeof(double) * lcol.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->SM, sM.data(), sizeof(double) * sM.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->SN, sN.data(), sizeof(double) * sN.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->SI, sI.data(), sizeof(double) * sI.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->SF, sF.data(), sizeof(double) * sF.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->SB, sB.data(), sizeof(double) * sB.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->dinv, di.data(), sizeof(double) * N, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->H, Hr.data(), sizeof(double) * Hr.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->y10, y10, sizeof(double) * d.n_m * d.n_l, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemsetAsync(h->X, 0, sizeof(double2) * nst, h->stream) != cudaSuccess || cudaMemsetAsync(h->cnt, 0, sizeof(unsigned) * B, h->stream) != cudaSuccess ||
+		cudaMemsetAsync(h->status, 0, sizeof(int), h->stream) != cudaSuccess) {
 		set_error("device upload failed");
 		return fail(QPC_ERR_CUDA);
 	}
 	auto attr = [](auto kern) { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SB_SMEM); };
 	attr(k_ar_sinv_blk<2>); attr(k_ar_sinv_blk<3>); attr(k_ar_sinv_blk<4>); attr(k_ar_sinv_blk<5>); attr(k_ar_sinv_blk<6>); attr(k_ar_sinv_blk<7>);
 	attr(k_ar_sinv_blk<8>);
+	if ((rc = wait_on(h->stream))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }

@@ -57,6 +57,11 @@ inline int wait_on(cudaStream_t st)
 	}
 }
 
+// Copies to the device and fills go through the stream of the work that reads them (cudaMemcpyAsync, cudaMemsetAsync):
+// a plain cudaMemcpy or cudaMemset belongs to the legacy stream, may return before the transfer has reached the device,
+// and the library's streams, which do not block on that one, would not wait for it.  The host side of such a copy is
+// kept until the stream has been waited for.
+
 // device -> host copy of a result: wait (bounded) for the work queued before it, then
 // copy.  Waiting first means the copy never blocks on queued work (a copy into pageable
 // memory may block inside the driver until the stream reaches it, without a bound), and a

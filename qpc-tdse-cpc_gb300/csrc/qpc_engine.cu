@@ -1006,13 +1006,14 @@ static int need_chains(qpc_lgwz* h)
 		if ((rc = dalloc(&h->spf_ff, sf.size())) || (rc = dalloc(&h->spb_ff, sb.size())) ||
 			(rc = dalloc(&h->spf_c, nblk_c * N * P)) || (rc = dalloc(&h->spb_c, nblk_c * N * P)))
 			return rc;
-		if (cudaMemcpy(h->spf_ff, sf.data(), sizeof(double2) * sf.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-			cudaMemcpy(h->spb_ff, sb.data(), sizeof(double2) * sb.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-			cudaMemset(h->spf_c, 0, sizeof(double2) * nblk_c * N * P) != cudaSuccess ||
-			cudaMemset(h->spb_c, 0, sizeof(double2) * nblk_c * N * P) != cudaSuccess) {
+		if (cudaMemcpyAsync(h->spf_ff, sf.data(), sizeof(double2) * sf.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+			cudaMemcpyAsync(h->spb_ff, sb.data(), sizeof(double2) * sb.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+			cudaMemsetAsync(h->spf_c, 0, sizeof(double2) * nblk_c * N * P, h->stream) != cudaSuccess ||
+			cudaMemsetAsync(h->spb_c, 0, sizeof(double2) * nblk_c * N * P, h->stream) != cudaSuccess) {
 			set_error("initial device copies failed");
 			return QPC_ERR_CUDA;
 		}
+		if ((rc = wait_on(h->stream))) return rc;
 	}
 	h->ffh = std::vector<double2>();
 	h->chains_ready = true;
@@ -1193,12 +1194,12 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 		(rc = dalloc(&h->status, 1)) || (rc = dalloc(&h->red, (size_t)h->B * M * L * 2)) ||
 		(rc = dalloc(&h->ntf, h->B)) || (rc = dalloc(&h->ntt, h->B)))
 		return fail(rc);
-	if (cudaMemcpy(h->S, S, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->R, R, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->Vh, Vh.data(), sizeof(double) * Vh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->lamp, lamp.data(), sizeof(double) * lamp.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->ff, ffh.data(), sizeof(double2) * ffh.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemset(h->hostlay, 0, sizeof(double2) * sl) != cudaSuccess || cudaMemset(h->status, 0, sizeof(int)) != cudaSuccess) {
+	if (cudaMemcpyAsync(h->S, S, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->R, R, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->Vh, Vh.data(), sizeof(double) * Vh.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->lamp, lamp.data(), sizeof(double) * lamp.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemcpyAsync(h->ff, ffh.data(), sizeof(double2) * ffh.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+		cudaMemsetAsync(h->hostlay, 0, sizeof(double2) * sl, h->stream) != cudaSuccess || cudaMemsetAsync(h->status, 0, sizeof(int), h->stream) != cudaSuccess) {
 		set_error("initial device copies failed");
 		return fail(QPC_ERR_CUDA);
 	}
@@ -1228,11 +1229,12 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 		std::vector<int> id(h->B);
 		for (int k = 0; k < h->B; ++k) id[k] = k;
 		if ((rc = dalloc(&h->ffmap, h->B)) || (rc = dalloc(&h->ffmap_id, h->B))) return fail(rc);
-		if (cudaMemcpy(h->ffmap_id, id.data(), sizeof(int) * h->B, cudaMemcpyHostToDevice) != cudaSuccess) {
+		if (cudaMemcpyAsync(h->ffmap_id, id.data(), sizeof(int) * h->B, cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
 			set_error("initial device copies failed");
 			return fail(QPC_ERR_CUDA);
 		}
 		h->ffmap_cur = h->ffmap_id;
+		if ((rc = wait_on(h->stream))) return fail(rc);	// before id goes
 	}
 	const char* ltc = getenv("QPC_LTRANS_TC");
 	h->lt_kb = (ltc && atoi(ltc) == 0) ? 0 : ltrans_kb(L);
@@ -1246,11 +1248,12 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 		std::vector<int> fex((size_t)M * 2 * 2 * h->lt_kb);
 		ltrans_digits(Vh.data(), M, L, np, h->lt_kb, dig.data(), fex.data());
 		if ((rc = dalloc(&h->lt_dig, dig.size())) || (rc = dalloc(&h->lt_fex, fex.size()))) return fail(rc);
-		if (cudaMemcpy(h->lt_dig, dig.data(), sizeof(uint16_t) * dig.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-			cudaMemcpy(h->lt_fex, fex.data(), sizeof(int) * fex.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+		if (cudaMemcpyAsync(h->lt_dig, dig.data(), sizeof(uint16_t) * dig.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+			cudaMemcpyAsync(h->lt_fex, fex.data(), sizeof(int) * fex.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
 			set_error("initial device copies failed");
 			return fail(QPC_ERR_CUDA);
 		}
+		if ((rc = wait_on(h->stream))) return fail(rc);	// before dig and fex go
 	}
 	size_t smem = sizeof(double2) * 2 * TR * (L | 1);
 	h->chain_smem = sizeof(double) * (size_t)N * NE;
@@ -1270,13 +1273,14 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 		int64_t* one = nullptr;
 		std::vector<int64_t> ones((size_t)N, 1);
 		if ((rc = dalloc(&one, (size_t)N))) return fail(rc);
-		if (cudaMemcpy(one, ones.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice) != cudaSuccess) { cudaFree(one); set_error("initial device copies failed"); return fail(QPC_ERR_CUDA); }
+		if (cudaMemcpyAsync(one, ones.data(), sizeof(int64_t) * N, cudaMemcpyHostToDevice, h->stream) != cudaSuccess) { cudaFree(one); set_error("initial device copies failed"); return fail(QPC_ERR_CUDA); }
 		in.fieldfree = [&](double2* X, double2* wk, int J, int fi) { return fieldfree_columns(h, X, wk, J, fi, one); };
 		rc = pos_create(in, &h->pos);
 		cudaFree(one);
 		if (rc) return fail(rc);
 	}
 	if (!h->pos) if ((rc = need_chains(h))) return fail(rc);
+	if ((rc = wait_on(h->stream))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }
@@ -1745,7 +1749,7 @@ static int mask_prepare(qpc_lgwz* h)
 	if (h->mLrow) return QPC_OK;
 	const int N = h->N, P = h->P, NE = P + 1;
 	std::vector<double> S((size_t)N * NE), Lc((size_t)N * NE);
-	QPC_CUDA(cudaMemcpy(S.data(), h->S, sizeof(double) * S.size(), cudaMemcpyDeviceToHost));
+	if (int rc = copy_to_host(S.data(), h->S, sizeof(double) * S.size(), h->stream)) return rc;
 	int bad = qpc_cholesky_band(N, P, S.data(), Lc.data());
 	if (bad) { set_error("S is not positive definite (pivot %d)", bad); return QPC_ERR_SINGULAR; }
 	std::vector<double> lrow((size_t)N * P, 0.0), lcol((size_t)N * P, 0.0), di(N);
@@ -1760,10 +1764,10 @@ static int mask_prepare(qpc_lgwz* h)
 	if ((rc = dalloc(&h->mM, (size_t)N * NE)) || (rc = dalloc(&h->mLrow, (size_t)N * P)) || (rc = dalloc(&h->mLcol, (size_t)N * P)) ||
 		(rc = dalloc(&h->mdinv, (size_t)N)))
 		return rc;
-	QPC_CUDA(cudaMemcpy(h->mLrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(h->mLcol, lcol.data(), sizeof(double) * lcol.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(h->mdinv, di.data(), sizeof(double) * N, cudaMemcpyHostToDevice));
-	return QPC_OK;
+	QPC_CUDA(cudaMemcpyAsync(h->mLrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice, h->stream));
+	QPC_CUDA(cudaMemcpyAsync(h->mLcol, lcol.data(), sizeof(double) * lcol.size(), cudaMemcpyHostToDevice, h->stream));
+	QPC_CUDA(cudaMemcpyAsync(h->mdinv, di.data(), sizeof(double) * N, cudaMemcpyHostToDevice, h->stream));
+	return wait_stream(h);
 }
 
 // c <- S^-1 (M c) on the resident state with the band in h->mM, enqueued on st; inside a run

@@ -549,10 +549,10 @@ int qpc_mlp_create(int32_t n_in, int32_t n_hidden, int32_t n_layers, int32_t n_o
 					W[(size_t)e * h->nW + h->offW[j] + (size_t)nn * h->Ks[j] + k] = (j == 0 && k >= n_in) ? 0.f : (float)((2.0 * u - 1.0) * bound);
 				}
 		}
-	if (cudaMemcpy(h->W, W.data(), sizeof(float) * tw, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemset(h->b, 0, sizeof(float) * tb) != cudaSuccess || cudaMemset(h->mW, 0, sizeof(float) * tw) != cudaSuccess ||
-		cudaMemset(h->vW, 0, sizeof(float) * tw) != cudaSuccess || cudaMemset(h->mb, 0, sizeof(float) * tb) != cudaSuccess ||
-		cudaMemset(h->vb, 0, sizeof(float) * tb) != cudaSuccess) {
+	if (cudaMemcpyAsync(h->W, W.data(), sizeof(float) * tw, cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemsetAsync(h->b, 0, sizeof(float) * tb, h->st) != cudaSuccess || cudaMemsetAsync(h->mW, 0, sizeof(float) * tw, h->st) != cudaSuccess ||
+		cudaMemsetAsync(h->vW, 0, sizeof(float) * tw, h->st) != cudaSuccess || cudaMemsetAsync(h->mb, 0, sizeof(float) * tb, h->st) != cudaSuccess ||
+		cudaMemsetAsync(h->vb, 0, sizeof(float) * tb, h->st) != cudaSuccess) {
 		set_error("device upload failed");
 		return fail(QPC_ERR_CUDA);
 	}
@@ -584,21 +584,23 @@ static int params_io(qpc_mlp* h, int32_t member, float* host, bool get)
 {
 	if (!h || !host || member < 0 || member >= h->E) { set_error("bad arguments"); return QPC_ERR_ARGS; }
 	cudaSetDevice(h->dev);
+	if (int rc = wait_on(h->st)) return rc;
+	std::vector<std::vector<float>> w(h->J);
 	long o = 0;
 	for (int j = 0; j < h->J; ++j) {
 		const size_t nw = (size_t)h->Ns[j] * h->Ks[j];
 		float* dW = h->W + (size_t)member * h->nW + h->offW[j];
 		float* db = h->b + (size_t)member * h->nb + h->offb[j];
 		if (get) {
-			QPC_CUDA(cudaMemcpy(host + o, dW, sizeof(float) * nw, cudaMemcpyDeviceToHost));
-			QPC_CUDA(cudaMemcpy(host + o + nw, db, sizeof(float) * h->Ns[j], cudaMemcpyDeviceToHost));
+			if (int rc = copy_to_host(host + o, dW, sizeof(float) * nw, h->st)) return rc;
+			if (int rc = copy_to_host(host + o + nw, db, sizeof(float) * h->Ns[j], h->st)) return rc;
 		} else {
-			std::vector<float> w(host + o, host + o + nw);
+			w[j].assign(host + o, host + o + nw);	// kept until the copies are done
 			if (j == 0)
 				for (int nn = 0; nn < h->Ns[j]; ++nn)
-					for (int k = h->n_in; k < h->K0; ++k) w[(size_t)nn * h->K0 + k] = 0.f;
-			QPC_CUDA(cudaMemcpy(dW, w.data(), sizeof(float) * nw, cudaMemcpyHostToDevice));
-			QPC_CUDA(cudaMemcpy(db, host + o + nw, sizeof(float) * h->Ns[j], cudaMemcpyHostToDevice));
+					for (int k = h->n_in; k < h->K0; ++k) w[j][(size_t)nn * h->K0 + k] = 0.f;
+			QPC_CUDA(cudaMemcpyAsync(dW, w[j].data(), sizeof(float) * nw, cudaMemcpyHostToDevice, h->st));
+			QPC_CUDA(cudaMemcpyAsync(db, host + o + nw, sizeof(float) * h->Ns[j], cudaMemcpyHostToDevice, h->st));
 		}
 		o += nw + h->Ns[j];
 	}

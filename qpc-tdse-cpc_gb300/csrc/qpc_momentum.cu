@@ -294,10 +294,11 @@ __global__ void k_ts_acc(int mode, const double2* __restrict__ W, const double2*
 	work[idx] = cadd(work[idx], t);
 }
 
-template <class T> int upload(T** d, const T* h, size_t n)
+// the copy is in flight: the caller waits on st before h goes
+template <class T> int upload(T** d, const T* h, size_t n, cudaStream_t st)
 {
 	if (int rc = dalloc(d, n)) return rc;
-	QPC_CUDA(cudaMemcpy(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(*d, h, sizeof(T) * n, cudaMemcpyHostToDevice, st));
 	return QPC_OK;
 }
 
@@ -436,18 +437,17 @@ int pcs_table(qpc_pcs* h, const double* ijl)
 	scratch tmp(h->st);
 	double* raw;
 	if ((rc = tmp.get(&raw, (size_t)nk * nl * n))) return rc;
-	QPC_CUDA(cudaStreamSynchronize(h->st));
-	QPC_CUDA(cudaMemcpy(raw, ijl, sizeof(double) * (size_t)nk * nl * n, cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(raw, ijl, sizeof(double) * (size_t)nk * nl * n, cudaMemcpyHostToDevice, h->st));
 	std::vector<int> lm(nch);
 	for (int c = 0; c < nch; ++c) lm[c] = std::abs(d.m0 + c / d.n_l) + c % d.n_l;
-	if ((rc = upload(&h->lmap, lm.data(), lm.size())) || (rc = dalloc(&h->status, 1))) return rc;
+	if ((rc = upload(&h->lmap, lm.data(), lm.size(), h->st)) || (rc = dalloc(&h->status, 1))) return rc;
 	QPC_CUDA(cudaMallocHost(&h->hstatus, sizeof(int)));
 	bool ok = nl <= 65535;
 	for (int k0 = 0; ok && k0 < n; k0 += TCK) {
 		h->seg.emplace_back();
 		if ((rc = tc_make(h->seg.back(), nullptr, raw, n, (long)nl * n, 1, nk, n, nl, -1, nullptr, 0, true, h->st, &ok, k0, std::min(n, k0 + TCK)))) return rc;
 	}
-	if (ok) return QPC_OK;
+	if (ok) return wait_on(h->st);
 	for (tc_store& t : h->seg) t.release();
 	h->seg.clear();
 	if ((rc = dalloc(&h->ijlT, (size_t)nl * n * nk))) return rc;
@@ -545,10 +545,11 @@ int qpc_pcs_create(const qpc_dims* dims, const qpc_kgrid* g, const double* kr, c
 		cudaEventCreate(&h->ev1) != cudaSuccess) { set_error("stream or event creation failed"); return fail(QPC_ERR_CUDA); }
 	const int nl = h->nl, nk = g->nkr, nch = dims->n_m * dims->n_l;
 	if ((rc = pcs_table(h, ijl))) return fail(rc);
-	if ((rc = upload(&h->plm, plm, (size_t)g->nkt * nch))) return fail(rc);
-	if ((rc = upload(&h->kr, kr, (size_t)nk))) return fail(rc);
-	if ((rc = upload(&h->exm, (const double2*)exm, (size_t)g->nkp * dims->n_m))) return fail(rc);
-	if ((rc = upload(&h->cps, (const double2*)cps, (size_t)nk * nl))) return fail(rc);
+	if ((rc = upload(&h->plm, plm, (size_t)g->nkt * nch, h->st))) return fail(rc);
+	if ((rc = upload(&h->kr, kr, (size_t)nk, h->st))) return fail(rc);
+	if ((rc = upload(&h->exm, (const double2*)exm, (size_t)g->nkp * dims->n_m, h->st))) return fail(rc);
+	if ((rc = upload(&h->cps, (const double2*)cps, (size_t)nk * nl, h->st))) return fail(rc);
+	if ((rc = wait_on(h->st))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }
@@ -609,20 +610,20 @@ int qpc_tsurff_create(const qpc_dims* dims, const qpc_kgrid* g, const double* kr
 		cudaEventCreate(&h->ev1) != cudaSuccess) { set_error("stream or event creation failed"); return fail(QPC_ERR_CUDA); }
 	const int nch = dims->n_m * dims->n_l, B = h->B;
 	std::vector<int> ibv(ib, ib + nb);
-	if ((rc = upload(&h->ib, nb ? ibv.data() : nullptr, nb))) return fail(rc);
-	if ((rc = upload(&h->b0, b0, nb)) || (rc = upload(&h->br, br, nb))) return fail(rc);
-	if ((rc = upload(&h->j0, j0, (size_t)g->nkr * h->nl)) || (rc = upload(&h->jr, jr, (size_t)g->nkr * h->nl))) return fail(rc);
+	if ((rc = upload(&h->ib, nb ? ibv.data() : nullptr, nb, h->st))) return fail(rc);
+	if ((rc = upload(&h->b0, b0, nb, h->st)) || (rc = upload(&h->br, br, nb, h->st))) return fail(rc);
+	if ((rc = upload(&h->j0, j0, (size_t)g->nkr * h->nl, h->st)) || (rc = upload(&h->jr, jr, (size_t)g->nkr * h->nl, h->st))) return fail(rc);
 	std::vector<double> yT((size_t)nch * g->nkt);
 	for (int t = 0; t < g->nkt; ++t)
 		for (int c = 0; c < nch; ++c) yT[(size_t)c * g->nkt + t] = y0[(size_t)t * nch + c];
-	if ((rc = upload(&h->y0T, yT.data(), yT.size()))) return fail(rc);
-	if ((rc = upload(&h->pm, pmat, (size_t)3 * nch))) return fail(rc);
-	if ((rc = upload(&h->e0, (const double2*)e0, (size_t)g->nkp * dims->n_m))) return fail(rc);
+	if ((rc = upload(&h->y0T, yT.data(), yT.size(), h->st))) return fail(rc);
+	if ((rc = upload(&h->pm, pmat, (size_t)3 * nch, h->st))) return fail(rc);
+	if ((rc = upload(&h->e0, (const double2*)e0, (size_t)g->nkp * dims->n_m, h->st))) return fail(rc);
 	std::vector<double> ct(g->nkt), st(g->nkt), cp(g->nkp), sp(g->nkp);
 	for (int i = 0; i < g->nkt; ++i) { ct[i] = std::cos(kt[i]); st[i] = std::sin(kt[i]); }
 	for (int i = 0; i < g->nkp; ++i) { cp[i] = std::cos(kp[i]); sp[i] = std::sin(kp[i]); }
-	if ((rc = upload(&h->kr, kr, g->nkr)) || (rc = upload(&h->coskt, ct.data(), ct.size())) || (rc = upload(&h->sinkt, st.data(), st.size())) ||
-		(rc = upload(&h->coskp, cp.data(), cp.size())) || (rc = upload(&h->sinkp, sp.data(), sp.size())))
+	if ((rc = upload(&h->kr, kr, g->nkr, h->st)) || (rc = upload(&h->coskt, ct.data(), ct.size(), h->st)) || (rc = upload(&h->sinkt, st.data(), st.size(), h->st)) ||
+		(rc = upload(&h->coskp, cp.data(), cp.size(), h->st)) || (rc = upload(&h->sinkp, sp.data(), sp.size(), h->st)))
 		return fail(rc);
 	if ((rc = dalloc(&h->temp, (size_t)B * nch)) || (rc = dalloc(&h->temq, (size_t)B * nch)) ||
 		(rc = dalloc(&h->U, (size_t)B * g->nkr * nch)) || (rc = dalloc(&h->W, (size_t)B * g->nkr * g->nkt * dims->n_m)) ||
@@ -630,7 +631,8 @@ int qpc_tsurff_create(const qpc_dims* dims, const qpc_kgrid* g, const double* kr
 		(rc = dalloc(&h->dclock, (size_t)4 * B)) || (rc = dalloc(&h->da1, (size_t)2 * B)) || (rc = dalloc(&h->dact, (size_t)B)))
 		return fail(rc);
 	h->clock.assign((size_t)4 * B, 0.0);
-	if (cudaMemset(h->work, 0, sizeof(double2) * (size_t)B * g->nkr * g->nkt * g->nkp) != cudaSuccess) { set_error("cudaMemset failed"); return fail(QPC_ERR_CUDA); }
+	if (cudaMemsetAsync(h->work, 0, sizeof(double2) * (size_t)B * g->nkr * g->nkt * g->nkp, h->st) != cudaSuccess) { set_error("cudaMemset failed"); return fail(QPC_ERR_CUDA); }
+	if ((rc = wait_on(h->st))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }

@@ -272,10 +272,10 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 					W[(size_t)m * p->nW + (((odd ? g0 : 0) + l / G) * nE + k) * G + l % G] = v;
 				}
 	if ((rc = dalloc(&p->lmap, lm.size())) || (rc = dalloc(&p->V, V.size())) || (rc = dalloc(&p->W, std::max<size_t>(W.size(), 1))) || (rc = dalloc(&p->lamp, (size_t)M * std::max(p->npair, 1)))) return rc;
-	QPC_CUDA(cudaMemcpy(p->lmap, lm.data(), sizeof(int) * lm.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(p->V, V.data(), sizeof(int2) * V.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(p->W, W.data(), sizeof(int2) * W.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(p->lamp, in.lamp, sizeof(double) * M * std::max(p->npair, 1), cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(p->lmap, lm.data(), sizeof(int) * lm.size(), cudaMemcpyHostToDevice, in.stream));
+	QPC_CUDA(cudaMemcpyAsync(p->V, V.data(), sizeof(int2) * V.size(), cudaMemcpyHostToDevice, in.stream));
+	QPC_CUDA(cudaMemcpyAsync(p->W, W.data(), sizeof(int2) * W.size(), cudaMemcpyHostToDevice, in.stream));
+	QPC_CUDA(cudaMemcpyAsync(p->lamp, in.lamp, sizeof(double) * M * std::max(p->npair, 1), cudaMemcpyHostToDevice, in.stream));
 	for (int i = 0; i < 2; ++i)
 		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
 	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT))) return rc;
@@ -284,7 +284,7 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 	cudaFuncSetAttribute(k_angle<3, 32, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	cudaFuncSetAttribute(k_angle<2, 32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	cudaFuncSetAttribute(k_angle<4, 32, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-	return QPC_OK;
+	return wait_on(in.stream);	// the tables' copies
 }
 
 } // namespace

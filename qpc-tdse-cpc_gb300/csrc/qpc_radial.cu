@@ -723,7 +723,7 @@ void lay_out(band_store& b, int N, int w, int wf, bool cx)
 	b.stride = o;
 }
 
-int upload(band_store& b, size_t bytes)
+int upload(band_store& b, size_t bytes, cudaStream_t st)
 {
 	const size_t nt = b.td.size();
 	int rc;
@@ -733,8 +733,8 @@ int upload(band_store& b, size_t bytes)
 		if ((rc = dalloc(&b.A, bytes))) return rc;
 		b.cap = bytes;
 	}
-	QPC_CUDA(cudaMemcpy(b.d_td, b.td.data(), sizeof(int4) * nt, cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(b.d_off, b.off.data(), sizeof(long) * nt, cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(b.d_td, b.td.data(), sizeof(int4) * nt, cudaMemcpyHostToDevice, st));
+	QPC_CUDA(cudaMemcpyAsync(b.d_off, b.off.data(), sizeof(long) * nt, cudaMemcpyHostToDevice, st));
 	return QPC_OK;
 }
 
@@ -883,7 +883,7 @@ int store_banded_impl(radial_ops* p, band_store& b, const double* A, long si, lo
 		b.prof = as_doubles(prof);
 	}
 	lay_out(b, p->N, w, wf, false);
-	if (int rc = upload(b, (size_t)b.stride)) return rc;
+	if (int rc = upload(b, (size_t)b.stride, st)) return rc;
 	k_store<false><<<dim3(p->ntile, 1), 256, 0, st>>>(nullptr, A, si, sj, p->N, w, std::ldexp(1.0, 56 - b.ea), b.d_td, b.d_off, b.A, b.stride);
 	QPC_CUDA(cudaGetLastError());
 	return QPC_OK;
@@ -949,7 +949,7 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 			if (p->nff > 1) { w = std::min(std::min(WMAX, N - 1), w + 8); wf = std::min(w, wf + 12); }	// the other potentials' bands, checked below
 			lay_out(p->F, N, w, wf, true);
 			if (!(*ok = (size_t)p->F.stride * nlh * p->nff <= (size_t)16 << 30)) return QPC_OK;
-			if ((rc = upload(p->F, (size_t)p->F.stride * nlh * p->nff))) return rc;
+			if ((rc = upload(p->F, (size_t)p->F.stride * nlh * p->nff, st))) return rc;
 		}
 		k_store<true><<<dim3(p->ntile, nlh), 256, 0, st>>>(Fb, nullptr, 0, 0, N, p->F.w, std::ldexp(1.0, 56), p->F.d_td, p->F.d_off,
 			p->F.A + (size_t)fi * nlh * p->F.stride, p->F.stride);

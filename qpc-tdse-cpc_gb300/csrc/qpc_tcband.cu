@@ -478,11 +478,11 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 	size_t* d_at;
 	if ((rc = tmp.get(&d_tile, tile_of.size())) || (rc = tmp.get(&d_at, at.size()))) return rc;
 	if ((rc = dalloc(&t.d_list, list.size())) || (rc = dalloc(&t.d_first, first.size())) || (rc = dalloc(&t.d_off, off.size())) || (rc = dalloc(&t.A, o * nop))) return rc;
-	QPC_CUDA(cudaMemcpy(t.d_list, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(t.d_first, first.data(), sizeof(int4) * first.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(t.d_off, off.data(), sizeof(size_t) * off.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(d_tile, tile_of.data(), sizeof(int) * tile_of.size(), cudaMemcpyHostToDevice));
-	QPC_CUDA(cudaMemcpy(d_at, at.data(), sizeof(size_t) * at.size(), cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(t.d_list, list.data(), sizeof(int2) * list.size(), cudaMemcpyHostToDevice, st));
+	QPC_CUDA(cudaMemcpyAsync(t.d_first, first.data(), sizeof(int4) * first.size(), cudaMemcpyHostToDevice, st));
+	QPC_CUDA(cudaMemcpyAsync(t.d_off, off.data(), sizeof(size_t) * off.size(), cudaMemcpyHostToDevice, st));
+	QPC_CUDA(cudaMemcpyAsync(d_tile, tile_of.data(), sizeof(int) * tile_of.size(), cudaMemcpyHostToDevice, st));
+	QPC_CUDA(cudaMemcpyAsync(d_at, at.data(), sizeof(size_t) * at.size(), cudaMemcpyHostToDevice, st));
 	k_tc_planes<DB><<<dim3((unsigned)list.size(), nop), 256, 0, st>>>(m, t.d_list, d_tile, d_at, t.stride, t.A, t.cx);
 	QPC_CUDA(cudaGetLastError());
 	auto attr = [](auto kern) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM); };

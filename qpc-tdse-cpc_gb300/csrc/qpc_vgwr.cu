@@ -841,7 +841,8 @@ int device_transforms(qpc_vgwr* h, std::vector<int>& chmap, std::vector<double> 
 			if (!ns) {	// no partner set: Z is zero on the block, the transform is the identity
 				std::vector<double> I((size_t)na * na, 0.0);
 				for (int i = 0; i < na; ++i) I[(size_t)i * na + i] = 1.0;
-				QPC_CUDA(cudaMemcpy(ub[base][b][0], I.data(), sizeof(double) * I.size(), cudaMemcpyHostToDevice));
+				QPC_CUDA(cudaMemcpyAsync(ub[base][b][0], I.data(), sizeof(double) * I.size(), cudaMemcpyHostToDevice, h->st));
+				if ((rc = wait_on(h->st))) return rc;
 				continue;
 			}
 			std::vector<double> Ccm((size_t)na * ns);	// column-major na x ns
@@ -851,7 +852,7 @@ int device_transforms(qpc_vgwr* h, std::vector<int>& chmap, std::vector<double> 
 			if ((rc = scratch(&A, Ccm.size())) || (rc = scratch(&Sg, (size_t)ns)) || (rc = scratch(&Ucm, (size_t)na * na)) ||
 				(rc = scratch(&rwork, (size_t)ns)))
 				return rc;
-			QPC_CUDA(cudaMemcpy(A, Ccm.data(), sizeof(double) * Ccm.size(), cudaMemcpyHostToDevice));
+			QPC_CUDA(cudaMemcpyAsync(A, Ccm.data(), sizeof(double) * Ccm.size(), cudaMemcpyHostToDevice, h->st));
 			int lwork = 0;
 			if (cusolverDnDgesvd_bufferSize(sol, na, ns, &lwork) != CUSOLVER_STATUS_SUCCESS) { set_error("gesvd buffer size failed"); return QPC_ERR_CUDA; }
 			if ((rc = scratch(&work, (size_t)std::max(lwork, 1)))) return rc;
@@ -861,12 +862,11 @@ int device_transforms(qpc_vgwr* h, std::vector<int>& chmap, std::vector<double> 
 			}
 			k_vg_transpose<<<(unsigned)(((long)na * na + 255) / 256), 256, 0, h->st>>>(Ucm, na, ub[base][b][0]);
 			QPC_CUDA(cudaGetLastError());
-			if ((rc = wait_on(h->st))) return rc;
 			int info = 0;
-			QPC_CUDA(cudaMemcpy(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost));
+			if ((rc = copy_to_host(&info, d_info, sizeof(int), h->st))) return rc;
 			if (info) { set_error("gesvd info %d", info); return QPC_ERR_NUMERIC; }
 			std::vector<double> sg(ns);
-			QPC_CUDA(cudaMemcpy(sg.data(), Sg, sizeof(double) * ns, cudaMemcpyDeviceToHost));
+			if ((rc = copy_to_host(sg.data(), Sg, sizeof(double) * ns, h->st))) return rc;
 			for (int k = 0; k < ns; ++k) {
 				lam[cx][o + k] = sg[k];
 				lam[cx][o + na + k] = -sg[k];
@@ -889,7 +889,7 @@ int device_transforms(qpc_vgwr* h, std::vector<int>& chmap, std::vector<double> 
 			}
 			double *ds = nullptr, *ux2 = nullptr, *uy1 = nullptr;
 			if ((rc = scratch(&ds, (size_t)n)) || (rc = scratch(&ux2, (size_t)n * n)) || (rc = scratch(&uy1, (size_t)n * n))) return rc;
-			QPC_CUDA(cudaMemcpy(ds, sgn.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+			QPC_CUDA(cudaMemcpyAsync(ds, sgn.data(), sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
 			const unsigned g = (unsigned)(((long)n * n + 255) / 256);
 			QPC_CUDA(cudaMemcpyAsync(h->tm[0][b][st], ub[0][b][st], sizeof(double) * n * n, cudaMemcpyDeviceToDevice, h->st));
 			QPC_CUDA(cudaMemcpyAsync(h->tm[1][b][st], ub[1][b][st], sizeof(double) * n * n, cudaMemcpyDeviceToDevice, h->st));
@@ -971,10 +971,11 @@ int make_pos(qpc_vgwr* h, const std::vector<int>& chmap, const double* Ri)
 	int* did = nullptr;
 	int rc;
 	if ((rc = dalloc(&done, n)) || (rc = dalloc(&did, n)) || (rc = dalloc(&h->ntts, (size_t)h->B))) { cudaFree(done); cudaFree(did); return rc; }
-	if (cudaMemcpy(done, one.data(), sizeof(long long) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(did, id.data(), sizeof(int) * n, cudaMemcpyHostToDevice) != cudaSuccess) { set_error("upload"); rc = QPC_ERR_CUDA; }
+	if (cudaMemcpyAsync(done, one.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemcpyAsync(did, id.data(), sizeof(int) * n, cudaMemcpyHostToDevice, h->st) != cudaSuccess) { set_error("upload"); rc = QPC_ERR_CUDA; }
 	in.fieldfree = [&](double2* X, double2* wk, int J, int) { return fieldfree_columns(h, X, wk, J, done, did); };
 	if (!rc) rc = vpos_create(in, &h->pos);
+	if (const int w = wait_on(h->st)) rc = rc ? rc : w;	// the copies, where nothing was made
 	cudaFree(done); cudaFree(did);
 	return rc;
 }
@@ -1039,7 +1040,7 @@ int qpc_vgwr_create(const qpc_dims* dims, double dt, const double* S, const doub
 		(rc = dalloc(&h->X, nst)) || (rc = dalloc(&h->W, nst)) || (rc = dalloc(&h->U, nst * (NE + 1))) || (rc = dalloc(&h->ntt, (size_t)h->B)) ||
 		(rc = dalloc(&h->perm, (size_t)h->B)) || (rc = dalloc(&h->nrm, (size_t)h->B)))
 		return fail(rc);
-	if (cudaMemcpy(h->chmap, chmap.data(), sizeof(int) * nch, cudaMemcpyHostToDevice) != cudaSuccess) { set_error("upload"); return fail(QPC_ERR_CUDA); }
+	if (cudaMemcpyAsync(h->chmap, chmap.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, h->st) != cudaSuccess) { set_error("upload"); return fail(QPC_ERR_CUDA); }
 	// the transforms' GEMMs: exact bf16 digit slices on the tensor cores (default), or the FP64
 	// DFMA kernel (QPC_VG_GEMM=dfma)
 	if (const char* e = std::getenv("QPC_VG_GEMM")) h->slices = std::strcmp(e, "dfma") != 0;
@@ -1051,18 +1052,19 @@ int qpc_vgwr_create(const qpc_dims* dims, double dt, const double* S, const doub
 	// angular eigensystems and the transform matrices, block by block on the device
 	std::vector<double> lam[4];
 	if ((rc = device_transforms(h, chmap, lam))) return fail(rc);
-	if (cudaMemcpy(h->S, S, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->Ri, Rinv, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->D, D, sizeof(double) * N * NE, cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->Lrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemcpy(h->Dinv, dinv.data(), sizeof(double) * dinv.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-		cudaMemset(h->X, 0, sizeof(double2) * nst) != cudaSuccess) {
+	if (cudaMemcpyAsync(h->S, S, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemcpyAsync(h->Ri, Rinv, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemcpyAsync(h->D, D, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemcpyAsync(h->Lrow, lrow.data(), sizeof(double) * lrow.size(), cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemcpyAsync(h->Dinv, dinv.data(), sizeof(double) * dinv.size(), cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
+		cudaMemsetAsync(h->X, 0, sizeof(double2) * nst, h->st) != cudaSuccess) {
 		set_error("device upload failed");
 		return fail(QPC_ERR_CUDA);
 	}
 	for (int c = 0; c < 4; ++c)
-		if (cudaMemcpy(h->lam[c], lam[c].data(), sizeof(double) * nch, cudaMemcpyHostToDevice) != cudaSuccess) { set_error("upload"); return fail(QPC_ERR_CUDA); }
+		if (cudaMemcpyAsync(h->lam[c], lam[c].data(), sizeof(double) * nch, cudaMemcpyHostToDevice, h->st) != cudaSuccess) { set_error("upload"); return fail(QPC_ERR_CUDA); }
 	if ((rc = make_pos(h, chmap, Rinv))) return fail(rc);
+	if ((rc = wait_on(h->st))) return fail(rc);
 	*out = h;
 	return QPC_OK;
 }
@@ -1113,7 +1115,7 @@ static int dipole_setup(qpc_vgwr* h)
 	if (h->dpairs) return QPC_OK;
 	const int nl = h->d.n_l, nm = h->d.n_m, m0 = h->d.m0;
 	std::vector<int> chmap(h->nch), inv(h->nch);
-	QPC_CUDA(cudaMemcpy(chmap.data(), h->chmap, sizeof(int) * h->nch, cudaMemcpyDeviceToHost));
+	if (int rc = copy_to_host(chmap.data(), h->chmap, sizeof(int) * h->nch, h->st)) return rc;
 	for (int t = 0; t < h->nch; ++t) inv[chmap[t]] = t;
 	std::vector<int2> pairs;
 	std::vector<double> coef;
@@ -1137,10 +1139,10 @@ static int dipole_setup(qpc_vgwr* h)
 	h->dnblk = std::max(1, std::min(64, (304 + h->B - 1) / h->B));
 	if (int rc = dalloc(&h->dpart, (size_t)h->B * h->dnblk)) return rc;
 	if (!pairs.empty()) {
-		QPC_CUDA(cudaMemcpy(h->dpairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice));
-		QPC_CUDA(cudaMemcpy(h->dcoef, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice));
+		QPC_CUDA(cudaMemcpyAsync(h->dpairs, pairs.data(), sizeof(int2) * pairs.size(), cudaMemcpyHostToDevice, h->st));
+		QPC_CUDA(cudaMemcpyAsync(h->dcoef, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, h->st));
 	}
-	return QPC_OK;
+	return wait_on(h->st);
 }
 
 static int run_impl(qpc_vgwr* h, const double* atab, int64_t ld, const int64_t* nt_field, const int64_t* nt_total,

@@ -256,7 +256,7 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	double* R = nullptr;
 	if ((rc = dalloc(&R, nb))) return rc;
 	struct guard { double* p; ~guard() { cudaFree(p); } } g{R};
-	QPC_CUDA(cudaMemcpy(R, neg.data(), sizeof(double) * nb, cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(R, neg.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, st));
 	if ((rc = radial_create(&p->ops, radial_setup{N, in.P, in.nlh, 1, in.S, R, false, in.fieldfree, st, 0}, nch, ok)) || !*ok) return rc;
 	if ((rc = dalloc(&p->om, N)) || (rc = dalloc(&p->rinv, N))) return rc;
 	k_negate<<<(N + 255) / 256, 256, 0, st>>>(p->ops.r, p->rinv, N);
@@ -288,7 +288,7 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	std::vector<int> lm(nch);
 	for (int t = 0; t < nch; ++t) lm[t] = in.chmap[t] % in.n_l + std::abs(in.m0 + in.chmap[t] / in.n_l);
 	if ((rc = dalloc(&p->lmap, nch))) return rc;
-	QPC_CUDA(cudaMemcpy(p->lmap, lm.data(), sizeof(int) * nch, cudaMemcpyHostToDevice));
+	QPC_CUDA(cudaMemcpyAsync(p->lmap, lm.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, st));
 	const long nvec = (long)p->B * nch;
 	for (int i = 0; i < 2; ++i)
 		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
