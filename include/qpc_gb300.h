@@ -304,6 +304,14 @@ int qpc_lgwz_set_profiling(qpc_lgwz* h, int on);
 int qpc_lgwz_get_tuning(qpc_lgwz* h, int32_t* out);
 int qpc_lgwz_kernel_times(qpc_lgwz* h, double* ms, int64_t* launches);
 
+/* Which kernels a handle has and its last run took: out[0] = 1: it holds the operators of the position basis
+ * (0: the banded solves serve every run); out[1] = the last run: 1 position basis, 0 banded solves, -1 none yet;
+ * out[2], out[3], out[4] = 1: digit planes for the tensor cores of the field-free step, of the way into the
+ * basis, of the way back; out[5] = QPC_PRODUCT_* of the last position-basis run's first field-free step.
+ * out must hold 6 values. */
+enum { QPC_PRODUCT_NONE = 0, QPC_PRODUCT_ONE = 1, QPC_PRODUCT_MADD = 2, QPC_PRODUCT_DIGITS = 3 };
+int qpc_lgwz_get_path(qpc_lgwz* h, int32_t* out);
+
 /* ---------------------------------------------------------------- velocity gauge, elliptical
  * Replaces propagator_cn_hc_vgwr (spherical/propagator/cn_1e.hpp:812-951): initialize with
  * S, Rinv = <B|1/r|B>, D = <B_i|d/dr B_j> (upper entries of the anti-symmetric band) and H
@@ -320,6 +328,9 @@ int qpc_vgwr_put(qpc_vgwr* h, const double* coef);
 int qpc_vgwr_get(qpc_vgwr* h, double* coef);
 int qpc_vgwr_put_device(qpc_vgwr* h, const double* dev_coef);
 int qpc_vgwr_get_device(qpc_vgwr* h, double* dev_coef);
+/* out[0] = 1: diagonal radial couplings (0: banded solves); out[1], out[2] = 1: digit planes of the dense radial
+ * transform and of the one back.  out must hold 3 values. */
+int qpc_vgwr_get_path(qpc_vgwr* h, int32_t* out);
 int qpc_vgwr_dims(qpc_vgwr* h, qpc_dims* dims);
 int qpc_vgwr_propagate(qpc_vgwr* h, const double* ax_ti, const double* ax_tf, const double* ay_ti, const double* ay_tf);
 int qpc_vgwr_propagate_free(qpc_vgwr* h);
@@ -493,6 +504,8 @@ typedef struct qpc_pcs qpc_pcs;
 int qpc_pcs_create(const qpc_dims* dims, const qpc_kgrid* grid, const double* kr, const double* ijl, const double* plm,
 	const double* exm, const double* cps, qpc_pcs** out);
 int qpc_pcs_destroy(qpc_pcs* h);
+/* *segments = column segments of the projector's table kept as digit planes (0: FP64 sums) */
+int qpc_pcs_get_path(qpc_pcs* h, int32_t* segments);
 /* measure_lmd (kind QPC_SPEC_LMD), measure_prj (PMD) or measure_pad (PAD) of
  * momentum_1e.hpp:337-403 for n_inst wavefunctions c[inst][m][l][r] (device memory when
  * on_device != 0, else host).  out (host, complex128): LMD [inst][kr][im][il] =

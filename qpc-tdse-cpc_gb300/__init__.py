@@ -46,12 +46,13 @@ EXPORTS = (
     "qpc_sph_legendre", "qpc_pcs_tables", "qpc_tsurff_tables", "qpc_pcs_create", "qpc_pcs_destroy", "qpc_pcs_measure",
     "qpc_lgwz_pcs", "qpc_tsurff_create", "qpc_tsurff_destroy", "qpc_tsurff_clear", "qpc_tsurff_accumulate",
     "qpc_lgwz_tsurff", "qpc_vgwr_tsurff", "qpc_tsurff_get", "qpc_pcs_last_run", "qpc_tsurff_last_run",
-    "qpc_lgwz_create_ex", "qpc_pcs_tables_numeric",
+    "qpc_lgwz_create_ex", "qpc_pcs_tables_numeric", "qpc_lgwz_get_path", "qpc_vgwr_get_path", "qpc_pcs_get_path",
 )
 SPEC_LMD, SPEC_PMD, SPEC_PAD = 0, 1, 2
 TSURFF_FREE, TSURFF_Z, TSURFF_XY = 0, 1, 2
 NOALLOC_MAX_ELEMS = 1 << 20
 KERNELS = ("factor", "transform_fwd", "sweep", "transform_bwd", "fieldfree")
+PRODUCTS = (None, "k_band_one", "k_band_apply", "k_tc_apply")
 
 
 class QpcError(RuntimeError):
@@ -124,6 +125,9 @@ def load(path=None):
         "qpc_lgwz_set_profiling": (ctypes.c_int, [P, ctypes.c_int]),
         "qpc_lgwz_kernel_times": (ctypes.c_int, [P, P, P]),
         "qpc_lgwz_get_tuning": (ctypes.c_int, [P, P]),
+        "qpc_lgwz_get_path": (ctypes.c_int, [P, P]),
+        "qpc_vgwr_get_path": (ctypes.c_int, [P, P]),
+        "qpc_pcs_get_path": (ctypes.c_int, [P, P]),
         "qpc_fieldfree_noalloc": (ctypes.c_int, [P, P, P, P, P]),
         "qpc_lgwz_run_dipole": (ctypes.c_int, [P, P, i64, P, P, P, P, i64]),
         "qpc_hhg_spectrum": (ctypes.c_int, [P, i64, d, d, d, d, i32, P, P]),
@@ -567,6 +571,15 @@ class propagator_cn_hc_lgwz:
                 "coupling": {b: int(out[1 + b]) for b in range(32) if out[1 + b]},
                 "fieldfree": {b: int(out[33 + b]) for b in range(32) if out[33 + b]}}
 
+    def path(self):
+        """{"position": the handle holds the operators of the position basis, "last_run": "position" | "banded" | None,
+        "digits": (field-free, in, out) operators kept for the tensor cores, "product": the kernel of the last
+        position-basis run's first field-free step}"""
+        out = np.zeros(6, np.int32)
+        _check(load().qpc_lgwz_get_path(self._h, _ptr(out)))
+        return {"position": bool(out[0]), "last_run": {1: "position", 0: "banded"}.get(int(out[1])),
+                "digits": tuple(bool(v) for v in out[2:5]), "product": PRODUCTS[out[5]]}
+
     def kernel_times(self):
         """{kernel: (total ms, launches)} accumulated by run() while profiling is on."""
         ms = np.zeros(len(KERNELS))
@@ -915,6 +928,12 @@ class propagator_cn_hc_vgwr:
     def enable_profiling(self, on=True):
         _check(load().qpc_vgwr_set_profiling(self._h, int(bool(on))))
 
+    def path(self):
+        """{"position": diagonal radial couplings, "digits": (dense radial transform, back) kept for the tensor cores}"""
+        out = np.zeros(3, np.int32)
+        _check(load().qpc_vgwr_get_path(self._h, _ptr(out)))
+        return {"position": bool(out[0]), "digits": tuple(bool(v) for v in out[1:])}
+
     def kernel_times(self):
         """{"transform" | "coupling" | "fieldfree": (total ms, launch groups)} of run() while profiling is on."""
         ms = np.zeros(3)
@@ -1048,6 +1067,12 @@ class spectrum_c_pcs:
             self.close()
         except Exception:
             pass
+
+    def path(self):
+        """{"segments": column segments of the table kept as digit planes for the tensor cores (0: FP64 sums)}"""
+        out = np.zeros(1, np.int32)
+        _check(load().qpc_pcs_get_path(self._h, _ptr(out)))
+        return {"segments": int(out[0])}
 
     def _measure(self, kind, coef):
         n_m, n_l, _ = self.shape

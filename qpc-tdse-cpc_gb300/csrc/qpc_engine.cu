@@ -483,6 +483,7 @@ struct qpc_lgwz {
 	int* dperm = nullptr;		// device [B]: the instance of each sorted slot
 	// the state lives in st (r-major), in hostlay (the caller's order), or in both
 	bool st_valid = false, lay_valid = true;
+	int last_pos = -1;		// the last run: 1 position basis, 0 banded solves
 	size_t fac_elems = 0;
 	bool chains_ready = false;	// the banded solves' buffers exist
 	std::vector<double2> ffh;	// host copy of ff until they do
@@ -1527,6 +1528,7 @@ static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* 
 	QPC_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
 	// the position basis: plain runs, the absorbing mask, and the dipole of R itself (diagonal there)
 	const bool pos = h->pos && !tsf && (!F || std::memcmp(F, h->h_R.data(), sizeof(double) * h->h_R.size()) == 0);
+	h->last_pos = pos;
 	if (pos) {
 		if (int rc = need_lmajor(h)) return rc;
 		QPC_CUDA(cudaMemcpyAsync(h->dperm, perm.data(), sizeof(int) * B, cudaMemcpyHostToDevice, h->stream));
@@ -1915,6 +1917,16 @@ int qpc_lgwz_get_tuning(qpc_lgwz* h, int32_t* out)
 	if (!h || !out) { set_error("NULL argument"); return QPC_ERR_ARGS; }
 	out[0] = h->K;
 	for (int b = 0; b < 32; ++b) { out[1 + b] = h->gsel[1][b]; out[33 + b] = h->gsel[0][b]; }
+	return QPC_OK;
+}
+
+int qpc_lgwz_get_path(qpc_lgwz* h, int32_t* out)
+{
+	if (!h || !out) { set_error("NULL argument"); return QPC_ERR_ARGS; }
+	for (int i = 0; i < 6; ++i) out[i] = 0;
+	out[0] = h->pos != nullptr;
+	out[1] = h->last_pos;
+	if (h->pos) pos_report(h->pos, out + 2);
 	return QPC_OK;
 }
 

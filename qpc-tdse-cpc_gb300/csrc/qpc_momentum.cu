@@ -560,6 +560,13 @@ int qpc_pcs_destroy(qpc_pcs* h)
 	return QPC_OK;
 }
 
+int qpc_pcs_get_path(qpc_pcs* h, int32_t* segments)
+{
+	if (!h || !segments) { set_error("NULL argument"); return QPC_ERR_ARGS; }
+	*segments = (int32_t)h->seg.size();
+	return QPC_OK;
+}
+
 int qpc_pcs_measure(qpc_pcs* h, int32_t kind, const double* coef, int32_t on_device, int32_t n_inst, double* out)
 {
 	if (!h || !coef || !out || n_inst < 1 || kind < QPC_SPEC_LMD || kind > QPC_SPEC_PAD) { set_error("bad arguments"); return QPC_ERR_ARGS; }

@@ -226,6 +226,7 @@ struct pos_path {
 	int angle_g = 3;		// outputs per task of k_angle, PT = 32
 	bool angle_small = false;	// PT = 8, one output per task
 	bool angle_many = false;	// four blocks per SM
+	int product = QPC_PRODUCT_NONE;	// kernel of the last run's first field-free product
 };
 
 
@@ -318,6 +319,12 @@ void pos_destroy(pos_path* p)
 	p->K.release();
 	radial_destroy(&p->ops);
 	delete p;
+}
+
+void pos_report(const pos_path* p, int32_t out[4])
+{
+	out[0] = p->ops.F.has_tc; out[1] = p->ops.W.has_tc; out[2] = p->ops.X.has_tc;
+	out[3] = p->product;
 }
 
 #define POS_PROF(kind) struct prof_ { const pos_run& r; int k; prof_(const pos_run& r_, int k_) : r(r_), k(k_) { if (r.prof_begin) r.prof_begin(k, r.stream); } \
@@ -414,7 +421,8 @@ int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf)
 		if (p->nff > 1) a.amap = r.perm;
 		a.s0 = p->buf[cur]; a.e0 = p->ex[cur]; a.dst = p->buf[1 - cur]; a.edst = p->ex[1 - cur];
 		a.nta = r.ntt; a.step = s;
-		band_apply(a, true, p->ntile, st, &p->ops.F, r.status, r.stbit);
+		const int product = band_apply(a, true, p->ntile, st, &p->ops.F, r.status, r.stbit);
+		if (s == 0) p->product = product;
 		++*r.launches;
 	}
 	QPC_CUDA(cudaGetLastError());

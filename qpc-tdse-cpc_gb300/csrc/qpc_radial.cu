@@ -796,18 +796,22 @@ void band_attr()
 // without a second block (two fit), and, for few columns, warps that share a column and split its k so that a
 // block still has eight.
 template <bool CX>
-void dispatch(const band_args& a, int tiles, cudaStream_t st)
+int dispatch(const band_args& a, int tiles, cudaStream_t st)
 {
 	const int n = a.ncols;
 	const long per = (long)tiles * a.nchan;
 	auto blocks = [&](int cols) { return per * ((n + cols - 1) / cols); };
-	if (a.amap || n == 1) launch_after(k_band_one<CX>, dim3((unsigned)(tiles * n), (unsigned)a.nchan), 256, 0, st, a);
-	else if (n == 2) band_launch<2, 8, CX>(a, tiles, st);
+	if (a.amap || n == 1) {
+		launch_after(k_band_one<CX>, dim3((unsigned)(tiles * n), (unsigned)a.nchan), 256, 0, st, a);
+		return QPC_PRODUCT_ONE;
+	}
+	if (n == 2) band_launch<2, 8, CX>(a, tiles, st);
 	else if (n <= 4) band_launch<4, 8, CX>(a, tiles, st);
 	else if (n <= 8) band_launch<4, 4, CX>(a, tiles, st);
 	else if (n <= 16 || blocks(32) < 304) band_launch<4, 2, CX>(a, tiles, st);
 	else if (n <= 32 || (n > 64 && n <= 96) || blocks(64) < 608) band_launch<4, 1, CX>(a, tiles, st);
 	else band_launch<8, 1, CX>(a, tiles, st);
+	return QPC_PRODUCT_MADD;
 }
 
 template <int P>
@@ -1006,14 +1010,13 @@ static double madd_cost(const band_store& b, bool cx, int nchan, int ncols)
 	return 6.0 + k * TM * nchan * ((ncols + 7) & ~7) / 8e6;
 }
 
-void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st, const band_store* b, int* status, int stbit)
+int band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st, const band_store* b, int* status, int stbit)
 {
 	if (b && b->has_tc && !a.amap && (b->tc_always || tc_cost(b->tc, a.nchan, a.ncols) < madd_cost(*b, cx, a.nchan, a.ncols))) {
 		tc_apply(b->tc, a, status, stbit, st);
-		return;
+		return QPC_PRODUCT_DIGITS;
 	}
-	if (cx) dispatch<true>(a, tiles, st);
-	else dispatch<false>(a, tiles, st);
+	return cx ? dispatch<true>(a, tiles, st) : dispatch<false>(a, tiles, st);
 }
 
 int store_banded(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st, bool* ok)

@@ -107,7 +107,8 @@ int orthonormalise(double* Qt, int N, double* E, double* T, cudaStream_t st, boo
 band_args band_args_of(const radial_ops* p, const band_store& b, int nchan, int ncols);
 // status, stbit: device word or-ed with stbit when a wait of the tensor-core kernel ran out; b: the store behind a (its
 // planes are used where that is the faster way), or NULL
-void band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st, const band_store* b = nullptr, int* status = nullptr, int stbit = 0);
+// returns the kernel it took (QPC_PRODUCT_*)
+int band_apply(const band_args& a, bool cx, int tiles, cudaStream_t st, const band_store* b = nullptr, int* status = nullptr, int stbit = 0);
 // largest biased exponent of every TE rows of src [nvec][N]
 void exponents(const double2* src, int* ex, int N, int ntile, long nvec, cudaStream_t st);
 

@@ -1102,6 +1102,15 @@ int qpc_vgwr_put(qpc_vgwr* h, const double* coef) { return vg_copy(h, coef, null
 int qpc_vgwr_get(qpc_vgwr* h, double* coef) { return vg_copy(h, nullptr, coef, cudaMemcpyDeviceToHost); }
 int qpc_vgwr_put_device(qpc_vgwr* h, const double* c) { return vg_copy(h, c, nullptr, cudaMemcpyDeviceToDevice); }
 int qpc_vgwr_get_device(qpc_vgwr* h, double* c) { return vg_copy(h, nullptr, c, cudaMemcpyDeviceToDevice); }
+int qpc_vgwr_get_path(qpc_vgwr* h, int32_t* out)
+{
+	if (!h || !out) { set_error("NULL argument"); return QPC_ERR_ARGS; }
+	out[0] = h->pos != nullptr;
+	out[1] = out[2] = 0;
+	if (h->pos) vpos_report(h->pos, out + 1);
+	return QPC_OK;
+}
+
 int qpc_vgwr_dims(qpc_vgwr* h, qpc_dims* dims)
 {
 	if (!h || !dims) { set_error("NULL argument"); return QPC_ERR_ARGS; }

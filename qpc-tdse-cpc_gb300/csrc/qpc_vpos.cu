@@ -339,6 +339,11 @@ void vpos_destroy(vpos_path* p)
 	delete p;
 }
 
+void vpos_report(const vpos_path* p, int32_t out[2])
+{
+	out[0] = p->TD.has_tc; out[1] = p->TI.has_tc;
+}
+
 namespace {
 
 struct prof_scope {

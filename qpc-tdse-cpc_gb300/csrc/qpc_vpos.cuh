@@ -26,6 +26,8 @@ struct vpos_setup {
 // *out = nullptr with QPC_OK when the sizes or operators do not suit it
 int vpos_create(const vpos_setup& in, vpos_path** out);
 void vpos_destroy(vpos_path* p);
+// digit planes of the dense transform and of the one back (0 or 1)
+void vpos_report(const vpos_path* p, int32_t out[2]);
 
 struct vpos_run {
 	double2* X;		// [slot][nch][N], engine channel order, in and out
