@@ -27,13 +27,16 @@ __device__ __forceinline__ int2 quant(double v, int E)
 	return make_int2(hi, (int)(x - ((long long)hi << 28)));
 }
 
-// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^61; nf: the operand was not finite
+// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^63; nf: the operand was not finite.  Two bits of m beside
+// h, or from |h| = 2^61 on (a sum of 32 in units of the column's power of two; rows of a dense orthogonal matrix reach
+// sqrt(N)) h alone, whose 62 bits leave m below the rounding
 __device__ __forceinline__ double to_double(long long h, long long m, int s, bool nf)
 {
-	long long q = (h << 2) | (m >> 26);
+	const bool wide = (unsigned long long)(h + (1ll << 61)) >> 62;
+	long long q = wide ? h : (h << 2) | (m >> 26);
 	unsigned long long a = q < 0 ? 0ull - (unsigned long long)q : (unsigned long long)q;
 	const int lz = __clzll((long long)a);
-	const int e = 1023 + 63 - lz + s - 2;
+	const int e = 1023 + 63 - lz + s - (wide ? 0 : 2);
 	a <<= (lz & 63);
 	unsigned long long b = ((unsigned long long)(unsigned)(e - 1) << 52) + (a >> 11) + ((a >> 10) & 1ull);
 	b |= (unsigned long long)q & 0x8000000000000000ull;

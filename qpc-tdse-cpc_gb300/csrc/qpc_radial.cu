@@ -872,7 +872,11 @@ int store_banded_impl(radial_ops* p, band_store& b, const double* A, long si, lo
 	double big = 0.0;
 	int w = p->N - 1, wf = p->N - 1;
 	*ok = true;
-	if (dense) b.ea = 0;	// orthogonal matrices
+	if (dense) {	// orthogonal matrices
+		b.ea = 0;
+		*ok = p->N <= DENSE_MAX;
+		if (!*ok) return QPC_OK;
+	}
 	else {
 		std::vector<unsigned long long> prof;
 		QPC_CUDA(cudaMemsetAsync(p->prof, 0, sizeof(unsigned long long) * (WMAX + 1), st));
@@ -883,6 +887,10 @@ int store_banded_impl(radial_ops* p, band_store& b, const double* A, long si, lo
 		if (!*ok) return QPC_OK;
 		std::frexp(big, &b.ea);
 		*ok = decay(prof, p->N, std::ldexp(1.0, b.ea), w, wf, 29);
+		if (!*ok) return QPC_OK;
+		double sum = -big;	// at least any row's sum of magnitudes
+		for (int d = 0; d <= std::min(w, WMAX); ++d) { double v; std::memcpy(&v, &prof[d], 8); sum += 2.0 * v; }
+		*ok = sum <= std::ldexp(SUM_MAX, b.ea);
 		if (!*ok) return QPC_OK;
 		b.prof = as_doubles(prof);
 	}
@@ -1024,10 +1032,10 @@ int store_banded(radial_ops* p, band_store& b, const double* A, long si, long sj
 	return store_banded_impl(p, b, A, si, sj, st, false, ok);
 }
 
-int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, int ncols, cudaStream_t st)
+int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, int ncols, cudaStream_t st, bool* ok)
 {
-	bool ok;
-	if (int rc = store_banded_impl(p, b, A, si, sj, st, true, &ok)) return rc;
+	if (int rc = store_banded_impl(p, b, A, si, sj, st, true, ok)) return rc;
+	if (!*ok) return QPC_OK;
 	const char* mode = std::getenv("QPC_POS_TC");
 	b.tc_always = mode && mode[0] == '1';
 	if (ncols < TC_MIN || (mode && mode[0] == '0')) return QPC_OK;

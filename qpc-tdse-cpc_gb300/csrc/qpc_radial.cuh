@@ -10,6 +10,11 @@
 namespace qpc {
 
 constexpr int WMAX = 176;	// widest band (either side of the diagonal) the products take
+// a product's sum is held in 63 bits, less than 128 in units of the column's and the operator's powers of two.  F~ is
+// unitary and stays below 27; the entries of any other band are added up at set-up, and a dense orthogonal matrix has rows
+// of norm 1, so at most sqrt(N)
+constexpr double SUM_MAX = 126.0;
+constexpr int DENSE_MAX = 15876;	// SUM_MAX^2
 
 struct band_args {
 	const char* A;		// operators, [set][nlh] of astride bytes
@@ -95,8 +100,8 @@ void radial_destroy(radial_ops* p);
 
 // A (device, FP64, element (i, j) at A[i si + j sj]) into b, banded where it falls off (ok), or dense
 int store_banded(radial_ops* p, band_store& b, const double* A, long si, long sj, cudaStream_t st, bool* ok);
-// an orthogonal matrix; ncols: most columns of a product
-int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, int ncols, cudaStream_t st);
+// an orthogonal matrix (ok: N at most DENSE_MAX); ncols: most columns of a product
+int store_dense(radial_ops* p, band_store& b, const double* A, long si, long sj, int ncols, cudaStream_t st, bool* ok);
 // A [N][N] = X^T B X for a symmetric band B, or for an anti-symmetric one given by its upper entries (device
 // [N][P+1]), zero beyond ~WMAX of the diagonal; Bx scratch [N][N]
 int project_band(const radial_ops* p, const double* B, bool anti, double* Bx, double* A, cudaStream_t st);

@@ -241,7 +241,8 @@ int momentum_basis(vpos_path* p, const vpos_setup& in, bool* ok)
 	*ok = hinfo == 0;
 	if (!*ok) return QPC_OK;
 	if ((rc = orthonormalise(Qt, N, A, T, st, ok)) || !*ok) return rc;
-	if ((rc = store_dense(&p->ops, p->TD, Qt, N, 1, p->B * p->nch, st)) || (rc = store_dense(&p->ops, p->TI, Qt, 1, N, p->B * p->nch, st))) return rc;
+	if ((rc = store_dense(&p->ops, p->TD, Qt, N, 1, p->B * p->nch, st, ok)) || !*ok) return rc;
+	if ((rc = store_dense(&p->ops, p->TI, Qt, 1, N, p->B * p->nch, st, ok)) || !*ok) return rc;
 	return wait_on(st);
 }
 
@@ -309,7 +310,7 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 int vpos_create(const vpos_setup& in, vpos_path** out)
 {
 	*out = nullptr;
-	if (in.P < 3 || in.P > 8 || std::max(in.nb[0], in.nb[1]) > NBMAX) return QPC_OK;
+	if (in.P < 3 || in.P > 8 || in.N > DENSE_MAX || std::max(in.nb[0], in.nb[1]) > NBMAX) return QPC_OK;
 	const double cols = (double)in.B * in.nch, N = in.N;
 	const double here = 2e-4 + cols * N * (48.0 * N + 30.0 * in.nch) / 6e12, there = std::max(38.8e-6 * N, cols * N * 1920.0 / 6e11);
 	if (here > there) return QPC_OK;
