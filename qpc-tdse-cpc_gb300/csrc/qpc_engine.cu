@@ -1403,17 +1403,13 @@ static void mask_enqueue(qpc_lgwz* h, cudaStream_t st, const int64_t* ntt, long 
 
 // the loop in the position basis; pf, pt: nt_field and nt_total in the sorted order of perm
 static int run_pos(qpc_lgwz* h, const std::vector<int64_t>& pf, const std::vector<int64_t>& pt, const std::vector<int>& perm, long smax, long ntt_max,
-	const double* mband, bool dipole, double* zlist, int64_t ldz)
+	bool mask, bool dipole, double* zlist, int64_t ldz)
 {
 	const int B = h->B;
-	if (mband) {
-		if (int rc = mask_prepare(h)) return rc;
-		QPC_CUDA(cudaMemcpyAsync(h->mM, mband, sizeof(double) * h->N * (h->P + 1), cudaMemcpyHostToDevice, h->stream));
-	}
 	if (int rc = wait_stream(h)) return rc;
 	pos_run r{};
 	r.state = h->hostlay; r.perm = h->dperm; r.ntf = h->ntf; r.ntt = h->ntt; r.ftab = h->ftab; r.ld = h->ld;
-	r.mask = mband ? h->mM : nullptr;
+	r.mask = mask;
 	r.z = dipole ? h->zdev : nullptr;
 	r.ldz = ldz;
 	r.launches = &h->launches;
@@ -1433,9 +1429,9 @@ static int run_pos(qpc_lgwz* h, const std::vector<int64_t>& pf, const std::vecto
 		};
 	}
 	h->st_valid = false;
-	QPC_CUDA(cudaEventRecord(h->ev0, h->stream));
+	if (!mask) QPC_CUDA(cudaEventRecord(h->ev0, h->stream));
 	if (int rc = pos_begin(h->pos, r)) return rc;
-	const long send = mband ? ntt_max + 1 : smax;
+	const long send = mask ? ntt_max + 1 : smax;
 	int Bc = 0, Bf = B;
 	while (Bc < B && pf[Bc] > 0) ++Bc;
 	for (long s = 0; s < send; ++s) {
@@ -1527,7 +1523,14 @@ static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* 
 	}
 	QPC_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
 	// the position basis: plain runs, the absorbing mask, and the dipole of R itself (diagonal there)
-	const bool pos = h->pos && !tsf && (!F || std::memcmp(F, h->h_R.data(), sizeof(double) * h->h_R.size()) == 0);
+	bool pos = h->pos && !tsf && (!F || std::memcmp(F, h->h_R.data(), sizeof(double) * h->h_R.size()) == 0);
+	if (pos && mband) {
+		// a mask that the fixed-point products do not suit (its size, or no fall-off) keeps the banded solves
+		if (int rc = mask_prepare(h)) return rc;
+		QPC_CUDA(cudaEventRecord(h->ev0, h->stream));
+		QPC_CUDA(cudaMemcpyAsync(h->mM, mband, sizeof(double) * h->N * (h->P + 1), cudaMemcpyHostToDevice, h->stream));
+		if (int rc = pos_mask(h->pos, h->mM, &h->launches, h->stream, &pos)) return rc;
+	}
 	h->last_pos = pos;
 	if (pos) {
 		if (int rc = need_lmajor(h)) return rc;
@@ -1565,7 +1568,7 @@ static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* 
 		h->ldz = ldz;
 		h->observing = !pos;
 	}
-	if (pos) return run_pos(h, pf, pt, perm, smax, ntt_max, mband, F != nullptr, zlist, ldz);
+	if (pos) return run_pos(h, pf, pt, perm, smax, ntt_max, mband != nullptr, F != nullptr, zlist, ldz);
 	// Instance groups (contiguous in the sorted order, balanced by work) on their
 	// own streams; within a group, the instances still in their pulse at step s
 	// are a prefix, and the field-free ones lie below a bound.

@@ -330,23 +330,23 @@ void pos_report(const pos_path* p, int32_t out[4])
 #define POS_PROF(kind) struct prof_ { const pos_run& r; int k; prof_(const pos_run& r_, int k_) : r(r_), k(k_) { if (r.prof_begin) r.prof_begin(k, r.stream); } \
 	~prof_() { if (r.prof_end) r.prof_end(k, r.stream); } } prof_scope_(r, kind)
 
+// X^T (M X): S^-1 is 1 in this basis
+int pos_mask(pos_path* p, const double* mask, int64_t* launches, cudaStream_t st, bool* ok)
+{
+	const size_t nn = (size_t)p->N * p->N;
+	scratch tmp(st);
+	double *Mx, *A;
+	int rc;
+	if ((rc = tmp.get(&Mx, nn)) || (rc = tmp.get(&A, nn)) || (rc = project_band(&p->ops, mask, false, Mx, A, st))) return rc;
+	*launches += 4;
+	return store_banded(&p->ops, p->K, A, p->N, 1, st, ok);
+}
+
 int pos_begin(pos_path* p, const pos_run& r)
 {
 	const int nchan = p->M * p->L;
 	const long nvec = (long)p->B * nchan;
 	cudaStream_t st = r.stream;
-	if (r.mask) {
-		// the mask X^T (M X) in this basis (S^-1 is 1 there)
-		const size_t nn = (size_t)p->N * p->N;
-		scratch tmp(st);
-		double *Mx, *A;
-		int rc;
-		if ((rc = tmp.get(&Mx, nn)) || (rc = tmp.get(&A, nn)) || (rc = project_band(&p->ops, r.mask, false, Mx, A, st))) return rc;
-		*r.launches += 4;
-		bool ok = false;
-		if ((rc = store_banded(&p->ops, p->K, A, p->N, 1, st, &ok))) return rc;
-		if (!ok) { set_error("the mask does not fall off the diagonal in the position basis"); return QPC_ERR_NUMERIC; }
-	}
 	if (r.z && !p->zpart) if (int rc = dalloc(&p->zpart, (size_t)pos_path::ZB * p->B * p->M * p->ntile * EPT)) return rc;
 	p->zcount = 0;
 	POS_PROF(QPC_KERNEL_TRANSFORM_FWD);

@@ -35,7 +35,7 @@ struct pos_run {
 	const int64_t *ntf, *ntt;	// device [B], by slot
 	const double* ftab;		// device [B][ld], by slot
 	long ld;
-	const double* mask;		// device band [N][P+1] applied (with S^-1) after every step, or nullptr
+	bool mask;			// the operator of pos_mask is applied after every step
 	double* z;			// device [B][ldz], the dipole of f(r) = r before every step, or nullptr
 	long ldz;
 	int64_t* launches;
@@ -44,6 +44,9 @@ struct pos_run {
 	std::function<void(int, cudaStream_t)> prof_begin, prof_end;	// per-kernel timing, or empty
 	cudaStream_t stream;
 };
+// the operator of a run's mask (device band [N][P+1]), before pos_begin of that run; ok = false: it does not suit the
+// fixed-point products
+int pos_mask(pos_path* p, const double* mask, int64_t* launches, cudaStream_t st, bool* ok);
 int pos_begin(pos_path* p, const pos_run& r);
 // loop step s: Bc slots (a prefix) may couple, Bf slots (a prefix) may take the field-free step
 int pos_step(pos_path* p, const pos_run& r, long s, int Bc, int Bf);

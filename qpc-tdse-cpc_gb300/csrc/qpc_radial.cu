@@ -883,9 +883,10 @@ int store_banded_impl(radial_ops* p, band_store& b, const double* A, long si, lo
 		k_profile<<<std::min(WMAX, p->N - 1) + 1, 128, 0, st>>>(A, si, sj, p->N, p->prof);
 		if (int rc = read_profile(p, st, prof)) return rc;
 		for (auto u : prof) { double v; std::memcpy(&v, &u, 8); big = std::max(big, v); }
-		*ok = big > 0.0 && big < 1e200;
+		*ok = big == 0.0 || (big > 1e-200 && big < 1e200);	// its power of two and the limbs' in FP64
 		if (!*ok) return QPC_OK;
-		std::frexp(big, &b.ea);
+		b.ea = 0;	// of zeros
+		if (big > 0.0) std::frexp(big, &b.ea);
 		*ok = decay(prof, p->N, std::ldexp(1.0, b.ea), w, wf, 29);
 		if (!*ok) return QPC_OK;
 		double sum = -big;	// at least any row's sum of magnitudes
