@@ -4,6 +4,7 @@
 #include "qpc_internal.h"
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cstdlib>
 #include <time.h>
 
 namespace qpc {
@@ -24,11 +25,27 @@ inline int check_device(int* dev)
 	return QPC_OK;
 }
 
+// QPC_ALLOC_MAX: device allocations above this many bytes fail, as they would on a full card (for tests of what happens then)
+inline bool alloc_refused(size_t bytes)
+{
+	const char* e = std::getenv("QPC_ALLOC_MAX");
+	return e && bytes > (size_t)std::atoll(e);
+}
+
+// a failure leaves no error behind for the next cudaGetLastError: some callers go on with less memory
 template <class T> inline int dalloc(T** p, size_t n)
 {
-	cudaError_t e = cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(n, 1));
-	if (e != cudaSuccess) { *p = nullptr; set_error("cudaMalloc(%zu bytes): %s", sizeof(T) * n, cudaGetErrorString(e)); return QPC_ERR_NOMEM; }
+	const size_t bytes = sizeof(T) * std::max<size_t>(n, 1);
+	cudaError_t e = alloc_refused(bytes) ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, bytes);
+	if (e != cudaSuccess) { cudaGetLastError(); *p = nullptr; set_error("cudaMalloc(%zu bytes): %s", sizeof(T) * n, cudaGetErrorString(e)); return QPC_ERR_NOMEM; }
 	return QPC_OK;
+}
+
+inline size_t free_bytes()
+{
+	size_t f = 0, total = 0;
+	if (cudaMemGetInfo(&f, &total) != cudaSuccess) { cudaGetLastError(); return 0; }
+	return f;
 }
 
 // bounded wait: poll the stream until its work is done, give up after

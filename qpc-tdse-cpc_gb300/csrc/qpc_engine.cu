@@ -486,7 +486,7 @@ struct qpc_lgwz {
 	int last_pos = -1;		// the last run: 1 position basis, 0 banded solves
 	size_t fac_elems = 0;
 	bool chains_ready = false;	// the banded solves' buffers exist
-	std::vector<double2> ffh;	// host copy of ff until they do
+	double2* lent[2] = {nullptr, nullptr};	// those of st, eo and wk that belong to pos
 	std::vector<double> h_lam;   // [M][L]
 	std::vector<double> h_P;     // [M][L][L]
 };
@@ -983,26 +983,41 @@ static void host_spikes(const double2* fac, size_t nblk, int N, int Q, int Ls, d
 		}
 }
 
+// the work vector of the banded solves, and eo: the position basis' buffers where the handle has them
+static int need_work(qpc_lgwz* h)
+{
+	if (h->wk) return QPC_OK;
+	if (!h->pos) return dalloc(&h->wk, state_len(h));
+	pos_buffers(h->pos, h->lent);
+	h->wk = h->lent[1];
+	if (!h->eo) h->eo = h->lent[0];
+	return QPC_OK;
+}
+
 // the buffers of the banded solves, made when a run first needs them
 static int need_chains(qpc_lgwz* h)
 {
 	if (h->chains_ready) return QPC_OK;
 	const int N = h->N, P = h->P, NE = P + 1;
-	const long sl = state_len(h);
 	int rc;
-	if ((!h->st && (rc = dalloc(&h->st, sl))) || (!h->eo && (rc = dalloc(&h->eo, sl))) || (!h->wk && (rc = dalloc(&h->wk, sl))) ||
-		(!h->fac && (rc = dalloc(&h->fac, h->fac_elems))))
-		return rc;
+	if ((rc = need_work(h)) || (!h->st && (rc = dalloc(&h->st, state_len(h)))) || (!h->eo && (rc = dalloc(&h->eo, state_len(h))))) return rc;
+	// less look-ahead where the factors find no room
+	while (!h->fac && (rc = dalloc(&h->fac, h->fac_elems))) {
+		if (h->K == 1) return rc;
+		h->fac_elems /= 2;
+		h->K /= 2;
+	}
 	if (h->seg_ok) {
-		const size_t nblk_ff = h->ffh.size() / ((size_t)N * NE), nblk_c = (size_t)h->K * h->B * h->M * h->npair;
-		std::vector<double2> sf(nblk_ff * N * P), sb(nblk_ff * N * P);
+		const size_t nblk_ff = (size_t)(h->hpi ? h->B : 1) * h->nlh, nblk_c = (size_t)h->K * h->B * h->M * h->npair;
+		std::vector<double2> ffh(nblk_ff * N * NE), sf(nblk_ff * N * P), sb(nblk_ff * N * P);
+		if ((rc = copy_to_host(ffh.data(), h->ff, sizeof(double2) * ffh.size(), h->stream))) return rc;
 		switch (P) {
-		case 3: host_spikes<3>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 4: host_spikes<4>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 5: host_spikes<5>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 6: host_spikes<6>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 7: host_spikes<7>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
-		case 8: host_spikes<8>(h->ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 3: host_spikes<3>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 4: host_spikes<4>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 5: host_spikes<5>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 6: host_spikes<6>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 7: host_spikes<7>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
+		case 8: host_spikes<8>(ffh.data(), nblk_ff, N, h->Q, h->Ls, sf.data(), sb.data()); break;
 		}
 		if ((rc = dalloc(&h->spf_ff, sf.size())) || (rc = dalloc(&h->spb_ff, sb.size())) ||
 			(rc = dalloc(&h->spf_c, nblk_c * N * P)) || (rc = dalloc(&h->spb_c, nblk_c * N * P)))
@@ -1016,7 +1031,6 @@ static int need_chains(qpc_lgwz* h)
 		}
 		if ((rc = wait_on(h->stream))) return rc;
 	}
-	h->ffh = std::vector<double2>();
 	h->chains_ready = true;
 	return QPC_OK;
 }
@@ -1266,7 +1280,6 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 	for (int g = 1; g <= P; ++g) if (P % g == 0 && (g <= 4 || g == P)) h->gcand.push_back(g);
 	if (h->seg_ok) h->gcand.push_back(QPC_SEG);	// the segmented solver
 	h->h_R.assign(R, R + (size_t)N * NE);
-	h->ffh.swap(ffh);
 	// the position basis, unless a switch asks for kernels of the banded solves (QPC_POS=1 keeps it all the same)
 	const char* ps = getenv("QPC_POS");
 	if (ps ? atoi(ps) != 0 : !getenv("QPC_CHAIN_G") && !getenv("QPC_LTRANS_TC")) {
@@ -1278,7 +1291,7 @@ static int create_impl(const qpc_dims* dims, double dt, const double* S, const d
 		in.fieldfree = [&](double2* X, double2* wk, int J, int fi) { return fieldfree_columns(h, X, wk, J, fi, one); };
 		rc = pos_create(in, &h->pos);
 		cudaFree(one);
-		if (rc) return fail(rc);
+		if (rc && rc != QPC_ERR_NOMEM) return fail(rc);	// no room for it: the banded solves need less
 	}
 	if (!h->pos) if ((rc = need_chains(h))) return fail(rc);
 	if ((rc = wait_on(h->stream))) return fail(rc);
@@ -1306,7 +1319,8 @@ int qpc_lgwz_destroy(qpc_lgwz* h)
 	cudaFree(h->S); cudaFree(h->R); cudaFree(h->Vh); cudaFree(h->lamp); cudaFree(h->ff); cudaFree(h->lt_dig); cudaFree(h->lt_fex);
 	cudaFree(h->ffmap); cudaFree(h->ffmap_id);
 	cudaFree(h->spf_c); cudaFree(h->spb_c); cudaFree(h->spf_ff); cudaFree(h->spb_ff);
-	cudaFree(h->st); cudaFree(h->eo); cudaFree(h->wk); cudaFree(h->hostlay); cudaFree(h->fac);
+	for (double2* p : {h->st, h->eo, h->wk}) if (p != h->lent[0] && p != h->lent[1]) cudaFree(p);
+	cudaFree(h->hostlay); cudaFree(h->fac);
 	cudaFree(h->status); cudaFree(h->red); cudaFree(h->ntf); cudaFree(h->ntt); cudaFree(h->ftab);
 	cudaFree(h->obsF); cudaFree(h->obs); cudaFree(h->dl); cudaFree(h->y10d); cudaFree(h->zdev);
 	cudaFree(h->mM); cudaFree(h->mLrow); cudaFree(h->mLcol); cudaFree(h->mdinv); cudaFree(h->slotmap);
@@ -1529,7 +1543,10 @@ static int run_impl(qpc_lgwz* h, const double* ftab, int64_t ld, const int64_t* 
 		if (int rc = mask_prepare(h)) return rc;
 		QPC_CUDA(cudaEventRecord(h->ev0, h->stream));
 		QPC_CUDA(cudaMemcpyAsync(h->mM, mband, sizeof(double) * h->N * (h->P + 1), cudaMemcpyHostToDevice, h->stream));
-		if (int rc = pos_mask(h->pos, h->mM, &h->launches, h->stream, &pos)) return rc;
+		if (int rc = pos_mask(h->pos, h->mM, &h->launches, h->stream, &pos)) {
+			if (rc != QPC_ERR_NOMEM) return rc;
+			pos = false;
+		}
 	}
 	h->last_pos = pos;
 	if (pos) {
@@ -1806,7 +1823,7 @@ int qpc_lgwz_mask(qpc_lgwz* h, const double* M)
 	if (int rc = wait_stream(h)) return rc;
 	if (int rc = mask_prepare(h)) return rc;
 	if (int rc = need_rmajor(h)) return rc;
-	if (!h->wk) if (int rc = dalloc(&h->wk, (size_t)state_len(h))) return rc;
+	if (int rc = need_work(h)) return rc;
 	h->lay_valid = false;
 	QPC_CUDA(cudaMemcpyAsync(h->mM, M, sizeof(double) * N * NE, cudaMemcpyHostToDevice, h->stream));
 	mask_enqueue(h, h->stream, nullptr, 0);

@@ -104,21 +104,6 @@ __global__ void __launch_bounds__(256) k_pcs_join(const double2* __restrict__ P,
 		if (kr0 + i < nkr) Q[(inst * nkr + kr0 + i) * nch + ch] = cmul(cps[(size_t)(kr0 + i) * nl_tot + l], t[tx][i]);
 }
 
-// ijlT[l][r][kr] = ijl[kr][l][r]
-__global__ void __launch_bounds__(256) k_pcs_transpose(const double* __restrict__ ijl, double* __restrict__ ijlT, int nkr, int nl, int n_r)
-{
-	__shared__ double t[32][33];
-	const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-	for (int l = blockIdx.z; l < nl; l += gridDim.z) {
-		__syncthreads();
-		for (int i = ty; i < 32; i += 8)
-			if (k0 + i < nkr && r0 + tx < n_r) t[i][tx] = ijl[((size_t)(k0 + i) * nl + l) * n_r + r0 + tx];
-		__syncthreads();
-		for (int i = ty; i < 32; i += 8)
-			if (r0 + i < n_r && k0 + tx < nkr) ijlT[((size_t)l * n_r + r0 + i) * nkr + k0 + tx] = t[tx][i];
-	}
-}
-
 // With Q = cps <ijl|c>:
 // LMD[inst][kr][ch] = sqrt(2/pi) Q                                   (measure_lmd, 386-403)
 // PMD[inst][kr][kt][kp] = sqrt(2/pi) sum_m exm[kp][m] sum_l plm Q     (measure_prj, 337-355)
@@ -428,6 +413,18 @@ int pcs_run(qpc_pcs* h, int kind, const double2* c, int n_inst, double* out)
 	return QPC_OK;
 }
 
+// ijlT[l][r][kr] = ijl[kr][l][r]
+int plain_table(qpc_pcs* h, const double* ijl)
+{
+	const size_t n = h->d.n_r, nl = h->nl, nk = h->nkr;
+	std::vector<double> t(nl * n * nk);
+	for (size_t k = 0; k < nk; ++k)
+		for (size_t l = 0; l < nl; ++l)
+			for (size_t r = 0; r < n; ++r) t[(l * n + r) * nk + k] = ijl[(k * nl + l) * n + r];
+	if (int rc = upload(&h->ijlT, t.data(), t.size(), h->st)) return rc;
+	return wait_on(h->st);
+}
+
 // the projector's table on the device: digit planes where it suits them, or transposed for k_pcs_proj
 int pcs_table(qpc_pcs* h, const double* ijl)
 {
@@ -436,7 +433,7 @@ int pcs_table(qpc_pcs* h, const double* ijl)
 	int rc;
 	scratch tmp(h->st);
 	double* raw;
-	if ((rc = tmp.get(&raw, (size_t)nk * nl * n))) return rc;
+	if (tmp.get(&raw, (size_t)nk * nl * n)) return plain_table(h, ijl);
 	QPC_CUDA(cudaMemcpyAsync(raw, ijl, sizeof(double) * (size_t)nk * nl * n, cudaMemcpyHostToDevice, h->st));
 	std::vector<int> lm(nch);
 	for (int c = 0; c < nch; ++c) lm[c] = std::abs(d.m0 + c / d.n_l) + c % d.n_l;
@@ -450,10 +447,8 @@ int pcs_table(qpc_pcs* h, const double* ijl)
 	if (ok) return wait_on(h->st);
 	for (tc_store& t : h->seg) t.release();
 	h->seg.clear();
-	if ((rc = dalloc(&h->ijlT, (size_t)nl * n * nk))) return rc;
-	k_pcs_transpose<<<dim3((n + 31) / 32, (nk + 31) / 32, std::min(nl, 65535)), 256, 0, h->st>>>(raw, h->ijlT, nk, nl, n);
-	QPC_CUDA(cudaGetLastError());
-	return wait_on(h->st);
+	tmp.release();
+	return plain_table(h, ijl);
 }
 
 // one accumulate, enqueued on st without a wait: the surface values come from c (host layout

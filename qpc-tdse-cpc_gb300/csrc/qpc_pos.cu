@@ -321,6 +321,11 @@ void pos_destroy(pos_path* p)
 	delete p;
 }
 
+void pos_buffers(const pos_path* p, double2* out[2])
+{
+	out[0] = p->buf[0]; out[1] = p->buf[1];
+}
+
 void pos_report(const pos_path* p, int32_t out[4])
 {
 	out[0] = p->ops.F.has_tc; out[1] = p->ops.W.has_tc; out[2] = p->ops.X.has_tc;

@@ -25,6 +25,8 @@ struct pos_setup {
 // *out = nullptr with QPC_OK when the operators do not suit the path
 int pos_create(const pos_setup& in, pos_path** out);
 void pos_destroy(pos_path* p);
+// its two state-sized buffers, which hold nothing between runs
+void pos_buffers(const pos_path* p, double2* out[2]);
 // digit planes of F~, W = X^T S and X (0 or 1), and the kernel of the last run's first field-free product (QPC_PRODUCT_*)
 void pos_report(const pos_path* p, int32_t out[4]);
 

@@ -961,7 +961,8 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 			if (!(*ok = decay(prof, N, 1.0, w, wf, 29))) return QPC_OK;
 			if (p->nff > 1) { w = std::min(std::min(WMAX, N - 1), w + 8); wf = std::min(w, wf + 12); }	// the other potentials' bands, checked below
 			lay_out(p->F, N, w, wf, true);
-			if (!(*ok = (size_t)p->F.stride * nlh * p->nff <= (size_t)16 << 30)) return QPC_OK;
+			// resident for the handle's life: at most 16 GB, and a quarter of what is free (more handles and the caller's own data share the card)
+			if (!(*ok = (size_t)p->F.stride * nlh * p->nff <= std::min<size_t>((size_t)16 << 30, free_bytes() / 4))) return QPC_OK;
 			if ((rc = upload(p->F, (size_t)p->F.stride * nlh * p->nff, st))) return rc;
 		}
 		k_store<true><<<dim3(p->ntile, nlh), 256, 0, st>>>(Fb, nullptr, 0, 0, N, p->F.w, std::ldexp(1.0, 56), p->F.d_td, p->F.d_off,

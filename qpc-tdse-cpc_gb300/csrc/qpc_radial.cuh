@@ -94,7 +94,8 @@ struct radial_ops {
 };
 
 // ok = false (with QPC_OK): S not positive definite, eigenvalues not apart, or an operator that does not fall off
-// within WMAX of the diagonal (or takes more than 16 GB)
+// within WMAX of the diagonal (or takes more than 16 GB,
+// or more than a quarter of the free memory)
 int radial_create(radial_ops* p, const radial_setup& in, int nmap, bool* ok);
 void radial_destroy(radial_ops* p);
 
@@ -122,10 +123,16 @@ struct scratch {
 	cudaStream_t st;
 	std::vector<void*> ptr;
 	explicit scratch(cudaStream_t s) : st(s) {}
-	~scratch() { for (void* q : ptr) cudaFreeAsync(q, st); }
+	~scratch() { release(); }
+	void release()
+	{
+		for (void* q : ptr) cudaFreeAsync(q, st);
+		ptr.clear();
+	}
 	template <class T> int get(T** q, size_t n)
 	{
-		if (cudaMallocAsync((void**)q, sizeof(T) * std::max<size_t>(n, 1), st) != cudaSuccess) {
+		const size_t bytes = sizeof(T) * std::max<size_t>(n, 1);
+		if (alloc_refused(bytes) || cudaMallocAsync((void**)q, bytes, st) != cudaSuccess) {
 			cudaGetLastError();
 			set_error("set-up scratch of %zu bytes", sizeof(T) * n);
 			return QPC_ERR_NOMEM;

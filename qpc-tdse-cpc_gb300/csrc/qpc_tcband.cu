@@ -473,7 +473,7 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 		t.work.push_back(work);
 	}
 	t.stride = o;
-	if (o * nop > (size_t)4 << 30) return QPC_OK;
+	if (o * nop > std::min<size_t>((size_t)4 << 30, free_bytes() / 8)) return QPC_OK;
 	int* d_tile;
 	size_t* d_at;
 	if ((rc = tmp.get(&d_tile, tile_of.size())) || (rc = tmp.get(&d_at, at.size()))) return rc;
@@ -500,18 +500,20 @@ int make(tc_store& t, const make_args& m, int nop, const double* prof, cudaStrea
 int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, long sj, int nrow, int N, int nop, int w, const double* prof, int ea,
 	bool rows, cudaStream_t st, bool* ok, int kb, int ke)
 {
+	t.release();
 	*ok = false;
 	make_args m{Fb, A, sop, si, sj, nrow, N, w, ea, nullptr, kb, ke < 0 ? N : ke};
 	int rc;
 	if (rows) {
-		if ((rc = dalloc(&t.ear, (size_t)nrow * nop))) return rc;
+		if (dalloc(&t.ear, (size_t)nrow * nop)) return QPC_OK;
 		k_tc_rows<<<dim3(nrow, nop), 32, 0, st>>>(m, t.ear);
 		QPC_CUDA(cudaGetLastError());
 		m.ear = t.ear;
 	}
 	rc = make<8>(t, m, nop, prof, st, ok);
 	if (!rc && !*ok) rc = make<7>(t, m, nop, prof, st, ok);
-	return rc;
+	if (rc || !*ok) { *ok = false; t.release(); }
+	return rc == QPC_ERR_NOMEM ? QPC_OK : rc;
 }
 
 namespace {

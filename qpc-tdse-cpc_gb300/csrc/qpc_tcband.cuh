@@ -8,7 +8,8 @@ namespace qpc {
 // w: half-band, or -1 for a dense one; rows: each row under its own
 // largest exponent in place of ea; kb, ke: the columns that take part (kb a multiple of 32).
 // prof: largest |entry| per distance as in radial_create (NULL: every entry counts).  ok = false: an exact sum could
-// exceed 2^24, or the planes would take more than 4 GB.
+// exceed 2^24, the planes would take more than 4 GB or an eighth of the free memory, or there is no room for them (t is
+// empty then, and the products go without).
 int tc_make(tc_store& t, const double2* Fb, const double* A, long sop, long si, long sj, int nrow, int N, int nop, int w, const double* prof, int ea,
 	bool rows, cudaStream_t st, bool* ok, int kb = 0, int ke = -1);
 

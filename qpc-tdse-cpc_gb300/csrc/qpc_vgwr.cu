@@ -954,6 +954,7 @@ int make_pos(qpc_vgwr* h, const std::vector<int>& chmap, const double* Ri)
 	if (ps ? std::atoi(ps) == 0 : std::getenv("QPC_VG_GEMM") || std::getenv("QPC_OZ_TC") || std::getenv("QPC_OZ_TMA")) return QPC_OK;
 	vpos_setup in{};
 	in.N = h->N; in.P = h->P; in.nch = h->nch; in.nlh = h->nlh; in.B = h->B; in.n_l = h->d.n_l; in.m0 = h->d.m0; in.dt = h->dt;
+	in.buf[0] = h->U; in.buf[1] = h->U + (size_t)h->B * h->nch * h->N;	// the banded solves' scratch, p + 2 states long
 	in.S = h->S; in.D = h->D; in.Ri = Ri; in.chmap = chmap.data(); in.stream = h->st;
 	for (int b = 0; b < 2; ++b) {
 		in.off[b] = h->off[b]; in.na[b] = h->na[b]; in.nb[b] = h->nb[b];
@@ -977,7 +978,7 @@ int make_pos(qpc_vgwr* h, const std::vector<int>& chmap, const double* Ri)
 	if (!rc) rc = vpos_create(in, &h->pos);
 	if (const int w = wait_on(h->st)) rc = rc ? rc : w;	// the copies, where nothing was made
 	cudaFree(done); cudaFree(did);
-	return rc;
+	return rc == QPC_ERR_NOMEM ? QPC_OK : rc;	// no room for it: the banded solves need none of it
 }
 
 } // namespace

@@ -221,7 +221,8 @@ int momentum_basis(vpos_path* p, const vpos_setup& in, bool* ok)
 	if ((rc = project_band(&p->ops, in.D, true, T, A, st))) return rc;
 	k_hermitian<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(A, N, H);
 	cusolverDnHandle_t sol = nullptr;
-	if (cusolverDnCreate(&sol) != CUSOLVER_STATUS_SUCCESS) { set_error("cusolverDnCreate failed"); return QPC_ERR_CUDA; }
+	// without room for its handle or work space: as any allocation that fails
+	if (cusolverDnCreate(&sol) != CUSOLVER_STATUS_SUCCESS) { cudaGetLastError(); set_error("cusolverDnCreate failed"); return QPC_ERR_NOMEM; }
 	struct guard { cusolverDnHandle_t s; ~guard() { cusolverDnDestroy(s); } } g{sol};
 	int lwork = 0;
 	if (cusolverDnSetStream(sol, st) != CUSOLVER_STATUS_SUCCESS ||
@@ -230,8 +231,10 @@ int momentum_basis(vpos_path* p, const vpos_setup& in, bool* ok)
 		return QPC_ERR_CUDA;
 	}
 	if ((rc = tmp.get(&work, (size_t)std::max(lwork, 1)))) return rc;
-	if (cusolverDnZheevd(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, H, N, w, work, lwork, info) != CUSOLVER_STATUS_SUCCESS) {
+	const cusolverStatus_t cs = cusolverDnZheevd(sol, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, H, N, w, work, lwork, info);
+	if (cs != CUSOLVER_STATUS_SUCCESS) {
 		set_error("heevd failed");
+		if (cs == CUSOLVER_STATUS_ALLOC_FAILED) { cudaGetLastError(); return QPC_ERR_NOMEM; }
 		return QPC_ERR_CUDA;
 	}
 	k_pairs<<<(N + 1) / 2, 128, 0, st>>>(H, w, N, Qt, p->om);
@@ -291,8 +294,10 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 	if ((rc = dalloc(&p->lmap, nch))) return rc;
 	QPC_CUDA(cudaMemcpyAsync(p->lmap, lm.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, st));
 	const long nvec = (long)p->B * nch;
-	for (int i = 0; i < 2; ++i)
-		if ((rc = dalloc(&p->buf[i], (size_t)nvec * N)) || (rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
+	for (int i = 0; i < 2; ++i) {
+		p->buf[i] = in.buf[i];
+		if ((rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
+	}
 	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT)) || (rc = dalloc(&p->status, 1))) return rc;
 	QPC_CUDA(cudaMallocHost(&p->hstatus, sizeof(int)));
 	*p->hstatus = 0;
@@ -332,7 +337,7 @@ void vpos_destroy(vpos_path* p)
 {
 	if (!p) return;
 	cudaFree(p->om); cudaFree(p->rinv); cudaFree(p->tab); cudaFree(p->lmap);
-	for (int i = 0; i < 2; ++i) { cudaFree(p->buf[i]); cudaFree(p->ex[i]); }
+	for (int i = 0; i < 2; ++i) cudaFree(p->ex[i]);
 	cudaFree(p->exin); cudaFree(p->status);
 	if (p->hstatus) cudaFreeHost(p->hstatus);
 	p->TD.release(); p->TI.release();

@@ -19,6 +19,7 @@ struct vpos_setup {
 	const double* tm[5][2][2];	// device, see qpc_vgwr.cu
 	const double* lam[4];		// device, engine order
 	double2 gam[4][2][2];
+	double2* buf[2];		// two state-sized buffers of the caller's, used within a run only
 	std::function<int(double2*, double2*, int, int)> fieldfree;	// on J vectors X[J][nlh][N]
 	cudaStream_t stream;
 };
