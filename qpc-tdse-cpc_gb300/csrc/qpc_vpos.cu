@@ -200,6 +200,7 @@ struct vpos_path {
 	int* exin = nullptr;
 	size_t smem = 0;
 	int *status = nullptr, *hstatus = nullptr;	// a tensor-core wait ran out (device, pinned)
+	bool on_tensor_cores() const { return TD.has_tc || TI.has_tc; }	// either transform may have planes without the other
 	cudaStream_t stream = nullptr;
 };
 
@@ -299,6 +300,7 @@ int build(vpos_path* p, const vpos_setup& in, bool* ok)
 		if ((rc = dalloc(&p->ex[i], (size_t)nvec * p->ntile * EPT))) return rc;
 	}
 	if ((rc = dalloc(&p->exin, (size_t)nvec * p->ntile * EPT)) || (rc = dalloc(&p->status, 1))) return rc;
+	QPC_CUDA(cudaMemsetAsync(p->status, 0, sizeof(int), st));
 	QPC_CUDA(cudaMallocHost(&p->hstatus, sizeof(int)));
 	*p->hstatus = 0;
 	p->smem = sizeof(double2) * 32 * std::max(in.nb[0], in.nb[1]);
@@ -415,7 +417,7 @@ void fieldfree(vpos_path* p, const vpos_run& r, int src, long s, int k0, int n)
 int vpos_begin(vpos_path* p, const vpos_run& r)
 {
 	prof_scope ps(r, 0);
-	if (p->TD.has_tc) QPC_CUDA(cudaMemsetAsync(p->status, 0, sizeof(int), p->stream));
+	if (p->on_tensor_cores()) QPC_CUDA(cudaMemsetAsync(p->status, 0, sizeof(int), p->stream));
 	exponents(r.X, p->exin, p->N, p->ntile, (long)p->B * p->nch, p->stream);
 	band_args a = band_args_of(&p->ops, p->ops.W, p->nch, p->B);
 	a.s0 = r.X; a.e0 = p->exin; a.dst = p->buf[0]; a.edst = p->ex[0];
@@ -473,7 +475,7 @@ int vpos_end(vpos_path* p, const vpos_run& r)
 	band_apply(a, false, p->ntile, p->stream);
 	++*r.launches;
 	QPC_CUDA(cudaGetLastError());
-	if (p->TD.has_tc) QPC_CUDA(cudaMemcpyAsync(p->hstatus, p->status, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
+	if (p->on_tensor_cores()) QPC_CUDA(cudaMemcpyAsync(p->hstatus, p->status, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
 	return QPC_OK;
 }
 
