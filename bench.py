@@ -175,10 +175,33 @@ def band_digit_flops(n_r, n_l, B, per=15.5):
     return total * n_l * B
 
 
-def pos_roofline(ktimes, n_r, n_l, B):
-    """the step's dominant kernel in the position basis"""
+def band_entries(n_r, n_l, w=110, wf=56):
+    """entries of the field-free operators as k_band_one and k_band_apply hold them (p = 6, csrc/qpc_radial.cu): (two complex
+    28-bit limbs, 16 bytes, 12 multiply-adds a column, within wf rows of the diagonal where an entry is above 2^-29;
+    one, 8 bytes, 4 multiply-adds, out to w)"""
+    near = sum(min(wf, r) + min(wf, n_r - 1 - r) + 1 for r in range(n_r))
+    return n_l * near, n_l * (sum(min(w, r) + min(w, n_r - 1 - r) + 1 for r in range(n_r)) - near)
+
+
+def pos_roofline(ktimes, n_r, n_l, B, product="k_tc_apply"):
+    """the step's dominant kernel in the position basis; product: the kernel of the field-free step, as the handle
+    reports it"""
     ms, n = ktimes["fieldfree"]
     peaks = load_peaks()
+    if product != "k_tc_apply":
+        # integer multiply-adds: one column is bound by the operators' bytes, several by the multiply-adds
+        launch_ms = ms / n
+        near, far = band_entries(n_r, n_l)
+        by, mads = 16.0 * near + 8.0 * far + 32.0 * B * n_l * n_r, B * (12.0 * near + 4.0 * far)
+        roof = {"kernel": "%s (banded field-free products, integer limbs)" % product, "launch_ms": launch_ms, "traffic": None,
+                "bytes_per_launch": by, "multiply_adds_per_launch": mads}
+        if product == "k_band_one":
+            ach, peak = by / (launch_ms * 1e-3) / 1e9, peaks.get("hbm_gbs")
+            return dict(roof, bound="hbm", achieved=ach, peak=peak, unit="GB/s", frac=ach / peak if peak else None,
+                        peak_source="MEASURED_PEAKS.json hbm_gbs")
+        ach = mads / (launch_ms * 1e-3) / 1e12
+        return dict(roof, bound="integer multiply-adds", achieved=ach, peak=8.0, unit="T multiply-adds/s", frac=ach / 8.0,
+                    peak_source="26 wide multiply-adds a cycle and SM, measured (csrc/qpc_radial.cu)")
     fl, bf = band_digit_flops(n_r, n_l, B), peaks.get("bf16_tflops")
     launch_ms = ms / n
     ach = fl / (launch_ms * 1e-3) / 1e12
@@ -316,7 +339,7 @@ def run_engine(args, sync=None):
     if roof["hbm"]["achieved_gbs"] and peaks.get("hbm_gbs"):
         roof["hbm"]["frac"] = roof["hbm"]["achieved_gbs"] / peaks["hbm_gbs"]
     if not ktimes["factor"][1] and ktimes["fieldfree"][1]:  # no factorisations: the position basis
-        roof = pos_roofline(ktimes, n_r, n_l, B)
+        roof = pos_roofline(ktimes, n_r, n_l, B, prop.path()["product"])
         roof["fp64_equivalent"] = {"flops_per_wf_step": path_flops(n_r, p, n_l), "achieved_tflops": path_tflops,
                                    "ratio_to_fp64_peak": path_tflops / fp64_peak()["tflops"], "note": "FP64 flops of the banded solves this replaces"}
     kt = {k: {"ms_total": v[0], "launches": v[1]} for k, v in ktimes.items()}
