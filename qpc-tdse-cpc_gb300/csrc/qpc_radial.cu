@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 	auto emit = [&](int cl, long long hr, long long mr, long long hi, long long mi) {
 		const int c = col0 + cl;
 		if (c >= p.ncols || (p.nta && !(p.step < p.nta[c]))) return;
-		const int E = sE[cl], s = p.ea + E - 1078;
+		const int E = sE[cl], s = p.ea + E - 1078 + (p.er && row < p.N ? p.er[row] : 0);
 		const double2 y = make_double2(to_double(hr, mr, s, E == 0x7ff), to_double(hi, mi, s, E == 0x7ff));
 		const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 		if (row < p.N) p.dst[o * p.N + row] = y;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(256, 4) k_band_one(const band_args p)
 #pragma unroll
 	for (int w = 1; w < 8; ++w) { rh += red[w][0][lane]; rm += red[w][1][lane]; ih += red[w][2][lane]; im += red[w][3][lane]; }
 	flush(rh, rm); flush(ih, im);
-	const int row = tile * TM + lane, s = p.ea + E - 1078;
+	const int row = tile * TM + lane, s = p.ea + E - 1078 + (p.er && row < p.N ? p.er[row] : 0);
 	const double2 y = make_double2(to_double(rh, rm, s, E == 0x7ff), to_double(ih, im, s, E == 0x7ff));
 	const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 	if (row < p.N) p.dst[o * p.N + row] = y;
@@ -618,6 +618,22 @@ __global__ void k_profile(const double* __restrict__ A, long si, long sj, int N,
 	}
 	for (int o = 16; o; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
 	if ((threadIdx.x & 31) == 0) atomicMax(prof + d, (unsigned long long)__double_as_longlong(big));
+}
+
+// each row under its own power of two: A(i, j) = out[i][j] 2^er[i], |out| < 1
+__global__ void __launch_bounds__(128) k_scale_rows(const double* __restrict__ A, long si, long sj, int N, double* __restrict__ out, int* __restrict__ er)
+{
+	const int i = blockIdx.x;
+	__shared__ double part[4];
+	double big = 0.0;
+	for (int j = threadIdx.x; j < N; j += 128) big = fmax(big, fabs(A[i * si + j * sj]));
+	for (int o = 16; o; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+	if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = big;
+	__syncthreads();
+	big = fmax(fmax(part[0], part[1]), fmax(part[2], part[3]));
+	const int e = big > 0.0 && big < 1e200 ? ilogb(big) + 1 : 0;
+	if (threadIdx.x == 0) er[i] = e;
+	for (int j = threadIdx.x; j < N; j += 128) out[(long)i * N + j] = ldexp(A[i * si + j * sj], -e);
 }
 
 // columns j0 .. j0+J of F~ (G[jj][l][i]) into the band Fb[l][i][2 WMAX + 1], with the profile
@@ -913,15 +929,22 @@ int build(radial_ops* p, const radial_setup& in, int nmap, bool* ok)
 	scratch tmp(st);
 	double* Yt = nullptr;
 	if ((rc = eigenvectors(p, in, tmp, &Yt, ok)) || !*ok) return rc;
-	if ((rc = store_banded(p, p->W, Yt, N, 1, st, ok)) || !*ok) return rc;
-	if ((rc = store_banded(p, p->X, p->Xt, 1, N, st, ok)) || !*ok) return rc;
+	// The rows of W = X^T S go with sqrt(h) and those of X with 1 / sqrt(h), h the grid's local spacing: one power of two for
+	// all would leave the rows of a graded grid's fine end log2 sqrt(h_max / h_min) bits fewer.  W also forms F~ below.
+	double *Ws, *Xs;
+	if ((rc = dalloc(&p->W.er, N)) || (rc = dalloc(&p->X.er, N)) || (rc = tmp.get(&Ws, (size_t)N * N)) || (rc = tmp.get(&Xs, (size_t)N * N))) return rc;
+	k_scale_rows<<<N, 128, 0, st>>>(Yt, N, 1, N, Ws, p->W.er);
+	k_scale_rows<<<N, 128, 0, st>>>(p->Xt, 1, N, N, Xs, p->X.er);
+	QPC_CUDA(cudaGetLastError());
+	if ((rc = store_banded(p, p->W, Ws, N, 1, st, ok)) || !*ok) return rc;
+	if ((rc = store_banded(p, p->X, Xs, N, 1, st, ok)) || !*ok) return rc;
 	const char* mode = std::getenv("QPC_POS_TC");	// 0: multiply-adds only, 1: tensor cores wherever they can
 	const bool always = mode && mode[0] == '1';
 	p->F.tc_always = p->W.tc_always = p->X.tc_always = always;
 	const bool tcp = p->nff == 1 && (always || (in.batch >= TC_MIN && N >= 128 && !(mode && mode[0] == '0')));
 	if (tcp) {
-		if ((rc = tc_make(p->W.tc, nullptr, Yt, 0, N, 1, N, N, 1, p->W.w, p->W.prof.data(), p->W.ea, false, st, &p->W.has_tc))) return rc;
-		if ((rc = tc_make(p->X.tc, nullptr, p->Xt, 0, 1, N, N, N, 1, p->X.w, p->X.prof.data(), p->X.ea, false, st, &p->X.has_tc))) return rc;
+		if ((rc = tc_make(p->W.tc, nullptr, Ws, 0, N, 1, N, N, 1, p->W.w, p->W.prof.data(), p->W.ea, false, st, &p->W.has_tc))) return rc;
+		if ((rc = tc_make(p->X.tc, nullptr, Xs, 0, N, 1, N, N, 1, p->X.w, p->X.prof.data(), p->X.ea, false, st, &p->X.has_tc))) return rc;
 	}
 	// F~_l, a set of columns at a time: the engine's field-free solve on the eigenvectors, then X^T S
 	const int J = (int)std::min<long>(N, std::max<long>(32, (64l << 20) / ((long)N * nlh * 16)));
@@ -1004,7 +1027,7 @@ void exponents(const double2* src, int* ex, int N, int ntile, long nvec, cudaStr
 band_args band_args_of(const radial_ops* p, const band_store& b, int nchan, int ncols)
 {
 	band_args a{};
-	a.A = b.A; a.astride = b.stride; a.td = b.d_td; a.toff = b.d_off; a.ea = b.ea;
+	a.A = b.A; a.astride = b.stride; a.td = b.d_td; a.toff = b.d_off; a.ea = b.ea; a.er = b.er;
 	a.N = p->N; a.ntile = p->ntile; a.nchan = nchan; a.ncols = ncols;
 	a.lmap = p->zero;
 	return a;

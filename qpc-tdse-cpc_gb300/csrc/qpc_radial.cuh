@@ -24,6 +24,7 @@ struct band_args {
 	const int* lmap;	// channel -> operator of a set
 	const int* amap;	// destination slot -> set (NULL: one set)
 	int ea;			// |A| <= 2^ea
+	const int* er;		// times 2^er of the row (NULL: 1)
 	int N, ntile, nchan, ncols;
 	const double2 *s0, *s1;	// [slot][nchan][N]; s1 where par[slot] is odd
 	const int *e0, *e1;	// largest biased exponent of every TE rows, [slot][nchan][ntile * EPT]
@@ -58,6 +59,7 @@ struct tc_store {
 // td = (first, first with hi limbs, end of those, end) at byte off
 struct band_store {
 	int w = 0, ea = 0;
+	int* er = nullptr;		// the rows' own powers of two (device [N]), or NULL
 	long stride = 0;		// bytes of one operator
 	std::vector<int4> td;
 	std::vector<long> off;
@@ -68,7 +70,7 @@ struct band_store {
 	std::vector<double> prof;	// largest entry per distance, as laid out
 	tc_store tc;			// the same for the tensor cores, for batches
 	bool has_tc = false, tc_always = false;
-	void release() { tc.release(); has_tc = false; cudaFree(d_td); cudaFree(d_off); cudaFree(A); d_td = nullptr; d_off = nullptr; A = nullptr; }
+	void release() { tc.release(); has_tc = false; cudaFree(d_td); cudaFree(d_off); cudaFree(A); cudaFree(er); d_td = nullptr; d_off = nullptr; A = nullptr; er = nullptr; }
 };
 
 // what radial_create reads: device bands S, R [N][P+1] (R: the operator the basis diagonalises, its eigenvalues
