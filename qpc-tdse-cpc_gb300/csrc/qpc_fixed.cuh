@@ -27,12 +27,14 @@ __device__ __forceinline__ int2 quant(double v, int E)
 	return make_int2(hi, (int)(x - ((long long)hi << 28)));
 }
 
-// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^63; nf: the operand was not finite.  Two bits of m beside
-// h, or from |h| = 2^61 on (a sum of 32 in units of the column's power of two; rows of a dense orthogonal matrix reach
-// sqrt(N)) h alone, whose 62 bits leave m below the rounding
+// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^61, or 2^63 if WIDE; nf: the operand was not finite.  Two
+// bits of m beside h, or from |h| = 2^61 on h alone, whose 62 bits leave m below the rounding.  2^61 is a sum of 32 in
+// units of the column's power of two: rows of a dense orthogonal matrix reach sqrt(N), k_angle 8, k_couple 21, F~ 27 (where
+// WIDE would cost 0.5 % of a step)
+template <bool WIDE>
 __device__ __forceinline__ double to_double(long long h, long long m, int s, bool nf)
 {
-	const bool wide = (unsigned long long)(h + (1ll << 61)) >> 62;
+	const bool wide = WIDE && (unsigned long long)(h + (1ll << 61)) >> 62;
 	long long q = wide ? h : (h << 2) | (m >> 26);
 	unsigned long long a = q < 0 ? 0ull - (unsigned long long)q : (unsigned long long)q;
 	const int lz = __clzll((long long)a);

@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 	auto emit = [&](int cl, long long hr, long long mr, long long hi, long long mi) {
 		const int c = col0 + cl;
 		if (c >= p.ncols || (p.nta && !(p.step < p.nta[c]))) return;
-		const int E = sE[cl], s = p.ea + E - 1078 + (p.er && row < p.N ? p.er[row] : 0);
-		const double2 y = make_double2(to_double(hr, mr, s, E == 0x7ff), to_double(hi, mi, s, E == 0x7ff));
+		const int E = sE[cl], s = p.ea + E - 1078 + (!CX && p.er && row < p.N ? p.er[row] : 0);
+		const double2 y = make_double2(to_double<!CX>(hr, mr, s, E == 0x7ff), to_double<!CX>(hi, mi, s, E == 0x7ff));
 		const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 		if (row < p.N) p.dst[o * p.N + row] = y;
 		const int e = group_max(row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);
@@ -325,8 +325,8 @@ __global__ void __launch_bounds__(256, 4) k_band_one(const band_args p)
 #pragma unroll
 	for (int w = 1; w < 8; ++w) { rh += red[w][0][lane]; rm += red[w][1][lane]; ih += red[w][2][lane]; im += red[w][3][lane]; }
 	flush(rh, rm); flush(ih, im);
-	const int row = tile * TM + lane, s = p.ea + E - 1078 + (p.er && row < p.N ? p.er[row] : 0);
-	const double2 y = make_double2(to_double(rh, rm, s, E == 0x7ff), to_double(ih, im, s, E == 0x7ff));
+	const int row = tile * TM + lane, s = p.ea + E - 1078 + (!CX && p.er && row < p.N ? p.er[row] : 0);
+	const double2 y = make_double2(to_double<!CX>(rh, rm, s, E == 0x7ff), to_double<!CX>(ih, im, s, E == 0x7ff));
 	const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 	if (row < p.N) p.dst[o * p.N + row] = y;
 	const int e = group_max(row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);

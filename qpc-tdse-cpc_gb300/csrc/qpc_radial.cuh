@@ -24,7 +24,7 @@ struct band_args {
 	const int* lmap;	// channel -> operator of a set
 	const int* amap;	// destination slot -> set (NULL: one set)
 	int ea;			// |A| <= 2^ea
-	const int* er;		// times 2^er of the row (NULL: 1)
+	const int* er;		// times 2^er of the row (real operators; NULL: 1)
 	int N, ntile, nchan, ncols;
 	const double2 *s0, *s1;	// [slot][nchan][N]; s1 where par[slot] is odd
 	const int *e0, *e1;	// largest biased exponent of every TE rows, [slot][nchan][ntile * EPT]

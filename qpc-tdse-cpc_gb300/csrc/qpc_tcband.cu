@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_apply(const band_args p, cons
 			const int row = tile * TR + qr * 32 + lane;
 			const bool in = row < t.nrow;
 			const uint32_t tl = tmem + ((uint32_t)(qr * 32) << 16);
-			const int ea = (t.ear ? (in ? t.ear[(long)p.lmap[ch] * t.nrow + row] : 0) : t.ea) + (p.er && in ? p.er[row] : 0);
+			const int ea = (t.ear ? (in ? t.ear[(long)p.lmap[ch] * t.nrow + row] : 0) : t.ea) + (!CX && p.er && in ? p.er[row] : 0);
 			const int nexo = (t.nrow + TM - 1) / TM * EPT;
 #pragma unroll 1
 			for (int b = 0; b < 2; ++b) {
