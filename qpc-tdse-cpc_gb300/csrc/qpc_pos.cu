@@ -25,6 +25,7 @@ namespace qpc {
 namespace {
 
 constexpr int LMAX = 128;	// most l channels
+constexpr int GRID_Y = 65535;	// most channels of a launch
 
 // ------------------------------------------------------------------ the local part of a step
 // One block: PT positions of one (slot, m), all l; PT lanes of a warp hold the positions, the 32 / PT groups of lanes
@@ -290,12 +291,12 @@ int build(pos_path* p, const pos_setup& in, bool* ok)
 
 } // namespace
 
-// The path is taken when 3 <= p <= 8, 2 <= n_l <= LMAX and radial_create finds the operators to suit it.
+// The path is taken when 3 <= p <= 8, 2 <= n_l <= LMAX, the channels fit the second dimension of a grid and radial_create finds the operators to suit it.
 // Everything else keeps the banded solves.
 int pos_create(const pos_setup& in, pos_path** out)
 {
 	*out = nullptr;
-	if (in.L > LMAX || in.L < 2 || in.P < 3 || in.P > 8) return QPC_OK;
+	if (in.L > LMAX || in.L < 2 || in.P < 3 || in.P > 8 || (long)in.M * in.L > GRID_Y || in.nlh > GRID_Y) return QPC_OK;
 	auto* p = new (std::nothrow) pos_path();
 	if (!p) { set_error("host allocation"); return QPC_ERR_NOMEM; }
 	p->N = in.N; p->P = in.P; p->L = in.L; p->M = in.M; p->m0 = in.m0; p->B = in.B; p->nlh = in.nlh; p->npair = in.npair;
