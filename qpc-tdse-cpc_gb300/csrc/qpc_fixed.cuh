@@ -10,6 +10,9 @@ constexpr int TM = 32;		// rows (positions) of a tile, one per lane
 constexpr int KC = 16;		// k per chunk of the stored operators
 constexpr int TE = 8;		// rows that share a recorded exponent
 constexpr int EPT = TM / TE;
+// largest exponent of a column whose product is formed: a sum of 2^5 units stays finite.  Beyond (5.6e306, infinities, NaN)
+// the product is NaN, which a run reports
+constexpr int EMAX = 2041;
 
 __device__ __forceinline__ int bexp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
 
@@ -27,7 +30,8 @@ __device__ __forceinline__ int2 quant(double v, int E)
 	return make_int2(hi, (int)(x - ((long long)hi << 28)));
 }
 
-// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^61, or 2^63 if WIDE; nf: the operand was not finite.  Two
+// (h + m 2^-28) 2^s rounded to double, m in [0, 2^28), |h| < 2^61, or 2^63 if WIDE (infinite from 2^1024 on: an operator may
+// grow its column); nf: the operand's exponent was above EMAX.  Two
 // bits of m beside h, or from |h| = 2^61 on h alone, whose 62 bits leave m below the rounding.  2^61 is a sum of 32 in
 // units of the column's power of two: rows of a dense orthogonal matrix reach sqrt(N), k_angle 8, k_couple 21, F~ 27 (where
 // WIDE would cost 0.5 % of a step)
@@ -42,6 +46,7 @@ __device__ __forceinline__ double to_double(long long h, long long m, int s, boo
 	a <<= (lz & 63);
 	unsigned long long b = ((unsigned long long)(unsigned)(e - 1) << 52) + (a >> 11) + ((a >> 10) & 1ull);
 	b |= (unsigned long long)q & 0x8000000000000000ull;
+	if (WIDE && e > 2046) b = 0x7ff0000000000000ull;
 	if (q == 0 || e < 1) b = 0ull;
 	if (nf) b = 0x7ff8000000000000ull;
 	return __longlong_as_double((long long)b);

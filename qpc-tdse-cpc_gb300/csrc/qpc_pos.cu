@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256, BPS) k_angle(const angle_args p)
 			if (g < no) {
 				const int s = e - 1078;
 				b[(2 * (k0 + g) + (odd ? 1 : 0)) * PT + lane] =
-					make_double2(to_double<false>(h[g][0], mm[g][0], s, e == 0x7ff), to_double<false>(h[g][1], mm[g][1], s, e == 0x7ff));
+					make_double2(to_double<false>(h[g][0], mm[g][0], s, e > EMAX), to_double<false>(h[g][1], mm[g][1], s, e > EMAX));
 			}
 	}
 	__syncthreads();
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(256, BPS) k_angle(const angle_args p)
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
 				const int s = e - 1078, l = 2 * (o0 + g) + odd;
-				const double2 v = make_double2(to_double<false>(h[g][0], mm[g][0], s, e == 0x7ff), to_double<false>(h[g][1], mm[g][1], s, e == 0x7ff));
+				const double2 v = make_double2(to_double<false>(h[g][0], mm[g][0], s, e > EMAX), to_double<false>(h[g][1], mm[g][1], s, e > EMAX));
 				if (in) y[(long)l * N] = v;
 				int x = in ? max(bexp(v.x), bexp(v.y)) : 0;
 #pragma unroll

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256, 2) k_band_apply(const band_args p)
 		const int c = col0 + cl;
 		if (c >= p.ncols || (p.nta && !(p.step < p.nta[c]))) return;
 		const int E = sE[cl], s = p.ea + E - 1078 + (!CX && p.er && row < p.N ? p.er[row] : 0);
-		const double2 y = make_double2(to_double<!CX>(hr, mr, s, E == 0x7ff), to_double<!CX>(hi, mi, s, E == 0x7ff));
+		const double2 y = make_double2(to_double<!CX>(hr, mr, s, E > EMAX), to_double<!CX>(hi, mi, s, E > EMAX));
 		const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 		if (row < p.N) p.dst[o * p.N + row] = y;
 		const int e = group_max(row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256, 4) k_band_one(const band_args p)
 	for (int w = 1; w < 8; ++w) { rh += red[w][0][lane]; rm += red[w][1][lane]; ih += red[w][2][lane]; im += red[w][3][lane]; }
 	flush(rh, rm); flush(ih, im);
 	const int row = tile * TM + lane, s = p.ea + E - 1078 + (!CX && p.er && row < p.N ? p.er[row] : 0);
-	const double2 y = make_double2(to_double<!CX>(rh, rm, s, E == 0x7ff), to_double<!CX>(ih, im, s, E == 0x7ff));
+	const double2 y = make_double2(to_double<!CX>(rh, rm, s, E > EMAX), to_double<!CX>(ih, im, s, E > EMAX));
 	const long o = (long)(p.dmap ? p.dmap[c] : c) * p.nchan + ch;
 	if (row < p.N) p.dst[o * p.N + row] = y;
 	const int e = group_max(row < p.N ? max(bexp(y.x), bexp(y.y)) : 0);

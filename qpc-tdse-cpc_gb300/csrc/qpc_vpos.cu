@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(CW * 32, 2) k_couple(const set_args p)
 #pragma unroll
 		for (int g = 0; g < G; ++g)
 			if (g < no) {
-				const double2 v = make_double2(to_double<false>(h[g][0], m[g][0], e - 1078, e == 0x7ff), to_double<false>(h[g][1], m[g][1], e - 1078, e == 0x7ff));
+				const double2 v = make_double2(to_double<false>(h[g][0], m[g][0], e - 1078, e > EMAX), to_double<false>(h[g][1], m[g][1], e - 1078, e > EMAX));
 				const int ch = (set ? na : 0) + o0 + g;
 				if (in) p.out[base + (long)ch * N] = v;
 				const int x = group_max(in ? max(bexp(v.x), bexp(v.y)) : 0);

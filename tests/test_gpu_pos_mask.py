@@ -80,3 +80,15 @@ def test_paths_in_turn(q, monkeypatch):
     assert pa == ["banded"] * 7 and pb == ["position", "banded", "position", "position", "banded", "position", "position"]
     for k, (x, y) in enumerate(zip(a, b)):
         assert rel_l2(y / np.abs(x).max(), x / np.abs(x).max()) < 1e-12, k
+
+
+@pytest.mark.parametrize("state,scale", [(1e200, 1e150), (1e150, 1e190)])
+def test_overflow_is_reported(q, monkeypatch, state, scale):
+    """a mask that grows the state past the largest double"""
+    def calls(prop, R, mask):
+        prop.put(state * prop.get())
+        with pytest.raises(q.QpcError) as e:
+            prop.run_ex(_f(3, 1), np.ones(B), np.ones(B), mask=scale * mask)
+        return e.value.code
+
+    assert _both(q, monkeypatch, calls) == [5, 5]
