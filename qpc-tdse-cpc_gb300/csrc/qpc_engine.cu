@@ -921,8 +921,9 @@ template <int P>
 void set_seg_smem_attr(qpc_lgwz* h)
 {
 	for (int cpl = 0; cpl < 2; ++cpl) {
+		// whatever its size: the default limit of 48 KB holds the kernel's static arrays too
 		const size_t smem = h->seg_smem[cpl];
-		if (smem <= 48 * 1024 || !raise_attr(h->dev, 100 + 4 * P + 2 * cpl + (h->seg_sfac[cpl] ? 1 : 0), smem)) continue;
+		if (!raise_attr(h->dev, 100 + 4 * P + 2 * cpl + (h->seg_sfac[cpl] ? 1 : 0), smem)) continue;
 		if (cpl && h->seg_sfac[1]) cudaFuncSetAttribute(k_chain_seg<P, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 		if (cpl && !h->seg_sfac[1]) cudaFuncSetAttribute(k_chain_seg<P, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 		if (!cpl && h->seg_sfac[0]) cudaFuncSetAttribute(k_chain_seg<P, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
