@@ -86,15 +86,19 @@ def test_both_paths_share_buffers(q, monkeypatch):
     n_r, n_l, B = 400, 21, 256
     _, S, R, H = _grid(q, n_r, 6, n_l)
     state, factors = 16 * n_r * n_l * B, 16 * n_r * 7 * (n_l // 2) * B
-    prop = q.propagator_cn_hc_lgwz().initialize(n_r, 6, n_l, S, R, H, 0.05, n_inst=B)
-    prop.put(np.ones((B, 1, n_l, n_r), complex))
     f = np.zeros((B, 2))
-    prop.run_dipole(f, np.ones(B), np.ones(B), R)
-    torch.cuda.synchronize()
-    before = torch.cuda.mem_get_info()[0]
-    prop.run_dipole(f, np.ones(B), np.ones(B), 0.5 * R)
-    assert prop.path()["last_run"] == "banded"
-    torch.cuda.synchronize()
-    used = before - torch.cuda.mem_get_info()[0]
-    prop.close()
-    assert used < factors + 1.6 * state, (used / state, factors / state)
+    used = []
+    for _ in range(3):	# free memory is a whole-device figure that other processes move too
+        prop = q.propagator_cn_hc_lgwz().initialize(n_r, 6, n_l, S, R, H, 0.05, n_inst=B)
+        prop.put(np.ones((B, 1, n_l, n_r), complex))
+        prop.run_dipole(f, np.ones(B), np.ones(B), R)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        prop.run_dipole(f, np.ones(B), np.ones(B), 0.5 * R)
+        assert prop.path()["last_run"] == "banded"
+        torch.cuda.synchronize()
+        used.append(before - torch.cuda.mem_get_info()[0])
+        prop.close()
+        if used[-1] < factors + 1.6 * state:
+            return
+    pytest.fail("%s states beside the factors" % [(u - factors) / state for u in used])
